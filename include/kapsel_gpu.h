@@ -422,7 +422,7 @@ int kapsel_gpu_launches_per_step(kapsel_ctx *ctx);
 const char *kapsel_gpu_kernel_name(int i);
 /* The kernel of timing slot i for this context's pass variants: with the
    fused y/z plane kernels (pass variant y = 3) slot 6 is k_yzw_c2r, slot 10
-   k_zyw_force, and slots 5 and 11 are empty ("", no launch). */
+   k_zyw_r2c, and slots 5 and 11 are empty ("", no launch). */
 const char *kapsel_gpu_step_kernel_name(kapsel_ctx *ctx, int i);
 
 /* The context's CUDA stream (a cudaStream_t), for recording events around

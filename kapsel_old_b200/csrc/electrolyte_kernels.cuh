@@ -158,44 +158,6 @@ __global__ void __launch_bounds__(256) k_x_fwd_op(Geo g, Twiddles<R> tw, const C
   }
 }
 
-// Forward z transform of real fields, kz < nkeep kept:
-// in [c][rows][pitch] (planes in_cstride apart) -> out [c][rows][ostride], k < nkeep.
-template <typename R>
-__global__ void __launch_bounds__(256) k_z_r2c(Geo g, Twiddles<R> tw, const R *__restrict__ in, int in_pitch,
-                                               size_t in_cstride, Cx<R> *__restrict__ out, int nkeep, int ostride) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int M = g.M;
-  constexpr int ES = ZROWS + 1;
-  Cx<R> *twm = reinterpret_cast<Cx<R> *>(smem_raw);
-  Cx<R> *twz = twm + M;
-  Cx<R> *S = twz + g.NZ;    // [M][ES]
-  Cx<R> *scr = S + M * ES;  // FFT scratch, then the output tile [ZROWS][nkeep+1]
-  load_twiddles(twm, tw.m, M);
-  load_twiddles(twz, tw.z, g.NZ);
-  const int c = blockIdx.y;
-  const size_t rows = (size_t)g.NX * g.NY;
-  const size_t row0 = (size_t)blockIdx.x * ZROWS;
-  const R *src = in + c * in_cstride;
-  for (int it = threadIdx.x; it < ZROWS * M; it += blockDim.x) {
-    const int n = it & (M - 1), rr = it >> g.lm;
-    const R *r = src + (row0 + rr) * (size_t)in_pitch + 2 * n;
-    S[n * ES + rr] = {r[0], r[1]};
-  }
-  __syncthreads();
-  fft2_smem<R, 1, ZROWS>(S, scr, g.lm, 1, ES, twm);
-  const int TA = nkeep + 1;
-  for (int it = threadIdx.x; it < ZROWS * nkeep; it += blockDim.x) {
-    const int rr = it % ZROWS, k = it / ZROWS;
-    scr[rr * TA + k] = r2c_post(S + rr, ES, k, M, twz);
-  }
-  __syncthreads();
-  Cx<R> *dst = out + c * rows * ostride + row0 * ostride;
-  for (int it = threadIdx.x; it < ZROWS * nkeep; it += blockDim.x) {
-    const int k = it % nkeep, rr = it / nkeep;
-    dst[rr * ostride + k] = scr[rr * TA + k];
-  }
-}
-
 // Hermitian completion of the kz = 0 and kz = NZ/2 planes of full spectra
 // [c][NX][NY][M+1], as the Ooura inverse (rdft3dsort isgn<0,
 // fftsg3d.c:645-668) reads them: on each plane one half is kept and the

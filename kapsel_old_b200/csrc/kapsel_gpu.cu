@@ -13,8 +13,8 @@
 //   7 k_z_c2r              inverse z -> u* (real)
 //   8 (k_z_c2r blocks)     AB2 / Euler positions and orientations
 //   9 k_particles_hydro_velocity  hydro force+torque gather, LJ, gravity, velocity, thermostat
-//  10 k_particles_scatter  phi, phi*u_p
-//  11 k_z_force            clamp, f = up - phi u*, forward z, clear phi/up
+//  10 k_particles_scatter  phi, phi*u_p, clamp, f = up - phi u*
+//  11 k_z_force            forward z of f, f cleared
 //  12 k_y_pass<fwd>        forward y (3 comps)
 //  13 k_x_force_to_zeta    forward x, solenoidal projection, zeta += zeta(f), uk_dc += f(0)
 // The 20 3D FFTs of the reference become 14 pruned ones because
@@ -294,7 +294,7 @@ struct BoxBase {
   int xsplit = 0;
   virtual bool xsplit_ok(int xs) const = 0;
   virtual void set_xsplit(int xs) = 0;
-  // the step runs the fused y/z plane kernels (k_yzw_c2r, k_zyw_force)
+  // the step runs the fused y/z plane kernels (k_yzw_c2r, k_zyw_r2c)
   virtual bool fused_yz() const { return false; }
   virtual int alloc_el() = 0;
   virtual int alloc_obl() = 0;
@@ -394,7 +394,7 @@ struct Box : BoxBase {
   Cx<R> *bufA = nullptr;  // I1-shaped, 5 comps [c][NX][KYc][TS]
   Cx<R> *bufB = nullptr;  // I2-shaped, 5 comps [c][NX][NY][TS]
   R *ustar = nullptr;     // [3][NX][NY][NZ]
-  R *phiup = nullptr;     // [4][NX][NY][NZ]
+  R *phiup = nullptr;     // [4][NX][NY][NZ], all zero between steps
   Cx<R> *twbuf = nullptr;
   Twiddles<R> tw;
   static constexpr int KCX = 4;                         // x-pass kz tile
@@ -402,6 +402,9 @@ struct Box : BoxBase {
   size_t smem_xu = 0, smem_xadv = 0, smem_xf = 0, smem_y = 0, smem_zp = 0, smem_zc = 0, smem_zf = 0, smem_zr = 0;
 
   size_t npts() const { return (size_t)g.NX * g.NY * g.NZ; }
+  // rigidity force of the Navier_Stokes and Electrolyte steps, [3][NX][NY][NZ]
+  // (the Lees-Edwards step scatters phi and phi u_p into the whole of phiup)
+  R *force() const { return phiup + npts(); }
 
   // x passes with compile-time NX for NX = 32..256 (the runtime-NX kernels otherwise)
   template <int LX, int XS>
@@ -485,33 +488,39 @@ struct Box : BoxBase {
   }
 
   // warp-level z kernels for NZ = 64, 128, 256 (zw = log2(NZ/2)); 0: block-level
-  static constexpr int ZNW = sizeof(R) == 4 ? 8 : 4;  // warps per block
+  int nsm = 0;
+  static constexpr int ZNW = sizeof(R) == 4 ? 8 : 4;  // warps per block at most
   int zw = 0;
-  int zw_grid_p = 0, zw_grid_c = 0, zw_grid_f = 0;
-  size_t zw_sm_p = 0, zw_sm_c = 0, zw_sm_f = 0;
+  // launch shape of a warp-level z kernel with `tasks` row groups to do
+  struct ZPlan {
+    int nw = 0, grid = 0;
+    size_t sm = 0;
+  };
+  ZPlan zp_p, zp_c, zp_f;
+  template <typename K>
+  int zplan(K kern, int tasks, size_t warp_bytes, ZPlan &p) {
+    KCHECK(allow_smem(kern, warp_bytes * ZNW));
+    int dev = 0, occ = 0;
+    KCHECK(cudaGetDevice(&dev));
+    KCHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    p.nw = ZNW;
+    p.sm = warp_bytes * p.nw;
+    KCHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, p.nw * 32, p.sm));
+    p.grid = std::min((tasks + p.nw - 1) / p.nw, std::max(occ, 1) * nsm);
+    return 0;
+  }
 
   template <int LM>
   int zw_setup() {
     using Z = ZL<LM>;
-    const size_t line = sizeof(Cx<R>) * Z::RW * Z::LS * ZNW;
-    // FP64: the prefetching products kernel; FP32: four line groups per warp
-    zw_sm_p = sizeof(R) == 8 ? sizeof(Cx<R>) * (size_t)ZProd<R, LM>::WARP * ZNW : 4 * line;
-    zw_sm_c = line;
-    zw_sm_f = 3 * line;
-    auto kp = sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW> : k_zw_products<R, LM, ZNW>;
-    KCHECK(allow_smem(kp, zw_sm_p));
-    KCHECK(allow_smem(k_zw_c2r<R, LM, ZNW>, zw_sm_c));
-    KCHECK(allow_smem(k_zw_force<R, LM, ZNW>, zw_sm_f));
-    int dev = 0, nsm = 0, op = 0, oc = 0, of = 0;
-    KCHECK(cudaGetDevice(&dev));
-    KCHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    KCHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&op, kp, ZNW * 32, zw_sm_p));
-    KCHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&oc, k_zw_c2r<R, LM, ZNW>, ZNW * 32, zw_sm_c));
-    KCHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&of, k_zw_force<R, LM, ZNW>, ZNW * 32, zw_sm_f));
+    const size_t line = sizeof(Cx<R>) * Z::RW * Z::LS;  // one line group
     const int groups = g.NX * g.NY / Z::RW;
-    zw_grid_p = std::min((groups + ZNW - 1) / ZNW, std::max(op, 1) * nsm);
-    zw_grid_c = std::min((3 * groups + ZNW - 1) / ZNW, std::max(oc, 1) * nsm);
-    zw_grid_f = std::min((groups + ZNW - 1) / ZNW, std::max(of, 1) * nsm);
+    // FP64: the prefetching products kernel; FP32: four line groups per warp
+    int rc = zplan(sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW> : k_zw_products<R, LM, ZNW>, groups,
+                   sizeof(R) == 8 ? sizeof(Cx<R>) * (size_t)ZProd<R, LM>::WARP : 4 * line, zp_p);
+    if (!rc) rc = zplan(k_zw_c2r<R, LM, ZNW>, 3 * groups, line, zp_c);
+    if (!rc) rc = zplan(k_zw_r2c<R, LM, ZNW, true, false>, 3 * groups, line, zp_f);
+    if (rc) return rc;
     zw = LM;
     yz_ly = 0;
     if (g.KYc < g.NY) {
@@ -527,13 +536,12 @@ struct Box : BoxBase {
   static constexpr int YZNW = sizeof(R) == 4 ? KAPSEL_YZ_NW : 4;  // warps per block
   int yz_ly = 0;
   size_t yz_sm = 0;
-  unsigned *plane_count = nullptr;  // [NX] readers of phi per x plane (k_zyw_force)
   template <int LY, int LM>
   int yz_setup() {
     const size_t sm = YZ<R, LY, LM>::smem(YZNW);
     if (sm > 227 * 1024) return 0;
     KCHECK(allow_smem(k_yzw_c2r<R, LY, LM, false, YZNW>, sm));
-    KCHECK(allow_smem(k_zyw_force<R, LY, LM, false, YZNW>, sm));
+    KCHECK(allow_smem(k_zyw_r2c<R, LY, LM, true, YZNW>, sm));
     yz_sm = sm;
     yz_ly = LY;
     return 0;
@@ -546,8 +554,8 @@ struct Box : BoxBase {
   }
   template <int LY, int LM>
   void zy_force_l(bool pdl) {
-    launch_k(pdl, k_zyw_force<R, LY, LM, false, YZNW>, dim3(3 * g.NX), dim3(YZNW * 32), yz_sm, stream, g, tw, phiup,
-             (const R *)ustar, bufA, plane_count);
+    launch_k(pdl, k_zyw_r2c<R, LY, LM, true, YZNW>, dim3(3 * g.NX), dim3(YZNW * 32), yz_sm, stream, g, tw, force(),
+             npts(), bufA);
   }
   // bufA (x real, ky compact) -> u*, with the position update in extra blocks
   template <int LM>
@@ -561,7 +569,7 @@ struct Box : BoxBase {
     else if (zw == 6) yz_c2r_m<6>(pdl, pts, euler);
     else yz_c2r_m<7>(pdl, pts, euler);
   }
-  // phi/up, u* -> force spectra in bufA (x real, ky compact)
+  // rigidity force -> its spectra in bufA (x real, ky compact)
   template <int LM>
   void zy_force_m(bool pdl) {
     if (yz_ly == 5) zy_force_l<5, LM>(pdl);
@@ -575,19 +583,19 @@ struct Box : BoxBase {
   }
   template <int LM>
   void zw_products(bool pdl) {
-    launch_k(pdl, sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW> : k_zw_products<R, LM, ZNW>, dim3(zw_grid_p),
-             dim3(ZNW * 32), zw_sm_p, stream, g, tw, bufB);
+    launch_k(pdl, sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW> : k_zw_products<R, LM, ZNW>, dim3(zp_p.grid),
+             dim3(zp_p.nw * 32), zp_p.sm, stream, g, tw, bufB);
   }
   template <int LM>
   void zw_c2r(bool pdl, DPart *pts, int euler) {
-    const int posblk = pts ? (Np + ZNW * 32 - 1) / (ZNW * 32) : 0;
-    launch_k(pdl, k_zw_c2r<R, LM, ZNW>, dim3(zw_grid_c + posblk), dim3(ZNW * 32), zw_sm_c, stream, g, tw,
-             (const Cx<R> *)bufB, ustar, npts(), g.NZ, 3, zw_grid_c, pp, pts, euler, status);
+    const int posblk = pts ? (Np + zp_c.nw * 32 - 1) / (zp_c.nw * 32) : 0;
+    launch_k(pdl, k_zw_c2r<R, LM, ZNW>, dim3(zp_c.grid + posblk), dim3(zp_c.nw * 32), zp_c.sm, stream, g, tw,
+             (const Cx<R> *)bufB, ustar, npts(), g.NZ, 3, zp_c.grid, pp, pts, euler, status);
   }
   template <int LM>
   void zw_force(bool pdl) {
-    launch_k(pdl, k_zw_force<R, LM, ZNW>, dim3(zw_grid_f), dim3(ZNW * 32), zw_sm_f, stream, g, tw, phiup,
-             (const R *)ustar, bufB);
+    launch_k(pdl, k_zw_r2c<R, LM, ZNW, true, false>, dim3(zp_f.grid), dim3(zp_f.nw * 32), zp_f.sm, stream, g, tw,
+             force(), npts(), bufB, 3);
   }
   // dispatch on the compile-time line length
   void zdisp_products(bool pdl) {
@@ -610,7 +618,7 @@ struct Box : BoxBase {
     if (zw == 5) zw_force<5>(pdl);
     else if (zw == 6) zw_force<6>(pdl);
     else if (zw == 7) zw_force<7>(pdl);
-    else launch_k(pdl, k_z_force<R>, dim3(gz()), dim3(256), smem_zf, stream, g, tw, phiup, (const R *)ustar, bufB);
+    else launch_k(pdl, k_z_force<R>, dim3(gz()), dim3(256), smem_zf, stream, g, tw, force(), bufB);
   }
 
   int alloc() override {
@@ -624,8 +632,6 @@ struct Box : BoxBase {
     KCHECK(cudaMalloc(&bufB, sizeof(Cx<R>) * nbuf * nB));
     KCHECK(cudaMalloc(&ustar, sizeof(R) * 3 * npts()));
     KCHECK(cudaMalloc(&phiup, sizeof(R) * 4 * npts()));
-    KCHECK(cudaMalloc(&plane_count, sizeof(unsigned) * g.NX));
-    KCHECK(cudaMemset(plane_count, 0, sizeof(unsigned) * g.NX));
     KCHECK(cudaMemset(zeta, 0, sizeof(Cx<R>) * 2 * nz));
     KCHECK(cudaMemset(ustar, 0, sizeof(R) * 3 * npts()));
     KCHECK(cudaMemset(phiup, 0, sizeof(R) * 4 * npts()));
@@ -715,7 +721,6 @@ struct Box : BoxBase {
   static constexpr int YNW = 4;
   static constexpr int YSLOTS = sizeof(R) == 4 ? 1 : 2;
   int yw_occ[2][2] = {{0, 0}, {0, 0}};  // blocks per SM, [inverse][full spectrum]
-  int nsm = 0;
   template <bool INV, int LY, bool FULL>
   void yw_launch(const Geo &gg, int nc, const Cx<R> *in, Cx<R> *out, bool pdl) {
     using Y = ZL<LY>;
@@ -848,7 +853,7 @@ struct Box : BoxBase {
     k_z_c2r<R><<<dim3(gz(), 3), 256, smem_zc, stream>>>(g, tw, bufB, out, cstride, pitch, PPar{}, nullptr, 0, nullptr);
   }
 
-  // f (from phi/up and u*) -> zeta update, launches 11-13
+  // f -> zeta update, launches 11-13
   void launch_force_to_zeta() {
     zdisp_force(false);
     launch_y<false>(g, 3, bufB, bufA);
@@ -885,7 +890,7 @@ struct Box : BoxBase {
     x_advect<0>(pdl);
     mark();
     // ymode 3: the inverse y and z c2r as one launch (k_yzw_c2r), and the
-    // force's z and y passes as one (k_zyw_force); their y slots stay empty
+    // force's z and y passes as one (k_zyw_r2c); their y slots stay empty
     const bool yzf = fused_yz();
     if (!yzf) launch_y<true>(g, 3, bufA, bufB, pdl);
     mark();
@@ -906,8 +911,8 @@ struct Box : BoxBase {
                (const R *)ustar, (const int *)cells, noise, euler, status, partial_p, arrivals,
                nc ? nc_corr : (double *)nullptr, ovl);
       mark();
-      launch_k(pdl, k_particles_scatter<R>, dim3(Np * PCL), dim3(256), 0, stream, pp, (const DPart *)parts,
-               (const int *)cells, phiup, status, (const unsigned *)ovl);
+      launch_k(pdl, k_particles_scatter<R, true>, dim3(Np * PCL), dim3(256), 0, stream, pp, (const DPart *)parts,
+               (const int *)cells, force(), (const R *)ustar, status, (const unsigned *)ovl);
       mark();
       if (yzf)
         zy_force(pdl);
@@ -941,7 +946,7 @@ struct Box : BoxBase {
     cudaMemsetAsync(uk_dc, 0, sizeof(double) * 3, stream);
     if (Np > 0) {
       launch_cells();
-      k_particles_scatter<R><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, phiup, status);
+      k_particles_scatter<R, true><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, force(), ustar, status);
       launch_force_to_zeta();
     }
     cudaMemsetAsync(uk_dc, 0, sizeof(double) * 3, stream);
@@ -1288,7 +1293,7 @@ struct Box : BoxBase {
     if (Np > 0) {
       k_particles_hydro_velocity<R><<<Np * pp.hyd_pcl, pp.hyd_threads, 0, stream>>>(pp, parts, ustar, cells, nullptr, euler, status,
                                                                   partial_p, arrivals);
-      k_particles_scatter<R><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, phiup, status);
+      k_particles_scatter<R, true><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, force(), ustar, status);
       launch_force_to_zeta();
     }
   }
@@ -1589,7 +1594,6 @@ struct Box : BoxBase {
     cudaFree(ustar);
     cudaFree(phiup);
     cudaFree(twbuf);
-    cudaFree(plane_count);
   }
 };
 
@@ -1829,7 +1833,7 @@ int Box<R>::phi_up_host(double *phi, double *up0, double *up1, double *up2) {
   KCHECK(cudaMalloc(&d, sizeof(R) * 4 * npt));
   KCHECK(cudaMemsetAsync(d, 0, sizeof(R) * 4 * npt, stream));
   launch_cells();
-  if (Np > 0) k_particles_scatter<R><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, d, status);
+  if (Np > 0) k_particles_scatter<R><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, d, nullptr, status);
   k_clamp_phi<R><<<592, 256, 0, stream>>>(npt, d);
   KCHECK(cudaGetLastError());
   std::vector<R> h(4 * npt);
@@ -1848,7 +1852,7 @@ int Box<R>::phi_only_host(double *phi) {
   KCHECK(cudaMalloc(&d, sizeof(R) * 4 * npt));
   KCHECK(cudaMemsetAsync(d, 0, sizeof(R) * 4 * npt, stream));
   launch_cells();
-  if (Np > 0) k_particles_scatter<R><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, d, status);
+  if (Np > 0) k_particles_scatter<R><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, d, nullptr, status);
   KCHECK(cudaGetLastError());
   std::vector<R> h(npt);
   KCHECK(cudaMemcpyAsync(h.data(), d, sizeof(R) * npt, cudaMemcpyDeviceToHost, stream));
@@ -2803,7 +2807,7 @@ const char *kapsel_gpu_step_kernel_name(kapsel_ctx *ctx, int i) {
   if (ctx && ctx->box->fused_yz()) {
     if (i == 5 || i == 11) return "";  // y passes inside the fused launches
     if (i == 6) return "k_yzw_c2r";
-    if (i == 10) return "k_zyw_force";
+    if (i == 10) return "k_zyw_r2c";
   }
   return kKernelNames[i];
 }

@@ -675,10 +675,36 @@ __device__ __forceinline__ void offset_from_base(const int rm[3], const int xi[3
   }
 }
 
+// The rigidity force at one point from its summed profile and phi u_p:
+// f = up' - phi' u* with the phi > 1 clamp (Make_f_particle_dt_nonsole,
+// f_particle.h:41-64; make_phi.cxx:278-297).
 template <typename R>
+__device__ __forceinline__ void store_force(R *__restrict__ force, const R *__restrict__ ustar, size_t npts, size_t im,
+                                            R acc, R (&up)[3]) {
+  R us[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) us[d] = __ldg(ustar + d * npts + im);
+  if (acc > R(1)) {
+    const R inv = R(1) / acc;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) up[d] *= inv;
+    acc = R(1);
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) force[d * npts + im] = up[d] - acc * us[d];
+}
+
+// FORCE = 0 stores phi and phi u_p: out[4][N].  FORCE = 1 (the steps) stores
+// the rigidity force instead: out[3][N].  The owner of a point holds its
+// complete sums, so it can form the force there and then, from u* values the
+// gather has just brought into L2; the z pass that follows then reads its
+// own force component only (not phi, up and u*, the last two by a second,
+// dependent round trip where phi is set) and has no clamp to apply.  The
+// scatter gains three loads and loses one store per point.
+template <typename R, bool FORCE = false>
 __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *__restrict__ parts,
-                                                           const int *__restrict__ cells, R *__restrict__ phiup,
-                                                           int *__restrict__ status,
+                                                           const int *__restrict__ cells, R *__restrict__ out,
+                                                           const R *__restrict__ ustar, int *__restrict__ status,
                                                            const unsigned *__restrict__ ovl = nullptr) {
   __shared__ NbShared nb[NB_MAX];
   pdl_begin();
@@ -746,9 +772,13 @@ __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *
         }
       }
       const size_t im = ((size_t)rm[0] * p.N[1] + rm[1]) * p.N[2] + rm[2];
-      reinterpret_cast<float *>(phiup)[im] = acc;
+      if constexpr (FORCE) {
+        store_force<R>(out, ustar, npts, im, acc, up);
+      } else {
+        out[im] = acc;
 #pragma unroll
-      for (int d = 0; d < 3; ++d) reinterpret_cast<float *>(phiup)[(1 + d) * npts + im] = up[d];
+        for (int d = 0; d < 3; ++d) out[(1 + d) * npts + im] = up[d];
+      }
     }
   } else
   for (int m = first; m < p.S; m += stride) {
@@ -795,9 +825,13 @@ __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *
       }
     }
     const size_t im = ((size_t)rm[0] * p.N[1] + rm[1]) * p.N[2] + rm[2];
-    phiup[im] = (R)acc;
+    if constexpr (FORCE) {
+      store_force<R>(out, ustar, npts, im, acc, up);
+    } else {
+      out[im] = (R)acc;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) phiup[(1 + d) * npts + im] = (R)up[d];
+      for (int d = 0; d < 3; ++d) out[(1 + d) * npts + im] = (R)up[d];
+    }
   }
 }
 

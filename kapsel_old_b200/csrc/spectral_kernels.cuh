@@ -346,14 +346,13 @@ __global__ void __launch_bounds__(256) k_z_c2r(Geo g, Twiddles<R> tw, const Cx<R
   }
 }
 
-// z pass of the rigidity force (Make_f_particle_dt_nonsole, f_particle.h:41-64,
-// with the phi > 1 clamp of make_phi.cxx:278-297 applied on the fly):
-// f = up' - phi' u*, forward z transform, kz < TZ kept -> out [3][NX][NY][TZ].
-// The scattered phi/up fields are cleared where they were written, so they are
-// all-zero again for the next scatter.  grid (NX*NY/ZROWS).
+// z pass of the rigidity force f [3][N] (all three components of ZROWS rows
+// per block): forward z, kz < TZ kept -> out [3][NX][NY][TZ].  f is set back to
+// zero where it was not, so it is all zero again for the next scatter.
+// grid (NX*NY/ZROWS).
 template <typename R>
-__global__ void __launch_bounds__(256) k_z_force(Geo g, Twiddles<R> tw, R *__restrict__ phiup,
-                                                 const R *__restrict__ ustar, Cx<R> *__restrict__ out) {
+__global__ void __launch_bounds__(256) k_z_force(Geo g, Twiddles<R> tw, R *__restrict__ force,
+                                                 Cx<R> *__restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
   const int M = g.M;
@@ -368,37 +367,15 @@ __global__ void __launch_bounds__(256) k_z_force(Geo g, Twiddles<R> tw, R *__res
   const size_t row0 = (size_t)blockIdx.x * ZROWS;
   for (int it = threadIdx.x; it < ZROWS * M; it += blockDim.x) {
     const int n = it & (M - 1), rr = it >> g.lm;
-    const size_t o = (row0 + rr) * g.NZ + 2 * n;
-    R ph[2], up[3][2], us[3][2];
+    Cx<R> *f = reinterpret_cast<Cx<R> *>(force + (row0 + rr) * g.NZ + 2 * n);  // an element pair
+    Cx<R> v[3];
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      ph[e] = phiup[o + e];
+    for (int d = 0; d < 3; ++d) v[d] = f[d * (npts / 2)];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        up[d][e] = phiup[(1 + d) * npts + o + e];
-        us[d][e] = ustar[d * npts + o + e];
-      }
+    for (int d = 0; d < 3; ++d) {
+      S[n * ES + rr * 3 + d] = v[d];
+      if (v[d].x != R(0) || v[d].y != R(0)) f[d * (npts / 2)] = {R(0), R(0)};
     }
-    R f[3][2];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      R p = ph[e];
-      if (p > R(1)) {
-        const R inv = R(1) / p;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) up[d][e] *= inv;
-        p = R(1);
-      }
-#pragma unroll
-      for (int d = 0; d < 3; ++d) f[d][e] = up[d][e] - p * us[d][e];
-      if (ph[e] != R(0)) {
-        phiup[o + e] = R(0);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) phiup[(1 + d) * npts + o + e] = R(0);
-      }
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) S[n * ES + rr * 3 + d] = {f[d][0], f[d][1]};
   }
   __syncthreads();
   fft2_smem<R, 1, NS>(S, scr, g.lm, 1, ES, twm);
@@ -441,6 +418,45 @@ __global__ void __launch_bounds__(256) k_z_r2c_full(Geo g, Twiddles<R> tw, const
   for (int it = threadIdx.x; it < ZROWS * (M + 1); it += blockDim.x) {
     const int k = it % (M + 1), rr = it / (M + 1);
     out[(row0 + rr) * (M + 1) + k] = r2c_post(S + rr, ES, k, M, twz);
+  }
+}
+
+// Forward z transform of real fields, kz < nkeep kept:
+// in [c][rows][pitch] (planes in_cstride apart) -> out [c][rows][ostride], k < nkeep.
+template <typename R>
+__global__ void __launch_bounds__(256) k_z_r2c(Geo g, Twiddles<R> tw, const R *__restrict__ in, int in_pitch,
+                                               size_t in_cstride, Cx<R> *__restrict__ out, int nkeep, int ostride) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_begin();
+  const int M = g.M;
+  constexpr int ES = ZROWS + 1;
+  Cx<R> *twm = reinterpret_cast<Cx<R> *>(smem_raw);
+  Cx<R> *twz = twm + M;
+  Cx<R> *S = twz + g.NZ;    // [M][ES]
+  Cx<R> *scr = S + M * ES;  // FFT scratch, then the output tile [ZROWS][nkeep+1]
+  load_twiddles(twm, tw.m, M);
+  load_twiddles(twz, tw.z, g.NZ);
+  const int c = blockIdx.y;
+  const size_t rows = (size_t)g.NX * g.NY;
+  const size_t row0 = (size_t)blockIdx.x * ZROWS;
+  const R *src = in + c * in_cstride;
+  for (int it = threadIdx.x; it < ZROWS * M; it += blockDim.x) {
+    const int n = it & (M - 1), rr = it >> g.lm;
+    const R *r = src + (row0 + rr) * (size_t)in_pitch + 2 * n;
+    S[n * ES + rr] = {r[0], r[1]};
+  }
+  __syncthreads();
+  fft2_smem<R, 1, ZROWS>(S, scr, g.lm, 1, ES, twm);
+  const int TA = nkeep + 1;
+  for (int it = threadIdx.x; it < ZROWS * nkeep; it += blockDim.x) {
+    const int rr = it % ZROWS, k = it / ZROWS;
+    scr[rr * TA + k] = r2c_post(S + rr, ES, k, M, twz);
+  }
+  __syncthreads();
+  Cx<R> *dst = out + c * rows * ostride + row0 * ostride;
+  for (int it = threadIdx.x; it < ZROWS * nkeep; it += blockDim.x) {
+    const int k = it % nkeep, rr = it / nkeep;
+    dst[rr * ostride + k] = scr[rr * TA + k];
   }
 }
 

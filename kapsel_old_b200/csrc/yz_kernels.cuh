@@ -126,90 +126,48 @@ __global__ void __launch_bounds__(NW * 32) k_yzw_c2r(Geo g, Twiddles<R> tw, cons
   }
 }
 
-// Rigidity force of component c = blockIdx.x / NX on plane x, z forward, then
-// forward y: f_c = up_c' - phi' u*_c with the phi > 1 clamp (as k_zw_force),
-// out [c][NX][KYc][TS].  up_c is cleared where phi is non-zero by the
-// component's own block; phi, which the blocks of all three components of
-// the plane read, by the last of them to finish reading (plane_count[x],
-// zero between launches), from the bit mask of non-zero element pairs that
-// every block gathers while it reads phi.
-template <typename R, int LY, int LM, bool FULLY, int NW>
-__global__ void __launch_bounds__(NW * 32) k_zyw_force(Geo g, Twiddles<R> tw, R *__restrict__ phiup,
-                                                       const R *__restrict__ ustar, Cx<R> *__restrict__ out,
-                                                       unsigned *__restrict__ plane_count) {
+// Forward z, then forward y, of plane (c, x) = blockIdx.x of real fields
+// in[c][NX][NY][NZ] (planes in_cstride apart) -> out [c][NX][KYc][TS], as
+// k_zw_r2c followed by the forward k_yw_pass.  CLEAR as in k_zw_r2c.  At
+// 128^3 in FP32 the rigidity force takes 26 us this way; with phi, up and u*
+// read here (phi by all three component blocks of a plane) it took 35 us.
+template <typename R, int LY, int LM, bool CLEAR, int NW>
+__global__ void __launch_bounds__(NW * 32) k_zyw_r2c(Geo g, Twiddles<R> tw, R *__restrict__ in, size_t in_cstride,
+                                                     Cx<R> *__restrict__ out) {
   using P = YZ<R, LY, LM>;
   using Y = typename P::Y;
   using Z = typename P::Z;
   using YL = typename P::YL;
   using V2 = typename Vec2<R>::T;
-  constexpr int NI = Z::RW * Z::M / 32;           // element pairs per lane and row group
-  constexpr int MASKW = P::NY * Z::M / 32;        // mask words of the plane
+  constexpr int NI = Z::RW * Z::M / 32;  // element pairs per lane and row group
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned nzmask[MASKW];
-  __shared__ int last_reader;
   pdl_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Cx<R> *plane = reinterpret_cast<Cx<R> *>(smem_raw);
   Cx<R> *slot = plane + P::NY * P::PS + warp * P::SLOT;
   const int pl = blockIdx.x;  // c * NX + x
   const int c = pl / g.NX, x = pl - c * g.NX;
-  const size_t npts = (size_t)g.NX * P::NY * Z::NZ;
-  const size_t row_base = (size_t)x * P::NY;
-  R *upc = phiup + (size_t)(1 + c) * npts;
-  const R *usc = ustar + (size_t)c * npts;
+  R *src = in + c * in_cstride + (size_t)x * P::NY * Z::NZ;
   {
     Cx<R> wf[Z::N1];
     wfft_twiddles<R, LM, 1>(tw.m, wf);
-    // phi of the warp's next row group is loaded while the current one is
-    // transformed
-    V2 ph_next[NI];
-    if (warp < P::NG)
+    // the warp's next row group is loaded while the current one is transformed
+    V2 next[NI];
+    auto load_group = [&](int grp) {
 #pragma unroll
       for (int h = 0; h < NI; ++h)
-        ph_next[h] = *reinterpret_cast<const V2 *>(phiup + (row_base + (size_t)warp * Z::RW) * Z::NZ +
-                                                   2 * (size_t)(lane + 32 * h));
+        next[h] = *reinterpret_cast<const V2 *>(src + (size_t)grp * Z::RW * Z::NZ + 2 * (lane + 32 * h));
+    };
+    if (warp < P::NG) load_group(warp);
     for (int grp = warp; grp < P::NG; grp += NW) {
-      const size_t row0 = row_base + (size_t)grp * Z::RW;
-      // all of the lane's loads first (up and u* where phi is non-zero), so
-      // that they are in flight together
-      V2 ph[NI], up[NI], us[NI];
-#pragma unroll
-      for (int h = 0; h < NI; ++h) ph[h] = ph_next[h];
-      if (grp + NW < P::NG)
-#pragma unroll
-        for (int h = 0; h < NI; ++h)
-          ph_next[h] = *reinterpret_cast<const V2 *>(phiup + (row0 + (size_t)NW * Z::RW) * Z::NZ +
-                                                     2 * (size_t)(lane + 32 * h));
-#pragma unroll
-      for (int h = 0; h < NI; ++h) {
-        const size_t o = row0 * Z::NZ + 2 * (size_t)(lane + 32 * h);
-        up[h] = us[h] = V2{R(0), R(0)};
-        if (ph[h].x != R(0) || ph[h].y != R(0)) {
-          up[h] = *reinterpret_cast<const V2 *>(upc + o);
-          us[h] = *reinterpret_cast<const V2 *>(usc + o);
-        }
-      }
+      R *row = src + (size_t)grp * Z::RW * Z::NZ;
 #pragma unroll
       for (int h = 0; h < NI; ++h) {
         const int i = lane + 32 * h, rr = i >> LM, n = i & (Z::M - 1);
-        const size_t o = row0 * Z::NZ + 2 * (size_t)i;
-        const bool nz = ph[h].x != R(0) || ph[h].y != R(0);
-        const unsigned bits = __ballot_sync(0xffffffffu, nz);
-        if (lane == 0) nzmask[grp * NI + h] = bits;
-        R p0 = ph[h].x, p1 = ph[h].y;
-        if (p0 > R(1)) {
-          const R inv = R(1) / p0;
-          up[h].x *= inv;
-          p0 = R(1);
-        }
-        if (p1 > R(1)) {
-          const R inv = R(1) / p1;
-          up[h].y *= inv;
-          p1 = R(1);
-        }
-        slot[rr * Z::LS + zpos<LM>(n)] = {up[h].x - p0 * us[h].x, up[h].y - p1 * us[h].y};
-        if (nz) *reinterpret_cast<V2 *>(upc + o) = V2{R(0), R(0)};
+        slot[rr * Z::LS + zpos<LM>(n)] = {next[h].x, next[h].y};
+        if (CLEAR && (next[h].x != R(0) || next[h].y != R(0))) *reinterpret_cast<V2 *>(row + 2 * i) = V2{R(0), R(0)};
       }
+      if (grp + NW < P::NG) load_group(grp + NW);
       __syncwarp();
       wfft<R, LM, 1>(slot, wf);
       for (int i = lane; i < Z::RW * Z::TZ; i += 32) {
@@ -220,40 +178,24 @@ __global__ void __launch_bounds__(NW * 32) k_zyw_force(Geo g, Twiddles<R> tw, R 
     }
   }
   __syncthreads();
-  // every phi value of this block has been read (and used) above
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last_reader = atomicAdd(plane_count + x, 1u) == 2u;
-  }
-  {
-    Cx<R> w[Y::N1];
-    wfft_twiddles<R, LY, 1>(tw.y, w);
-    const Cx<R> zero = {R(0), R(0)};
-    for (int b = warp; b < P::NB; b += NW) {
-      const int col0 = b * Y::RW, ncols = min(Y::RW, Z::TZ - col0);
-      for (int i = lane; i < P::NY * Y::RW; i += 32) {
-        const int r = i >> Y::LR, col = i & (Y::RW - 1);
-        slot[YL::template base<LY>(col) + zpos<LY>(r)] = col < ncols ? plane[r * P::PS + col0 + col] : zero;
-      }
-      __syncwarp();
-      wfft<R, LY, 1, YL>(slot, w);
-      Cx<R> *dst = out + (size_t)pl * g.KYc * g.TS + col0;
-      for (int i = lane; i < g.KYc * Y::RW; i += 32) {
-        const int r = i >> Y::LR, col = i & (Y::RW - 1);
-        const int j = full_from_compact(r, g.TY, g.KYc, P::NY);
-        if (col < ncols) dst[(size_t)r * g.TS + col] = slot[YL::template base<LY>(col) + zpos<LY>(j)];
-      }
-      __syncwarp();
+  Cx<R> w[Y::N1];
+  wfft_twiddles<R, LY, 1>(tw.y, w);
+  const Cx<R> zero = {R(0), R(0)};
+  for (int b = warp; b < P::NB; b += NW) {
+    const int col0 = b * Y::RW, ncols = min(Y::RW, Z::TZ - col0);
+    for (int i = lane; i < P::NY * Y::RW; i += 32) {
+      const int r = i >> Y::LR, col = i & (Y::RW - 1);
+      slot[YL::template base<LY>(col) + zpos<LY>(r)] = col < ncols ? plane[r * P::PS + col0 + col] : zero;
     }
-  }
-  __syncthreads();
-  if (last_reader) {
-    __threadfence();
-    // element pair q of the plane (row q / M, pair q % M) is mask bit q
-    R *phi = phiup + row_base * Z::NZ;
-    for (int wd = warp; wd < MASKW; wd += NW)
-      if ((nzmask[wd] >> lane) & 1u) *reinterpret_cast<V2 *>(phi + 2 * (size_t)(wd * 32 + lane)) = V2{R(0), R(0)};
-    if (threadIdx.x == 0) plane_count[x] = 0u;
+    __syncwarp();
+    wfft<R, LY, 1, YL>(slot, w);
+    Cx<R> *dst = out + (size_t)pl * g.KYc * g.TS + col0;
+    for (int i = lane; i < g.KYc * Y::RW; i += 32) {
+      const int r = i >> Y::LR, col = i & (Y::RW - 1);
+      const int j = full_from_compact(r, g.TY, g.KYc, P::NY);
+      if (col < ncols) dst[(size_t)r * g.TS + col] = slot[YL::template base<LY>(col) + zpos<LY>(j)];
+    }
+    __syncwarp();
   }
 }
 

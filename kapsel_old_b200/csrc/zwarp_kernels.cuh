@@ -131,7 +131,7 @@ __device__ __forceinline__ void wpack_c2r(const Cx<R> *A, Cx<R> *Zl, const Cx<R>
 template <typename R, int LM>
 __device__ __forceinline__ Cx<R> wunpack_r2c(const Cx<R> *Zl, int k, const Cx<R> *__restrict__ twz) {
   using Z = ZL<LM>;
-  const Cx<R> zk = Zl[zpos<LM>(k)];
+  const Cx<R> zk = Zl[zpos<LM>(k & (Z::M - 1))];  // Z[M] is Z[0]
   const Cx<R> zm = cconj(Zl[zpos<LM>((Z::M - k) & (Z::M - 1))]);
   const Cx<R> e = cadd(zk, zm), d = csub(zk, zm);
   const Cx<R> t = cmul_mi(cmul(d, twz[k]));
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products(Geo g, Twiddles<R> tw, 
   constexpr int GL = Z::RW * Z::LS, KP = Z::RW * Z::M / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * 4 * GL;
   Cx<R> wi[Z::N1], wf[Z::N1], wk[Z::KW];
   wfft_twiddles<R, LM, -1>(tw.m, wi);
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products(Geo g, Twiddles<R> tw, 
   const size_t cstr = rows * Z::TS;
   const int ngroups = (int)(rows / Z::RW);
   const R sc = R(g.inv_n);
-  for (int grp = blockIdx.x * NW + warp; grp < ngroups; grp += gridDim.x * NW) {
+  for (int grp = blockIdx.x * nw + warp; grp < ngroups; grp += gridDim.x * nw) {
     const size_t row0 = (size_t)grp * Z::RW;
 #pragma unroll
     for (int c = 0; c < 3; ++c)
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products_pf(Geo g, Twiddles<R> t
   using P = ZProd<R, LM>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * P::WARP;
   Cx<R> *stage = buf + 4 * P::GL;  // [3][RW][TS]
   Cx<R> wi[Z::N1], wf[Z::N1], wk[Z::KW];
@@ -266,9 +266,9 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products_pf(Geo g, Twiddles<R> t
   const size_t rows = (size_t)g.NX * g.NY;
   const size_t cstr = rows * Z::TS;
   const int ngroups = (int)(rows / Z::RW);
-  const int gstride = gridDim.x * NW;
+  const int gstride = gridDim.x * nw;
   const R sc = R(g.inv_n);
-  int grp = blockIdx.x * NW + warp;
+  int grp = blockIdx.x * nw + warp;
   auto issue = [&](int gq) {
     const size_t r0 = (size_t)gq * Z::RW;
 #pragma unroll
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
     if (parts && n < pp.Np) position_update_one(pp, parts, n, euler, status);
     return;
   }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   // one line group per warp: the packing reads the rows straight from global
   // memory, and the small footprint keeps more warps resident
   Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * Z::RW * Z::LS;
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
   const size_t rows = (size_t)g.NX * g.NY;
   const int ngroups = (int)(rows / Z::RW);
   const R sc = R(g.inv_n);
-  for (int task = blockIdx.x * NW + warp; task < ncomp * ngroups; task += nblk * NW) {
+  for (int task = blockIdx.x * nw + warp; task < ncomp * ngroups; task += nblk * nw) {
     const int c = task / ngroups;
     const size_t row0 = (size_t)(task - c * ngroups) * Z::RW;
     const Cx<R> *src = in + c * rows * Z::TS + row0 * Z::TS;
@@ -382,96 +382,46 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
   }
 }
 
-// One element pair of the rigidity force: phi > 1 clamp, f = up' - phi' u*
-// into the three padded lines, and phi/up cleared where phi was written.
-template <typename R, int LM>
-__device__ __forceinline__ void zw_force_item(Cx<R> *buf, R *__restrict__ phiup, size_t npts, size_t row0, int i,
-                                              typename Vec2<R>::T ph, typename Vec2<R>::T (&up)[3],
-                                              const typename Vec2<R>::T (&us)[3]) {
+// Forward z of real fields in[c][rows][NZ] (planes in_cstride apart), kz < TZ
+// kept, or all M + 1 (FULL), -> out [c][rows][TS].  Tasks (component, row
+// group), one line group per warp, as k_zw_c2r.  All element pairs of a row
+// group are loaded before the first is used.  CLEAR: the field is set back to
+// zero where it was not (the rigidity force, which only the points under a
+// particle's profile carry, is all zero again for the next scatter).
+template <typename R, int LM, int NW, bool CLEAR, bool FULL>
+__global__ void __launch_bounds__(NW * 32) k_zw_r2c(Geo g, Twiddles<R> tw, R *__restrict__ in, size_t in_cstride,
+                                                    Cx<R> *__restrict__ out, int ncomp) {
   using Z = ZL<LM>;
   using V2 = typename Vec2<R>::T;
-  const int rr = i >> LM, n = i & (Z::M - 1);
-  const size_t o = row0 * Z::NZ + 2 * (size_t)i;
-  R p0 = ph.x, p1 = ph.y;
-  if (p0 > R(1)) {
-    const R inv = R(1) / p0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) up[d].x *= inv;
-    p0 = R(1);
-  }
-  if (p1 > R(1)) {
-    const R inv = R(1) / p1;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) up[d].y *= inv;
-    p1 = R(1);
-  }
-#pragma unroll
-  for (int d = 0; d < 3; ++d)
-    buf[(d * Z::RW + rr) * Z::LS + zpos<LM>(n)] = {up[d].x - p0 * us[d].x, up[d].y - p1 * us[d].y};
-  if (ph.x != R(0) || ph.y != R(0)) {
-    const V2 zero = {R(0), R(0)};
-    *reinterpret_cast<V2 *>(phiup + o) = zero;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) *reinterpret_cast<V2 *>(phiup + (1 + d) * npts + o) = zero;
-  }
-}
-
-// Rigidity force (as k_z_force): f = up' - phi' u* with the phi > 1 clamp,
-// phi/up cleared where written, forward z, kz < TZ kept -> out [3][rows][TZ].
-// phi >= 0 at every point and up is zero wherever phi is, so clearing both
-// values of an element pair when either phi is non-zero is exact.
-template <typename R, int LM, int NW>
-__global__ void __launch_bounds__(NW * 32) k_zw_force(Geo g, Twiddles<R> tw, R *__restrict__ phiup,
-                                                      const R *__restrict__ ustar, Cx<R> *__restrict__ out) {
-  using Z = ZL<LM>;
-  using V2 = typename Vec2<R>::T;
+  constexpr int NK = FULL ? Z::M + 1 : Z::TZ, OS = (NK + 3) & ~3;
+  constexpr int NI = Z::RW * Z::M / 32;  // element pairs per lane
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * 3 * Z::RW * Z::LS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * Z::RW * Z::LS;
   Cx<R> wf[Z::N1];
   wfft_twiddles<R, LM, 1>(tw.m, wf);
   const size_t rows = (size_t)g.NX * g.NY;
-  const size_t npts = rows * Z::NZ;
   const int ngroups = (int)(rows / Z::RW);
-  constexpr int NI = Z::RW * Z::M / 32;  // element pairs per lane
-  for (int grp = blockIdx.x * NW + warp; grp < ngroups; grp += gridDim.x * NW) {
-    const size_t row0 = (size_t)grp * Z::RW;
-    // phi first, all of the lane's element pairs at once: where phi is zero
-    // up is zero too and f = up - phi u* = 0, so up and u* are read only
-    // where a particle's profile reaches (about an eighth of the points at
-    // a solid fraction of 0.14); the rest of the pass is unchanged
-    V2 ph[NI];
+  for (int task = blockIdx.x * nw + warp; task < ncomp * ngroups; task += gridDim.x * nw) {
+    const int c = task / ngroups;
+    const size_t row0 = (size_t)(task - c * ngroups) * Z::RW;
+    R *src = in + c * in_cstride + row0 * Z::NZ;
+    V2 v[NI];
 #pragma unroll
-    for (int h = 0; h < NI; ++h)
-      ph[h] = *reinterpret_cast<const V2 *>(phiup + row0 * Z::NZ + 2 * (size_t)(lane + 32 * h));
-#pragma unroll 1
+    for (int h = 0; h < NI; ++h) v[h] = *reinterpret_cast<const V2 *>(src + 2 * (lane + 32 * h));
+#pragma unroll
     for (int h = 0; h < NI; ++h) {
-      const int i = lane + 32 * h;
-      const size_t o = row0 * Z::NZ + 2 * (size_t)i;
-      V2 up[3], us[3];
-      if (ph[h].x != R(0) || ph[h].y != R(0)) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          up[d] = *reinterpret_cast<const V2 *>(phiup + (1 + d) * npts + o);
-          us[d] = *reinterpret_cast<const V2 *>(ustar + d * npts + o);
-        }
-      } else {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) up[d] = us[d] = V2{R(0), R(0)};
-      }
-      zw_force_item<R, LM>(buf, phiup, npts, row0, i, ph[h], up, us);
+      const int i = lane + 32 * h, rr = i >> LM, n = i & (Z::M - 1);
+      buf[rr * Z::LS + zpos<LM>(n)] = {v[h].x, v[h].y};
+      if (CLEAR && (v[h].x != R(0) || v[h].y != R(0))) *reinterpret_cast<V2 *>(src + 2 * i) = V2{R(0), R(0)};
     }
     __syncwarp();
-#pragma unroll
-    for (int d = 0; d < 3; ++d) wfft<R, LM, 1>(buf + d * Z::RW * Z::LS, wf);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      Cx<R> *dst = out + d * rows * Z::TS + row0 * Z::TS;
-      for (int i = lane; i < Z::RW * Z::TZ; i += 32) {
-        const int rr = i / Z::TZ, k = i - rr * Z::TZ;
-        dst[rr * Z::TS + k] = wunpack_r2c<R, LM>(buf + (d * Z::RW + rr) * Z::LS, k, tw.z);
-      }
+    wfft<R, LM, 1>(buf, wf);
+    Cx<R> *dst = out + c * rows * OS + row0 * OS;
+    for (int i = lane; i < Z::RW * NK; i += 32) {
+      const int rr = i / NK, k = i - rr * NK;
+      dst[rr * OS + k] = wunpack_r2c<R, LM>(buf + rr * Z::LS, k, tw.z);
     }
     __syncwarp();
   }
