@@ -960,7 +960,7 @@ struct Box : BoxBase {
   size_t sm_xo6 = 0, sm_xo3 = 0, sm_xof = 0;
 
   int alloc_obl() override {
-    const size_t N = npts(), nst = OB_PART + 2 * (size_t)OB_RED_BLOCKS;
+    const size_t N = npts(), nst = OB_SIZE;
     KCHECK(cudaMalloc(&ob6, sizeof(R) * 6 * N));
     KCHECK(cudaMalloc(&obB, sizeof(R) * 3 * N));
     KCHECK(cudaMalloc(&obst, sizeof(double) * nst));
@@ -1007,23 +1007,20 @@ struct Box : BoxBase {
     k_x_obl_inv<R, KCX, 3><<<gx(), 256, sm_xo3, stream>>>(g, tw, zeta, uk_dc, obst, bufA);
     launch_y<true>(g, 3, bufA, bufB);
     k_z_c2r<R><<<dim3(gz(), 3), 256, smem_zc, stream>>>(g, tw, bufB, ob6, N, g.NZ, PPar{}, nullptr, 0, nullptr);
-    // deformation: degree_oblique, grid reset, Cartesian u (ustar), Shear_rate_eff
-    k_obl_degree<<<1, 32, 0, stream>>>(op, obst);
-    k_obl_remap<R><<<pb, 256, 0, stream>>>(op, (const double *)obst, (const R *)ob6, obB);
-    k_obl_to_cart<R><<<pb, 256, 0, stream>>>(op, (const double *)obst, (const R *)obB, ustar);
-    k_obl_srate_partial<R><<<OB_RED_BLOCKS, 256, 0, stream>>>(op, (const R *)ustar, obst);
-    k_obl_srate_final<<<1, 32, 0, stream>>>(op, obst, OB_RED_BLOCKS);
+    // deformation: degree_oblique, grid reset, Cartesian u (ustar), Shear_rate_eff,
+    // positions
+    k_obl_to_cart<R><<<pb, 256, 0, stream>>>(op, (const double *)obst, (const R *)ob6, ustar);
+    k_obl_srate_position<R><<<1, 1024, 0, stream>>>(op, (const R *)ustar, obst, pp, parts, euler, status);
     if (Np > 0) {
-      k_obl_position<<<(Np + 127) / 128, 128, 0, stream>>>(pp, parts, euler, (const double *)obst, status);
-      k_obl_hydro_velocity<R><<<Np, 256, 0, stream>>>(pp, parts, (const R *)ustar, (const int *)cells, noise, euler,
+      k_obl_hydro_velocity<R><<<Np, 512, 0, stream>>>(pp, parts, (const R *)ustar, (const int *)cells, noise, euler,
                                                        (const double *)obst, status);
       k_obl_scatter<R><<<Np * PCL, 256, 0, stream>>>(pp, (const DPart *)parts, (const int *)cells,
                                                       (const double *)obst, phiup);
     }
     // f = up - phi u (Cartesian), u += U2u_oblique(f), forward, Solenoidal_uk_OBL,
     // contra2co, U_k2zeta_k_OBL
-    k_obl_force<R><<<pb, 256, 0, stream>>>(N, phiup, (const R *)ustar, ob6);
-    k_obl_add_force<R><<<pb, 256, 0, stream>>>(op, (const double *)obst, (const R *)ob6, obB);
+    k_obl_force<R><<<pb, 256, 0, stream>>>(N, phiup, (const R *)ustar, ob6 + 3 * N);
+    k_obl_add_force<R><<<pb, 256, 0, stream>>>(op, (const double *)obst, (const R *)(ob6 + 3 * N), (const R *)ob6, obB);
     k_z_r2c<R><<<dim3(gz(), 3), 256, smem_zc, stream>>>(g, tw, obB, g.NZ, N, bufB, g.TZ, g.TS);
     launch_y<false>(g, 3, bufB, bufA);
     k_x_obl_fwd<R, KCX, 0><<<gx(), 256, sm_xof, stream>>>(g, tw, bufA, zeta, uk_dc, obst);

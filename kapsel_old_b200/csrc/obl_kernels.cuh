@@ -4,7 +4,7 @@
 // State that changes every step lives in device memory so that the step can
 // be captured into a CUDA graph: ObState[0] = degree_oblique (input.cxx:271),
 // [1] = Shear_rate_eff, [2] = 1 when this step reset the oblique grid,
-// [3] = Shear_strain_realized (sp_3d_ns.cxx:600), [8..] reduction partials.
+// [3] = Shear_strain_realized (sp_3d_ns.cxx:600).
 //
 // k-space operators (one mode at a time, retained 2/3 box only; the
 // reference truncates zeta at the start of every step, operate_omega.cxx:
@@ -32,8 +32,7 @@
 
 namespace kapsel {
 
-enum { OB_DEG = 0, OB_SRATE = 1, OB_REMAP = 2, OB_STRAIN = 3, OB_PART = 8 };
-constexpr int OB_RED_BLOCKS = 296;
+enum { OB_DEG = 0, OB_SRATE = 1, OB_REMAP = 2, OB_STRAIN = 3, OB_SIZE = 8 };
 
 struct OblPar {
   double shear_rate;  // Shear_rate of the DC external field
@@ -307,40 +306,29 @@ __global__ void k_obl_cross(size_t n, const R *__restrict__ uw, R *__restrict__ 
   }
 }
 
-// degree_oblique += Shear_rate dt, Shear_rate_eff = Shear_rate, and the grid
-// reset when it reaches 1 (sp_3d_ns.cxx:261,278-303).  One thread.  The
-// product and the sum are rounded separately, as the reference computes them.
-__global__ void k_obl_degree(OblPar o, double *__restrict__ st) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double deg = __dadd_rn(st[OB_DEG], __dmul_rn(o.shear_rate, o.dt));
-  const int remap = deg >= 1.0;
-  if (remap) deg = __dsub_rn(deg, 1.0);
-  st[OB_DEG] = deg;
-  st[OB_SRATE] = o.shear_rate;
-  st[OB_REMAP] = (double)remap;
+// degree_oblique of this step, += Shear_rate dt, and whether it reaches 1,
+// where the grid is reset (sp_3d_ns.cxx:261,278-303).  The product and the
+// sum are rounded separately, as the reference computes them.
+__device__ __forceinline__ double obl_next_degree(const OblPar &o, const double *__restrict__ st, bool &remap) {
+  const double deg = __dadd_rn(st[OB_DEG], __dmul_rn(o.shear_rate, o.dt));
+  remap = deg >= 1.0;
+  return remap ? __dsub_rn(deg, 1.0) : deg;
 }
 
-// Grid reset (sp_3d_ns.cxx:279-302): when the step passed degree_oblique = 1,
-// out[0](i', j) = u0(i, j) + u1(i, j), out[1..2](i', j) = u(i, j) with
-// i' = i + j - NY/2 (mod NX); otherwise a copy.
+// Row (i, j) of the oblique-grid u of this step in the field before the grid
+// reset (sp_3d_ns.cxx:279-302): itself, or with i' = i + j - NY/2 (mod NX)
+// the row that the reset moves to i.
+__device__ __forceinline__ size_t obl_source_row(const OblPar &o, bool remap, int i, int j) {
+  const int a = remap ? (i - (j - o.NY / 2)) & (o.NX - 1) : i;  // NX is a power of two
+  return (size_t)a * o.NY + j;
+}
+// The three components at point s: the reset also adds u1 to u0.
 template <typename R>
-__global__ void k_obl_remap(OblPar o, const double *__restrict__ st, const R *__restrict__ in, R *__restrict__ out) {
-  const size_t n = (size_t)o.NX * o.NY * o.NZ;
-  const bool remap = st[OB_REMAP] != 0.0;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(e % o.NZ);
-    const int j = (int)((e / o.NZ) % o.NY);
-    const int id = (int)(e / ((size_t)o.NZ * o.NY));
-    if (!remap) {
-      for (int c = 0; c < 3; ++c) out[c * n + e] = in[c * n + e];
-      continue;
-    }
-    const int i = ((id - (j - o.NY / 2)) % o.NX + o.NX) % o.NX;
-    const size_t s = ((size_t)i * o.NY + j) * o.NZ + k;
-    out[e] = in[s] + in[n + s];
-    out[n + e] = in[n + s];
-    out[2 * n + e] = in[2 * n + s];
-  }
+__device__ __forceinline__ void obl_source(const R *__restrict__ in, size_t n, size_t s, bool remap, R v[3]) {
+  v[0] = in[s];
+  v[1] = in[n + s];
+  v[2] = in[2 * n + s];
+  if (remap) v[0] += v[1];
 }
 
 // Interpolation weights of row j (U_oblique2u, fft_wrapper.h:292-300):
@@ -354,27 +342,41 @@ __device__ __forceinline__ int obl_row_o2c(int j, int NY, double deg, double &al
   return io;
 }
 
-// U_oblique2u (fft_wrapper.h:265-325): oblique-grid contravariant u -> the
+// degree_oblique of this step, the grid reset and U_oblique2u
+// (fft_wrapper.h:265-325) in one pass: oblique-grid contravariant u -> the
 // Cartesian u of the sheared frame plus the mean shear flow S (y - NY/2).
-// out(i_ob) from in(i), in(i + sign) where i_ob = i + shift (mod NX).
+// out(i_ob) from in(i), in(i + sign) where i_ob = i + shift (mod NX).  The
+// new degree is only computed here; k_obl_srate_position stores it.  One
+// warp per row of NZ points, which share the interpolation weights; the
+// reset is an index into the field before it, so no copy of the field is
+// made (three launches and 24 + 24 bytes a point before: 44 us at 128^3 in
+// FP32 against 13).
 template <typename R>
-__global__ void k_obl_to_cart(OblPar o, const double *__restrict__ st, const R *__restrict__ in, R *__restrict__ out) {
+__global__ void __launch_bounds__(256) k_obl_to_cart(OblPar o, const double *__restrict__ st, const R *__restrict__ in,
+                                                     R *__restrict__ out) {
   const size_t n = (size_t)o.NX * o.NY * o.NZ;
-  const double deg = st[OB_DEG], srate = st[OB_SRATE];
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(e % o.NZ);
-    const int j = (int)((e / o.NZ) % o.NY);
-    const int iob = (int)(e / ((size_t)o.NZ * o.NY));
+  bool remap;
+  const double deg = obl_next_degree(o, st, remap), srate = o.shear_rate;
+  const int lane = threadIdx.x & 31;
+  for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < o.NX * o.NY;
+       row += (gridDim.x * blockDim.x) >> 5) {
+    const int j = row & (o.NY - 1), iob = row / o.NY;
     double alpha, sign;
     const int io = obl_row_o2c(j, o.NY, deg, alpha, sign);
     const double beta = 1. - alpha;
-    const int i = ((iob - io) % o.NX + o.NX) % o.NX;
-    const int ip = ((i + (int)sign) % o.NX + o.NX) % o.NX;
-    const size_t s = ((size_t)i * o.NY + j) * o.NZ + k, sp = ((size_t)ip * o.NY + j) * o.NZ + k;
-    const double w1 = beta * (double)in[n + s] + alpha * (double)in[n + sp];
-    out[e] = (R)((beta * (double)in[s] + alpha * (double)in[sp]) + deg * w1 + srate * ((double)j - o.NY / 2.));
-    out[n + e] = (R)w1;
-    out[2 * n + e] = (R)(beta * (double)in[2 * n + s] + alpha * (double)in[2 * n + sp]);
+    const int i = (iob - io) & (o.NX - 1);
+    const int ip = (i + (int)sign) & (o.NX - 1);
+    const size_t s = obl_source_row(o, remap, i, j) * o.NZ, sp = obl_source_row(o, remap, ip, j) * o.NZ;
+    for (int k = lane; k < o.NZ; k += 32) {
+      R a[3], b[3];
+      obl_source(in, n, s + k, remap, a);
+      obl_source(in, n, sp + k, remap, b);
+      const size_t e = (size_t)row * o.NZ + k;
+      const double w1 = beta * (double)a[1] + alpha * (double)b[1];
+      out[e] = (R)((beta * (double)a[0] + alpha * (double)b[0]) + deg * w1 + srate * ((double)j - o.NY / 2.));
+      out[n + e] = (R)w1;
+      out[2 * n + e] = (R)(beta * (double)a[2] + alpha * (double)b[2]);
+    }
   }
 }
 
@@ -396,67 +398,41 @@ __global__ void k_obl_force(size_t n, R *__restrict__ phiup, const R *__restrict
   }
 }
 
-// u += U2u_oblique(f) (fft_wrapper.h:204-263, f_particle.h:83-99): the
+// out = u + U2u_oblique(f) (fft_wrapper.h:204-263, f_particle.h:83-99): the
 // Cartesian force interpolated back to the oblique grid, as contravariant
-// components.
+// components, added to the (reset, see obl_source_row) oblique-grid u.
 template <typename R>
-__global__ void k_obl_add_force(OblPar o, const double *__restrict__ st, const R *__restrict__ f, R *__restrict__ u) {
+__global__ void __launch_bounds__(256) k_obl_add_force(OblPar o, const double *__restrict__ st,
+                                                       const R *__restrict__ f, const R *__restrict__ u,
+                                                       R *__restrict__ out) {
   const size_t n = (size_t)o.NX * o.NY * o.NZ;
   const double deg = st[OB_DEG];
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(e % o.NZ);
-    const int j = (int)((e / o.NZ) % o.NY);
-    const int i = (int)(e / ((size_t)o.NZ * o.NY));
+  const bool remap = st[OB_REMAP] != 0.0;
+  const int lane = threadIdx.x & 31;
+  for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < o.NX * o.NY;
+       row += (gridDim.x * blockDim.x) >> 5) {
+    const int j = row & (o.NY - 1), i = row / o.NY;
     double sign = (double)(j - o.NY / 2);
     if (!(sign == 0)) sign = sign / fabs(sign);
     const double jd = (double)(j - o.NY / 2);
     const int io = (int)((double)(int)(sign * deg * jd) * sign);
     const double alpha = (deg * jd - (double)io) * sign, beta = 1. - alpha;
-    const int iob = ((i + io) % o.NX + o.NX) % o.NX;
-    const int iobp = ((iob + (int)sign) % o.NX + o.NX) % o.NX;
-    const size_t s = ((size_t)iob * o.NY + j) * o.NZ + k, sp = ((size_t)iobp * o.NY + j) * o.NZ + k;
-    const double g1 = beta * (double)f[n + s] + alpha * (double)f[n + sp];
-    const double g0 = (beta * (double)f[s] + alpha * (double)f[sp]) - deg * g1;
-    const double g2 = beta * (double)f[2 * n + s] + alpha * (double)f[2 * n + sp];
-    u[e] = (R)((double)u[e] + g0);
-    u[n + e] = (R)((double)u[n + e] + g1);
-    u[2 * n + e] = (R)((double)u[2 * n + e] + g2);
+    const int iob = (i + io) & (o.NX - 1);
+    const int iobp = (iob + (int)sign) & (o.NX - 1);
+    const size_t s = ((size_t)iob * o.NY + j) * o.NZ, sp = ((size_t)iobp * o.NY + j) * o.NZ;
+    const size_t su = obl_source_row(o, remap, i, j) * o.NZ;
+    for (int k = lane; k < o.NZ; k += 32) {
+      R v[3];
+      obl_source(u, n, su + k, remap, v);
+      const double g1 = beta * (double)f[n + s + k] + alpha * (double)f[n + sp + k];
+      const double g0 = (beta * (double)f[s + k] + alpha * (double)f[sp + k]) - deg * g1;
+      const double g2 = beta * (double)f[2 * n + s + k] + alpha * (double)f[2 * n + sp + k];
+      const size_t e = (size_t)row * o.NZ + k;
+      out[e] = (R)((double)v[0] + g0);
+      out[n + e] = (R)((double)v[1] + g1);
+      out[2 * n + e] = (R)((double)v[2] + g2);
+    }
   }
-}
-
-// Calc_shear_rate_eff (sp_3d_ns.h:174-196): the mean of d u0/dy over the
-// NY-1 interior y differences, in two launches (partial sums per block,
-// compensated, then the final sum by one block).
-template <typename R>
-__global__ void __launch_bounds__(256) k_obl_srate_partial(OblPar o, const R *__restrict__ u0, double *__restrict__ st) {
-  __shared__ double sh[2 * 32];
-  const size_t nterm = (size_t)o.NX * (o.NY - 1) * o.NZ;
-  KSum s{0.0, 0.0};
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nterm; e += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(e % o.NZ);
-    const int j = (int)((e / o.NZ) % (o.NY - 1));
-    const int i = (int)(e / ((size_t)o.NZ * (o.NY - 1)));
-    const size_t a = ((size_t)i * o.NY + j) * o.NZ + k;
-    s.add(((double)u0[a + o.NZ] - (double)u0[a]) / o.dx);
-  }
-  KSum v[1] = {s};
-  block_reduce<1>(v, sh);
-  if (threadIdx.x == 0) {
-    st[OB_PART + 2 * blockIdx.x] = v[0].s;
-    st[OB_PART + 2 * blockIdx.x + 1] = v[0].c;
-  }
-}
-__global__ void k_obl_srate_final(OblPar o, double *__restrict__ st, int nblocks) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  KSum s{0.0, 0.0};
-  double c = 0.0;
-  for (int b = 0; b < nblocks; ++b) {
-    s.add(st[OB_PART + 2 * b]);
-    c += st[OB_PART + 2 * b + 1];
-  }
-  const double srate = (s.s + (s.c + c)) * o.srate_scale;
-  st[OB_SRATE] = srate;
-  st[OB_STRAIN] += srate * o.dt;
 }
 
 // ---------------------------------------------------------------------------
@@ -467,18 +443,17 @@ __global__ void k_obl_srate_final(OblPar o, double *__restrict__ st, int nblocks
 // x is shifted by degree_oblique NY cells.
 __device__ __forceinline__ int obl_stencil_point(const StencilBase &b, const int *cell, const PPar &p, double deg,
                                                  int rm[3], double r[3]) {
-  double signY = (double)(b.xi[1] + cell[1]);
-  rm[1] = (b.xi[1] + cell[1] + p.N[1]) % p.N[1];
-  signY -= (double)rm[1];
-  int sign = (int)signY;
-  if (!(sign == 0)) sign = sign / abs(sign);
+  const int jy = b.xi[1] + cell[1];
+  rm[1] = jy & (p.N[1] - 1);  // N is a power of two
+  const int sign = (jy > rm[1]) - (jy < rm[1]);
   const double xo = (double)b.xi[0] - (double)sign * deg * (double)p.N[1] + b.res[0] / p.DX + (double)cell[0] +
                     (double)(4 * p.N[0]);
-  double xm = fmod(xo, (double)p.N[0]);
-  if (xm < 0.0) xm += (double)p.N[0];  // only past 4 box lengths of shift; keeps the index inside the field
+  // xo modulo N: exact in this form too for a power of two, in three
+  // operations where fmod takes a long division
+  const double xm = xo - (double)p.N[0] * floor(xo * (1.0 / (double)p.N[0]));
   rm[0] = min((int)xm, p.N[0] - 1);
   const double xres = xm - (double)rm[0];
-  rm[2] = (b.xi[2] + cell[2] + p.N[2]) % p.N[2];
+  rm[2] = (b.xi[2] + cell[2]) & (p.N[2] - 1);
   r[0] = (double)cell[0] * p.DX - xres * p.DX;
   r[1] = (double)cell[1] * p.DX - b.res[1];
   r[2] = (double)cell[2] * p.DX - b.res[2];
@@ -499,25 +474,72 @@ __device__ __forceinline__ int pbc_obl(double *x, const PPar &p, double deg) {
   return sign;
 }
 
-// MD_solver_position_Euler_OBL / _AB2_OBL (particle_solver.cxx:292-346).
-__global__ void k_obl_position(PPar p, DPart *__restrict__ parts, int euler, const double *__restrict__ st,
-                               int *__restrict__ status) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= p.Np || p.frozen) return;
-  DPart &a = parts[n];
+// MD_solver_position_Euler_OBL / _AB2_OBL (particle_solver.cxx:292-346) of
+// one particle.
+__device__ __forceinline__ void obl_position_one(const PPar &p, DPart &a, int euler, double deg, double srate,
+                                                 int *__restrict__ status) {
   const double hdt = 0.5 * p.dt;
   for (int d = 0; d < 3; ++d) {
     const double dx = euler ? p.dt * a.v[d] : hdt * (3.0 * a.v[d] - a.v_old[d]);
     a.x_nopbc[d] += dx;
     a.x[d] += dx;
   }
-  const int sign = pbc_obl(a.x, p, st[OB_DEG]);
-  const double dvx = -(double)sign * st[OB_SRATE] * p.L[1];
+  const int sign = pbc_obl(a.x, p, deg);
+  const double dvx = -(double)sign * srate * p.L[1];
   a.v[0] += dvx;
   a.v_old[0] += dvx;
   for (int d = 0; d < 3; ++d)
     if (!(a.x[d] >= 0.0 && a.x[d] < p.L[d])) atomicExch(status, -6);
   if (p.rotation) orientation_update(p, a, euler);
+}
+
+// One block: the new degree_oblique and reset flag into the state, then
+// Calc_shear_rate_eff (sp_3d_ns.h:174-196), then the particle positions,
+// which need both.  The mean of d u0/dy over the NY - 1 interior y
+// differences of a column telescopes to its last value less its first, so
+// only two of NY rows of u0 are read; the column terms are summed
+// compensated, per thread, then over the block.  Measured at 128^3 with 256
+// particles, FP32: 10 us, where the sum over all differences, its final sum
+// and the positions took 28 + 31 + 6 us as three launches.
+template <typename R>
+__global__ void __launch_bounds__(1024) k_obl_srate_position(OblPar o, const R *__restrict__ u0, double *__restrict__ st,
+                                                             PPar p, DPart *__restrict__ parts, int euler,
+                                                             int *__restrict__ status) {
+  __shared__ double sh[2 * 32];
+  __shared__ double state[2];
+  const int cols = o.NX * o.NZ;
+  const size_t plane = (size_t)o.NY * o.NZ, last = (size_t)(o.NY - 1) * o.NZ;
+  KSum s{0.0, 0.0};
+  constexpr int B = 8;  // columns of a thread whose loads are in flight together
+  for (int e0 = threadIdx.x; e0 < cols; e0 += B * blockDim.x) {
+    R lo[B], hi[B];
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const int e = e0 + b * blockDim.x;
+      lo[b] = hi[b] = R(0);
+      if (e < cols) {
+        const size_t a = (size_t)(e / o.NZ) * plane + (e & (o.NZ - 1));
+        lo[b] = u0[a];
+        hi[b] = u0[a + last];
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < B; ++b) s.add(((double)hi[b] - (double)lo[b]) / o.dx);
+  }
+  KSum v[1] = {s};
+  block_reduce<1>(v, sh);
+  if (threadIdx.x == 0) {
+    bool remap;
+    const double deg = obl_next_degree(o, st, remap);
+    const double srate = (v[0].s + v[0].c) * o.srate_scale;
+    st[OB_DEG] = state[0] = deg;
+    st[OB_REMAP] = remap ? 1.0 : 0.0;
+    st[OB_SRATE] = state[1] = srate;
+    st[OB_STRAIN] += srate * o.dt;
+  }
+  __syncthreads();
+  if (p.frozen) return;
+  for (int n = threadIdx.x; n < p.Np; n += blockDim.x) obl_position_one(p, parts[n], euler, state[0], state[1], status);
 }
 
 // Distance0_OBL (interaction.h:39-65): x12 = LE-image of x2 - x1.
@@ -544,14 +566,16 @@ __device__ __forceinline__ double distance_obl(const double *x1, const double *x
 // velocity, Force_OBL (particle_solver.h:111-128: all-pairs LJ,
 // md_force.cxx:136-179, then gravity), MD_solver_velocity_Euler_OBL /
 // _AB2_hydro_OBL (particle_solver.cxx:348-440) and the thermostat kick.
-// One block per particle; the pair forces are summed by thread 0 in the
-// reference's order (partner index ascending).
+// One block per particle.  The threads of the block share the partners of
+// the pair force as they share the stencil points (one thread walking all
+// of them, each step a dependent load, was 85% of the kernel: 171 us at
+// 128^3 with 256 particles, 20 us now); every sum is compensated.
 template <typename R>
-__global__ void __launch_bounds__(256) k_obl_hydro_velocity(PPar p, DPart *__restrict__ parts,
+__global__ void __launch_bounds__(512) k_obl_hydro_velocity(PPar p, DPart *__restrict__ parts,
                                                             const R *__restrict__ u, const int *__restrict__ cells,
                                                             const double *__restrict__ noise, int euler,
                                                             const double *__restrict__ st, int *__restrict__ status) {
-  __shared__ double sh[2 * 6 * 32];
+  __shared__ double sh[2 * 9 * 32];
   const int n = blockIdx.x;
   DPart &a = parts[n];
   const double deg = st[OB_DEG], srate = st[OB_SRATE];
@@ -560,14 +584,15 @@ __global__ void __launch_bounds__(256) k_obl_hydro_velocity(PPar p, DPart *__res
   const double wp[3] = {a.omega[0], a.omega[1], a.omega[2]};
   const StencilBase b = stencil_base(xp, p);
   const size_t npts = (size_t)p.N[0] * p.N[1] * p.N[2];
-  KSum acc[6];
-  for (int i = 0; i < 6; ++i) acc[i] = {0.0, 0.0};
+  KSum acc[9];
+  for (int i = 0; i < 9; ++i) acc[i] = {0.0, 0.0};
   for (int m = threadIdx.x; m < p.S; m += blockDim.x) {
     int rm[3];
     double r[3];
     const int sign = obl_stencil_point(b, cells + 3 * m, p, deg, rm, r);
     const double dist = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
     const double ph = (double)prof_phi<R>(dist, p);
+    if (ph == 0.0) continue;  // a zero term: skip its loads
     double vr[3] = {0.0, 0.0, 0.0};
     if (p.rotation) {
       vr[0] = wp[1] * r[2] - wp[2] * r[1];
@@ -584,11 +609,8 @@ __global__ void __launch_bounds__(256) k_obl_hydro_velocity(PPar p, DPart *__res
     acc[4].add(r[2] * fp[0] - r[0] * fp[2]);
     acc[5].add(r[0] * fp[1] - r[1] * fp[0]);
   }
-  block_reduce<6>(acc, sh);
-  if (threadIdx.x != 0) return;
-  double fr[3] = {0.0, 0.0, 0.0};
-  if (p.lj_on) {
-    for (int j = 0; j < p.Np; ++j) {
+  if (p.lj_on)
+    for (int j = threadIdx.x; j < p.Np; j += blockDim.x) {
       if (j == n) continue;
       double x12[3];
       const double rij = j < n ? distance_obl(parts[j].x, xp, p, deg, x12) : distance_obl(xp, parts[j].x, p, deg, x12);
@@ -599,13 +621,13 @@ __global__ void __launch_bounds__(256) k_obl_hydro_velocity(PPar p, DPart *__res
         if (p.lj_powers >= 1) dmy = dmy * dmy;
         if (p.lj_powers >= 2) dmy = dmy * (s * s) * (s * s) * (s * s);
         const double f = p.lj_coeff / (rij * rij) * (2.0 * dmy * dmy - dmy);
-        for (int d = 0; d < 3; ++d) {
-          const double d1 = f * -x12[d];
-          fr[d] = j < n ? fr[d] - d1 : fr[d] + d1;
-        }
+        for (int d = 0; d < 3; ++d) acc[6 + d].add(j < n ? f * x12[d] : f * -x12[d]);
       }
     }
-  }
+  block_reduce<9>(acc, sh);
+  if (threadIdx.x != 0) return;
+  double fr[3];
+  for (int d = 0; d < 3; ++d) fr[d] = acc[6 + d].s + acc[6 + d].c;
   fr[p.gdir] -= p.grav;
   double fh[3], th[3];
   for (int d = 0; d < 3; ++d) {
