@@ -127,10 +127,25 @@ __device__ __forceinline__ void cp_async_cx(Cx<R> *smem, const Cx<R> *gmem) {
 // Programmatic dependent launch: let the next kernel of the stream start its
 // launch now, then wait until the previous kernel has finished and its
 // writes are visible.  Both are no-ops when the kernel was launched without
-// the programmatic-serialization attribute.
+// the programmatic-serialization attribute.  It is the first statement of a
+// kernel: with constant loads (twiddles) placed between the two, loads of the
+// previous kernel's output through `const __restrict__` arguments, which the
+// compiler may take for memory that never changes while the kernel runs, were
+// moved up across the wait (wrong results).  Hiding every pointer from that
+// assumption made it correct again, and slower than this form (128^3 mixed
+// step 158 -> 160 us, 256^3 1813 -> 1877 us).
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// A pointer to an earlier launch's data that the compiler cannot take for an
+// argument of this kernel (see above).  It goes by way of the global address,
+// so that the result is known to be global memory.
+template <typename T>
+__device__ __forceinline__ T *pdl_fresh(T *p) {
+  size_t a = __cvta_generic_to_global(p);
+  asm volatile("" : "+l"(a)::"memory");
+  return reinterpret_cast<T *>(__cvta_global_to_generic(a));
 }
 
 // Cooperative copy of a twiddle table (n entries) into shared memory.

@@ -148,6 +148,28 @@ std::vector<int> sekibun(double A, double A_XI, double DX) {
   return out;
 }
 
+// The offsets the particle kernels visit: those of the Sekibun list (which
+// reaches RADIUS + HXI + 1.7321 DX) that can lie inside a profile's support,
+// RADIUS + HXI, for some position of the centre within its cell.  phi is
+// exactly zero at the others (1935 offsets, 1256 kept at a = 5, xi = 2).  On
+// a grid that the support nearly spans a far offset folds back to a near
+// point, and the whole list is kept.
+std::vector<short4> stencil_cells(const std::vector<int> &sek, double A, double A_XI, const int N[3]) {
+  const double sup = A + 0.5 * A_XI;  // in cells
+  const bool all = std::min(N[0], std::min(N[1], N[2])) < 2.0 * sup + 4.0;
+  std::vector<short4> out;
+  for (size_t m = 0; m + 2 < sek.size(); m += 3) {
+    double near2 = 0.0;  // the centre is 0..1 cells past its cell's origin
+    for (int d = 0; d < 3; ++d) {
+      const double c = sek[m + d], n = c > 0 ? c - 1.0 : -c;
+      near2 += n * n;
+    }
+    if (all || std::sqrt(near2) < sup * (1.0 + 1e-5))
+      out.push_back(make_short4((short)sek[m], (short)sek[m + 1], (short)sek[m + 2], 0));
+  }
+  return out;
+}
+
 template <typename R, bool INVERSE>
 __global__ void k_col_pass(Geo g, const Cx<R> *twn, int logn, int n, const Cx<R> *in, Cx<R> *out,
                            long long line_stride, long long elem_stride, int nlines, int lines_per_plane,
@@ -186,7 +208,7 @@ struct BoxBase {
   int Np = 0, S = 0;
   cudaStream_t stream = nullptr;
   DPart *parts = nullptr;
-  int *cells = nullptr;
+  short4 *cells = nullptr;  // stencil offsets of the particle kernels (pp.S of them)
   double *uk_dc = nullptr;
   int *status = nullptr;
   double *partial_p = nullptr;  // [Np][PCL][18] partial force sums
@@ -491,22 +513,26 @@ struct Box : BoxBase {
   int nsm = 0;
   static constexpr int ZNW = sizeof(R) == 4 ? 8 : 4;  // warps per block at most
   int zw = 0;
-  // launch shape of a warp-level z kernel with `tasks` row groups to do
+  // launch shape of a warp-level z kernel
   struct ZPlan {
-    int nw = 0, grid = 0;
+    int nw = 0, cap = 0;  // warps per block; blocks the GPU holds at once
     size_t sm = 0;
+    int grid(int tasks) const { return std::min((tasks + nw - 1) / nw, cap); }
   };
   ZPlan zp_p, zp_c, zp_f;
+  ZPlan zp_pu, zp_q, zp_qf, zp_fl, zp_cb;  // Electrolyte
+  ZPlan zp_x, zp_of;                       // Lees-Edwards
   template <typename K>
-  int zplan(K kern, int tasks, size_t warp_bytes, ZPlan &p) {
-    KCHECK(allow_smem(kern, warp_bytes * ZNW));
+  int zplan(K kern, size_t warp_bytes, ZPlan &p) {
+    p.nw = ZNW;
+    while (p.nw > 1 && warp_bytes * p.nw > 227 * 1024) p.nw >>= 1;
+    KCHECK(allow_smem(kern, warp_bytes * p.nw));
     int dev = 0, occ = 0;
     KCHECK(cudaGetDevice(&dev));
     KCHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    p.nw = ZNW;
     p.sm = warp_bytes * p.nw;
     KCHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, p.nw * 32, p.sm));
-    p.grid = std::min((tasks + p.nw - 1) / p.nw, std::max(occ, 1) * nsm);
+    p.cap = std::max(occ, 1) * nsm;
     return 0;
   }
 
@@ -514,12 +540,22 @@ struct Box : BoxBase {
   int zw_setup() {
     using Z = ZL<LM>;
     const size_t line = sizeof(Cx<R>) * Z::RW * Z::LS;  // one line group
-    const int groups = g.NX * g.NY / Z::RW;
     // FP64: the prefetching products kernel; FP32: four line groups per warp
-    int rc = zplan(sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW> : k_zw_products<R, LM, ZNW>, groups,
-                   sizeof(R) == 8 ? sizeof(Cx<R>) * (size_t)ZProd<R, LM>::WARP : 4 * line, zp_p);
-    if (!rc) rc = zplan(k_zw_c2r<R, LM, ZNW>, 3 * groups, line, zp_c);
-    if (!rc) rc = zplan(k_zw_r2c<R, LM, ZNW, true, false>, 3 * groups, line, zp_f);
+    const size_t prod = sizeof(R) == 8 ? sizeof(Cx<R>) * (size_t)ZProd<R, LM>::WARP : 4 * line;
+    int rc = zplan(sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW> : k_zw_products<R, LM, ZNW>, prod, zp_p);
+    if (!rc) rc = zplan(k_zw_c2r<R, LM, ZNW>, line, zp_c);
+    if (!rc) rc = zplan(k_zw_r2c<R, LM, ZNW, true, false>, line, zp_f);
+    if (!rc && prm.eq == KAPSEL_EQ_ELECTROLYTE) {
+      rc = zplan(sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW, true> : k_zw_products<R, LM, ZNW, true>, prod, zp_pu);
+      if (!rc) rc = zplan(k_zw_charge<R, LM, ZNW, false>, line, zp_q);
+      if (!rc) rc = zplan(k_zw_charge<R, LM, ZNW, true>, line, zp_qf);
+      if (!rc) rc = zplan(k_zw_flux<R, LM, ZNW>, 3 * line, zp_fl);
+      if (!rc) rc = zplan(k_zw_coulomb<R, LM, ZNW>, 3 * line, zp_cb);
+    }
+    if (!rc && prm.eq == KAPSEL_EQ_SHEAR_LE) {
+      rc = zplan(k_zw_cross<R, LM, ZNW>, 6 * line, zp_x);
+      if (!rc) rc = zplan(k_zw_obl_force<R, LM, ZNW>, 3 * line, zp_of);
+    }
     if (rc) return rc;
     zw = LM;
     yz_ly = 0;
@@ -547,27 +583,27 @@ struct Box : BoxBase {
     return 0;
   }
   template <int LY, int LM>
-  void yz_c2r_l(bool pdl, DPart *pts, int euler) {
+  void yz_c2r_l(bool pdl, R *out, DPart *pts, int euler) {
     const int posblk = pts ? (Np + YZNW * 32 - 1) / (YZNW * 32) : 0;
     launch_k(pdl, k_yzw_c2r<R, LY, LM, false, YZNW>, dim3(3 * g.NX + posblk), dim3(YZNW * 32), yz_sm, stream, g, tw,
-             (const Cx<R> *)bufA, ustar, npts(), g.NZ, 3 * g.NX, pp, pts, euler, status);
+             (const Cx<R> *)bufA, out, npts(), g.NZ, 3 * g.NX, pp, pts, euler, status);
   }
   template <int LY, int LM>
   void zy_force_l(bool pdl) {
     launch_k(pdl, k_zyw_r2c<R, LY, LM, true, YZNW>, dim3(3 * g.NX), dim3(YZNW * 32), yz_sm, stream, g, tw, force(),
              npts(), bufA);
   }
-  // bufA (x real, ky compact) -> u*, with the position update in extra blocks
+  // bufA (x real, ky compact) -> real fields, with the position update in extra blocks
   template <int LM>
-  void yz_c2r_m(bool pdl, DPart *pts, int euler) {
-    if (yz_ly == 5) yz_c2r_l<5, LM>(pdl, pts, euler);
-    else if (yz_ly == 6) yz_c2r_l<6, LM>(pdl, pts, euler);
-    else yz_c2r_l<7, LM>(pdl, pts, euler);
+  void yz_c2r_m(bool pdl, R *out, DPart *pts, int euler) {
+    if (yz_ly == 5) yz_c2r_l<5, LM>(pdl, out, pts, euler);
+    else if (yz_ly == 6) yz_c2r_l<6, LM>(pdl, out, pts, euler);
+    else yz_c2r_l<7, LM>(pdl, out, pts, euler);
   }
-  void yz_c2r(bool pdl, DPart *pts, int euler) {
-    if (zw == 5) yz_c2r_m<5>(pdl, pts, euler);
-    else if (zw == 6) yz_c2r_m<6>(pdl, pts, euler);
-    else yz_c2r_m<7>(pdl, pts, euler);
+  void yz_c2r(bool pdl, R *out, DPart *pts, int euler) {
+    if (zw == 5) yz_c2r_m<5>(pdl, out, pts, euler);
+    else if (zw == 6) yz_c2r_m<6>(pdl, out, pts, euler);
+    else yz_c2r_m<7>(pdl, out, pts, euler);
   }
   // rigidity force -> its spectra in bufA (x real, ky compact)
   template <int LM>
@@ -583,19 +619,24 @@ struct Box : BoxBase {
   }
   template <int LM>
   void zw_products(bool pdl) {
-    launch_k(pdl, sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW> : k_zw_products<R, LM, ZNW>, dim3(zp_p.grid),
-             dim3(zp_p.nw * 32), zp_p.sm, stream, g, tw, bufB);
+    launch_k(pdl, sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW> : k_zw_products<R, LM, ZNW>,
+             dim3(zp_p.grid(zgroups<LM>())), dim3(zp_p.nw * 32), zp_p.sm, stream, g, tw, bufB, (R *)nullptr);
   }
   template <int LM>
-  void zw_c2r(bool pdl, DPart *pts, int euler) {
+  int zgroups() const {
+    return g.NX * g.NY / ZL<LM>::RW;
+  }
+  template <int LM>
+  void zw_c2r(bool pdl, int nc, R *out, DPart *pts, int euler) {
+    const int nblk = zp_c.grid(nc * zgroups<LM>());
     const int posblk = pts ? (Np + zp_c.nw * 32 - 1) / (zp_c.nw * 32) : 0;
-    launch_k(pdl, k_zw_c2r<R, LM, ZNW>, dim3(zp_c.grid + posblk), dim3(zp_c.nw * 32), zp_c.sm, stream, g, tw,
-             (const Cx<R> *)bufB, ustar, npts(), g.NZ, 3, zp_c.grid, pp, pts, euler, status);
+    launch_k(pdl, k_zw_c2r<R, LM, ZNW>, dim3(nblk + posblk), dim3(zp_c.nw * 32), zp_c.sm, stream, g, tw,
+             (const Cx<R> *)bufB, out, npts(), g.NZ, nc, nblk, pp, pts, euler, status);
   }
   template <int LM>
   void zw_force(bool pdl) {
-    launch_k(pdl, k_zw_r2c<R, LM, ZNW, true, false>, dim3(zp_f.grid), dim3(zp_f.nw * 32), zp_f.sm, stream, g, tw,
-             force(), npts(), bufB, 3);
+    launch_k(pdl, k_zw_r2c<R, LM, ZNW, true, false>, dim3(zp_f.grid(3 * zgroups<LM>())), dim3(zp_f.nw * 32), zp_f.sm,
+             stream, g, tw, force(), npts(), bufB, 3);
   }
   // dispatch on the compile-time line length
   void zdisp_products(bool pdl) {
@@ -604,14 +645,16 @@ struct Box : BoxBase {
     else if (zw == 7) zw_products<7>(pdl);
     else launch_k(pdl, k_z_products<R>, dim3(gz()), dim3(256), smem_zp, stream, g, tw, bufB);
   }
-  void zdisp_c2r(bool pdl, DPart *pts, int euler) {
-    if (zw == 5) zw_c2r<5>(pdl, pts, euler);
-    else if (zw == 6) zw_c2r<6>(pdl, pts, euler);
-    else if (zw == 7) zw_c2r<7>(pdl, pts, euler);
+  // z c2r of nc components in bufB into real fields, with the position update
+  // in extra blocks when pts is not null
+  void zdisp_c2r(bool pdl, int nc, R *out, DPart *pts, int euler) {
+    if (zw == 5) zw_c2r<5>(pdl, nc, out, pts, euler);
+    else if (zw == 6) zw_c2r<6>(pdl, nc, out, pts, euler);
+    else if (zw == 7) zw_c2r<7>(pdl, nc, out, pts, euler);
     else {
       const int posblk = pts ? (Np + 255) / 256 : 0;
-      launch_k(pdl, k_z_c2r<R>, dim3(gz() + posblk, 3), dim3(256), smem_zc, stream, g, tw, (const Cx<R> *)bufB,
-               ustar, npts(), g.NZ, pp, pts, euler, status);
+      launch_k(pdl, k_z_c2r<R>, dim3(gz() + posblk, nc), dim3(256), smem_zc, stream, g, tw, (const Cx<R> *)bufB, out,
+               npts(), g.NZ, pp, pts, euler, status);
     }
   }
   void zdisp_force(bool pdl) {
@@ -620,14 +663,36 @@ struct Box : BoxBase {
     else if (zw == 7) zw_force<7>(pdl);
     else launch_k(pdl, k_z_force<R>, dim3(gz()), dim3(256), smem_zf, stream, g, tw, force(), bufB);
   }
+  // inverse y and z of three spectra in bufA (x real) into real fields: one
+  // launch over planes where the plane kernels are on (pass variant y = 3),
+  // else two
+  bool planes() const { return ymode == 3 && zw && yz_ly; }
+  void inverse3(bool pdl, R *out, DPart *pts = nullptr, int euler = 0) {
+    if (planes()) {
+      yz_c2r(pdl, out, pts, euler);
+    } else {
+      launch_y<true>(g, 3, bufA, bufB, pdl);
+      zdisp_c2r(pdl, 3, out, pts, euler);
+    }
+  }
+  // forward z and y of the rigidity force into bufA (x real)
+  void forward_force(bool pdl) {
+    if (planes()) {
+      zy_force(pdl);
+    } else {
+      zdisp_force(pdl);
+      launch_y<false>(g, 3, bufB, bufA, pdl);
+    }
+  }
 
   int alloc() override {
     const size_t nz = (size_t)g.KXc * g.KYc * g.TS;
     const size_t nA = (size_t)g.NX * g.KYc * g.TS;
     const size_t nB = (size_t)g.NX * g.NY * g.TS;
     KCHECK(cudaMalloc(&zeta, sizeof(Cx<R>) * 2 * nz));
-    // the Lees-Edwards advection term carries u and the vorticity: 6 spectra
-    const int nbuf = prm.eq == KAPSEL_EQ_SHEAR_LE ? 6 : 5;
+    // 6 spectra: the Lees-Edwards advection term carries u and the vorticity,
+    // the Electrolyte one the fluxes of both species
+    const int nbuf = prm.eq == KAPSEL_EQ_NAVIER_STOKES ? 5 : 6;
     KCHECK(cudaMalloc(&bufA, sizeof(Cx<R>) * nbuf * nA));
     KCHECK(cudaMalloc(&bufB, sizeof(Cx<R>) * nbuf * nB));
     KCHECK(cudaMalloc(&ustar, sizeof(R) * 3 * npts()));
@@ -854,10 +919,9 @@ struct Box : BoxBase {
   }
 
   // f -> zeta update, launches 11-13
-  void launch_force_to_zeta() {
-    zdisp_force(false);
-    launch_y<false>(g, 3, bufB, bufA);
-    x_force(false, bufA);
+  void launch_force_to_zeta(bool pdl = false) {
+    forward_force(pdl);
+    x_force(pdl, bufA);
   }
 
   void launch_step(const double *noise, int euler, cudaEvent_t *ev = nullptr) override {
@@ -898,9 +962,9 @@ struct Box : BoxBase {
     // when profiling, so that each launch is timed separately)
     const bool fuse_pos = Np > 0 && !ev;
     if (yzf)
-      yz_c2r(pdl, fuse_pos ? parts : (DPart *)nullptr, euler);
+      yz_c2r(pdl, ustar, fuse_pos ? parts : (DPart *)nullptr, euler);
     else
-      zdisp_c2r(pdl, fuse_pos ? parts : (DPart *)nullptr, euler);
+      zdisp_c2r(pdl, 3, ustar, fuse_pos ? parts : (DPart *)nullptr, euler);
     mark();
     if (Np > 0) {
       if (!fuse_pos) k_particles_position<<<(Np + 127) / 128, 128, 0, stream>>>(pp, parts, euler, status);
@@ -908,11 +972,11 @@ struct Box : BoxBase {
       mark();
       if (nc) launch_nearcontact();  // timed with the position slot when profiling
       launch_k(pdl, k_particles_hydro_velocity<R>, dim3(Np * pp.hyd_pcl), dim3(pp.hyd_threads), 0, stream, pp, parts,
-               (const R *)ustar, (const int *)cells, noise, euler, status, partial_p, arrivals,
+               (const R *)ustar, (const short4 *)cells, noise, euler, status, partial_p, arrivals,
                nc ? nc_corr : (double *)nullptr, ovl);
       mark();
       launch_k(pdl, k_particles_scatter<R, true>, dim3(Np * PCL), dim3(256), 0, stream, pp, (const DPart *)parts,
-               (const int *)cells, force(), (const R *)ustar, status, (const unsigned *)ovl);
+               (const short4 *)cells, force(), (const R *)ustar, status, (const unsigned *)ovl);
       mark();
       if (yzf)
         zy_force(pdl);
@@ -957,7 +1021,81 @@ struct Box : BoxBase {
   R *obB = nullptr;        // [3][N]: contravariant u on the oblique grid
   double *obst = nullptr;  // degree_oblique, Shear_rate_eff, ... (obl_kernels.cuh)
   OblPar op{};
-  size_t sm_xo6 = 0, sm_xo3 = 0, sm_xof = 0;
+  size_t sm_xo6 = 0, sm_xoa = 0, sm_xof = 0;
+  template <int LX>
+  int obl_x_setup() {
+    KCHECK(allow_smem(k_x_obl_inv<R, KCX, LX>, sm_xo6));
+    KCHECK(allow_smem(k_x_obl_update<R, KCX, 1, LX>, sm_xoa));
+    KCHECK(allow_smem(k_x_obl_update<R, KCX, 0, LX>, sm_xof));
+    return 0;
+  }
+  // the x passes with compile-time NX: 0 the first inverse, 1 the advection
+  // update, 2 the end of the step
+  template <int LX>
+  void obl_x_l(bool pdl, int which) {
+    if (which == 0)
+      launch_k(pdl, k_x_obl_inv<R, KCX, LX>, gx(), dim3(256), sm_xo6, stream, g, tw, (const Cx<R> *)zeta,
+               (const double *)uk_dc, (const double *)obst, bufA);
+    else if (which == 1)
+      launch_k(pdl, k_x_obl_update<R, KCX, 1, LX>, gx(), dim3(256), sm_xoa, stream, g, tw, bufA, zeta, uk_dc,
+               (const double *)obst);
+    else
+      launch_k(pdl, k_x_obl_update<R, KCX, 0, LX>, gx(), dim3(256), sm_xof, stream, g, tw, bufA, zeta, uk_dc,
+               (const double *)obst);
+  }
+  void obl_x(bool pdl, int which) {
+    switch (g.NX) {
+      case 32: obl_x_l<5>(pdl, which); return;
+      case 64: obl_x_l<6>(pdl, which); return;
+      case 128: obl_x_l<7>(pdl, which); return;
+      case 256: obl_x_l<8>(pdl, which); return;
+      default: obl_x_l<0>(pdl, which);
+    }
+  }
+  template <int LM>
+  void zw_cross(bool pdl) {
+    launch_k(pdl, k_zw_cross<R, LM, ZNW>, dim3(zp_x.grid(zgroups<LM>())), dim3(zp_x.nw * 32), zp_x.sm, stream, g, tw,
+             bufB);
+  }
+  template <int LM>
+  void zw_obl_force(bool pdl) {
+    launch_k(pdl, k_zw_obl_force<R, LM, ZNW>, dim3(zp_of.grid(zgroups<LM>())), dim3(zp_of.nw * 32), zp_of.sm, stream,
+             g, tw, op, (const double *)obst, (const R *)phiup, (const R *)ustar, (const R *)ob6, bufB);
+  }
+  // bufB: inverse z of u and the vorticity, u x omega, forward z.  One launch
+  // where the warp-level z kernels exist for this NZ.
+  void obl_cross_z(bool pdl) {
+    const size_t N = npts();
+    if (zw_avail == 5) zw_cross<5>(pdl);
+    else if (zw_avail == 6) zw_cross<6>(pdl);
+    else if (zw_avail == 7) zw_cross<7>(pdl);
+    else {
+      launch_k(pdl, k_z_c2r<R>, dim3(gz(), 6), dim3(256), smem_zc, stream, g, tw, (const Cx<R> *)bufB, ob6, N, g.NZ,
+               PPar{}, (DPart *)nullptr, 0, (int *)nullptr);
+      launch_k(pdl, k_obl_cross<R>, dim3(592), dim3(256), 0, stream, N, (const R *)ob6, obB);
+      launch_k(pdl, k_z_r2c<R>, dim3(gz(), 3), dim3(256), smem_zc, stream, g, tw, (const R *)obB, g.NZ, N, bufB, g.TZ,
+               g.TS);
+    }
+  }
+  // f = up - phi u (Cartesian), u += U2u_oblique(f), forward z into bufB, and
+  // phi/up back to zero
+  void obl_force_z(bool pdl) {
+    const size_t N = npts();
+    if (zw_avail) {
+      if (zw_avail == 5) zw_obl_force<5>(pdl);
+      else if (zw_avail == 6) zw_obl_force<6>(pdl);
+      else zw_obl_force<7>(pdl);
+      if (Np > 0)
+        launch_k(pdl, k_obl_clear<R>, dim3(Np * PCL), dim3(256), 0, stream, pp, (const DPart *)parts,
+                 (const short4 *)cells, (const double *)obst, phiup);
+      return;
+    }
+    launch_k(pdl, k_obl_force<R>, dim3(592), dim3(256), 0, stream, N, phiup, (const R *)ustar, ob6 + 3 * N);
+    launch_k(pdl, k_obl_add_force<R>, dim3(592), dim3(256), 0, stream, op, (const double *)obst,
+             (const R *)(ob6 + 3 * N), (const R *)ob6, obB);
+    launch_k(pdl, k_z_r2c<R>, dim3(gz(), 3), dim3(256), smem_zc, stream, g, tw, (const R *)obB, g.NZ, N, bufB, g.TZ,
+             g.TS);
+  }
 
   int alloc_obl() override {
     const size_t N = npts(), nst = OB_SIZE;
@@ -969,13 +1107,18 @@ struct Box : BoxBase {
     KCHECK(cudaMemset(obst, 0, sizeof(double) * nst));
     const size_t C = sizeof(Cx<R>);
     sm_xo6 = C * (g.NX + (size_t)2 * g.KXc * KCX + (size_t)2 * g.NX * 6 * KCX);
-    sm_xo3 = C * (g.NX + (size_t)2 * g.KXc * KCX + (size_t)2 * g.NX * 3 * KCX);
+    sm_xoa = C * (g.NX + (size_t)2 * g.KXc * KCX + (size_t)2 * g.NX * 3 * KCX);
     sm_xof = C * (g.NX + (size_t)2 * g.NX * 3 * KCX);
     if (sm_xo6 > 227 * 1024 || smem_zc > 227 * 1024) return KAPSEL_ERANGE;
-    KCHECK(allow_smem(k_x_obl_inv<R, KCX, 6>, sm_xo6));
-    KCHECK(allow_smem(k_x_obl_inv<R, KCX, 3>, sm_xo3));
-    KCHECK(allow_smem(k_x_obl_fwd<R, KCX, 1>, sm_xof));
-    KCHECK(allow_smem(k_x_obl_fwd<R, KCX, 0>, sm_xof));
+    int rc = 0;
+    switch (g.NX) {
+      case 32: rc = obl_x_setup<5>(); break;
+      case 64: rc = obl_x_setup<6>(); break;
+      case 128: rc = obl_x_setup<7>(); break;
+      case 256: rc = obl_x_setup<8>(); break;
+      default: rc = obl_x_setup<0>();
+    }
+    if (rc) return rc;
     KCHECK(allow_smem(k_z_r2c<R>, smem_zc));
     op.shear_rate = prm.shear_rate;
     op.dt = prm.dt;
@@ -992,38 +1135,32 @@ struct Box : BoxBase {
 
   // Time_evolution_hydro_OBL (sp_3d_ns.cxx:214-390).
   void launch_step_obl(const double *noise, int euler) {
-    const size_t N = npts();
-    const int pb = 592;
+    const bool pdl = use_pdl;
     // NS_solver_slavedEuler_Shear_OBL: u and omega of the truncated zeta, u x omega,
-    // forward, shear correction, curl and the slaved-Euler step
-    k_x_obl_inv<R, KCX, 6><<<gx(), 256, sm_xo6, stream>>>(g, tw, zeta, uk_dc, obst, bufA);
-    launch_y<true>(g, 6, bufA, bufB);
-    k_z_c2r<R><<<dim3(gz(), 6), 256, smem_zc, stream>>>(g, tw, bufB, ob6, N, g.NZ, PPar{}, nullptr, 0, nullptr);
-    k_obl_cross<R><<<pb, 256, 0, stream>>>(N, ob6, obB);
-    k_z_r2c<R><<<dim3(gz(), 3), 256, smem_zc, stream>>>(g, tw, obB, g.NZ, N, bufB, g.TZ, g.TS);
-    launch_y<false>(g, 3, bufB, bufA);
-    k_x_obl_fwd<R, KCX, 1><<<gx(), 256, sm_xof, stream>>>(g, tw, bufA, zeta, uk_dc, obst);
-    // FIX_CELL on uk_dc, u = Zeta_k2u_k_OBL(zeta, uk_dc), A_k2a
-    k_x_obl_inv<R, KCX, 3><<<gx(), 256, sm_xo3, stream>>>(g, tw, zeta, uk_dc, obst, bufA);
-    launch_y<true>(g, 3, bufA, bufB);
-    k_z_c2r<R><<<dim3(gz(), 3), 256, smem_zc, stream>>>(g, tw, bufB, ob6, N, g.NZ, PPar{}, nullptr, 0, nullptr);
+    // forward, shear correction, curl and the slaved-Euler step; then FIX_CELL on
+    // uk_dc, u = Zeta_k2u_k_OBL(zeta, uk_dc), A_k2a
+    obl_x(false, 0);
+    launch_y<true>(g, 6, bufA, bufB, pdl);
+    obl_cross_z(pdl);
+    launch_y<false>(g, 3, bufB, bufA, pdl);
+    obl_x(pdl, 1);
+    inverse3(pdl, ob6);
     // deformation: degree_oblique, grid reset, Cartesian u (ustar), Shear_rate_eff,
     // positions
-    k_obl_to_cart<R><<<pb, 256, 0, stream>>>(op, (const double *)obst, (const R *)ob6, ustar);
-    k_obl_srate_position<R><<<1, 1024, 0, stream>>>(op, (const R *)ustar, obst, pp, parts, euler, status);
+    launch_k(pdl, k_obl_to_cart<R>, dim3(592), dim3(256), 0, stream, op, (const double *)obst, (const R *)ob6, ustar);
+    launch_k(pdl, k_obl_srate_position<R>, dim3(1), dim3(1024), 0, stream, op, (const R *)ustar, obst, pp, parts, euler,
+             status);
     if (Np > 0) {
-      k_obl_hydro_velocity<R><<<Np, 512, 0, stream>>>(pp, parts, (const R *)ustar, (const int *)cells, noise, euler,
-                                                       (const double *)obst, status);
-      k_obl_scatter<R><<<Np * PCL, 256, 0, stream>>>(pp, (const DPart *)parts, (const int *)cells,
-                                                      (const double *)obst, phiup);
+      launch_k(pdl, k_obl_hydro_velocity<R>, dim3(Np), dim3(512), 0, stream, pp, parts, (const R *)ustar,
+               (const short4 *)cells, noise, euler, (const double *)obst, status);
+      launch_k(pdl, k_obl_scatter<R>, dim3(Np * PCL), dim3(256), 0, stream, pp, (const DPart *)parts,
+               (const short4 *)cells, (const double *)obst, phiup);
     }
     // f = up - phi u (Cartesian), u += U2u_oblique(f), forward, Solenoidal_uk_OBL,
     // contra2co, U_k2zeta_k_OBL
-    k_obl_force<R><<<pb, 256, 0, stream>>>(N, phiup, (const R *)ustar, ob6 + 3 * N);
-    k_obl_add_force<R><<<pb, 256, 0, stream>>>(op, (const double *)obst, (const R *)(ob6 + 3 * N), (const R *)ob6, obB);
-    k_z_r2c<R><<<dim3(gz(), 3), 256, smem_zc, stream>>>(g, tw, obB, g.NZ, N, bufB, g.TZ, g.TS);
-    launch_y<false>(g, 3, bufB, bufA);
-    k_x_obl_fwd<R, KCX, 0><<<gx(), 256, sm_xof, stream>>>(g, tw, bufA, zeta, uk_dc, obst);
+    obl_force_z(pdl);
+    launch_y<false>(g, 3, bufB, bufA, pdl);
+    obl_x(pdl, 2);
   }
 
   int oblique_state(double *out) override {
@@ -1042,7 +1179,6 @@ struct Box : BoxBase {
 
   // ---- Electrolyte branch (two ion species) --------------------------------
   Cx<R> *conc_k = nullptr;  // [2][KXc][KYc][TS]
-  Cx<R> *rho_k = nullptr;   // [KXc][KYc][TS]
   R *phiq = nullptr;        // [5][N]: phi, surface charge, normal x/y/z
   R *creal = nullptr;       // [2][N]
   R *gradr = nullptr;       // [3][N]
@@ -1067,7 +1203,6 @@ struct Box : BoxBase {
     const size_t nz = (size_t)g.KXc * g.KYc * g.TS, N = npts();
     const size_t nfull = (size_t)g.NX * g.NY * gF.TS;
     KCHECK(cudaMalloc(&conc_k, sizeof(Cx<R>) * 2 * nz));
-    KCHECK(cudaMalloc(&rho_k, sizeof(Cx<R>) * nz));
     KCHECK(cudaMalloc(&phiq, sizeof(R) * 5 * N));
     KCHECK(cudaMalloc(&creal, sizeof(R) * 2 * N));
     KCHECK(cudaMalloc(&gradr, sizeof(R) * 3 * N));
@@ -1077,7 +1212,7 @@ struct Box : BoxBase {
     KCHECK(cudaMalloc(&F1, sizeof(Cx<R>) * 3 * nfull));
     KCHECK(cudaMalloc(&F2, sizeof(Cx<R>) * 3 * nfull));
     KCHECK(cudaMalloc(&scal, sizeof(double) * 8));
-    KCHECK(cudaMalloc(&partial, sizeof(double) * 2 * RED_BLOCKS));
+    KCHECK(cudaMalloc(&partial, sizeof(double) * std::max(2 * RED_BLOCKS, Np * PCL)));
     KCHECK(cudaMalloc(&total_solute, sizeof(double) * 2));
     KCHECK(cudaMemset(conc_k, 0, sizeof(Cx<R>) * 2 * nz));
     KCHECK(cudaMemset(scal, 0, sizeof(double) * 8));
@@ -1093,14 +1228,12 @@ struct Box : BoxBase {
     if (sm_el > 227 * 1024) return KAPSEL_ERANGE;
     const int sm = (int)sm_el;
     KCHECK(allow_smem(k_x_inv_op<R, KCX, XI_IDENT, 2, 2>, sm));
-    KCHECK(allow_smem(k_x_inv_op<R, KCX, XI_IDENT, 3, 3>, sm));
-    KCHECK(allow_smem(k_x_inv_op<R, KCX, XI_GRADPSI, 1, 3>, sm));
     KCHECK(allow_smem(k_x_inv_op<R, KCX, XI_GRADDIFF, 1, 3>, sm));
-    KCHECK(allow_smem(k_x_fwd_op<R, KCX, XF_STORE, 1>, sm));
     KCHECK(allow_smem(k_x_fwd_op<R, KCX, XF_CONCUPD, 3>, sm));
-    KCHECK(allow_smem(k_x_fwd_op<R, KCX, XF_GRADPSI_FULL, 1>, sm));
     KCHECK(allow_smem(k_x_fwd_op<R, KCX, XF_PSI_FULL, 1>, sm));
     KCHECK(allow_smem(k_x_inv_op<R, KCX, XI_IDENT, 1, 1>, sm));
+    KCHECK(allow_smem(k_x_poisson<R, KCX, 0>, sm));
+    KCHECK(allow_smem(k_x_poisson<R, KCX, 1>, sm));
     KCHECK(allow_smem(k_z_r2c<R>, sm));
     KCHECK(allow_smem(k_z_c2r<R>, sm));
     KCHECK(allow_smem(k_y_pass<R, true, KCY>, sm));
@@ -1117,31 +1250,89 @@ struct Box : BoxBase {
   bool ext_on() const { return prm.e_ext[0] != 0.0 || prm.e_ext[1] != 0.0 || prm.e_ext[2] != 0.0; }
 
   // real c_n = A_k2a_out(conc_k[n]) for both species
-  void el_conc_real() {
+  void el_conc_real(bool pdl = false) {
     const size_t nz = (size_t)g.KXc * g.KYc * g.TS;
-    k_x_inv_op<R, KCX, XI_IDENT, 2, 2><<<gx(), 256, sm_el, stream>>>(g, tw, conc_k, nz, bufA, KOp{});
-    launch_y<true>(g, 2, bufA, bufB);
-    k_z_c2r<R><<<dim3(gz(), 2), 256, sm_el, stream>>>(g, tw, bufB, creal, npts(), g.NZ, PPar{}, nullptr, 0, nullptr);
+    launch_k(pdl, k_x_inv_op<R, KCX, XI_IDENT, 2, 2>, gx(), dim3(256), sm_xinv(2, 2), stream, g, tw,
+             (const Cx<R> *)conc_k, nz, bufA, KOp{});
+    launch_y<true>(g, 2, bufA, bufB, pdl);
+    zdisp_c2r(pdl, 2, creal, nullptr, 0);
   }
-  // surface-charge scale s0 = sum|Z_e| / (sum|surf| DX3) (operate_electrolyte.cxx:217-241)
-  void el_surface_scale() {
-    k_reduce_partial<R, RED_ABS><<<RED_BLOCKS, 256, 0, stream>>>(npts(), phiq + npts(), nullptr, 0, 1, partial);
+  // dynamic shared memory of the x passes on the retained box
+  size_t sm_xinv(int nin, int nout) const {
+    return sizeof(Cx<R>) * (g.NX + (size_t)nin * g.KXc * KCX + (size_t)2 * g.NX * nout * KCX);
+  }
+  size_t sm_x3() const { return sizeof(Cx<R>) * (g.NX + (size_t)2 * g.NX * 3 * KCX); }
+  // surface-charge scale s0 = sum|Z_e| / (sum|surf| DX3) from the scatter's
+  // sums (operate_electrolyte.cxx:217-241)
+  void el_surface_scale(bool pdl = false) {
     const double dx3 = prm.dx * prm.dx * prm.dx;
-    k_reduce_final<<<1, 256, 0, stream>>>(partial, RED_BLOCKS, 1, 0, fabs(ze()) * Np, total_solute, dx3, scal);
+    launch_k(pdl, k_reduce_final, dim3(1), dim3(256), 0, stream, (const double *)partial, Np * PCL, 1, 0,
+             fabs(ze()) * Np, (const double *)total_solute, dx3, scal);
   }
   void el_scatter(int with_normal) {
     cudaMemsetAsync(phiq, 0, sizeof(R) * (with_normal ? 5 : 2) * npts(), stream);
-    if (Np > 0) k_particles_scatter_el<R><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, phiq, ze(), with_normal);
+    if (Np > 0)
+      k_particles_scatter_el<R><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, phiq, ze(), with_normal, partial);
   }
-  // forward transform of ncomp real fields, 2/3 modes kept, into bufA (I1 layout)
-  void el_forward_trunc(const R *real, int ncomp) {
-    k_z_r2c<R><<<dim3(gz(), ncomp), 256, sm_el, stream>>>(g, tw, real, g.NZ, npts(), bufB, g.TZ, g.TS);
-    launch_y<false>(g, ncomp, bufB, bufA);
+  // charge field of phiq, creal and scal, forward transformed (2/3 modes) in y
+  // and z: into component 0 of bufA.  Where the warp-level z kernels exist for
+  // this NZ the charge is formed inside the z pass.
+  template <int LM, bool FULL>
+  void zw_charge(bool pdl, int use_fac, R *keep, Cx<R> *out) {
+    const ZPlan &p = FULL ? zp_qf : zp_q;
+    launch_k(pdl, k_zw_charge<R, LM, ZNW, FULL>, dim3(p.grid(zgroups<LM>())), dim3(p.nw * 32), p.sm, stream, g, tw,
+             (const R *)phiq, (const R *)creal, (const double *)scal, use_fac, prm.valency_p, prm.valency_n, keep, out);
   }
-  // inverse of three I1-layout components in bufA into real fields
-  void el_inverse3(R *out) {
-    launch_y<true>(g, 3, bufA, bufB);
-    k_z_c2r<R><<<dim3(gz(), 3), 256, sm_el, stream>>>(g, tw, bufB, out, npts(), g.NZ, PPar{}, nullptr, 0, nullptr);
+  template <bool FULL>
+  void el_charge_z(bool pdl, int use_fac, R *keep, Cx<R> *out) {
+    if (zw_avail == 5) zw_charge<5, FULL>(pdl, use_fac, keep, out);
+    else if (zw_avail == 6) zw_charge<6, FULL>(pdl, use_fac, keep, out);
+    else if (zw_avail == 7) zw_charge<7, FULL>(pdl, use_fac, keep, out);
+    else {
+      const Geo &gg = FULL ? gF : g;
+      launch_k(pdl, k_el_charge<R>, dim3(592), dim3(256), 0, stream, npts(), (const R *)phiq, (const R *)creal,
+               (const double *)scal, use_fac, prm.valency_p, prm.valency_n, charge);
+      launch_k(pdl, k_z_r2c<R>, dim3(gz(), 1), dim3(256), sm_el, stream, gg, tw, (const R *)charge, g.NZ, npts(), out,
+               gg.TZ, gg.TS);
+    }
+  }
+  // inverse z, ion fluxes, forward z of both species in bufB
+  template <int LM>
+  void zw_flux(bool pdl, const FluxPar &fp) {
+    launch_k(pdl, k_zw_flux<R, LM, ZNW>, dim3(zp_fl.grid(2 * zgroups<LM>())), dim3(zp_fl.nw * 32), zp_fl.sm, stream, g,
+             tw, bufB, (const R *)creal, (const R *)gradr, (const R *)(phiq + 2 * npts()), (const R *)ureal, fp);
+  }
+  void el_flux_z(bool pdl, const FluxPar &fp) {
+    const size_t N = npts(), nB = (size_t)g.NX * g.NY * g.TS;
+    if (zw_avail == 5) zw_flux<5>(pdl, fp);
+    else if (zw_avail == 6) zw_flux<6>(pdl, fp);
+    else if (zw_avail == 7) zw_flux<7>(pdl, fp);
+    else
+      for (int n = 0; n < 2; ++n) {
+        Cx<R> *b = bufB + 3 * n * nB;
+        launch_k(pdl, k_z_c2r<R>, dim3(gz(), 3), dim3(256), sm_el, stream, g, tw, (const Cx<R> *)b, fluxr, N, g.NZ,
+                 PPar{}, (DPart *)nullptr, 0, (int *)nullptr);
+        launch_k(pdl, k_el_flux<R>, dim3(592), dim3(256), 0, stream, N, fluxr, (const R *)(creal + n * N),
+                 (const R *)gradr, (const R *)(phiq + 2 * N), (const R *)ureal, N, fp.L[n], fp.ve[n]);
+        launch_k(pdl, k_z_r2c<R>, dim3(gz(), 3), dim3(256), sm_el, stream, g, tw, (const R *)fluxr, g.NZ, N, b, g.TZ,
+                 g.TS);
+      }
+  }
+  // nonlinear-term centre in bufB, u real into ureal
+  template <int LM>
+  void zw_products_u(bool pdl) {
+    launch_k(pdl, sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW, true> : k_zw_products<R, LM, ZNW, true>,
+             dim3(zp_pu.grid(zgroups<LM>())), dim3(zp_pu.nw * 32), zp_pu.sm, stream, g, tw, bufB, ureal);
+  }
+  void el_products_z(bool pdl) {
+    if (zw_avail == 5) zw_products_u<5>(pdl);
+    else if (zw_avail == 6) zw_products_u<6>(pdl);
+    else if (zw_avail == 7) zw_products_u<7>(pdl);
+    else {
+      launch_k(pdl, k_z_c2r<R>, dim3(gz(), 3), dim3(256), sm_el, stream, g, tw, (const Cx<R> *)bufB, ureal, npts(),
+               g.NZ, PPar{}, (DPart *)nullptr, 0, (int *)nullptr);
+      launch_k(pdl, k_z_products<R>, dim3(gz()), dim3(256), smem_zp, stream, g, tw, bufB);
+    }
   }
 
   // NSsolute_solver_Euler (fluid_solver.cxx:306-326): Rhs_NS_Nernst_Planck
@@ -1149,37 +1340,35 @@ struct Box : BoxBase {
   // both ion concentrations (uk_dc is unchanged: its rhs is zero,
   // fluid_solver.cxx:176-178)
   void launch_el_fluid() {
-    const size_t N = npts(), nz = (size_t)g.KXc * g.KYc * g.TS;
-    const double ve[2] = {prm.valency_p, prm.valency_n}, L[2] = {prm.onsager_p, prm.onsager_n};
-    const double ieps = 1.0 / prm.dielectric;
-    const int pb = 592;
+    const size_t nz = (size_t)g.KXc * g.KYc * g.TS;
+    const bool pdl = use_pdl;
+    const double Nd = (double)npts();
     // Rhs_NS_Nernst_Planck: charge from the current conc and positions
     el_scatter(1);
-    el_surface_scale();
-    el_conc_real();
-    k_el_charge<R><<<pb, 256, 0, stream>>>(N, phiq, creal, scal, 0, ve[0], ve[1], charge);
-    el_forward_trunc(charge, 1);
-    k_x_fwd_op<R, KCX, XF_STORE, 1><<<gx(), 256, sm_el, stream>>>(g, tw, bufA, rho_k, 0, KOp{});
-    KOp gp{ieps, {prm.e_ext[0] * (double)N, prm.e_ext[1] * (double)N, prm.e_ext[2] * (double)N}};
-    k_x_inv_op<R, KCX, XI_GRADPSI, 1, 3><<<gx(), 256, sm_el, stream>>>(g, tw, rho_k, nz, bufA, gp);
-    el_inverse3(gradr);
+    el_surface_scale(pdl);
+    el_conc_real(pdl);
+    el_charge_z<false>(pdl, 0, nullptr, bufB);
+    launch_y<false>(g, 1, bufB, bufA, pdl);
+    const KOp gp{{1.0 / prm.dielectric, 0.0}, {prm.e_ext[0] * Nd, prm.e_ext[1] * Nd, prm.e_ext[2] * Nd}};
+    launch_k(pdl, k_x_poisson<R, KCX, 0>, gx(), dim3(256), sm_x3(), stream, g, tw, bufA, gp);
+    inverse3(pdl, gradr);
     // Rhs_NS_solute: u, the advection term and the explicit Euler update of zeta
-    x_zeta(false, zeta, uk_dc, bufA);
-    launch_y<true>(g, 3, bufA, bufB);
-    k_z_c2r<R><<<dim3(gz(), 3), 256, sm_el, stream>>>(g, tw, bufB, ureal, N, g.NZ, PPar{}, nullptr, 0, nullptr);
-    k_z_products<R><<<gz(), 256, smem_zp, stream>>>(g, tw, bufB);
-    launch_y<false>(g, 5, bufB, bufA);
-    x_advect<1>(false);
-    // ion fluxes and the Euler update of each concentration
-    for (int n = 0; n < 2; ++n) {
-      KOp dk{prm.kbt * L[n], {0, 0, 0}};
-      k_x_inv_op<R, KCX, XI_GRADDIFF, 1, 3><<<gx(), 256, sm_el, stream>>>(g, tw, conc_k + n * nz, nz, bufA, dk);
-      el_inverse3(fluxr);
-      k_el_flux<R><<<pb, 256, 0, stream>>>(N, fluxr, creal + n * N, gradr, phiq + 2 * N, ureal, N, L[n], ve[n]);
-      el_forward_trunc(fluxr, 3);
-      k_x_fwd_op<R, KCX, XF_CONCUPD, 3><<<gx(), 256, sm_el, stream>>>(g, tw, bufA, conc_k + n * nz, 0,
-                                                                         KOp{prm.dt, {0, 0, 0}});
-    }
+    x_zeta(pdl, zeta, uk_dc, bufA);
+    launch_y<true>(g, 3, bufA, bufB, pdl);
+    el_products_z(pdl);
+    launch_y<false>(g, 5, bufB, bufA, pdl);
+    x_advect<1>(pdl);
+    // ion fluxes and the Euler update of the concentrations, both species at once
+    const KOp dk{{prm.kbt * prm.onsager_p, prm.kbt * prm.onsager_n}, {0, 0, 0}};
+    dim3 gx2 = gx();
+    gx2.z = 2;
+    launch_k(pdl, k_x_inv_op<R, KCX, XI_GRADDIFF, 1, 3>, gx2, dim3(256), sm_xinv(1, 3), stream, g, tw,
+             (const Cx<R> *)conc_k, nz, bufA, dk);
+    launch_y<true>(g, 6, bufA, bufB, pdl);
+    el_flux_z(pdl, FluxPar{{prm.onsager_p, prm.onsager_n}, {prm.valency_p, prm.valency_n}});
+    launch_y<false>(g, 6, bufB, bufA, pdl);
+    launch_k(pdl, k_x_fwd_op<R, KCX, XF_CONCUPD, 3>, gx2, dim3(256), sm_x3(), stream, g, tw, (const Cx<R> *)bufA,
+             conc_k, nz, KOp{{prm.dt, 0.0}, {0, 0, 0}});
   }
   // Rescale_solute (solute_rhs.cxx:99-128) at the current positions: the
   // factors total[n] / (sum (1 - phi) c_n DX3) into scal[1..2], conc_k scaled.
@@ -1188,33 +1377,51 @@ struct Box : BoxBase {
   void launch_el_rescale() {
     const size_t N = npts(), nz = (size_t)g.KXc * g.KYc * g.TS;
     const double dx3 = prm.dx * prm.dx * prm.dx;
+    const bool pdl = use_pdl;
     el_scatter(0);
-    el_surface_scale();
-    el_conc_real();
-    k_reduce_partial<R, RED_PHI_C><<<RED_BLOCKS, 256, 0, stream>>>(N, phiq, creal, N, 2, partial);
-    k_reduce_final<<<1, 256, 0, stream>>>(partial, RED_BLOCKS, 2, 1, 0.0, total_solute, dx3, scal);
-    k_scale_conc<R><<<592, 256, 0, stream>>>(nz, conc_k, scal);
+    el_surface_scale(pdl);
+    el_conc_real(pdl);
+    launch_k(pdl, k_reduce_partial<R, RED_PHI_C>, dim3(RED_BLOCKS), dim3(256), 0, stream, N, (const R *)phiq,
+             (const R *)creal, N, 2, partial);
+    launch_k(pdl, k_reduce_final, dim3(1), dim3(256), 0, stream, (const double *)partial, RED_BLOCKS, 2, 1, 0.0,
+             (const double *)total_solute, dx3, scal);
+    launch_k(pdl, k_scale_conc<R>, dim3(592), dim3(256), 0, stream, nz, conc_k, (const double *)scal);
   }
-  // Make_Coulomb_force_x_on_fluid (operate_electrolyte.cxx:90-177) from the
-  // charge field: the full (untruncated) potential gradient with the Ooura
-  // inverse semantics, then f = charge (-grad psi + E_ext), times `scale`,
-  // into fluxr
-  void launch_el_coulomb(double scale) {
+  // The full (untruncated) potential gradient of Make_Coulomb_force_x_on_fluid
+  // (operate_electrolyte.cxx:90-177), y-transformed, into F2; the charge field
+  // itself into charge.  use_fac: concentrations times the rescale factors.
+  void el_full_gradient(bool pdl, int use_fac) {
+    el_charge_z<true>(pdl, use_fac, charge, F2);
+    launch_y<false>(gF, 1, F2, F1, pdl);
+    launch_k(pdl, k_x_poisson<R, KCX, 1>, gxF(), dim3(256), sm_x3(), stream, gF, tw, F1,
+             KOp{{1.0 / prm.dielectric, 0.0}, {0, 0, 0}});
+    launch_y<true>(gF, 3, F1, F2, pdl);
+  }
+  // f = charge (-grad psi + E_ext) times `scale`, forward z and y into bufA
+  template <int LM>
+  void zw_coulomb(bool pdl, const double *e, double scale) {
+    launch_k(pdl, k_zw_coulomb<R, LM, ZNW>, dim3(zp_cb.grid(zgroups<LM>())), dim3(zp_cb.nw * 32), zp_cb.sm, stream, g,
+             tw, (const Cx<R> *)F2, (const R *)charge, e[0], e[1], e[2], scale, bufB);
+  }
+  // the same force density into the real field fluxr
+  void el_coulomb_real(bool pdl, double scale) {
     const size_t N = npts();
-    const double ieps = 1.0 / prm.dielectric;
-    const int pb = 592;
-    const size_t nfull = (size_t)g.NX * g.NY * gF.TS;
-    k_z_r2c<R><<<dim3(gz(), 1), 256, sm_el, stream>>>(gF, tw, charge, g.NZ, N, F2, gF.TZ, gF.TS);
-    launch_y<false>(gF, 1, F2, F1);
-    k_x_fwd_op<R, KCX, XF_GRADPSI_FULL, 1><<<gxF(), 256, sm_el, stream>>>(gF, tw, F1, F2, nfull,
-                                                                             KOp{ieps, {0, 0, 0}});
-    k_hermitian_planes<R><<<pb, 256, 0, stream>>>(gF, F2, 3);
-    k_x_inv_op<R, KCX, XI_IDENT, 3, 3><<<gxF(), 256, sm_el, stream>>>(gF, tw, F2, nfull, F1, KOp{});
-    launch_y<true>(gF, 3, F1, F2);
-    k_z_c2r<R><<<dim3(gz(), 3), 256, sm_el, stream>>>(gF, tw, F2, gradr, N, g.NZ, PPar{}, nullptr, 0, nullptr);
+    launch_k(pdl, k_z_c2r<R>, dim3(gz(), 3), dim3(256), sm_el, stream, gF, tw, (const Cx<R> *)F2, gradr, N, g.NZ,
+             PPar{}, (DPart *)nullptr, 0, (int *)nullptr);
     const bool ext = ext_on();
-    k_el_coulomb<R><<<pb, 256, 0, stream>>>(N, charge, gradr, ext ? prm.e_ext[0] : 0.0, ext ? prm.e_ext[1] : 0.0,
-                                            ext ? prm.e_ext[2] : 0.0, scale, fluxr);
+    launch_k(pdl, k_el_coulomb<R>, dim3(592), dim3(256), 0, stream, N, (const R *)charge, (const R *)gradr,
+             ext ? prm.e_ext[0] : 0.0, ext ? prm.e_ext[1] : 0.0, ext ? prm.e_ext[2] : 0.0, scale, fluxr);
+  }
+  void el_coulomb_forward(bool pdl, double scale) {
+    if (zw_avail == 5) zw_coulomb<5>(pdl, prm.e_ext, scale);
+    else if (zw_avail == 6) zw_coulomb<6>(pdl, prm.e_ext, scale);
+    else if (zw_avail == 7) zw_coulomb<7>(pdl, prm.e_ext, scale);
+    else {
+      el_coulomb_real(pdl, scale);
+      launch_k(pdl, k_z_r2c<R>, dim3(gz(), 3), dim3(256), sm_el, stream, g, tw, (const R *)fluxr, g.NZ, npts(), bufB,
+               g.TZ, g.TS);
+    }
+    launch_y<false>(g, 3, bufB, bufA, pdl);
   }
 
   // the Coulomb potential of the charge field (Conc_k2charge_field, A2a_k,
@@ -1226,7 +1433,7 @@ struct Box : BoxBase {
     k_z_r2c<R><<<dim3(gz(), 1), 256, sm_el, stream>>>(gF, tw, charge, g.NZ, N, F2, gF.TZ, gF.TS);
     launch_y<false>(gF, 1, F2, F1);
     k_x_fwd_op<R, KCX, XF_PSI_FULL, 1><<<gxF(), 256, sm_el, stream>>>(gF, tw, F1, F2, nfull,
-                                                                         KOp{1.0 / prm.dielectric, {0, 0, 0}});
+                                                                         KOp{{1.0 / prm.dielectric, 0.0}, {0, 0, 0}});
     k_hermitian_planes<R><<<592, 256, 0, stream>>>(gF, F2, 1);
     k_x_inv_op<R, KCX, XI_IDENT, 1, 1><<<gxF(), 256, sm_el, stream>>>(gF, tw, F2, nfull, F1, KOp{});
     launch_y<true>(gF, 1, F1, F2);
@@ -1270,28 +1477,27 @@ struct Box : BoxBase {
   }
 
   void launch_step_el(int euler) {
-    const size_t N = npts();
-    const double ve[2] = {prm.valency_p, prm.valency_n};
+    const bool pdl = use_pdl;
     launch_el_fluid();
     if (Np > 0) k_particles_position<<<(Np + 127) / 128, 128, 0, stream>>>(pp, parts, euler, status);
     launch_cells();
     // Rescale_solute at the new positions, then the Coulomb force (the
     // charge from the concentrations before the scaling times the factors)
     launch_el_rescale();
-    k_el_charge<R><<<592, 256, 0, stream>>>(N, phiq, creal, scal, 1, ve[0], ve[1], charge);
-    launch_el_coulomb(prm.dt / prm.rho);
-    // u += f dt/rho; Solenoidal_u: in k-space zeta += zeta(sol f), uk_dc += f(0)
-    el_forward_trunc(fluxr, 3);
-    x_force(false, bufA);
-    // u (real) of the updated zeta, then the particle part of the step
-    x_zeta(false, zeta, uk_dc, bufA);
-    launch_y<true>(g, 3, bufA, bufB);
-    k_z_c2r<R><<<dim3(gz(), 3), 256, smem_zc, stream>>>(g, tw, bufB, ustar, N, g.NZ, PPar{}, nullptr, 0, nullptr);
+    el_full_gradient(pdl, 1);
+    el_coulomb_forward(pdl, prm.dt / prm.rho);
+    // u += f dt/rho; Solenoidal_u: in k-space zeta += zeta(sol f), uk_dc +=
+    // f(0), and on the same tiles u_k of the updated zeta
+    x_force_next(pdl);
+    // u (real), then the particle part of the step
+    inverse3(pdl, ustar);
     if (Np > 0) {
-      k_particles_hydro_velocity<R><<<Np * pp.hyd_pcl, pp.hyd_threads, 0, stream>>>(pp, parts, ustar, cells, nullptr, euler, status,
-                                                                  partial_p, arrivals);
-      k_particles_scatter<R, true><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, force(), ustar, status);
-      launch_force_to_zeta();
+      launch_k(pdl, k_particles_hydro_velocity<R>, dim3(Np * pp.hyd_pcl), dim3(pp.hyd_threads), 0, stream, pp, parts,
+               (const R *)ustar, (const short4 *)cells, (const double *)nullptr, euler, status, partial_p, arrivals,
+               (double *)nullptr, ovl);
+      launch_k(pdl, k_particles_scatter<R, true>, dim3(Np * PCL), dim3(256), 0, stream, pp, (const DPart *)parts,
+               (const short4 *)cells, force(), (const R *)ustar, status, (const unsigned *)ovl);
+      launch_force_to_zeta(pdl);
     }
   }
 
@@ -1549,8 +1755,8 @@ struct Box : BoxBase {
     el_scatter(0);
     el_surface_scale();
     el_conc_real();
-    k_el_charge<R><<<592, 256, 0, stream>>>(N, phiq, creal, scal, 0, prm.valency_p, prm.valency_n, charge);
-    launch_el_coulomb(1.0);
+    el_full_gradient(false, 0);
+    el_coulomb_real(false, 1.0);
     KCHECK(cudaGetLastError());
     std::vector<R> h(3 * N);
     KCHECK(cudaMemcpyAsync(h.data(), fluxr, sizeof(R) * h.size(), cudaMemcpyDeviceToHost, stream));
@@ -1573,7 +1779,6 @@ struct Box : BoxBase {
     cudaFree(obB);
     cudaFree(obst);
     cudaFree(conc_k);
-    cudaFree(rho_k);
     cudaFree(phiq);
     cudaFree(creal);
     cudaFree(gradr);
@@ -1861,7 +2066,7 @@ int Box<R>::phi_only_host(double *phi) {
 
 template <typename R>
 __global__ void k_gather_only(PPar p, const DPart *__restrict__ parts, const R *__restrict__ u,
-                              const int *__restrict__ cells, double *__restrict__ out) {
+                              const short4 *__restrict__ cells, double *__restrict__ out) {
   __shared__ double sh[2 * 6 * 32];
   const int n = blockIdx.x;
   const DPart &a = parts[n];
@@ -1873,7 +2078,7 @@ __global__ void k_gather_only(PPar p, const DPart *__restrict__ parts, const R *
   for (int m = threadIdx.x; m < p.S; m += blockDim.x) {
     int rm[3];
     double r[3], dist;
-    stencil_point(b, cells + 3 * m, xp, p, rm, r, dist);
+    stencil_point(b, load_cell(cells, m), xp, p, rm, r, dist);
     const double ph = (double)prof_phi<R>(dist, p);
     double vr[3] = {0.0, 0.0, 0.0};
     if (p.rotation) {
@@ -2087,14 +2292,15 @@ int kapsel_gpu_create(const kapsel_params *p, kapsel_ctx **out) {
 
   // particle constants: Set_global_parameters (input.cxx:274-431)
   PPar &pp = b->pp;
-  std::vector<int> cells = sekibun(p->a, p->a_xi, p->dx);
+  const std::vector<int> sek = sekibun(p->a, p->a_xi, p->dx);
   b->Np = p->n_particles;
-  b->S = (int)cells.size() / 3;
+  b->S = (int)sek.size() / 3;
   pp.Np = b->Np;
-  pp.S = b->S;
   pp.N[0] = g.NX;
   pp.N[1] = g.NY;
   pp.N[2] = g.NZ;
+  const std::vector<short4> cells = stencil_cells(sek, p->a, p->a_xi, pp.N);
+  pp.S = (int)cells.size();
   for (int d = 0; d < 3; ++d) {
     pp.L[d] = L[d];
     pp.invL[d] = 1.0 / L[d];
@@ -2171,8 +2377,8 @@ int kapsel_gpu_create(const kapsel_params *p, kapsel_ctx **out) {
   if (cudaMallocHost(&b->parts_host, sizeof(DPart) * np1) != cudaSuccess) return KAPSEL_ENOMEM;
   if (cudaMallocHost(&b->status_host, sizeof(int)) != cudaSuccess) return KAPSEL_ENOMEM;
   if (cudaMemset(b->parts, 0, sizeof(DPart) * np1) != cudaSuccess) return KAPSEL_ECUDA;
-  if (cudaMalloc(&b->cells, sizeof(int) * cells.size()) != cudaSuccess) return KAPSEL_ENOMEM;
-  if (cudaMemcpy(b->cells, cells.data(), sizeof(int) * cells.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+  if (cudaMalloc(&b->cells, sizeof(short4) * cells.size()) != cudaSuccess) return KAPSEL_ENOMEM;
+  if (cudaMemcpy(b->cells, cells.data(), sizeof(short4) * cells.size(), cudaMemcpyHostToDevice) != cudaSuccess)
     return KAPSEL_ECUDA;
   if (cudaMalloc(&b->uk_dc, sizeof(double) * 3) != cudaSuccess) return KAPSEL_ENOMEM;
   cudaMemset(b->uk_dc, 0, sizeof(double) * 3);

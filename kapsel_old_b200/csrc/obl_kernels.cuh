@@ -29,6 +29,7 @@
 
 #include "particle_kernels.cuh"
 #include "spectral_kernels.cuh"
+#include "zwarp_kernels.cuh"
 
 namespace kapsel {
 
@@ -89,53 +90,46 @@ __device__ __forceinline__ void obl_zeta_to_u(int KXi, int kz, R kx, R ky, R kzr
 }
 
 // ---------------------------------------------------------------------------
-// x pass, inverse, from the compact zeta:
-//   NOUT = 6: contravariant u (Zeta_k2u_k_OBL, k = 0 from uk_dc) and the
-//             contravariant vorticity (Zeta_k2omega_k_OBL), for the advection
-//             term (Zeta_k2u_cpuky / Zeta_k2omega_OBL, operate_omega.h:144-172);
-//   NOUT = 3: u after the FIX_CELL reset of uk_dc (sp_3d_ns.cxx:240-253).
-// IK2 and the metric use degree_oblique at the start of the step.
-// out I1: [NOUT][NX][KYc][TS].  grid (KYc, ceil(TZ/KC)).
-template <typename R, int KC, int NOUT>
+// x pass, inverse, from the compact zeta: contravariant u (Zeta_k2u_k_OBL,
+// k = 0 from uk_dc) and the contravariant vorticity (Zeta_k2omega_k_OBL), for
+// the advection term (Zeta_k2u_cpuky / Zeta_k2omega_OBL, operate_omega.h:
+// 144-172).  IK2 and the metric use degree_oblique at the start of the step.
+// out I1: [6][NX][KYc][TS].  grid (KYc, ceil(TZ/KC)).
+template <typename R, int KC, int LX = 0>
 __global__ void __launch_bounds__(256) k_x_obl_inv(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ zeta,
-                                                   double *__restrict__ uk_dc, const double *__restrict__ st,
+                                                   const double *__restrict__ uk_dc, const double *__restrict__ st,
                                                    Cx<R> *__restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int W = NOUT * KC;
+  pdl_begin();
+  const int NXv = LX > 0 ? (1 << LX) : g.NX, LXv = LX > 0 ? LX : g.lx;
+  constexpr int W = 6 * KC;
   Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
-  Cx<R> *Zt = twx + g.NX;           // [2][KXc][KC]
-  Cx<R> *U = Zt + 2 * g.KXc * KC;   // [NX][NOUT*KC]
-  Cx<R> *scr = U + g.NX * W;
-  __shared__ double ukd[3];
+  Cx<R> *Zt = twx + NXv;            // [2][KXc][KC]
+  Cx<R> *U = Zt + 2 * g.KXc * KC;   // [NX][6*KC]
+  Cx<R> *scr = U + NXv * W;
   const int iy = blockIdx.x;
   const int kz0 = blockIdx.y * KC;
   const int ncol = min(KC, g.TZ - kz0);
   const size_t zplane = (size_t)g.KXc * g.KYc * g.TS;
+  load_twiddles(twx, tw.x, NXv);
+  zeta = pdl_fresh(zeta);
+  uk_dc = pdl_fresh(uk_dc);
+  st = pdl_fresh(st);
   for (int it = threadIdx.x; it < 2 * g.KXc * KC; it += blockDim.x) {
     const int col = it % KC, rest = it / KC, ix = rest % g.KXc, c = rest / g.KXc;
     if (col < ncol) cp_async_cx(Zt + it, zeta + c * zplane + ((size_t)ix * g.KYc + iy) * g.TS + kz0 + col);
   }
-  load_twiddles(twx, tw.x, g.NX);
-  const bool has_k0 = (iy == 0 && blockIdx.y == 0);
-  if (threadIdx.x < 3) {
-    double v = has_k0 ? uk_dc[threadIdx.x] : 0.0;
-    if (NOUT == 3 && has_k0 && g.fix_cell[threadIdx.x]) {
-      v = 0.0;
-      uk_dc[threadIdx.x] = 0.0;
-    }
-    ukd[threadIdx.x] = v;
-  }
+  const double deg = st[OB_DEG];
   cp_async_wait_all();
   __syncthreads();
-  const double deg = st[OB_DEG];
   const int KYi = signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY);
   const R ky = R(g.wave[1] * KYi);
-  for (int it = threadIdx.x; it < g.NX * KC; it += blockDim.x) {
+  for (int it = threadIdx.x; it < NXv * KC; it += blockDim.x) {
     const int col = it % KC, i = it / KC;
-    Cx<R> o[NOUT];
+    Cx<R> o[6];
 #pragma unroll
-    for (int c = 0; c < NOUT; ++c) o[c] = {R(0), R(0)};
-    const int KXi = signed_k(i, g.NX);
+    for (int c = 0; c < 6; ++c) o[c] = {R(0), R(0)};
+    const int KXi = signed_k(i, NXv);
     if (col < ncol && abs(KXi) < g.TX) {
       const int ix = KXi >= 0 ? KXi : KXi + g.KXc;
       const int kz = kz0 + col;
@@ -143,71 +137,87 @@ __global__ void __launch_bounds__(256) k_x_obl_inv(Geo g, Twiddles<R> tw, const 
       const Cx<R> z0 = Zt[ix * KC + col], z1 = Zt[(g.KXc + ix) * KC + col];
       const double k2 = obl_k2(g, deg, KXi, KYi, kz);
       const R ik2 = k2 > 0.0 ? R(1.0 / k2) : R(0);
-      Cx<R> u[3];
-      obl_zeta_to_u(KXi, kz, kx, ky, kzr, ik2, R(deg), z0, z1, u);
+      obl_zeta_to_u(KXi, kz, kx, ky, kzr, ik2, R(deg), z0, z1, o);
       if (KXi == 0 && KYi == 0 && kz == 0) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) u[d] = {R(ukd[d]), R(0)};
+        for (int d = 0; d < 3; ++d) o[d] = {R(uk_dc[d]), R(0)};
       }
-#pragma unroll
-      for (int d = 0; d < 3; ++d) o[d] = u[d];
-      if (NOUT == 6) {
-        Cx<R> w[3];
-        obl_omega(KXi, kz, kx, ky, kzr, z0, z1, w);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) o[(3 + d) % NOUT] = w[d];
-      }
+      obl_omega(KXi, kz, kx, ky, kzr, z0, z1, o + 3);
     }
 #pragma unroll
-    for (int c = 0; c < NOUT; ++c) U[i * W + c * KC + col] = o[c];
+    for (int c = 0; c < 6; ++c) U[i * W + c * KC + col] = o[c];
   }
   __syncthreads();
-  fft2_smem<R, -1, W>(U, scr, g.lx, 1, W, twx);
-  for (int it = threadIdx.x; it < NOUT * g.NX * KC; it += blockDim.x) {
-    const int col = it % KC, rest = it / KC, x = rest & (g.NX - 1), c = rest >> g.lx;
-    if (col < ncol) out[(((size_t)c * g.NX + x) * g.KYc + iy) * g.TS + kz0 + col] = U[x * W + c * KC + col];
+  fft2_smem<R, -1, W, LX>(U, scr, LXv, 1, W, twx);
+  for (int it = threadIdx.x; it < 6 * NXv * KC; it += blockDim.x) {
+    const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LXv;
+    if (col < ncol) out[(((size_t)c * NXv + x) * g.KYc + iy) * g.TS + kz0 + col] = U[x * W + c * KC + col];
   }
 }
 
-// ---------------------------------------------------------------------------
-// x pass, forward, of three spectra in (I1 layout) with the update of zeta:
-//   ADV = 1: in = the advection term u x omega.  A -= 2 S_eff (1, deg, 0) u^y_k
+// x passes of three spectra on one tile of (ky, kz chunk), in place on buf
+// (I1 layout), with the update of zeta between them:
+//   ADV = 1: buf = the advection term u x omega.  A -= 2 S_eff (1, deg, 0) u^y_k
 //            (operate_omega.cxx:155-164; u^y_k of the zeta at the start of the
 //            step, recomputed here), curl (U_k2rotation_k, fft_wrapper.cxx:
 //            679-722), Omega_k2zeta_k_OBL (fft_wrapper.cxx:175-197) and the
 //            slaved-Euler step with the oblique K2 (fluid_solver.cxx:398-430);
-//   ADV = 0: in = the contravariant u of the end of the step: Solenoidal_uk_OBL
+//            then the FIX_CELL reset of uk_dc, u of the updated zeta
+//            (sp_3d_ns.cxx:240-253) and its inverse x transform.  (The second
+//            half was a launch of its own that read zeta back: 16 + 15 us at
+//            128^3 in FP32.)
+//   ADV = 0: buf = the contravariant u of the end of the step: Solenoidal_uk_OBL
 //            (operate_omega.cxx:222-263), contra2co (fft_wrapper.h:327-361),
 //            U_k2zeta_k_OBL with uk_dc = co2contra(u_co(0)) (fft_wrapper.cxx:
 //            341-406), all with the updated degree_oblique.
 // grid (KYc, ceil(TZ/KC)).
-template <typename R, int KC, int ADV>
-__global__ void __launch_bounds__(256) k_x_obl_fwd(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ in,
-                                                   Cx<R> *__restrict__ zeta, double *__restrict__ uk_dc,
-                                                   const double *__restrict__ st) {
+template <typename R, int KC, int ADV, int LX = 0>
+__global__ void __launch_bounds__(256) k_x_obl_update(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ buf,
+                                                      Cx<R> *__restrict__ zeta, double *__restrict__ uk_dc,
+                                                      const double *__restrict__ st) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_begin();
+  const int NXv = LX > 0 ? (1 << LX) : g.NX, LXv = LX > 0 ? LX : g.lx;
   constexpr int W = 3 * KC;
   Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
-  Cx<R> *Pb = twx + g.NX;  // [NX][3*KC]
-  Cx<R> *scr = Pb + g.NX * W;
+  Cx<R> *Pb = twx + NXv;             // [NX][3*KC]
+  Cx<R> *scr = Pb + NXv * W;
+  Cx<R> *Zs = scr + NXv * W;         // [2][KXc][KC] (ADV only)
+  __shared__ double uks[2][3];       // uk_dc at the start, and after FIX_CELL
   const int iy = blockIdx.x;
   const int kz0 = blockIdx.y * KC;
   const int ncol = min(KC, g.TZ - kz0);
-  const size_t cstr = (size_t)g.NX * g.KYc * g.TS;
+  const size_t cstr = (size_t)NXv * g.KYc * g.TS;
   const size_t zplane = (size_t)g.KXc * g.KYc * g.TS;
-  for (int it = threadIdx.x; it < 3 * g.NX * KC; it += blockDim.x) {
-    const int col = it % KC, rest = it / KC, x = rest & (g.NX - 1), c = rest >> g.lx;
+  load_twiddles(twx, tw.x, NXv);
+  buf = pdl_fresh(buf);
+  zeta = pdl_fresh(zeta);
+  uk_dc = pdl_fresh(uk_dc);
+  st = pdl_fresh(st);
+  for (int it = threadIdx.x; it < 3 * NXv * KC; it += blockDim.x) {
+    const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LXv;
     Cx<R> *d = Pb + x * W + c * KC + col;
     if (col < ncol)
-      cp_async_cx(d, in + c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col);
+      cp_async_cx(d, buf + c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col);
     else
       *d = {R(0), R(0)};
   }
-  load_twiddles(twx, tw.x, g.NX);
+  if (ADV) {
+    for (int it = threadIdx.x; it < 2 * g.KXc * KC; it += blockDim.x) {
+      const int col = it % KC, rest = it / KC, ix = rest % g.KXc, c = rest / g.KXc;
+      if (col < ncol) cp_async_cx(Zs + it, zeta + c * zplane + ((size_t)ix * g.KYc + iy) * g.TS + kz0 + col);
+    }
+    if (iy == 0 && blockIdx.y == 0 && threadIdx.x < 3) {
+      const double v = uk_dc[threadIdx.x];
+      uks[0][threadIdx.x] = v;
+      uks[1][threadIdx.x] = g.fix_cell[threadIdx.x] ? 0.0 : v;
+      uk_dc[threadIdx.x] = uks[1][threadIdx.x];
+    }
+  }
+  const double deg = st[OB_DEG], s_eff = ADV ? st[OB_SRATE] : 0.0;
   cp_async_wait_all();
   __syncthreads();
-  fft2_smem<R, 1, W>(Pb, scr, g.lx, 1, W, twx);
-  const double deg = st[OB_DEG];
+  fft2_smem<R, 1, W, LX>(Pb, scr, LXv, 1, W, twx);
   const R degr = R(deg);
   const int KYi = signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY);
   const R ky = R(g.wave[1] * KYi);
@@ -215,7 +225,7 @@ __global__ void __launch_bounds__(256) k_x_obl_fwd(Geo g, Twiddles<R> tw, const 
     const int col = it % KC, ix = it / KC;
     if (col >= ncol) continue;
     const int KXi = ix < g.TX ? ix : ix - g.KXc;
-    const int i = KXi >= 0 ? KXi : KXi + g.NX;
+    const int i = KXi >= 0 ? KXi : KXi + NXv;
     const int kz = kz0 + col;
     const size_t o = ((size_t)ix * g.KYc + iy) * g.TS + kz;
     const Cx<R> *p = Pb + i * W + col;
@@ -224,11 +234,11 @@ __global__ void __launch_bounds__(256) k_x_obl_fwd(Geo g, Twiddles<R> tw, const 
     const R ik2 = k2 > 0.0 ? R(1.0 / k2) : R(0);
     const bool k0 = (KXi == 0 && KYi == 0 && kz == 0);
     if (ADV) {
-      Cx<R> z0 = zeta[o], z1 = zeta[zplane + o];
+      Cx<R> z0 = Zs[ix * KC + col], z1 = Zs[(g.KXc + ix) * KC + col];
       Cx<R> uo[3];
       obl_zeta_to_u(KXi, kz, kx, ky, kzr, ik2, degr, z0, z1, uo);
-      const R uy_re = k0 ? R(uk_dc[1]) : uo[1].x, uy_im = k0 ? R(0) : uo[1].y;
-      const R s2 = R(2.0 * st[OB_SRATE]), s2d = R(2.0 * st[OB_SRATE] * deg);
+      const R uy_re = k0 ? R(uks[0][1]) : uo[1].x, uy_im = k0 ? R(0) : uo[1].y;
+      const R s2 = R(2.0 * s_eff), s2d = R(2.0 * s_eff * deg);
       const Cx<R> a0 = {p[0].x - s2 * uy_re, p[0].y - s2 * uy_im};
       const Cx<R> a1 = {p[KC].x - s2d * uy_re, p[KC].y - s2d * uy_im};
       const Cx<R> a2 = p[2 * KC];
@@ -254,6 +264,8 @@ __global__ void __launch_bounds__(256) k_x_obl_fwd(Geo g, Twiddles<R> tw, const 
       z1 = {z1.x + dmy * (z1.x - c1 * f1.x), z1.y + dmy * (z1.y - c1 * f1.y)};
       zeta[o] = z0;
       zeta[zplane + o] = z1;
+      Zs[ix * KC + col] = z0;
+      Zs[(g.KXc + ix) * KC + col] = z1;
     } else {
       Cx<R> u0 = p[0], u1 = p[KC], u2 = p[2 * KC];
       const R kxc = (R(1) + degr * degr) * kx - degr * ky;
@@ -289,6 +301,33 @@ __global__ void __launch_bounds__(256) k_x_obl_fwd(Geo g, Twiddles<R> tw, const 
       }
     }
   }
+  if (!ADV) return;
+  __syncthreads();
+  for (int it = threadIdx.x; it < NXv * KC; it += blockDim.x) {
+    const int col = it % KC, i = it / KC;
+    Cx<R> u[3] = {{R(0), R(0)}, {R(0), R(0)}, {R(0), R(0)}};
+    const int KXi = signed_k(i, NXv);
+    if (col < ncol && abs(KXi) < g.TX) {
+      const int ix = KXi >= 0 ? KXi : KXi + g.KXc;
+      const int kz = kz0 + col;
+      const R kx = R(g.wave[0] * KXi), kzr = R(g.wave[2] * kz);
+      const double k2 = obl_k2(g, deg, KXi, KYi, kz);
+      const R ik2 = k2 > 0.0 ? R(1.0 / k2) : R(0);
+      obl_zeta_to_u(KXi, kz, kx, ky, kzr, ik2, degr, Zs[ix * KC + col], Zs[(g.KXc + ix) * KC + col], u);
+      if (KXi == 0 && KYi == 0 && kz == 0) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) u[d] = {R(uks[1][d]), R(0)};
+      }
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) Pb[i * W + d * KC + col] = u[d];
+  }
+  __syncthreads();
+  fft2_smem<R, -1, W, LX>(Pb, scr, LXv, 1, W, twx);
+  for (int it = threadIdx.x; it < 3 * NXv * KC; it += blockDim.x) {
+    const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LXv;
+    if (col < ncol) buf[c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col] = Pb[x * W + c * KC + col];
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -297,6 +336,8 @@ __global__ void __launch_bounds__(256) k_x_obl_fwd(Geo g, Twiddles<R> tw, const 
 // u x omega (operate_omega.cxx:131-150): uw = [u0 u1 u2 w0 w1 w2] -> out[3].
 template <typename R>
 __global__ void k_obl_cross(size_t n, const R *__restrict__ uw, R *__restrict__ out) {
+  pdl_begin();
+  uw = pdl_fresh(uw);
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const R u1 = uw[i], u2 = uw[n + i], u3 = uw[2 * n + i];
     const R w1 = uw[3 * n + i], w2 = uw[4 * n + i], w3 = uw[5 * n + i];
@@ -354,6 +395,9 @@ __device__ __forceinline__ int obl_row_o2c(int j, int NY, double deg, double &al
 template <typename R>
 __global__ void __launch_bounds__(256) k_obl_to_cart(OblPar o, const double *__restrict__ st, const R *__restrict__ in,
                                                      R *__restrict__ out) {
+  pdl_begin();
+  st = pdl_fresh(st);
+  in = pdl_fresh(in);
   const size_t n = (size_t)o.NX * o.NY * o.NZ;
   bool remap;
   const double deg = obl_next_degree(o, st, remap), srate = o.shear_rate;
@@ -385,6 +429,9 @@ __global__ void __launch_bounds__(256) k_obl_to_cart(OblPar o, const double *__r
 // cleared for the next scatter.
 template <typename R>
 __global__ void k_obl_force(size_t n, R *__restrict__ phiup, const R *__restrict__ u, R *__restrict__ f) {
+  pdl_begin();
+  phiup = pdl_fresh(phiup);
+  u = pdl_fresh(u);
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     R ph = phiup[i];
     R up[3] = {phiup[n + i], phiup[2 * n + i], phiup[3 * n + i]};
@@ -405,6 +452,10 @@ template <typename R>
 __global__ void __launch_bounds__(256) k_obl_add_force(OblPar o, const double *__restrict__ st,
                                                        const R *__restrict__ f, const R *__restrict__ u,
                                                        R *__restrict__ out) {
+  pdl_begin();
+  st = pdl_fresh(st);
+  f = pdl_fresh(f);
+  u = pdl_fresh(u);
   const size_t n = (size_t)o.NX * o.NY * o.NZ;
   const double deg = st[OB_DEG];
   const bool remap = st[OB_REMAP] != 0.0;
@@ -441,22 +492,22 @@ __global__ void __launch_bounds__(256) k_obl_add_force(OblPar o, const double *_
 // Relative_coord_check_stepover_Y (make_phi.h:198-236): mesh index and offset
 // of one Sekibun point; returns the y image crossing (-1, 0, 1), across which
 // x is shifted by degree_oblique NY cells.
-__device__ __forceinline__ int obl_stencil_point(const StencilBase &b, const int *cell, const PPar &p, double deg,
+__device__ __forceinline__ int obl_stencil_point(const StencilBase &b, const Cell &cell, const PPar &p, double deg,
                                                  int rm[3], double r[3]) {
-  const int jy = b.xi[1] + cell[1];
+  const int jy = b.xi[1] + cell.d[1];
   rm[1] = jy & (p.N[1] - 1);  // N is a power of two
   const int sign = (jy > rm[1]) - (jy < rm[1]);
-  const double xo = (double)b.xi[0] - (double)sign * deg * (double)p.N[1] + b.res[0] / p.DX + (double)cell[0] +
+  const double xo = (double)b.xi[0] - (double)sign * deg * (double)p.N[1] + b.res[0] / p.DX + (double)cell.d[0] +
                     (double)(4 * p.N[0]);
   // xo modulo N: exact in this form too for a power of two, in three
   // operations where fmod takes a long division
   const double xm = xo - (double)p.N[0] * floor(xo * (1.0 / (double)p.N[0]));
   rm[0] = min((int)xm, p.N[0] - 1);
   const double xres = xm - (double)rm[0];
-  rm[2] = (b.xi[2] + cell[2]) & (p.N[2] - 1);
-  r[0] = (double)cell[0] * p.DX - xres * p.DX;
-  r[1] = (double)cell[1] * p.DX - b.res[1];
-  r[2] = (double)cell[2] * p.DX - b.res[2];
+  rm[2] = (b.xi[2] + cell.d[2]) & (p.N[2] - 1);
+  r[0] = (double)cell.d[0] * p.DX - xres * p.DX;
+  r[1] = (double)cell.d[1] * p.DX - b.res[1];
+  r[2] = (double)cell.d[2] * p.DX - b.res[2];
   return sign;
 }
 
@@ -464,13 +515,13 @@ __device__ __forceinline__ int obl_stencil_point(const StencilBase &b, const int
 // sign; x is shifted by deg*Ly across a y boundary.
 __device__ __forceinline__ int pbc_obl(double *x, const PPar &p, double deg) {
   double signY = x[1];
-  x[1] = fmod(x[1] + p.L[1], p.L[1]);
+  x[1] = wrap_mod(x[1] + p.L[1], p.L[1]);
   signY -= x[1];
   int sign = (int)signY;
   if (!(sign == 0)) sign = sign / abs(sign);
   x[0] -= (double)sign * deg * p.L[1];
-  x[0] = fmod(x[0] + p.L[0], p.L[0]);
-  x[2] = fmod(x[2] + p.L[2], p.L[2]);
+  x[0] = wrap_mod(x[0] + p.L[0], p.L[0]);
+  x[2] = wrap_mod(x[2] + p.L[2], p.L[2]);
   return sign;
 }
 
@@ -499,7 +550,7 @@ __device__ __forceinline__ void obl_position_one(const PPar &p, DPart &a, int eu
 // differences of a column telescopes to its last value less its first, so
 // only two of NY rows of u0 are read; the column terms are summed
 // compensated, per thread, then over the block.  Measured at 128^3 with 256
-// particles, FP32: 10 us, where the sum over all differences, its final sum
+// particles, FP32: 12 us, where the sum over all differences, its final sum
 // and the positions took 28 + 31 + 6 us as three launches.
 template <typename R>
 __global__ void __launch_bounds__(1024) k_obl_srate_position(OblPar o, const R *__restrict__ u0, double *__restrict__ st,
@@ -507,6 +558,10 @@ __global__ void __launch_bounds__(1024) k_obl_srate_position(OblPar o, const R *
                                                              int *__restrict__ status) {
   __shared__ double sh[2 * 32];
   __shared__ double state[2];
+  pdl_begin();
+  u0 = pdl_fresh(u0);
+  st = pdl_fresh(st);
+  parts = pdl_fresh(parts);
   const int cols = o.NX * o.NZ;
   const size_t plane = (size_t)o.NY * o.NZ, last = (size_t)(o.NY - 1) * o.NZ;
   KSum s{0.0, 0.0};
@@ -524,14 +579,14 @@ __global__ void __launch_bounds__(1024) k_obl_srate_position(OblPar o, const R *
       }
     }
 #pragma unroll
-    for (int b = 0; b < B; ++b) s.add(((double)hi[b] - (double)lo[b]) / o.dx);
+    for (int b = 0; b < B; ++b) s.add((double)hi[b] - (double)lo[b]);
   }
   KSum v[1] = {s};
   block_reduce<1>(v, sh);
   if (threadIdx.x == 0) {
     bool remap;
     const double deg = obl_next_degree(o, st, remap);
-    const double srate = (v[0].s + v[0].c) * o.srate_scale;
+    const double srate = (v[0].s + v[0].c) / o.dx * o.srate_scale;
     st[OB_DEG] = state[0] = deg;
     st[OB_REMAP] = remap ? 1.0 : 0.0;
     st[OB_SRATE] = state[1] = srate;
@@ -569,13 +624,18 @@ __device__ __forceinline__ double distance_obl(const double *x1, const double *x
 // One block per particle.  The threads of the block share the partners of
 // the pair force as they share the stencil points (one thread walking all
 // of them, each step a dependent load, was 85% of the kernel: 171 us at
-// 128^3 with 256 particles, 20 us now); every sum is compensated.
+// 128^3 with 256 particles, 21 us now); every sum is compensated.
 template <typename R>
 __global__ void __launch_bounds__(512) k_obl_hydro_velocity(PPar p, DPart *__restrict__ parts,
-                                                            const R *__restrict__ u, const int *__restrict__ cells,
+                                                            const R *__restrict__ u, const short4 *__restrict__ cells,
                                                             const double *__restrict__ noise, int euler,
                                                             const double *__restrict__ st, int *__restrict__ status) {
   __shared__ double sh[2 * 9 * 32];
+  pdl_begin();
+  parts = pdl_fresh(parts);
+  u = pdl_fresh(u);
+  noise = pdl_fresh(noise);
+  st = pdl_fresh(st);
   const int n = blockIdx.x;
   DPart &a = parts[n];
   const double deg = st[OB_DEG], srate = st[OB_SRATE];
@@ -589,7 +649,7 @@ __global__ void __launch_bounds__(512) k_obl_hydro_velocity(PPar p, DPart *__res
   for (int m = threadIdx.x; m < p.S; m += blockDim.x) {
     int rm[3];
     double r[3];
-    const int sign = obl_stencil_point(b, cells + 3 * m, p, deg, rm, r);
+    const int sign = obl_stencil_point(b, load_cell(cells, m), p, deg, rm, r);
     const double dist = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
     const double ph = (double)prof_phi<R>(dist, p);
     if (ph == 0.0) continue;  // a zero term: skip its loads
@@ -674,8 +734,11 @@ __global__ void __launch_bounds__(512) k_obl_hydro_velocity(PPar p, DPart *__res
 // up += (v - sign S_eff Ly e_x + omega x r) phi_i.  PCL blocks per particle.
 template <typename R>
 __global__ void __launch_bounds__(256) k_obl_scatter(PPar p, const DPart *__restrict__ parts,
-                                                     const int *__restrict__ cells, const double *__restrict__ st,
+                                                     const short4 *__restrict__ cells, const double *__restrict__ st,
                                                      R *__restrict__ phiup) {
+  pdl_begin();
+  parts = pdl_fresh(parts);
+  st = pdl_fresh(st);
   const int n = blockIdx.x / PCL;
   const int stride = PCL * blockDim.x;
   const int first = (blockIdx.x % PCL) * blockDim.x + threadIdx.x;
@@ -689,9 +752,10 @@ __global__ void __launch_bounds__(256) k_obl_scatter(PPar p, const DPart *__rest
   for (int m = first; m < p.S; m += stride) {
     int rm[3];
     double r[3];
-    const int sign = obl_stencil_point(b, cells + 3 * m, p, deg, rm, r);
+    const int sign = obl_stencil_point(b, load_cell(cells, m), p, deg, rm, r);
     const double dist = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
     const double ph = (double)prof_phi<R>(dist, p);
+    if (ph == 0.0) continue;  // adds nothing
     double vr[3] = {0.0, 0.0, 0.0};
     if (p.rotation) {
       vr[0] = wp[1] * r[2] - wp[2] * r[1];
@@ -703,6 +767,182 @@ __global__ void __launch_bounds__(256) k_obl_scatter(PPar p, const DPart *__rest
     atomicAdd(phiup + npts + im, (R)(((vp[0] - (double)sign * srate * p.L[1]) + vr[0]) * ph));
     atomicAdd(phiup + 2 * npts + im, (R)((vp[1] + vr[1]) * ph));
     atomicAdd(phiup + 3 * npts + im, (R)((vp[2] + vr[2]) * ph));
+  }
+}
+
+// phi/up back to zero at every point the scatter of the same positions may
+// have written.
+template <typename R>
+__global__ void __launch_bounds__(256) k_obl_clear(PPar p, const DPart *__restrict__ parts,
+                                                   const short4 *__restrict__ cells, const double *__restrict__ st,
+                                                   R *__restrict__ phiup) {
+  pdl_begin();
+  parts = pdl_fresh(parts);
+  st = pdl_fresh(st);
+  const int n = blockIdx.x / PCL;
+  const double xp[3] = {parts[n].x[0], parts[n].x[1], parts[n].x[2]};
+  const StencilBase b = stencil_base(xp, p);
+  const double deg = st[OB_DEG];
+  const size_t npts = (size_t)p.N[0] * p.N[1] * p.N[2];
+  for (int m = (blockIdx.x % PCL) * blockDim.x + threadIdx.x; m < p.S; m += PCL * blockDim.x) {
+    int rm[3];
+    double r[3];
+    obl_stencil_point(b, load_cell(cells, m), p, deg, rm, r);
+    const size_t im = ((size_t)rm[0] * p.N[1] + rm[1]) * p.N[2] + rm[2];
+#pragma unroll
+    for (int d = 0; d < 4; ++d) phiup[d * npts + im] = R(0);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// z passes fused with the point operations between them (warp-level,
+// zwarp_kernels.cuh).
+
+// Inverse z of u and omega (components 0..2 and 3..5 of io), u x omega
+// (operate_omega.cxx:131-150), forward z into components 0..2.  None of the
+// nine real fields is stored (as three block-level launches over them this
+// took 60 + 14 + 30 us at 128^3 in FP32).
+template <typename R, int LM, int NW>
+__global__ void __launch_bounds__(NW * 32) k_zw_cross(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ io) {
+  using Z = ZL<LM>;
+  constexpr int GL = Z::RW * Z::LS, NI = Z::RW * Z::M / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_begin();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * 6 * GL;
+  Cx<R> wi[Z::N1], wk[Z::KW];
+  wfft_twiddles<R, LM, -1>(tw.m, wi);
+  wpre_twiddles<R, LM>(tw.z, wk);
+  io = pdl_fresh(io);
+  const size_t rows = (size_t)g.NX * g.NY, cstr = rows * Z::TS;
+  const int ngroups = (int)(rows / Z::RW);
+  const R sc = R(g.inv_n);
+  for (int grp = blockIdx.x * nw + warp; grp < ngroups; grp += gridDim.x * nw) {
+    Cx<R> *row = io + (size_t)grp * Z::RW * Z::TS;
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+      for (int rr = 0; rr < Z::RW; ++rr) wpack_c2r<R, LM>(row + c * cstr + rr * Z::TS, buf + c * GL + rr * Z::LS, wk);
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 6; ++c) wfft<R, LM, -1>(buf + c * GL, wi);
+#pragma unroll 2
+    for (int h = 0; h < NI; ++h) {
+      const int i = lane + 32 * h, at = (i >> LM) * Z::LS + zpos<LM>(i & (Z::M - 1));
+      Cx<R> v[6];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) v[c] = cscale(buf[c * GL + at], sc);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const int a = (d + 1) % 3, b = (d + 2) % 3;
+        buf[d * GL + at] = {v[a].x * v[3 + b].x - v[b].x * v[3 + a].x, v[a].y * v[3 + b].y - v[b].y * v[3 + a].y};
+      }
+    }
+    __syncwarp();
+    zw_forward3<R, LM>(buf, GL, tw, row, cstr);
+  }
+}
+
+// u + U2u_oblique(f) (k_obl_add_force) with the rigidity force formed at the
+// two source points of each term (k_obl_force's expressions, where phi is not
+// zero), forward z, kz < TZ kept -> out [3][rows][TS].  One pass over u and
+// phi where the force field and its sum with u were written and read back
+// (21 + 31 + 30 us at 128^3 in FP32).
+template <typename R, int LM, int NW>
+__global__ void __launch_bounds__(NW * 32) k_zw_obl_force(Geo g, Twiddles<R> tw, OblPar o,
+                                                          const double *__restrict__ st, const R *__restrict__ phiup,
+                                                          const R *__restrict__ ucart, const R *__restrict__ uobl,
+                                                          Cx<R> *__restrict__ out) {
+  using Z = ZL<LM>;
+  using V2 = typename Vec2<R>::T;
+  constexpr int GL = Z::RW * Z::LS, HR = Z::M / 32;  // element pairs per lane and row
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_begin();
+  st = pdl_fresh(st);
+  phiup = pdl_fresh(phiup);
+  ucart = pdl_fresh(ucart);
+  uobl = pdl_fresh(uobl);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * 3 * GL;
+  const double deg = st[OB_DEG];
+  const bool remap = st[OB_REMAP] != 0.0;
+  const size_t rows = (size_t)g.NX * g.NY, n = rows * Z::NZ, cstr = rows * Z::TS;
+  const int ngroups = (int)(rows / Z::RW);
+  // the force at the element pair at point s, with phi there
+  auto force = [&](size_t s, V2 ph, V2 (&f)[3]) {
+    R p0 = ph.x, p1 = ph.y, i0 = R(1), i1 = R(1);
+    if (p0 > R(1)) {
+      i0 = R(1) / p0;
+      p0 = R(1);
+    }
+    if (p1 > R(1)) {
+      i1 = R(1) / p1;
+      p1 = R(1);
+    }
+    V2 up[3], us[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      up[d] = *reinterpret_cast<const V2 *>(phiup + (1 + d) * n + s);
+      us[d] = *reinterpret_cast<const V2 *>(ucart + d * n + s);
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) f[d] = V2{up[d].x * i0 - p0 * us[d].x, up[d].y * i1 - p1 * us[d].y};
+  };
+  for (int grp = blockIdx.x * nw + warp; grp < ngroups; grp += gridDim.x * nw) {
+    const int row0 = grp * Z::RW, i = row0 / g.NY;
+#pragma unroll 1
+    for (int rr = 0; rr < Z::RW; ++rr) {
+      const int j = (row0 + rr) & (g.NY - 1);
+      double sign = (double)(j - o.NY / 2);
+      if (!(sign == 0)) sign = sign / fabs(sign);
+      const double jd = (double)(j - o.NY / 2);
+      const int io = (int)((double)(int)(sign * deg * jd) * sign);
+      const double alpha = (deg * jd - (double)io) * sign, beta = 1. - alpha;
+      const int iob = (i + io) & (o.NX - 1);
+      const int iobp = (iob + (int)sign) & (o.NX - 1);
+      const size_t s = ((size_t)iob * o.NY + j) * Z::NZ, sp = ((size_t)iobp * o.NY + j) * Z::NZ;
+      const size_t su = obl_source_row(o, remap, i, j) * Z::NZ;
+      V2 pa[HR], pb[HR], u[HR][3];
+#pragma unroll
+      for (int h = 0; h < HR; ++h) {
+        const int k = 2 * (lane + 32 * h);
+        pa[h] = *reinterpret_cast<const V2 *>(phiup + s + k);
+        pb[h] = *reinterpret_cast<const V2 *>(phiup + sp + k);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) u[h][d] = *reinterpret_cast<const V2 *>(uobl + d * n + su + k);
+      }
+#pragma unroll
+      for (int h = 0; h < HR; ++h) {
+        const int m = lane + 32 * h, k = 2 * m;
+        if (remap) {
+          u[h][0].x += u[h][1].x;
+          u[h][0].y += u[h][1].y;
+        }
+        const bool na = pa[h].x != R(0) || pa[h].y != R(0), nb = pb[h].x != R(0) || pb[h].y != R(0);
+        if (na || nb) {
+          const V2 zero = {R(0), R(0)};
+          V2 fa[3] = {zero, zero, zero}, fb[3] = {zero, zero, zero};
+          if (na) force(s + k, pa[h], fa);
+          if (nb) force(sp + k, pb[h], fb);
+          double gx[3], gy[3];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            gx[d] = beta * (double)fa[d].x + alpha * (double)fb[d].x;
+            gy[d] = beta * (double)fa[d].y + alpha * (double)fb[d].y;
+          }
+          gx[0] -= deg * gx[1];
+          gy[0] -= deg * gy[1];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            u[h][d].x = (R)((double)u[h][d].x + gx[d]);
+            u[h][d].y = (R)((double)u[h][d].y + gy[d]);
+          }
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) buf[d * GL + rr * Z::LS + zpos<LM>(m)] = {u[h][d].x, u[h][d].y};
+      }
+    }
+    __syncwarp();
+    zw_forward3<R, LM>(buf, GL, tw, out + (size_t)row0 * Z::TS, cstr);
   }
 }
 

@@ -82,6 +82,14 @@ struct StencilBase {
   int xi[3];
   double res[3];
 };
+// Offset of a stencil point, stored as four 16-bit integers (one 8-byte load).
+struct Cell {
+  int d[3];
+};
+__device__ __forceinline__ Cell load_cell(const short4 *__restrict__ cells, int m) {
+  const short4 c = __ldg(cells + m);
+  return {{c.x, c.y, c.z}};
+}
 __device__ __forceinline__ StencilBase stencil_base(const double *x, const PPar &p) {
   StencilBase b;
   const double idx = 1.0 / p.DX;
@@ -112,12 +120,12 @@ __device__ __forceinline__ double point_dist(const double *xp, const int rm[3], 
   }
   return __dsqrt_rn(s);
 }
-__device__ __forceinline__ void stencil_point(const StencilBase &b, const int *cell, const double *xp, const PPar &p,
+__device__ __forceinline__ void stencil_point(const StencilBase &b, const Cell &cell, const double *xp, const PPar &p,
                                               int rm[3], double r[3], double &dist) {
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    rm[d] = (b.xi[d] + cell[d] + p.N[d]) & (p.N[d] - 1);  // N is a power of two
-    r[d] = __dsub_rn(__dmul_rn((double)cell[d], p.DX), b.res[d]);
+    rm[d] = (b.xi[d] + cell.d[d] + p.N[d]) & (p.N[d] - 1);  // N is a power of two
+    r[d] = __dsub_rn(__dmul_rn((double)cell.d[d], p.DX), b.res[d]);
   }
   dist = point_dist(xp, rm, p);
 }
@@ -185,6 +193,15 @@ __device__ __forceinline__ void orientation_update(const PPar &p, DPart &a, int 
   qnormalize(a.q);
 }
 
+// fmod(v, L) of the periodic wraps.  The steps give v in [0, 2L), where the
+// difference is exact and is what fmod returns; fmod itself, a long division
+// in double, only for what is left (a NaN among it).
+__device__ __forceinline__ double wrap_mod(double v, double L) {
+  if (v >= 0.0 && v < L) return v;
+  if (v >= L && v < 2.0 * L) return v - L;
+  return fmod(v, L);
+}
+
 // MD_solver_position_Euler / _AB2 (particle_solver.cxx:36-88), PBC
 // (periodic_boundary.h:9-15), MD_solver_orientation_Euler / _AB2
 // (particle_rotation_solver.h:15-39).  One thread per particle.
@@ -197,7 +214,7 @@ __device__ __forceinline__ void position_update_one(const PPar &p, DPart *__rest
     const double dx = euler ? p.dt * a.v[d] : hdt * (3.0 * a.v[d] - a.v_old[d]);
     a.x_nopbc[d] += dx;
     a.x[d] += dx;
-    a.x[d] = fmod(a.x[d] + p.L[d], p.L[d]);
+    a.x[d] = wrap_mod(a.x[d] + p.L[d], p.L[d]);
     if (!(a.x[d] >= 0.0 && a.x[d] < p.L[d])) atomicExch(status, -6);
   }
   if (p.rotation) orientation_update(p, a, euler);
@@ -269,7 +286,7 @@ constexpr int HYD_PCL_MAX = 8;
 
 template <typename R>
 __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart *__restrict__ parts,
-                                                                  const R *__restrict__ u, const int *__restrict__ cells,
+                                                                  const R *__restrict__ u, const short4 *__restrict__ cells,
                                                                   const double *__restrict__ noise, int euler,
                                                                   int *__restrict__ status,
                                                                   double *__restrict__ partial,
@@ -318,13 +335,13 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
         ph[k] = 0.f;
         im[k] = 0;
         if (m < p.S) {
-          const int *cell = cells + 3 * m;
+          const Cell cell = load_cell(cells, m);
           int rm[3];
 #pragma unroll
-          for (int d = 0; d < 3; ++d) rm[d] = (b.xi[d] + cell[d] + p.N[d]) & (p.N[d] - 1);
+          for (int d = 0; d < 3; ++d) rm[d] = (b.xi[d] + cell.d[d] + p.N[d]) & (p.N[d] - 1);
           // phi is exactly zero beyond a + xi/2 (about half of the Sekibun
           // points): those terms add zeros, so their loads are skipped
-          ph[k] = prof_phi_f(offset_f(cell, resf, dxf, r[k]), rpf, rmf, dxf);
+          ph[k] = prof_phi_f(offset_f(cell.d, resf, dxf, r[k]), rpf, rmf, dxf);
           im[k] = ((size_t)rm[0] * p.N[1] + rm[1]) * p.N[2] + rm[2];
         }
       }
@@ -358,7 +375,7 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
   for (int m = first; m < p.S; m += stride) {
     int rm[3];
     double r[3], dist;
-    stencil_point(b, cells + 3 * m, xp, p, rm, r, dist);
+    stencil_point(b, load_cell(cells, m), xp, p, rm, r, dist);
     const double ph = (double)prof_phi<R>(dist, p);
     if (ph == 0.0) continue;  // a zero term: skip its loads
     const size_t im = ((size_t)rm[0] * p.N[1] + rm[1]) * p.N[2] + rm[2];
@@ -703,7 +720,7 @@ __device__ __forceinline__ void store_force(R *__restrict__ force, const R *__re
 // scatter gains three loads and loses one store per point.
 template <typename R, bool FORCE = false>
 __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *__restrict__ parts,
-                                                           const int *__restrict__ cells, R *__restrict__ out,
+                                                           const short4 *__restrict__ cells, R *__restrict__ out,
                                                            const R *__restrict__ ustar, int *__restrict__ status,
                                                            const unsigned *__restrict__ ovl = nullptr) {
   __shared__ NbShared nb[NB_MAX];
@@ -726,12 +743,12 @@ __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *
     const float dxf = (float)p.DX, rpf = (float)(p.RADIUS + p.HXI), rmf = (float)(p.RADIUS - p.HXI);
     const float resf[3] = {(float)b.res[0], (float)b.res[1], (float)b.res[2]};
     for (int m = first; m < p.S; m += stride) {
-      const int *cell = cells + 3 * m;
+      const Cell cell = load_cell(cells, m);
       int rm[3];
       float r[3];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) rm[d] = (b.xi[d] + cell[d] + p.N[d]) & (p.N[d] - 1);
-      const float ph = prof_phi_f(offset_f(cell, resf, dxf, r), rpf, rmf, dxf);
+      for (int d = 0; d < 3; ++d) rm[d] = (b.xi[d] + cell.d[d] + p.N[d]) & (p.N[d] - 1);
+      const float ph = prof_phi_f(offset_f(cell.d, resf, dxf, r), rpf, rmf, dxf);
       if (ph == 0.f) continue;
       bool own = true;
       for (int k = 0; k < nlow && own; ++k) {
@@ -784,7 +801,7 @@ __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *
   for (int m = first; m < p.S; m += stride) {
     int rm[3];
     double r[3], dist;
-    stencil_point(b, cells + 3 * m, xp, p, rm, r, dist);
+    stencil_point(b, load_cell(cells, m), xp, p, rm, r, dist);
     const double ph = (double)prof_phi<R>(dist, p);
     if (ph == 0.0) continue;
     bool own = true;

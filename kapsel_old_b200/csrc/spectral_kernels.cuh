@@ -107,12 +107,12 @@ __global__ void __launch_bounds__(256) k_x_zeta_to_u(Geo g, Twiddles<R> tw, cons
   const int kz0 = blockIdx.y * KC;
   const int ncol = min(KC, g.TZ - kz0);
   const size_t zplane = (size_t)g.KXc * g.KYc * g.TS;
+  load_twiddles(twx, tw.x, NXv);
   for (int it = threadIdx.x; it < 2 * g.KXc * KC; it += blockDim.x) {
     const int col = it % KC, rest = it / KC, ix = rest % g.KXc, c = rest / g.KXc;
     if (col < ncol)
       cp_async_cx(Zt + it, zeta + c * zplane + ((size_t)ix * g.KYc + iy) * g.TS + kz0 + col);
   }
-  load_twiddles(twx, tw.x, NXv);
   cp_async_wait_all();
   __syncthreads();
   const int KYi = signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY);
@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(256, 3) k_y_pass(Geo g, Twiddles<R> tw, const 
   constexpr int RSTEP = 256 / KC;
   const int col = threadIdx.x % KC, j0 = threadIdx.x / KC;
   const bool colok = col < ncol;
+  load_twiddles(twy, tw.y, g.NY);
   for (int j = j0; j < g.NY; j += RSTEP) {
     Cx<R> *d = Y + j * KC + col;
     int srow = j;
@@ -183,7 +184,6 @@ __global__ void __launch_bounds__(256, 3) k_y_pass(Geo g, Twiddles<R> tw, const 
     else
       *d = {R(0), R(0)};
   }
-  load_twiddles(twy, tw.y, g.NY);
   cp_async_wait_all();
   __syncthreads();
   fft2_smem<R, INVERSE ? -1 : 1, KC>(Y, scr, g.ly, 1, KC, twy);
@@ -247,12 +247,12 @@ __global__ void __launch_bounds__(256) k_z_products(Geo g, Twiddles<R> tw, Cx<R>
   const size_t rows = (size_t)g.NX * g.NY;
   const size_t row0 = (size_t)blockIdx.x * ZROWS;
   const size_t cstr = rows * g.TS;
+  load_twiddles(twm, tw.m, M);
+  load_twiddles(twz, tw.z, g.NZ);
   for (int it = threadIdx.x; it < NV * g.TZ; it += blockDim.x) {
     const int k = it % g.TZ, q = it / g.TZ, c = q % 3, rr = q / 3;
     cp_async_cx(A + q * TA + k, io + c * cstr + (row0 + rr) * g.TS + k);
   }
-  load_twiddles(twm, tw.m, M);
-  load_twiddles(twz, tw.z, g.NZ);
   cp_async_wait_all();
   __syncthreads();
   for (int it = threadIdx.x; it < NV * M; it += blockDim.x) {
@@ -321,12 +321,12 @@ __global__ void __launch_bounds__(256) k_z_c2r(Geo g, Twiddles<R> tw, const Cx<R
   const size_t rows = (size_t)g.NX * g.NY;
   const size_t row0 = (size_t)blockIdx.x * ZROWS;
   const Cx<R> *src = in + c * rows * g.TS + row0 * g.TS;
+  load_twiddles(twm, tw.m, M);
+  load_twiddles(twz, tw.z, g.NZ);
   for (int it = threadIdx.x; it < ZROWS * g.TZ; it += blockDim.x) {
     const int k = it % g.TZ, rr = it / g.TZ;
     cp_async_cx(A + rr * TA + k, src + rr * g.TS + k);
   }
-  load_twiddles(twm, tw.m, M);
-  load_twiddles(twz, tw.z, g.NZ);
   cp_async_wait_all();
   __syncthreads();
   for (int it = threadIdx.x; it < ZROWS * M; it += blockDim.x) {
@@ -361,10 +361,10 @@ __global__ void __launch_bounds__(256) k_z_force(Geo g, Twiddles<R> tw, R *__res
   Cx<R> *twz = twm + M;
   Cx<R> *S = twz + g.NZ;     // [M][ES], line = rr*3 + d
   Cx<R> *scr = S + M * ES;   // FFT scratch
-  load_twiddles(twm, tw.m, M);
-  load_twiddles(twz, tw.z, g.NZ);
   const size_t npts = (size_t)g.NX * g.NY * g.NZ;
   const size_t row0 = (size_t)blockIdx.x * ZROWS;
+  load_twiddles(twm, tw.m, M);
+  load_twiddles(twz, tw.z, g.NZ);
   for (int it = threadIdx.x; it < ZROWS * M; it += blockDim.x) {
     const int n = it & (M - 1), rr = it >> g.lm;
     Cx<R> *f = reinterpret_cast<Cx<R> *>(force + (row0 + rr) * g.NZ + 2 * n);  // an element pair
@@ -434,12 +434,12 @@ __global__ void __launch_bounds__(256) k_z_r2c(Geo g, Twiddles<R> tw, const R *_
   Cx<R> *twz = twm + M;
   Cx<R> *S = twz + g.NZ;    // [M][ES]
   Cx<R> *scr = S + M * ES;  // FFT scratch, then the output tile [ZROWS][nkeep+1]
-  load_twiddles(twm, tw.m, M);
-  load_twiddles(twz, tw.z, g.NZ);
   const int c = blockIdx.y;
   const size_t rows = (size_t)g.NX * g.NY;
   const size_t row0 = (size_t)blockIdx.x * ZROWS;
   const R *src = in + c * in_cstride;
+  load_twiddles(twm, tw.m, M);
+  load_twiddles(twz, tw.z, g.NZ);
   for (int it = threadIdx.x; it < ZROWS * M; it += blockDim.x) {
     const int n = it & (M - 1), rr = it >> g.lm;
     const R *r = src + (row0 + rr) * (size_t)in_pitch + 2 * n;
@@ -559,7 +559,8 @@ __global__ void __launch_bounds__(256) k_x_advect_update(Geo g, Twiddles<R> tw, 
   const int ncol = min(KC, g.TZ - kz0);
   const size_t cstr = (size_t)NXv * g.KYc * g.TS;
   const size_t zplane = (size_t)g.KXc * g.KYc * g.TS;
-  // stage the five product spectra (bit-reversed rows) and the zeta tile
+  load_twiddles(twx, tw.x, NXv);
+  // stage the five product spectra and the zeta tile
   if constexpr (sizeof(R) == 4 && KC % 2 == 0) {
     constexpr int KP = KC / 2;
     for (int it = threadIdx.x; it < 5 * NXv * KP; it += blockDim.x) {
@@ -585,7 +586,6 @@ __global__ void __launch_bounds__(256) k_x_advect_update(Geo g, Twiddles<R> tw, 
       if (col < ncol) cp_async_cx(Zs + it, zeta + c * zplane + ((size_t)ix * g.KYc + iy) * g.TS + kz0 + col);
     }
   }
-  load_twiddles(twx, tw.x, NXv);
   const bool has_k0 = (iy == 0 && blockIdx.y == 0);
   if (threadIdx.x < 3) {
     double v = 0.0;
@@ -686,6 +686,7 @@ __global__ void __launch_bounds__(256) k_x_force_to_zeta(Geo g, Twiddles<R> tw, 
   const int ncol = min(KC, g.TZ - kz0);
   const size_t cstr = (size_t)NXv * g.KYc * g.TS;
   const size_t zplane = (size_t)g.KXc * g.KYc * g.TS;
+  load_twiddles(twx, tw.x, NXv);
   if constexpr (sizeof(R) == 4 && KC % 2 == 0) {
     constexpr int KP = KC / 2;
     for (int it = threadIdx.x; it < 3 * NXv * KP; it += blockDim.x) {
@@ -711,7 +712,6 @@ __global__ void __launch_bounds__(256) k_x_force_to_zeta(Geo g, Twiddles<R> tw, 
       if (col < ncol) cp_async_cx(Zs + it, zeta + c * zplane + ((size_t)ix * g.KYc + iy) * g.TS + kz0 + col);
     }
   }
-  load_twiddles(twx, tw.x, NXv);
   cp_async_wait_all();
   __syncthreads();
   fft2_smem<R, 1, W3, LX, XS>(Pb, scr, LXv, 1, W3, twx);

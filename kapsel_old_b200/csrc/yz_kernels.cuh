@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(NW * 32) k_yzw_c2r(Geo g, Twiddles<R> tw, cons
 // Forward z, then forward y, of plane (c, x) = blockIdx.x of real fields
 // in[c][NX][NY][NZ] (planes in_cstride apart) -> out [c][NX][KYc][TS], as
 // k_zw_r2c followed by the forward k_yw_pass.  CLEAR as in k_zw_r2c.  At
-// 128^3 in FP32 the rigidity force takes 27 us this way; with phi, up and u*
+// 128^3 in FP32 the rigidity force takes 26 us this way; with phi, up and u*
 // read here (phi by all three component blocks of a plane) it took 35 us.
 template <typename R, int LY, int LM, bool CLEAR, int NW>
 __global__ void __launch_bounds__(NW * 32) k_zyw_r2c(Geo g, Twiddles<R> tw, R *__restrict__ in, size_t in_cstride,

@@ -110,10 +110,10 @@ __device__ __forceinline__ void wfft(Cx<R> *buf, const Cx<R> (&w)[ZL<LM>::N1]) {
   __syncwarp();
 }
 
-// c2r packing of one line of A[k], k < TZ (stride 1, shared or global) into the padded
+// c2r packing of one line of A[k], k < NK (stride 1, shared or global) into the padded
 // line Z: Z[k] = (A[k] + conj A[M-k]) + i (A[k] - conj A[M-k]) w_NZ^{-k}.
 // wk[j] = w_NZ^{-k} for this lane's k = lane + 32 j.
-template <typename R, int LM>
+template <typename R, int LM, int NK = ZL<LM>::TZ>
 __device__ __forceinline__ void wpack_c2r(const Cx<R> *A, Cx<R> *Zl, const Cx<R> (&wk)[ZL<LM>::KW]) {
   using Z = ZL<LM>;
   const int lane = threadIdx.x & 31;
@@ -121,8 +121,8 @@ __device__ __forceinline__ void wpack_c2r(const Cx<R> *A, Cx<R> *Zl, const Cx<R>
   for (int j = 0; j < Z::KW; ++j) {
     const int k = lane + 32 * j;
     const Cx<R> zero = {R(0), R(0)};
-    const Cx<R> a = k < Z::TZ ? A[k] : zero;
-    const Cx<R> b = (Z::M - k) < Z::TZ ? cconj(A[Z::M - k]) : zero;
+    const Cx<R> a = k < NK ? A[k] : zero;
+    const Cx<R> b = (Z::M - k) < NK ? cconj(A[Z::M - k]) : zero;
     Zl[zpos<LM>(k)] = cadd(cadd(a, b), cmul_pi(cmul(csub(a, b), wk[j])));
   }
 }
@@ -156,6 +156,14 @@ struct Vec2<double> {
   using T = double2;
 };
 
+template <typename R>
+__device__ __forceinline__ void store_u(R *o, size_t npts, R u1a, R u1b, R u2a, R u2b, R u3a, R u3b) {
+  using V2 = typename Vec2<R>::T;
+  *reinterpret_cast<V2 *>(o) = V2{u1a, u1b};
+  *reinterpret_cast<V2 *>(o + npts) = V2{u2a, u2b};
+  *reinterpret_cast<V2 *>(o + 2 * npts) = V2{u3a, u3b};
+}
+
 // ---------------------------------------------------------------------------
 // Nonlinear-term centre (as k_z_products): per row group, inverse z of the
 // three velocity components, the five products, forward z (kz < TZ kept).
@@ -166,13 +174,16 @@ struct Vec2<double> {
 // then in flight together instead of behind a staging copy, which cut the
 // long-scoreboard stalls per issue from 4.1 to 0.9 at the same 16 resident
 // warps per SM.
-template <typename R, int LM, int NW>
-__global__ void __launch_bounds__(NW * 32) k_zw_products(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ io) {
+// STORE: the velocity itself is also written, ureal[3][rows][NZ] (the
+// Electrolyte ion fluxes read it).
+template <typename R, int LM, int NW, bool STORE = false>
+__global__ void __launch_bounds__(NW * 32) k_zw_products(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ io,
+                                                         R *__restrict__ ureal) {
   using Z = ZL<LM>;
   constexpr int GL = Z::RW * Z::LS, KP = Z::RW * Z::M / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * 4 * GL;
   Cx<R> wi[Z::N1], wf[Z::N1], wk[Z::KW];
   wfft_twiddles<R, LM, -1>(tw.m, wi);
@@ -182,7 +193,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products(Geo g, Twiddles<R> tw, 
   const size_t cstr = rows * Z::TS;
   const int ngroups = (int)(rows / Z::RW);
   const R sc = R(g.inv_n);
-  for (int grp = blockIdx.x * nw + warp; grp < ngroups; grp += gridDim.x * nw) {
+  for (int grp = blockIdx.x * NW + warp; grp < ngroups; grp += gridDim.x * NW) {
     const size_t row0 = (size_t)grp * Z::RW;
 #pragma unroll
     for (int c = 0; c < 3; ++c)
@@ -198,6 +209,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products(Geo g, Twiddles<R> tw, 
       const int rr = i >> LM, n = rr * Z::LS + zpos<LM>(i & (Z::M - 1));
       const Cx<R> U1 = buf[n], U2 = buf[GL + n], U3 = buf[2 * GL + n];
       const R u1a = U1.x * sc, u1b = U1.y * sc, u2a = U2.x * sc, u2b = U2.y * sc, u3a = U3.x * sc, u3b = U3.y * sc;
+      if (STORE) store_u<R>(ureal + row0 * Z::NZ + 2 * i, rows * Z::NZ, u1a, u1b, u2a, u2b, u3a, u3b);
       buf[n] = {u2a * u3a, u2b * u3b};
       buf[GL + n] = {u3a * u1a, u3b * u1b};
       buf[2 * GL + n] = {u1a * u2a, u1b * u2b};
@@ -250,13 +262,14 @@ struct ZProd {
   static constexpr int KP = Z::RW * Z::M / 32;  // product elements per lane
 };
 
-template <typename R, int LM, int NW>
-__global__ void __launch_bounds__(NW * 32) k_zw_products_pf(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ io) {
+template <typename R, int LM, int NW, bool STORE = false>
+__global__ void __launch_bounds__(NW * 32) k_zw_products_pf(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ io,
+                                                            R *__restrict__ ureal) {
   using Z = ZL<LM>;
   using P = ZProd<R, LM>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * P::WARP;
   Cx<R> *stage = buf + 4 * P::GL;  // [3][RW][TS]
   Cx<R> wi[Z::N1], wf[Z::N1], wk[Z::KW];
@@ -266,9 +279,9 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products_pf(Geo g, Twiddles<R> t
   const size_t rows = (size_t)g.NX * g.NY;
   const size_t cstr = rows * Z::TS;
   const int ngroups = (int)(rows / Z::RW);
-  const int gstride = gridDim.x * nw;
+  const int gstride = gridDim.x * NW;
   const R sc = R(g.inv_n);
-  int grp = blockIdx.x * nw + warp;
+  int grp = blockIdx.x * NW + warp;
   auto issue = [&](int gq) {
     const size_t r0 = (size_t)gq * Z::RW;
 #pragma unroll
@@ -298,6 +311,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products_pf(Geo g, Twiddles<R> t
       const int rr = i >> LM, n = rr * Z::LS + zpos<LM>(i & (Z::M - 1));
       const Cx<R> U1 = buf[n], U2 = buf[P::GL + n], U3 = buf[2 * P::GL + n];
       const R u1a = U1.x * sc, u1b = U1.y * sc, u2a = U2.x * sc, u2b = U2.y * sc, u3a = U3.x * sc, u3b = U3.y * sc;
+      if (STORE) store_u<R>(ureal + row0 * Z::NZ + 2 * i, rows * Z::NZ, u1a, u1b, u2a, u2b, u3a, u3b);
       buf[n] = {u2a * u3a, u2b * u3b};
       buf[P::GL + n] = {u3a * u1a, u3b * u1b};
       buf[2 * P::GL + n] = {u1a * u2a, u1b * u2b};
@@ -352,7 +366,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
     if (parts && n < pp.Np) position_update_one(pp, parts, n, euler, status);
     return;
   }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // one line group per warp: the packing reads the rows straight from global
   // memory, and the small footprint keeps more warps resident
   Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * Z::RW * Z::LS;
@@ -362,7 +376,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
   const size_t rows = (size_t)g.NX * g.NY;
   const int ngroups = (int)(rows / Z::RW);
   const R sc = R(g.inv_n);
-  for (int task = blockIdx.x * nw + warp; task < ncomp * ngroups; task += nblk * nw) {
+  for (int task = blockIdx.x * NW + warp; task < ncomp * ngroups; task += nblk * NW) {
     const int c = task / ngroups;
     const size_t row0 = (size_t)(task - c * ngroups) * Z::RW;
     const Cx<R> *src = in + c * rows * Z::TS + row0 * Z::TS;
@@ -382,6 +396,26 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
   }
 }
 
+// Forward transform of three line groups held in buf (GL apart), kz < TZ kept,
+// row c, rr at dst + c * cstr + rr * TS.
+template <typename R, int LM>
+__device__ __forceinline__ void zw_forward3(Cx<R> *buf, int GL, const Twiddles<R> &tw, Cx<R> *__restrict__ dst,
+                                            size_t cstr) {
+  using Z = ZL<LM>;
+  const int lane = threadIdx.x & 31;
+  Cx<R> wf[Z::N1];
+  wfft_twiddles<R, LM, 1>(tw.m, wf);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) wfft<R, LM, 1>(buf + c * GL, wf);
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    for (int i = lane; i < Z::RW * Z::TZ; i += 32) {
+      const int rr = i / Z::TZ, k = i - rr * Z::TZ;
+      dst[c * cstr + rr * Z::TS + k] = wunpack_r2c<R, LM>(buf + c * GL + rr * Z::LS, k, tw.z);
+    }
+  __syncwarp();
+}
+
 // Forward z of real fields in[c][rows][NZ] (planes in_cstride apart), kz < TZ
 // kept, or all M + 1 (FULL), -> out [c][rows][TS].  Tasks (component, row
 // group), one line group per warp, as k_zw_c2r.  All element pairs of a row
@@ -397,13 +431,13 @@ __global__ void __launch_bounds__(NW * 32) k_zw_r2c(Geo g, Twiddles<R> tw, R *__
   constexpr int NI = Z::RW * Z::M / 32;  // element pairs per lane
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * Z::RW * Z::LS;
   Cx<R> wf[Z::N1];
   wfft_twiddles<R, LM, 1>(tw.m, wf);
   const size_t rows = (size_t)g.NX * g.NY;
   const int ngroups = (int)(rows / Z::RW);
-  for (int task = blockIdx.x * nw + warp; task < ncomp * ngroups; task += gridDim.x * nw) {
+  for (int task = blockIdx.x * NW + warp; task < ncomp * ngroups; task += gridDim.x * NW) {
     const int c = task / ngroups;
     const size_t row0 = (size_t)(task - c * ngroups) * Z::RW;
     R *src = in + c * in_cstride + row0 * Z::NZ;
