@@ -975,7 +975,7 @@ struct Box : BoxBase {
                (const R *)ustar, (const short4 *)cells, noise, euler, status, partial_p, arrivals,
                nc ? nc_corr : (double *)nullptr, ovl);
       mark();
-      launch_k(pdl, k_particles_scatter<R, true>, dim3(Np * PCL), dim3(256), 0, stream, pp, (const DPart *)parts,
+      launch_k(pdl, k_particles_scatter<R, true>, dim3(Np * pp.sc_pcl), dim3(256), 0, stream, pp, (const DPart *)parts,
                (const short4 *)cells, force(), (const R *)ustar, status, (const unsigned *)ovl);
       mark();
       if (yzf)
@@ -1010,7 +1010,7 @@ struct Box : BoxBase {
     cudaMemsetAsync(uk_dc, 0, sizeof(double) * 3, stream);
     if (Np > 0) {
       launch_cells();
-      k_particles_scatter<R, true><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, force(), ustar, status);
+      k_particles_scatter<R, true><<<Np * pp.sc_pcl, 256, 0, stream>>>(pp, parts, cells, force(), ustar, status);
       launch_force_to_zeta();
     }
     cudaMemsetAsync(uk_dc, 0, sizeof(double) * 3, stream);
@@ -1495,7 +1495,7 @@ struct Box : BoxBase {
       launch_k(pdl, k_particles_hydro_velocity<R>, dim3(Np * pp.hyd_pcl), dim3(pp.hyd_threads), 0, stream, pp, parts,
                (const R *)ustar, (const short4 *)cells, (const double *)nullptr, euler, status, partial_p, arrivals,
                (double *)nullptr, ovl);
-      launch_k(pdl, k_particles_scatter<R, true>, dim3(Np * PCL), dim3(256), 0, stream, pp, (const DPart *)parts,
+      launch_k(pdl, k_particles_scatter<R, true>, dim3(Np * pp.sc_pcl), dim3(256), 0, stream, pp, (const DPart *)parts,
                (const short4 *)cells, force(), (const R *)ustar, status, (const unsigned *)ovl);
       launch_force_to_zeta(pdl);
     }
@@ -2035,7 +2035,7 @@ int Box<R>::phi_up_host(double *phi, double *up0, double *up1, double *up2) {
   KCHECK(cudaMalloc(&d, sizeof(R) * 4 * npt));
   KCHECK(cudaMemsetAsync(d, 0, sizeof(R) * 4 * npt, stream));
   launch_cells();
-  if (Np > 0) k_particles_scatter<R><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, d, nullptr, status);
+  if (Np > 0) k_particles_scatter<R><<<Np * pp.sc_pcl, 256, 0, stream>>>(pp, parts, cells, d, nullptr, status);
   k_clamp_phi<R><<<592, 256, 0, stream>>>(npt, d);
   KCHECK(cudaGetLastError());
   std::vector<R> h(4 * npt);
@@ -2054,7 +2054,7 @@ int Box<R>::phi_only_host(double *phi) {
   KCHECK(cudaMalloc(&d, sizeof(R) * 4 * npt));
   KCHECK(cudaMemsetAsync(d, 0, sizeof(R) * 4 * npt, stream));
   launch_cells();
-  if (Np > 0) k_particles_scatter<R><<<Np * PCL, 256, 0, stream>>>(pp, parts, cells, d, nullptr, status);
+  if (Np > 0) k_particles_scatter<R><<<Np * pp.sc_pcl, 256, 0, stream>>>(pp, parts, cells, d, nullptr, status);
   KCHECK(cudaGetLastError());
   std::vector<R> h(npt);
   KCHECK(cudaMemcpyAsync(h.data(), d, sizeof(R) * npt, cudaMemcpyDeviceToHost, stream));
@@ -2353,10 +2353,20 @@ int kapsel_gpu_create(const kapsel_params *p, kapsel_ctx **out) {
   pp.noise_v = 1.439 * std::sqrt(zeta_drag * p->dt * p->kbt * p->alpha_v);
   pp.noise_o = 1.22 * std::sqrt(zeta_drag_rot * p->dt * p->kbt * p->alpha_o);
   pp.frozen = p->frozen ? 1 : 0;
-  // one gather block per particle: 512 threads when there are enough
-  // particles to fill the GPU, 1024 (two Sekibun points a thread) otherwise
+  // One gather block per particle.  Few particles: many threads each, since
+  // the block's latency is the kernel's.  Many: few threads, since a block's
+  // reduction costs as much per warp whatever the warp summed (8600
+  // particles at 256^3: 255 us with 512 threads, 193 with 256, 162 with 128,
+  // 159 with 64; 256 at 128^3: 15.7, 17.6, 23.6, 36).  The scatter's blocks
+  // each find the particle's neighbours first, so with enough particles to
+  // fill the GPU one block does all its points (336 us with four, 250 with
+  // two, 215 with one at 256^3; 14.9, 13.2, 15.4 at 128^3).
   pp.hyd_pcl = 1;
-  pp.hyd_threads = b->Np >= 128 ? 512 : 1024;
+  pp.hyd_threads = b->Np >= 1024 ? 128 : b->Np >= 128 ? 512 : 1024;
+  pp.sc_pcl = b->Np >= 1024 ? 1 : b->Np >= 128 ? 2 : PCL;
+  // a neighbour's centre is within two supports, a point within one
+  const double reach = 3.0 * (p->a + 0.5 * p->a_xi) + 4.0;
+  pp.near_wrap = std::min(g.NX, std::min(g.NY, g.NZ)) < 2.0 * reach ? 1 : 0;
   if (pp.frozen) pp.thermostat = 0;
   if (p->neighbor_lists < -1 || p->neighbor_lists > 1) return KAPSEL_EINVAL;
   b->mt.reset(new MT19937(p->mt_seed));

@@ -38,6 +38,8 @@ struct PPar {
   int frozen;               // positions and velocities held; forces still measured
   int hyd_pcl;              // gather blocks per particle (at most HYD_PCL_MAX)
   int hyd_threads;          // threads per gather block (at most 1024)
+  int sc_pcl;               // scatter blocks per particle
+  int near_wrap;            // a neighbour's offsets may pass half the box (small grids)
   // per-particle neighbour lists ([Np][NBL_MAX + 1]: count, then indices in
   // increasing order) built each step for large particle counts; null: the
   // pair searches scan all particles
@@ -226,38 +228,41 @@ __global__ void k_particles_position(PPar p, DPart *__restrict__ parts, int eule
   if (n < p.Np) position_update_one(p, parts, n, euler, status);
 }
 
+// Compensated sum over the lanes of a warp, valid in lane 0.
+__device__ __forceinline__ KSum warp_ksum(double s, double c) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double so = __shfl_down_sync(0xffffffffu, s, o);
+    const double co = __shfl_down_sync(0xffffffffu, c, o);
+    KSum k{s, c + co};
+    k.add(so);
+    s = k.s;
+    c = k.c;
+  }
+  return {s, c};
+}
+
 // Block reduction of NV compensated sums; result valid in thread 0.  Warps
-// reduce with shuffles, then thread i < NV adds value i over the warps.
+// reduce with shuffles, then warp i adds value i over the warps the same way
+// (five dependent additions where one thread adding up to 32 took 32).
 template <int NV>
 __device__ void block_reduce(KSum (&v)[NV], double *sh /* [2*NV][32] */) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    double s = v[i].s, c = v[i].c;
-    for (int o = 16; o > 0; o >>= 1) {
-      const double so = __shfl_down_sync(0xffffffffu, s, o);
-      const double co = __shfl_down_sync(0xffffffffu, c, o);
-      KSum k{s, c + co};
-      k.add(so);
-      s = k.s;
-      c = k.c;
-    }
+    const KSum k = warp_ksum(v[i].s, v[i].c);
     if (lane == 0) {
-      sh[(2 * i) * 32 + wid] = s;
-      sh[(2 * i + 1) * 32 + wid] = c;
+      sh[(2 * i) * 32 + wid] = k.s;
+      sh[(2 * i + 1) * 32 + wid] = k.c;
     }
   }
   __syncthreads();
-  if (threadIdx.x < NV) {
-    const int i = threadIdx.x;
-    KSum k{0.0, 0.0};
-    double cs = 0.0;
-    for (int w = 0; w < nw; ++w) {
-      k.add(sh[(2 * i) * 32 + w]);
-      cs += sh[(2 * i + 1) * 32 + w];
+  for (int i = wid; i < NV; i += nw) {
+    const KSum k = warp_ksum(lane < nw ? sh[(2 * i) * 32 + lane] : 0.0, lane < nw ? sh[(2 * i + 1) * 32 + lane] : 0.0);
+    if (lane == 0) {
+      sh[(2 * i) * 32] = k.s;
+      sh[(2 * i + 1) * 32] = k.c;
     }
-    sh[(2 * i) * 32] = k.s;
-    sh[(2 * i + 1) * 32] = k.c + cs;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -316,8 +321,7 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
     // mixed path: the point's offset from the sphere centre, its distance,
     // phi and the momentum-exchange terms in float (the offset is an integer
     // cell shift minus the centre's sub-cell residue, so it is exact to one
-    // float ulp); the per-thread and per-warp sums in float, every wider sum
-    // in double (compensated)
+    // float ulp); sums of GB points in float, every wider sum in double
     const float dxf = (float)p.DX, rpf = (float)(p.RADIUS + p.HXI), rmf = (float)(p.RADIUS - p.HXI);
     const float resf[3] = {(float)b.res[0], (float)b.res[1], (float)b.res[2]};
     const float vpf[3] = {(float)vp[0], (float)vp[1], (float)vp[2]};
@@ -370,31 +374,55 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
         f6[4] += r[k][2] * fp[0] - r[k][0] * fp[2];
         f6[5] += r[k][0] * fp[1] - r[k][1] * fp[0];
       }
-    }
-  } else
-  for (int m = first; m < p.S; m += stride) {
-    int rm[3];
-    double r[3], dist;
-    stencil_point(b, load_cell(cells, m), xp, p, rm, r, dist);
-    const double ph = (double)prof_phi<R>(dist, p);
-    if (ph == 0.0) continue;  // a zero term: skip its loads
-    const size_t im = ((size_t)rm[0] * p.N[1] + rm[1]) * p.N[2] + rm[2];
-    const double ug[3] = {(double)__ldg(u + im), (double)__ldg(u + npts + im), (double)__ldg(u + 2 * npts + im)};
-    double vr[3] = {0.0, 0.0, 0.0};
-    if (p.rotation) {
-      vr[0] = wp[1] * r[2] - wp[2] * r[1];
-      vr[1] = wp[2] * r[0] - wp[0] * r[2];
-      vr[2] = wp[0] * r[1] - wp[1] * r[0];
-    }
-    double fp[3];
+      // a batch is summed in float, the batches in double
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      fp[d] = ((vp[d] + vr[d]) - ug[d]) * ph;
-      a9[d] += fp[d];
+      for (int i = 0; i < 6; ++i) {
+        a9[i] += (double)f6[i];
+        f6[i] = 0.f;
+      }
     }
-    a9[3] += r[1] * fp[2] - r[2] * fp[1];
-    a9[4] += r[2] * fp[0] - r[0] * fp[2];
-    a9[5] += r[0] * fp[1] - r[1] * fp[0];
+  } else {
+    // the same in double, two points at a time
+    constexpr int GB2 = 2;
+    for (int m0 = first; m0 < p.S; m0 += GB2 * stride) {
+      double ph[GB2], r[GB2][3], ug[GB2][3];
+#pragma unroll
+      for (int k = 0; k < GB2; ++k) {
+        const int m = m0 + k * stride;
+        ph[k] = 0.0;
+        if (m >= p.S) continue;
+        int rm[3];
+        double dist;
+        stencil_point(b, load_cell(cells, m), xp, p, rm, r[k], dist);
+        const size_t im = ((size_t)rm[0] * p.N[1] + rm[1]) * p.N[2] + rm[2];
+        // phi is exactly zero from RADIUS + HXI on; the loads start before
+        // the profile's exponentials
+        if (dist < p.RADIUS + p.HXI) {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) ug[k][d] = (double)__ldg(u + d * npts + im);
+          ph[k] = (double)prof_phi<R>(dist, p);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < GB2; ++k) {
+        if (ph[k] == 0.0) continue;
+        double vr[3] = {0.0, 0.0, 0.0};
+        if (p.rotation) {
+          vr[0] = wp[1] * r[k][2] - wp[2] * r[k][1];
+          vr[1] = wp[2] * r[k][0] - wp[0] * r[k][2];
+          vr[2] = wp[0] * r[k][1] - wp[1] * r[k][0];
+        }
+        double fp[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          fp[d] = ((vp[d] + vr[d]) - ug[k][d]) * ph[k];
+          a9[d] += fp[d];
+        }
+        a9[3] += r[k][1] * fp[2] - r[k][2] * fp[1];
+        a9[4] += r[k][2] * fp[0] - r[k][0] * fp[2];
+        a9[5] += r[k][0] * fp[1] - r[k][1] * fp[0];
+      }
+    }
   }
   if (p.lj_on) {
     int mc[3];
@@ -459,12 +487,10 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
   }
   KSum acc[9];
   if constexpr (sizeof(R) == 4) {
-    // each thread's few hydro terms are summed in float; from the warp
-    // level up every sum is double (warp sums plain, the sum over the warps
+    // each batch of a thread's hydro terms is summed in float; from there up
+    // every sum is double (thread and warp sums plain, the sum over the warps
     // compensated)
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) a9[i] = (double)f6[i];
 #pragma unroll
     for (int i = 0; i < 9; ++i)
 #pragma unroll
@@ -473,12 +499,12 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
 #pragma unroll
       for (int i = 0; i < 9; ++i) sh[(2 * i) * 32 + wid] = a9[i];
     __syncthreads();
-    if (threadIdx.x < 9) {
-      const int i = threadIdx.x;
-      KSum k{0.0, 0.0};
-      for (int w = 0; w < nw; ++w) k.add(sh[(2 * i) * 32 + w]);
-      sh[(2 * i) * 32] = k.s;
-      sh[(2 * i + 1) * 32] = k.c;
+    for (int i = wid; i < 9; i += nw) {
+      const KSum k = warp_ksum(lane < nw ? sh[(2 * i) * 32 + lane] : 0.0, 0.0);
+      if (lane == 0) {
+        sh[(2 * i) * 32] = k.s;
+        sh[(2 * i + 1) * 32] = k.c;
+      }
     }
     __syncthreads();
     if (threadIdx.x == 0)
@@ -590,7 +616,8 @@ constexpr int NB_MAX = 64;  // overlapping neighbours per particle (more: KAPSEL
 
 struct NbShared {
   double x[3], v[3], w[3], res[3];
-  float resf[3];
+  float resf[3], vf[3], wf[3];
+  float base[3];  // cell of the scattering particle less this one's, nearest image
   int xi[3];
   int idx;
 };
@@ -606,6 +633,8 @@ __device__ void fill_candidate(const PPar &p, const DPart *__restrict__ parts, i
     e.w[d] = o.omega[d];
     e.res[d] = sb.res[d];
     e.resf[d] = (float)sb.res[d];
+    e.vf[d] = (float)o.v[d];
+    e.wf[d] = (float)o.omega[d];
     e.xi[d] = sb.xi[d];
   }
   e.idx = j;
@@ -696,11 +725,8 @@ __device__ __forceinline__ void offset_from_base(const int rm[3], const int xi[3
 // f = up' - phi' u* with the phi > 1 clamp (Make_f_particle_dt_nonsole,
 // f_particle.h:41-64; make_phi.cxx:278-297).
 template <typename R>
-__device__ __forceinline__ void store_force(R *__restrict__ force, const R *__restrict__ ustar, size_t npts, size_t im,
-                                            R acc, R (&up)[3]) {
-  R us[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) us[d] = __ldg(ustar + d * npts + im);
+__device__ __forceinline__ void store_force(R *__restrict__ force, size_t npts, size_t im, R acc, R (&up)[3],
+                                            const R (&us)[3]) {
   if (acc > R(1)) {
     const R inv = R(1) / acc;
 #pragma unroll
@@ -725,9 +751,9 @@ __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *
                                                            const unsigned *__restrict__ ovl = nullptr) {
   __shared__ NbShared nb[NB_MAX];
   pdl_begin();
-  const int n = blockIdx.x / PCL;
-  const int stride = PCL * blockDim.x;
-  const int first = (blockIdx.x % PCL) * blockDim.x + threadIdx.x;
+  const int n = blockIdx.x / p.sc_pcl;
+  const int stride = p.sc_pcl * blockDim.x;
+  const int first = (blockIdx.x % p.sc_pcl) * blockDim.x + threadIdx.x;
   const int nnb = ovl ? overlap_from_bits(p, parts, n, ovl, nb, status) : overlap_candidates(p, parts, n, nb, status);
   int nlow = 0;  // candidates with a lower index come first
   while (nlow < nnb && nb[nlow].idx < n) ++nlow;
@@ -742,20 +768,57 @@ __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *
     // mixed path: offset, distance, phi and phi*(v + omega x r) in float
     const float dxf = (float)p.DX, rpf = (float)(p.RADIUS + p.HXI), rmf = (float)(p.RADIUS - p.HXI);
     const float resf[3] = {(float)b.res[0], (float)b.res[1], (float)b.res[2]};
+    const float vf[3] = {(float)vp[0], (float)vp[1], (float)vp[2]}, wf[3] = {(float)wp[0], (float)wp[1], (float)wp[2]};
+    if (threadIdx.x < 3 * nnb) {
+      const int k = threadIdx.x / 3, d = threadIdx.x - 3 * k;
+      const int c = (b.xi[d] - nb[k].xi[d]) & (p.N[d] - 1);
+      nb[k].base[d] = (float)(c >= p.N[d] / 2 ? c - p.N[d] : c);
+    }
+    __syncthreads();
+    // A point is outside a neighbour's support for certain from this squared
+    // distance on (the margin covers the roundings of the distance below,
+    // which decides): that leaves the square root and the profile to the few
+    // neighbours whose support reaches the point.
+    const float far2 = rpf * rpf * (1.f + 1e-6f);
+    // the offset of the point from neighbour k and its squared length.
+    // Cell differences are small integers, exact in float; only on a small
+    // grid can one pass half the box and need its nearest image.
+    auto reach = [&](int k, const float (&cf)[3], float (&rj)[3]) -> float {
+      float s2 = 0.f;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        float c = cf[d] + nb[k].base[d];
+        if (p.near_wrap) {
+          const int ci = (int)c & (p.N[d] - 1);
+          c = (float)(ci >= p.N[d] / 2 ? ci - p.N[d] : ci);
+        }
+        rj[d] = __fsub_rn(__fmul_rn(c, dxf), nb[k].resf[d]);
+        s2 = d == 0 ? __fmul_rn(rj[d], rj[d]) : __fadd_rn(s2, __fmul_rn(rj[d], rj[d]));
+      }
+      return s2;
+    };
     for (int m = first; m < p.S; m += stride) {
       const Cell cell = load_cell(cells, m);
       int rm[3];
       float r[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) rm[d] = (b.xi[d] + cell.d[d] + p.N[d]) & (p.N[d] - 1);
-      const float ph = prof_phi_f(offset_f(cell.d, resf, dxf, r), rpf, rmf, dxf);
+      const float dist = offset_f(cell.d, resf, dxf, r);
+      if (!(dist < rpf)) continue;  // phi is exactly zero there
+      const size_t im = ((size_t)rm[0] * p.N[1] + rm[1]) * p.N[2] + rm[2];
+      float us[3];  // on their way while the profile and the owner are found
+      if constexpr (FORCE)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) us[d] = ustar[d * npts + im];
+      const float ph = prof_phi_f(dist, rpf, rmf, dxf);
       if (ph == 0.f) continue;
+      const float cf[3] = {(float)cell.d[0], (float)cell.d[1], (float)cell.d[2]};
       bool own = true;
       for (int k = 0; k < nlow && own; ++k) {
-        int cj[3];
         float rj[3];
-        offset_from_base(rm, nb[k].xi, p, cj);
-        const float dj = offset_f(cj, nb[k].resf, dxf, rj);
+        const float s2 = reach(k, cf, rj);
+        if (s2 >= far2) continue;
+        const float dj = __fsqrt_rn(s2);
         if (dj < rpf && prof_phi_f(dj, rpf, rmf, dxf) != 0.f) own = false;
       }
       if (!own) continue;
@@ -765,15 +828,15 @@ __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *
         float vr = 0.f;
         if (p.rotation) {
           const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
-          vr = (float)wp[d1] * r[d2] - (float)wp[d2] * r[d1];
+          vr = wf[d1] * r[d2] - wf[d2] * r[d1];
         }
-        up[d] = ((float)vp[d] + vr) * ph;
+        up[d] = (vf[d] + vr) * ph;
       }
       for (int k = nlow; k < nnb; ++k) {
-        int cj[3];
         float rj[3];
-        offset_from_base(rm, nb[k].xi, p, cj);
-        const float dj = offset_f(cj, nb[k].resf, dxf, rj);
+        const float s2 = reach(k, cf, rj);
+        if (s2 >= far2) continue;
+        const float dj = __fsqrt_rn(s2);
         if (!(dj < rpf)) continue;
         const float phj = prof_phi_f(dj, rpf, rmf, dxf);
         if (phj == 0.f) continue;
@@ -783,14 +846,13 @@ __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *
           float vr = 0.f;
           if (p.rotation) {
             const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
-            vr = (float)nb[k].w[d1] * rj[d2] - (float)nb[k].w[d2] * rj[d1];
+            vr = nb[k].wf[d1] * rj[d2] - nb[k].wf[d2] * rj[d1];
           }
-          up[d] += ((float)nb[k].v[d] + vr) * phj;
+          up[d] += (nb[k].vf[d] + vr) * phj;
         }
       }
-      const size_t im = ((size_t)rm[0] * p.N[1] + rm[1]) * p.N[2] + rm[2];
       if constexpr (FORCE) {
-        store_force<R>(out, ustar, npts, im, acc, up);
+        store_force<R>(out, npts, im, acc, up, us);
       } else {
         out[im] = acc;
 #pragma unroll
@@ -802,6 +864,12 @@ __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *
     int rm[3];
     double r[3], dist;
     stencil_point(b, load_cell(cells, m), xp, p, rm, r, dist);
+    if (!(dist < rsup)) continue;  // phi is exactly zero there
+    const size_t im = ((size_t)rm[0] * p.N[1] + rm[1]) * p.N[2] + rm[2];
+    R us[3];
+    if constexpr (FORCE)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) us[d] = ustar[d * npts + im];
     const double ph = (double)prof_phi<R>(dist, p);
     if (ph == 0.0) continue;
     bool own = true;
@@ -841,9 +909,8 @@ __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *
         up[d] += (nb[k].v[d] + vr) * phj;
       }
     }
-    const size_t im = ((size_t)rm[0] * p.N[1] + rm[1]) * p.N[2] + rm[2];
     if constexpr (FORCE) {
-      store_force<R>(out, ustar, npts, im, acc, up);
+      store_force<R>(out, npts, im, acc, up, us);
     } else {
       out[im] = (R)acc;
 #pragma unroll
