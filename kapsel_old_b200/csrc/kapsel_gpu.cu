@@ -2152,8 +2152,16 @@ __global__ void k_time_gate(unsigned long long ns) {
 // scaling of a trained network.
 struct kapsel_nc {
   cudaStream_t stream = nullptr;
-  float *params = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr, *loss = nullptr;
+  float *params = nullptr, *m = nullptr, *v = nullptr;
+  // gradient, loss and status word in one allocation
+  float *grad = nullptr, *loss = nullptr;
   int *status = nullptr;
+  // device rows of the largest call so far: three allocations and their
+  // return in every call were most of a 16384-row gradient's 820 us.  They
+  // belong to the object; calls on it take turns (mu).
+  std::mutex mu;
+  float *rows = nullptr;
+  size_t rows_cap = 0;
   long long adam_t = 0;
   nc::NcScale sc{};
   bool scaled = false;
@@ -3425,10 +3433,11 @@ int kapsel_nc_create(const float *params, kapsel_nc **out) {
   if (!h) return KAPSEL_ENOMEM;
   const size_t nb = sizeof(float) * nc::NPARAM;
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) return KAPSEL_ECUDA;
-  if (cudaMalloc(&h->params, nb) != cudaSuccess || cudaMalloc(&h->grad, nb) != cudaSuccess ||
-      cudaMalloc(&h->m, nb) != cudaSuccess || cudaMalloc(&h->v, nb) != cudaSuccess ||
-      cudaMalloc(&h->loss, sizeof(float)) != cudaSuccess || cudaMalloc(&h->status, sizeof(int)) != cudaSuccess)
+  if (cudaMalloc(&h->params, nb) != cudaSuccess || cudaMalloc(&h->grad, nb + 2 * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&h->m, nb) != cudaSuccess || cudaMalloc(&h->v, nb) != cudaSuccess)
     return KAPSEL_ENOMEM;
+  h->loss = h->grad + nc::NPARAM;
+  h->status = reinterpret_cast<int *>(h->grad + nc::NPARAM + 1);
   KCHECK(cudaMemcpyAsync(h->params, params, nb, cudaMemcpyHostToDevice, h->stream));
   KCHECK(cudaMemsetAsync(h->grad, 0, nb, h->stream));
   KCHECK(cudaMemsetAsync(h->m, 0, nb, h->stream));
@@ -3446,8 +3455,7 @@ int kapsel_nc_destroy(kapsel_nc *nc) {
   cudaFree(nc->grad);
   cudaFree(nc->m);
   cudaFree(nc->v);
-  cudaFree(nc->loss);
-  cudaFree(nc->status);
+  cudaFree(nc->rows);
   cudaStreamDestroy(nc->stream);
   delete nc;
   return 0;
@@ -3467,24 +3475,42 @@ int kapsel_nc_set_params(kapsel_nc *nc, const float *params) {
   return 0;
 }
 
-static int nc_status(kapsel_nc *nc) {
-  int st = 0;
-  KCHECK(cudaMemcpyAsync(&st, nc->status, sizeof(int), cudaMemcpyDeviceToHost, nc->stream));
-  KCHECK(cudaStreamSynchronize(nc->stream));
+// clears a non-zero status word after it has been read
+static int nc_clear(kapsel_nc *nc, int st) {
   if (st) {
     cudaMemsetAsync(nc->status, 0, sizeof(int), nc->stream);
     cudaStreamSynchronize(nc->stream);
   }
   return st;
 }
+static int nc_status(kapsel_nc *nc) {
+  int st = 0;
+  KCHECK(cudaMemcpyAsync(&st, nc->status, sizeof(int), cudaMemcpyDeviceToHost, nc->stream));
+  KCHECK(cudaStreamSynchronize(nc->stream));
+  return nc_clear(nc, st);
+}
+
+// device rows for n samples: inputs, targets or outputs, column weights
+static int nc_rows(kapsel_nc *nc, int n) {
+  if ((size_t)n <= nc->rows_cap) return 0;
+  cudaFree(nc->rows);
+  nc->rows = nullptr;
+  nc->rows_cap = 0;
+  if (cudaMalloc(&nc->rows, sizeof(float) * ((nc::IN + nc::OUT) * (size_t)n + nc::OUT)) != cudaSuccess) {
+    cudaGetLastError();
+    return KAPSEL_ENOMEM;
+  }
+  nc->rows_cap = (size_t)n;
+  return 0;
+}
 
 int kapsel_nc_forward(kapsel_nc *nc, const float *x, int n, float *y) {
   if (!nc || !x || !y || n < 0) return KAPSEL_EINVAL;
   if (n == 0) return 0;
-  float *dx = nullptr, *dy = nullptr;
-  if (cudaMallocAsync(&dx, sizeof(float) * nc::IN * n, nc->stream) != cudaSuccess ||
-      cudaMallocAsync(&dy, sizeof(float) * nc::OUT * n, nc->stream) != cudaSuccess)
-    return KAPSEL_ENOMEM;
+  std::lock_guard<std::mutex> turn(nc->mu);
+  const int rc = nc_rows(nc, n);
+  if (rc) return rc;
+  float *dx = nc->rows, *dy = dx + nc::IN * (size_t)n;
   KCHECK(cudaMemcpyAsync(dx, x, sizeof(float) * nc::IN * n, cudaMemcpyHostToDevice, nc->stream));
   nc::TileIO io{};
   io.x = dx;
@@ -3494,25 +3520,20 @@ int kapsel_nc_forward(kapsel_nc *nc, const float *x, int n, float *y) {
   nc::k_mlp_tile<false><<<(n + nc::TILE - 1) / nc::TILE, 256, nc::SMEM_ALLOC, nc->stream>>>(nc->params, io);
   KCHECK(cudaGetLastError());
   KCHECK(cudaMemcpyAsync(y, dy, sizeof(float) * nc::OUT * n, cudaMemcpyDeviceToHost, nc->stream));
-  cudaFreeAsync(dx, nc->stream);
-  cudaFreeAsync(dy, nc->stream);
-  KCHECK(cudaStreamSynchronize(nc->stream));
   return nc_status(nc);
 }
 
 int kapsel_nc_gradient(kapsel_nc *nc, const float *x, const float *y, const float *colw, int n, float *grad,
                        float *loss) {
   if (!nc || !x || !y || !colw || !grad || !loss || n <= 0) return KAPSEL_EINVAL;
-  float *dx = nullptr, *dy = nullptr, *dw = nullptr;
-  if (cudaMallocAsync(&dx, sizeof(float) * nc::IN * n, nc->stream) != cudaSuccess ||
-      cudaMallocAsync(&dy, sizeof(float) * nc::OUT * n, nc->stream) != cudaSuccess ||
-      cudaMallocAsync(&dw, sizeof(float) * nc::OUT, nc->stream) != cudaSuccess)
-    return KAPSEL_ENOMEM;
+  std::lock_guard<std::mutex> turn(nc->mu);
+  const int rc = nc_rows(nc, n);
+  if (rc) return rc;
+  float *dx = nc->rows, *dy = dx + nc::IN * (size_t)n, *dw = dy + nc::OUT * (size_t)n;
+  KCHECK(cudaMemsetAsync(nc->grad, 0, sizeof(float) * (nc::NPARAM + 1), nc->stream));  // and the loss
   KCHECK(cudaMemcpyAsync(dx, x, sizeof(float) * nc::IN * n, cudaMemcpyHostToDevice, nc->stream));
   KCHECK(cudaMemcpyAsync(dy, y, sizeof(float) * nc::OUT * n, cudaMemcpyHostToDevice, nc->stream));
   KCHECK(cudaMemcpyAsync(dw, colw, sizeof(float) * nc::OUT, cudaMemcpyHostToDevice, nc->stream));
-  KCHECK(cudaMemsetAsync(nc->grad, 0, sizeof(float) * nc::NPARAM, nc->stream));
-  KCHECK(cudaMemsetAsync(nc->loss, 0, sizeof(float), nc->stream));
   nc::TileIO io{};
   io.x = dx;
   io.y = dy;
@@ -3525,18 +3546,20 @@ int kapsel_nc_gradient(kapsel_nc *nc, const float *x, const float *y, const floa
   nc::k_mlp_tile<true><<<(n + nc::TILE - 1) / nc::TILE, 128, nc::SMEM_ALLOC, nc->stream>>>(nc->params, io);
   KCHECK(cudaGetLastError());
   KCHECK(cudaMemcpyAsync(grad, nc->grad, sizeof(float) * nc::NPARAM, cudaMemcpyDeviceToHost, nc->stream));
-  KCHECK(cudaMemcpyAsync(loss, nc->loss, sizeof(float), cudaMemcpyDeviceToHost, nc->stream));
-  KCHECK(cudaMemsetAsync(nc->grad, 0, sizeof(float) * nc::NPARAM, nc->stream));
-  cudaFreeAsync(dx, nc->stream);
-  cudaFreeAsync(dy, nc->stream);
-  cudaFreeAsync(dw, nc->stream);
+  // the loss and the status word after it in one copy
+  float tail[2];
+  KCHECK(cudaMemcpyAsync(tail, nc->loss, sizeof(tail), cudaMemcpyDeviceToHost, nc->stream));
   KCHECK(cudaStreamSynchronize(nc->stream));
-  return nc_status(nc);
+  *loss = tail[0];
+  int st;
+  memcpy(&st, &tail[1], sizeof(int));
+  return nc_clear(nc, st);
 }
 
 int kapsel_nc_train(kapsel_nc *nc, const float *x, const float *y, const float *colw, int n, int epochs, int batch,
                     float lr, unsigned int seed, float *loss_per_epoch) {
   if (!nc || !x || !y || !colw || n <= 0 || epochs <= 0 || batch <= 0 || !(lr > 0.f)) return KAPSEL_EINVAL;
+  std::lock_guard<std::mutex> turn(nc->mu);
   float *dx = nullptr, *dy = nullptr, *dw = nullptr;
   int *didx = nullptr;
   if (cudaMallocAsync(&dx, sizeof(float) * nc::IN * n, nc->stream) != cudaSuccess ||
