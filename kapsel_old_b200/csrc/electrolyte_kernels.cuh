@@ -10,151 +10,125 @@
 
 #include "particle_kernels.cuh"
 #include "spectral_kernels.cuh"
+#include "xtile_kernels.cuh"
 #include "zwarp_kernels.cuh"
 
 namespace kapsel {
 
-struct KOp {
-  double a[2];      // operator scale (1/eps, kBT*L, dt ...), of blockIdx.z
-  double e_amp[3];  // value subtracted from the real part of the k=0 mode (k_x_poisson)
-};
-
 enum { XI_IDENT = 0, XI_GRADDIFF = 2 };
-enum { XF_CONCUPD = 1, XF_PSI_FULL = 3 };
 
-// x pass, inverse, with a k-space operator on the (compact) input spectra:
-//   XI_IDENT     out_c = in_c                        (NOUT == NIN)
-//   XI_GRADDIFF  out_d = -i k_d a in_0                (Diffusion_flux_single,
-//                solute_rhs.cxx:214-234)
-// in: [NIN][KXc][KYc][TZ] (planes in_cstride apart), out I1: [NOUT][NX][KYc][TZ].
-// grid (KYc, ceil(TZ/KC), batches): batch z reads NIN planes and writes NOUT
-// components on from those of batch z - 1 (the two ion species in one launch).
-template <typename R, int KC, int OP, int NIN, int NOUT>
-__global__ void __launch_bounds__(256) k_x_inv_op(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ in,
-                                                  size_t in_cstride, Cx<R> *__restrict__ out, KOp op) {
+// x pass, inverse, of compact spectra with a k-space operator
+// (xtile_kernels.cuh).  A group computes one output component from what it reads
+// itself, so the block needs no shared tile:
+//   XI_IDENT     out_c = in_c                        (NOUT inputs)
+//   XI_GRADDIFF  out_d = -i k_d a in_0, three outputs per input
+//                (Diffusion_flux_single, solute_rhs.cxx:214-234)
+// in: [..][KXc][KYc][TS] (planes in_cstride apart), out I1: [..][NX][KYc][TS].
+// grid (ceil(TZ/CW), KYc, batches): batch z reads the next input (GRADDIFF) and
+// writes the next NOUT components (the two ion species in one launch).
+struct XOp {
+  double a[2];  // operator scale of batch z (kBT L)
+};
+template <typename R, int LX, int OP, int NOUT, bool FULL>
+__global__ void __launch_bounds__(NOUT * XT<R, LX>::TPG, XT<R, LX>::blocks(NOUT)) k_xw_inv_op(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ in,
+                                                         size_t in_cstride, Cx<R> *__restrict__ out, XOp op) {
+  using T = XT<R, LX, FULL>;
+  using X = ZL<LX>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  in += (size_t)blockIdx.z * NIN * in_cstride;
-  out += (size_t)blockIdx.z * NOUT * g.NX * g.KYc * g.TS;
-  constexpr int W = NOUT * KC;
-  Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
-  Cx<R> *Zt = twx + g.NX;            // [NIN][KXc][KC]
-  Cx<R> *U = Zt + NIN * g.KXc * KC;  // [NX][NOUT*KC]
-  Cx<R> *scr = U + g.NX * W;
-  const int iy = blockIdx.x;
-  const int kz0 = blockIdx.y * KC;
-  const int ncol = min(KC, g.TZ - kz0);
-  load_twiddles(twx, tw.x, g.NX);
   in = pdl_fresh(in);
-  for (int it = threadIdx.x; it < NIN * g.KXc * KC; it += blockDim.x) {
-    const int col = it % KC, rest = it / KC, ix = rest % g.KXc, c = rest / g.KXc;
-    if (col < ncol) cp_async_cx(Zt + it, in + c * in_cstride + ((size_t)ix * g.KYc + iy) * g.TS + kz0 + col);
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  const int KYi = signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY);
-  const R ky = R(g.wave[1] * KYi);
-  for (int it = threadIdx.x; it < g.NX * KC; it += blockDim.x) {
-    const int col = it % KC, i = it / KC;
-    Cx<R> o[NOUT];
+  const int grp = T::group();
+  Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + grp * T::EX;
+  const int iy = blockIdx.y, kz0 = blockIdx.x * T::CW, ncol = min(T::CW, g.TZ - kz0);
+  const size_t at = (size_t)iy * g.TS + kz0, row = (size_t)g.KYc * g.TS;
+  const Cx<R> *src = in + (OP == XI_IDENT ? grp : (int)blockIdx.z) * in_cstride + at;
+  const R ky = R(g.wave[1] * signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY));
+  const R a = OP == XI_IDENT ? R(1) : R(op.a[blockIdx.z]);
+  Cx<R> v[X::N1];
+  const int col = T::col();
 #pragma unroll
-    for (int c = 0; c < NOUT; ++c) o[c] = {R(0), R(0)};
-    const int KXi = signed_k(i, g.NX);
-    if (col < ncol && abs(KXi) < g.TX) {
-      const int ix = KXi >= 0 ? KXi : KXi + g.KXc;
-      const int kz = kz0 + col;
-      if (OP == XI_IDENT) {
-#pragma unroll
-        for (int c = 0; c < NOUT; ++c) o[c] = Zt[(c * g.KXc + ix) * KC + col];
-      } else {
-        const R kx = R(g.wave[0] * KXi), kzr = R(g.wave[2] * kz);
-        const Cx<R> a = Zt[ix * KC + col];
-        const R s = R(op.a[blockIdx.z]);
-        const Cx<R> v = {a.x * s, a.y * s};
-        const R kk[3] = {kx, ky, kzr};
-#pragma unroll
-        for (int d = 0; d < 3 && d < NOUT; ++d) o[d] = {kk[d] * v.y, -kk[d] * v.x};  // -i k v
-      }
+  for (int n1 = 0; n1 < X::N1; ++n1) {
+    const int ix = T::G::row(T::t() + X::N2 * n1);
+    v[n1] = ix >= 0 && col < ncol ? src[ix * row + col] : Cx<R>{R(0), R(0)};
+    if (OP == XI_GRADDIFF) {
+      const int KXi = ix < T::TX ? ix : ix - T::KXc;
+      const R k = grp == 0 ? R(g.wave[0] * KXi) : grp == 1 ? ky : R(g.wave[2] * (kz0 + col));
+      const Cx<R> q = {v[n1].x * a, v[n1].y * a};
+      v[n1] = {k * q.y, -k * q.x};  // -i k v
     }
-#pragma unroll
-    for (int c = 0; c < NOUT; ++c) U[i * W + c * KC + col] = o[c];
   }
-  __syncthreads();
-  fft2_smem<R, -1, W>(U, scr, g.lx, 1, W, twx);
-  for (int it = threadIdx.x; it < NOUT * g.NX * KC; it += blockDim.x) {
-    const int col = it % KC, rest = it / KC, x = rest & (g.NX - 1), c = rest >> g.lx;
-    if (col < ncol) out[(((size_t)c * g.NX + x) * g.KYc + iy) * g.TS + kz0 + col] = U[x * W + c * KC + col];
-  }
+  xfft<R, LX, -1>(v, ex, tw.x);
+  x_store<R, LX>(out + (size_t)(blockIdx.z * NOUT + grp) * T::NX * row + at, row, ncol, v);
 }
 
-// x pass, forward, of NIN spectra (I1 layout) with an operator on the kept modes:
-//   XF_CONCUPD       out[o] += a * (-i k.X)             (U_k2divergence_k + the
-//                    concentration part of Field_solver_Euler, fluid_solver.cxx:122-135)
-//   XF_PSI_FULL      out[o] = X_0 IK2 a                 (full spectrum: the Coulomb
-//                    potential of Output_avs_charge, avs_output.cxx:464-466)
-// grid (KYc, ceil(TZ/KC), batches): batch z reads the next NIN components and
-// updates the next output plane, out_cstride on.
-template <typename R, int KC, int OP, int NIN>
-__global__ void __launch_bounds__(256) k_x_fwd_op(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ in,
-                                                  Cx<R> *__restrict__ out, size_t out_cstride, KOp op) {
+// x pass, forward, of the three flux spectra of species z = blockIdx.z and the
+// Euler update of its concentration: conc += dt (-i k.F)  (U_k2divergence_k and
+// the concentration part of Field_solver_Euler, fluid_solver.cxx:122-135).
+// grid (ceil(TZ/CW), KYc, 2), three groups.
+template <typename R, int LX>
+__global__ void __launch_bounds__(3 * XT<R, LX>::TPG, XT<R, LX>::blocks(3)) k_xw_concupd(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ in,
+                                                   Cx<R> *__restrict__ conc, size_t conc_stride, double dtime) {
+  using T = XT<R, LX>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  in += (size_t)blockIdx.z * NIN * g.NX * g.KYc * g.TS;
-  out += blockIdx.z * out_cstride;
-  constexpr int W = NIN * KC;
-  Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
-  Cx<R> *Pb = twx + g.NX;  // [NX][NIN*KC]
-  Cx<R> *scr = Pb + g.NX * W;
-  const int iy = blockIdx.x;
-  const int kz0 = blockIdx.y * KC;
-  const int ncol = min(KC, g.TZ - kz0);
-  const size_t cstr = (size_t)g.NX * g.KYc * g.TS;
-  load_twiddles(twx, tw.x, g.NX);
   in = pdl_fresh(in);
-  out = pdl_fresh(out);
-  for (int it = threadIdx.x; it < NIN * g.NX * KC; it += blockDim.x) {
-    const int col = it % KC, rest = it / KC, x = rest & (g.NX - 1), c = rest >> g.lx;
-    Cx<R> *d = Pb + x * W + c * KC + col;
-    if (col < ncol)
-      cp_async_cx(d, in + c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col);
-    else
-      *d = {R(0), R(0)};
-  }
-  cp_async_wait_all();
+  conc = pdl_fresh(conc);
+  const int grp = T::group();
+  Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + grp * T::EX;
+  Cx<R> *S = reinterpret_cast<Cx<R> *>(smem_raw);  // [3][KXc][CW], a group's buffer each
+  const int iy = blockIdx.y, kz0 = blockIdx.x * T::CW, ncol = min(T::CW, g.TZ - kz0);
+  const size_t at = (size_t)iy * g.TS + kz0, row = (size_t)g.KYc * g.TS;
+  Cx<R> v[ZL<LX>::N1];
+  x_load<R, LX>(in + (size_t)(blockIdx.z * 3 + grp) * T::NX * row + at, row, ncol, v);
+  xfft<R, LX, 1>(v, ex, tw.x);
+  x_put<R, LX>(ex, v);
   __syncthreads();
-  fft2_smem<R, 1, W>(Pb, scr, g.lx, 1, W, twx);
-  const int KYi = signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY);
-  const R ky = R(g.wave[1] * KYi);
-  for (int it = threadIdx.x; it < g.KXc * KC; it += blockDim.x) {
-    const int col = it % KC, ix = it / KC;
-    if (col >= ncol) continue;
-    const int KXi = ix < g.TX ? ix : ix - g.KXc;
-    const int i = KXi >= 0 ? KXi : KXi + g.NX;
-    const int kz = kz0 + col;
-    const size_t o = ((size_t)ix * g.KYc + iy) * g.TS + kz;
-    const Cx<R> *p = Pb + i * W + col;
+  const R ky = R(g.wave[1] * signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY)), dt = R(dtime);
+  x_modes<R, LX>(kz0, ncol, [&](int ix, int KXi, int col, int kz) {
+    const Cx<R> *p = S + ix * T::CW + col;
+    const Cx<R> f0 = p[0], f1 = p[T::EX], f2 = p[2 * T::EX];
     const R kx = R(g.wave[0] * KXi), kzr = R(g.wave[2] * kz);
-    if (OP == XF_CONCUPD) {
-      const Cx<R> f0 = p[0], f1 = p[KC], f2 = p[2 * KC];
-      const Cx<R> dv = {kx * f0.y + ky * f1.y + kzr * f2.y, -(kx * f0.x + ky * f1.x + kzr * f2.x)};
-      const R dt = R(op.a[0]);
-      out[o] = {out[o].x + dt * dv.x, out[o].y + dt * dv.y};
-    } else {
-      const R k2 = kx * kx + ky * ky + kzr * kzr;
-      const R s = k2 > R(0) ? R(op.a[0]) / k2 : R(0);
-      out[o] = {p[0].x * s, p[0].y * s};
-    }
+    const Cx<R> dv = {kx * f0.y + ky * f1.y + kzr * f2.y, -(kx * f0.x + ky * f1.x + kzr * f2.x)};
+    Cx<R> *c = conc + blockIdx.z * conc_stride + ix * row + at + col;
+    *c = {c->x + dt * dv.x, c->y + dt * dv.y};
+  });
+}
+
+// x pass, forward, of the full charge spectrum into the Coulomb potential's,
+// out[o] = X IK2 a (Output_avs_charge, avs_output.cxx:464-466).
+// grid (ceil(TZ/CW), KYc), one group.
+template <typename R, int LX>
+__global__ void __launch_bounds__(XT<R, LX>::TPG, XT<R, LX>::blocks(1)) k_xw_psi(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ in,
+                                               Cx<R> *__restrict__ out, double a) {
+  using T = XT<R, LX, true>;
+  using X = ZL<LX>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw);
+  const int iy = blockIdx.y, kz0 = blockIdx.x * T::CW, ncol = min(T::CW, g.TZ - kz0);
+  const size_t at = (size_t)iy * g.TS + kz0, row = (size_t)g.KYc * g.TS;
+  Cx<R> v[X::N1];
+  x_load<R, LX>(in + at, row, ncol, v);
+  xfft<R, LX, 1>(v, ex, tw.x);
+  const R ky = R(g.wave[1] * signed_k(iy, g.NY));
+#pragma unroll
+  for (int n1 = 0; n1 < X::N1; ++n1) {
+    const R kx = R(g.wave[0] * signed_k(T::t() + X::N2 * n1, T::NX));
+    const R kz = R(g.wave[2] * (kz0 + T::col()));
+    const R k2 = kx * kx + ky * ky + kz * kz;
+    v[n1] = cscale(v[n1], k2 > R(0) ? R(a) / k2 : R(0));
   }
+  x_store<R, LX>(out + at, row, ncol, v);
 }
 
 // x passes of the potential gradient, in place on buf: forward x of the
 // charge spectrum (component 0), out_d = -i k_d rho IK2 / eps
 // (Charge_field_k2Coulomb_potential_k_PBC, A_k2da_k; operate_electrolyte.cxx:
-// 76-88), inverse x of the three components.  The tile of one (ky, kz chunk)
-// stays in shared memory between the two transforms, so the charge spectrum
-// and the gradient's are never stored (forward and inverse as two launches,
-// with the completion of the full spectrum as a third, took 9 + 14 us and
-// 17 + 4 + 31 us at 128^3 in FP32).
+// 76-88), inverse x of the three components.  The charge spectrum and the
+// gradient's are never stored (forward and inverse as two launches, with the
+// completion of the full spectrum as a third, took 9 + 14 us and 17 + 4 + 31
+// us at 128^3 in FP32).  A block owns three tiles of columns: each of its three
+// groups of threads does one tile's forward transform, then one component's
+// inverse transforms.
 //   FULL = 0  the 2/3 box; the k=0 mode is -e_amp (Add_constant_field_k,
 //             fluid_solver.cxx:228-241)
 //   FULL = 1  the whole half spectrum (Make_Coulomb_force_x_on_fluid keeps
@@ -167,67 +141,57 @@ __global__ void __launch_bounds__(256) k_x_fwd_op(Geo g, Twiddles<R> tw, const C
 //             except on the Nyquist lines, where the partner has the same
 //             positive wavenumber: the components along such a line change
 //             sign, the others are what they were.
-// grid (KYc, ceil(TZ/KC)).
-template <typename R, int KC, int FULL>
-__global__ void __launch_bounds__(256) k_x_poisson(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ buf, KOp op) {
+// grid (ceil(TZ/(3 CW)), KYc), three groups.
+struct POp {
+  double a;         // 1 / eps
+  double e_amp[3];  // minus the k=0 mode (FULL = 0)
+};
+template <typename R, int LX, bool FULL>
+__global__ void __launch_bounds__(3 * XT<R, LX>::TPG, XT<R, LX>::blocks(3)) k_xw_poisson(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ buf, POp op) {
+  using T = XT<R, LX, FULL>;
+  using X = ZL<LX>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  constexpr int W = 3 * KC;
-  Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
-  Cx<R> *P = twx + g.NX;     // [NX][KC] charge, later FFT scratch
-  Cx<R> *U = P + g.NX * W;   // FFT scratch, later [NX][3*KC]
-  const int iy = blockIdx.x;
-  const int kz0 = blockIdx.y * KC;
-  const int ncol = min(KC, g.TZ - kz0);
-  const size_t cstr = (size_t)g.NX * g.KYc * g.TS;
-  load_twiddles(twx, tw.x, g.NX);
   buf = pdl_fresh(buf);
-  for (int it = threadIdx.x; it < g.NX * KC; it += blockDim.x) {
-    const int col = it % KC, x = it / KC;
-    if (col < ncol)
-      cp_async_cx(P + it, buf + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col);
-    else
-      P[it] = {R(0), R(0)};
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  fft2_smem<R, 1, KC>(P, U, g.lx, 1, KC, twx);
+  const int grp = T::group();
+  Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + grp * T::EX;
+  Cx<R> *S = reinterpret_cast<Cx<R> *>(smem_raw) + 3 * T::EX;  // [3 tiles][KXc][CW]
+  const int iy = blockIdx.y, kz0 = blockIdx.x * 3 * T::CW;
+  const size_t at = (size_t)iy * g.TS + kz0, row = (size_t)g.KYc * g.TS, cstr = (size_t)T::NX * row;
   const int KYi = signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY);
   const R ky = R(g.wave[1] * KYi);
-  for (int it = threadIdx.x; it < g.NX * KC; it += blockDim.x) {
-    const int col = it % KC, i = it / KC;
-    const int KXi = signed_k(i, g.NX), kz = kz0 + col;
-    Cx<R> o[3] = {{R(0), R(0)}, {R(0), R(0)}, {R(0), R(0)}};
-    if (col < ncol && (FULL || abs(KXi) < g.TX)) {
-      const R kk[3] = {R(g.wave[0] * KXi), ky, R(g.wave[2] * kz)};
-      const R k2 = kk[0] * kk[0] + kk[1] * kk[1] + kk[2] * kk[2];
-      const R s = k2 > R(0) ? R(op.a[0]) / k2 : R(0);
-      const Cx<R> v = {P[it].x * s, P[it].y * s};
+  auto ncol = [&](int tile) { return min(T::CW, g.TZ - kz0 - tile * T::CW); };
+  Cx<R> v[X::N1];
+  x_load<R, LX>(buf + at + grp * T::CW, row, ncol(grp), v);
+  xfft<R, LX, 1>(v, ex, tw.x);
+  x_put<R, LX, FULL>(S + grp * T::MODES, v);
+  __syncthreads();
+#pragma unroll 1
+  for (int tile = 0; tile < 3; ++tile) {
+    if (ncol(tile) <= 0) break;
+    x_get<R, LX, FULL>(S + tile * T::MODES, v);
 #pragma unroll
-      for (int d = 0; d < 3; ++d) o[d] = {kk[d] * v.y, -kk[d] * v.x};  // -i k v
-      if (!FULL && KXi == 0 && KYi == 0 && kz == 0)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) o[d] = {R(-op.e_amp[d]), R(0)};
+    for (int n1 = 0; n1 < X::N1; ++n1) {
+      const int i = T::t() + X::N2 * n1, KXi = signed_k(i, T::NX);
+      const int kz = kz0 + tile * T::CW + T::col();
+      const R kx = R(g.wave[0] * KXi), kzr = R(g.wave[2] * kz);
+      const R k2 = kx * kx + ky * ky + kzr * kzr, k = grp == 0 ? kx : grp == 1 ? ky : kzr;
+      const R s = k2 > R(0) ? R(op.a) / k2 : R(0);
+      const Cx<R> q = {v[n1].x * s, v[n1].y * s};
+      Cx<R> o = {k * q.y, -k * q.x};  // -i k q
+      if (!FULL && KXi == 0 && KYi == 0 && kz == 0) o = {R(-op.e_amp[grp]), R(0)};
       if (FULL && (kz == 0 || kz == g.M)) {
-        const int n1h = g.NX / 2, n2h = g.NY / 2;
+        const int n1h = T::NX / 2, n2h = g.NY / 2;
         const bool edge = iy == 0 || iy == n2h;
         const bool keep = kz == 0 ? ((iy > 0 && iy < n2h) || (edge && i <= n1h)) : (iy > n2h || (edge && i >= n1h));
-        const bool nyq[3] = {i == n1h, iy == n2h, kz == g.M};
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          if (!keep && nyq[d]) o[d] = {-o[d].x, -o[d].y};
-          if (edge && (i == 0 || i == n1h)) o[d].y = R(0);
-        }
+        const bool nyquist = grp == 0 ? i == n1h : grp == 1 ? iy == n2h : kz == g.M;
+        if (!keep && nyquist) o = {-o.x, -o.y};
+        if (edge && (i == 0 || i == n1h)) o.y = R(0);
       }
+      v[n1] = o;
     }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) U[i * W + d * KC + col] = o[d];
-  }
-  __syncthreads();
-  fft2_smem<R, -1, W>(U, P, g.lx, 1, W, twx);
-  for (int it = threadIdx.x; it < 3 * g.NX * KC; it += blockDim.x) {
-    const int col = it % KC, rest = it / KC, x = rest & (g.NX - 1), c = rest >> g.lx;
-    if (col < ncol) buf[c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col] = U[x * W + c * KC + col];
+    xfft<R, LX, -1>(v, ex, tw.x);
+    x_store<R, LX>(buf + grp * cstr + at + tile * T::CW, row, ncol(tile), v);
   }
 }
 
@@ -494,9 +458,11 @@ __global__ void k_scale_conc(size_t nz, Cx<R> *__restrict__ conc, const double *
 }
 
 // ---------------------------------------------------------------------------
-// z passes fused with the point operations between them (warp-level, one row
-// group of every component per task; zwarp_kernels.cuh).  The real fields that
-// a point operation reads or writes and nothing else needs are never stored.
+// z passes fused with the point operations between them (warp-level,
+// zwarp_kernels.cuh: a row group's elements stay in the same lanes from the
+// inverse transform through the point operation to the forward one).  The real
+// fields that a point operation reads or writes and nothing else needs are
+// never stored.
 
 // Charge field of a row group (k_el_charge's expression) and its forward z
 // transform, kz < TZ or all M + 1 (FULL) kept -> out [rows][TS].  The charge
@@ -509,27 +475,27 @@ __global__ void __launch_bounds__(NW * 32) k_zw_charge(Geo g, Twiddles<R> tw, co
   using Z = ZL<LM>;
   using V2 = typename Vec2<R>::T;
   constexpr int NK = FULL ? Z::M + 1 : Z::TZ, OS = (NK + 3) & ~3;
-  constexpr int NI = Z::RW * Z::M / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * Z::RW * Z::LS;
-  Cx<R> wf[Z::N1];
-  wfft_twiddles<R, LM, 1>(tw.m, wf);
   phiq = pdl_fresh(phiq);
   creal = pdl_fresh(creal);
   scal = pdl_fresh(scal);
-  charge = pdl_fresh(charge);
+  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
+  int turn = 0;
+  Cx<R> w[Z::N1], wz[Z::N1];
+  wfft_twiddles<R, LM>(tw.m, w);
+  wpack_twiddles<R, LM>(tw.z, wz);
   const R qs = R(scal[0]);
   const R f0 = use_fac ? R(scal[1]) : R(1), f1 = use_fac ? R(scal[2]) : R(1);
   const size_t rows = (size_t)g.NX * g.NY, n = rows * Z::NZ;
   const int ngroups = (int)(rows / Z::RW);
   for (int grp = blockIdx.x * nw + warp; grp < ngroups; grp += gridDim.x * nw) {
-    const size_t row0 = (size_t)grp * Z::RW;
-#pragma unroll 4
-    for (int h = 0; h < NI; ++h) {
-      const int i = lane + 32 * h, rr = i >> LM, m = i & (Z::M - 1);
-      const size_t o = row0 * Z::NZ + 2 * i;
+    const size_t row = (size_t)grp * Z::RW + wl<LM>();
+    Cx<R> v[Z::N1];
+#pragma unroll
+    for (int n1 = 0; n1 < Z::N1; ++n1) {
+      const size_t o = row * Z::NZ + 2 * (wt<LM>() + Z::N2 * n1);
       const V2 ph = *reinterpret_cast<const V2 *>(phiq + o), sf = *reinterpret_cast<const V2 *>(phiq + n + o);
       const V2 c0 = *reinterpret_cast<const V2 *>(creal + o), c1 = *reinterpret_cast<const V2 *>(creal + n + o);
       const R wx = R(1) - ph.x, wy = R(1) - ph.y;
@@ -539,22 +505,16 @@ __global__ void __launch_bounds__(NW * 32) k_zw_charge(Geo g, Twiddles<R> tw, co
       q.y += R(ve0) * (f0 * c0.y) * wy;
       q.y += R(ve1) * (f1 * c1.y) * wy;
       if (charge) *reinterpret_cast<V2 *>(charge + o) = q;
-      buf[rr * Z::LS + zpos<LM>(m)] = {q.x, q.y};
+      v[n1] = {q.x, q.y};
     }
-    __syncwarp();
-    wfft<R, LM, 1>(buf, wf);
-    Cx<R> *dst = out + row0 * OS;
-    for (int i = lane; i < Z::RW * NK; i += 32) {
-      const int rr = i / NK, k = i - rr * NK;
-      dst[rr * OS + k] = wunpack_r2c<R, LM>(buf + rr * Z::LS, k, tw.z);
-    }
-    __syncwarp();
+    wfft<R, LM, 1>(v, ex, turn, w);
+    wunpack_r2c<R, LM, NK>(v, out + row * OS, wz, tw.z);
   }
 }
 
-// Inverse z of three components in io[3 s ..], the point operation, forward z
-// in place: the ion flux of species s = task / groups (k_el_flux's
-// expressions; both species in one launch).
+// Inverse z of three components in io[3 s ..], the ion flux of species s =
+// task / groups (k_el_flux's expressions), forward z in place; both species
+// in one launch.
 struct FluxPar {
   double L[2], ve[2];
 };
@@ -565,37 +525,36 @@ __global__ void __launch_bounds__(NW * 32) k_zw_flux(Geo g, Twiddles<R> tw, Cx<R
                                                      FluxPar fp) {
   using Z = ZL<LM>;
   using V2 = typename Vec2<R>::T;
-  constexpr int GL = Z::RW * Z::LS, NI = Z::RW * Z::M / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * 3 * GL;
-  Cx<R> wi[Z::N1], wk[Z::KW];
-  wfft_twiddles<R, LM, -1>(tw.m, wi);
-  wpre_twiddles<R, LM>(tw.z, wk);
   io = pdl_fresh(io);
   creal = pdl_fresh(creal);
   grad = pdl_fresh(grad);
   normal = pdl_fresh(normal);
   u = pdl_fresh(u);
+  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
+  int turn = 0;
+  Cx<R> w[Z::N1], wz[Z::N1];
+  wfft_twiddles<R, LM>(tw.m, w);
+  wpack_twiddles<R, LM>(tw.z, wz);
   const size_t rows = (size_t)g.NX * g.NY, n = rows * Z::NZ, cstr = rows * Z::TS;
   const int ngroups = (int)(rows / Z::RW);
   const R sc = R(g.inv_n);
   for (int task = blockIdx.x * nw + warp; task < 2 * ngroups; task += gridDim.x * nw) {
     const int s = task >= ngroups;
-    const size_t row0 = (size_t)(task - s * ngroups) * Z::RW;
-    Cx<R> *row = io + 3 * s * cstr + row0 * Z::TS;
+    const size_t row = (size_t)(task - s * ngroups) * Z::RW + wl<LM>();
+    Cx<R> *line = io + 3 * s * cstr + row * Z::TS;
     const R L = R(fp.L[s]), ve = R(fp.ve[s]);
+    Cx<R> f[3][Z::N1];
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-      for (int rr = 0; rr < Z::RW; ++rr) wpack_c2r<R, LM>(row + c * cstr + rr * Z::TS, buf + c * GL + rr * Z::LS, wk);
-    __syncwarp();
+    for (int c = 0; c < 3; ++c) {
+      wpack_c2r<R, LM>(line + c * cstr, f[c], wz);
+      wfft<R, LM, -1>(f[c], ex, turn, w);
+    }
 #pragma unroll
-    for (int c = 0; c < 3; ++c) wfft<R, LM, -1>(buf + c * GL, wi);
-#pragma unroll 2
-    for (int h = 0; h < NI; ++h) {
-      const int i = lane + 32 * h, at = (i >> LM) * Z::LS + zpos<LM>(i & (Z::M - 1));
-      const size_t o = row0 * Z::NZ + 2 * i;
+    for (int n1 = 0; n1 < Z::N1; ++n1) {
+      const size_t o = row * Z::NZ + 2 * (wt<LM>() + Z::N2 * n1);
       const V2 c = *reinterpret_cast<const V2 *>(creal + s * n + o);
       V2 gr[3], nv[3], uv[3];
 #pragma unroll
@@ -604,36 +563,38 @@ __global__ void __launch_bounds__(NW * 32) k_zw_flux(Geo g, Twiddles<R> tw, Cx<R
         nv[d] = *reinterpret_cast<const V2 *>(normal + d * n + o);
         uv[d] = *reinterpret_cast<const V2 *>(u + d * n + o);
       }
-      Cx<R> f[3];
+      Cx<R> x[3];
       R nx = R(0), ny = R(0);
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        const Cx<R> df = buf[d * GL + at];
-        f[d] = {df.x * sc + c.x * (L * (gr[d].x * ve)), df.y * sc + c.y * (L * (gr[d].y * ve))};
+        x[d] = {f[d][n1].x * sc + c.x * (L * (gr[d].x * ve)), f[d][n1].y * sc + c.y * (L * (gr[d].y * ve))};
         nx += nv[d].x * nv[d].x;
         ny += nv[d].y * nv[d].y;
       }
       if (nx > R(0)) {
-        const R dm = (f[0].x * nv[0].x + f[1].x * nv[1].x + f[2].x * nv[2].x) / nx;
+        const R dm = (x[0].x * nv[0].x + x[1].x * nv[1].x + x[2].x * nv[2].x) / nx;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) f[d].x -= nv[d].x * dm;
+        for (int d = 0; d < 3; ++d) x[d].x -= nv[d].x * dm;
       }
       if (ny > R(0)) {
-        const R dm = (f[0].y * nv[0].y + f[1].y * nv[1].y + f[2].y * nv[2].y) / ny;
+        const R dm = (x[0].y * nv[0].y + x[1].y * nv[1].y + x[2].y * nv[2].y) / ny;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) f[d].y -= nv[d].y * dm;
+        for (int d = 0; d < 3; ++d) x[d].y -= nv[d].y * dm;
       }
 #pragma unroll
-      for (int d = 0; d < 3; ++d) buf[d * GL + at] = {f[d].x + c.x * -uv[d].x, f[d].y + c.y * -uv[d].y};
+      for (int d = 0; d < 3; ++d) f[d][n1] = {x[d].x + c.x * -uv[d].x, x[d].y + c.y * -uv[d].y};
     }
-    __syncwarp();
-    zw_forward3<R, LM>(buf, GL, tw, row, cstr);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      wfft<R, LM, 1>(f[c], ex, turn, w);
+      wunpack_r2c<R, LM>(f[c], line + c * cstr, wz, tw.z);
+    }
   }
 }
 
-// Inverse z of the full-spectrum potential gradient in[3][rows][OS], the
+// Inverse z of the full-spectrum potential gradient in[3][rows][IS], the
 // Coulomb force (k_el_coulomb's expressions), forward z, kz < TZ kept ->
-// out [3][rows][TS].
+// out [3][rows][TS].  Tasks (component, row group).
 template <typename R, int LM, int NW>
 __global__ void __launch_bounds__(NW * 32) k_zw_coulomb(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ in,
                                                         const R *__restrict__ charge, double e0, double e1, double e2,
@@ -641,43 +602,39 @@ __global__ void __launch_bounds__(NW * 32) k_zw_coulomb(Geo g, Twiddles<R> tw, c
   using Z = ZL<LM>;
   using V2 = typename Vec2<R>::T;
   constexpr int NK = Z::M + 1, IS = (NK + 3) & ~3;
-  constexpr int GL = Z::RW * Z::LS, NI = Z::RW * Z::M / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * 3 * GL;
-  Cx<R> wi[Z::N1], wk[Z::KW];
-  wfft_twiddles<R, LM, -1>(tw.m, wi);
-  wpre_twiddles<R, LM>(tw.z, wk);
   in = pdl_fresh(in);
   charge = pdl_fresh(charge);
-  const size_t rows = (size_t)g.NX * g.NY, cstr = rows * Z::TS;
+  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
+  int turn = 0;
+  Cx<R> w[Z::N1], wz[Z::N1];
+  wfft_twiddles<R, LM>(tw.m, w);
+  wpack_twiddles<R, LM>(tw.z, wz);
+  const size_t rows = (size_t)g.NX * g.NY;
   const int ngroups = (int)(rows / Z::RW);
-  const R sc = R(g.inv_n), e[3] = {R(e0), R(e1), R(e2)};
-  for (int grp = blockIdx.x * nw + warp; grp < ngroups; grp += gridDim.x * nw) {
-    const size_t row0 = (size_t)grp * Z::RW;
+  const R sc = R(g.inv_n);
+  for (int task = blockIdx.x * nw + warp; task < 3 * ngroups; task += gridDim.x * nw) {
+    const int c = task / ngroups;
+    const size_t row = (size_t)(task - c * ngroups) * Z::RW + wl<LM>();
+    const R e = R(c == 0 ? e0 : c == 1 ? e1 : e2);
+    Cx<R> v[Z::N1];
+    wpack_c2r<R, LM, NK>(in + (c * rows + row) * IS, v, wz);
+    V2 q[Z::N1];
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-      for (int rr = 0; rr < Z::RW; ++rr)
-        wpack_c2r<R, LM, NK>(in + (c * rows + row0 + rr) * IS, buf + c * GL + rr * Z::LS, wk);
-    __syncwarp();
+    for (int n1 = 0; n1 < Z::N1; ++n1)
+      q[n1] = *reinterpret_cast<const V2 *>(charge + row * Z::NZ + 2 * (wt<LM>() + Z::N2 * n1));
+    wfft<R, LM, -1>(v, ex, turn, w);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) wfft<R, LM, -1>(buf + c * GL, wi);
-#pragma unroll 4
-    for (int h = 0; h < NI; ++h) {
-      const int i = lane + 32 * h, at = (i >> LM) * Z::LS + zpos<LM>(i & (Z::M - 1));
-      const V2 q = *reinterpret_cast<const V2 *>(charge + row0 * Z::NZ + 2 * i);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const Cx<R> gr = buf[d * GL + at];
-        R fx = -(gr.x * sc), fy = -(gr.y * sc);
-        fx += e[d];
-        fy += e[d];
-        buf[d * GL + at] = {(q.x * fx) * R(scale), (q.y * fy) * R(scale)};
-      }
+    for (int n1 = 0; n1 < Z::N1; ++n1) {
+      R fx = -(v[n1].x * sc), fy = -(v[n1].y * sc);
+      fx += e;
+      fy += e;
+      v[n1] = {(q[n1].x * fx) * R(scale), (q[n1].y * fy) * R(scale)};
     }
-    __syncwarp();
-    zw_forward3<R, LM>(buf, GL, tw, out + row0 * Z::TS, cstr);
+    wfft<R, LM, 1>(v, ex, turn, w);
+    wunpack_r2c<R, LM>(v, out + (c * rows + row) * Z::TS, wz, tw.z);
   }
 }
 

@@ -128,12 +128,11 @@ __device__ __forceinline__ void cp_async_cx(Cx<R> *smem, const Cx<R> *gmem) {
 // launch now, then wait until the previous kernel has finished and its
 // writes are visible.  Both are no-ops when the kernel was launched without
 // the programmatic-serialization attribute.  It is the first statement of a
-// kernel: with constant loads (twiddles) placed between the two, loads of the
-// previous kernel's output through `const __restrict__` arguments, which the
-// compiler may take for memory that never changes while the kernel runs, were
-// moved up across the wait (wrong results).  Hiding every pointer from that
-// assumption made it correct again, and slower than this form (128^3 mixed
-// step 158 -> 160 us, 256^3 1813 -> 1877 us).
+// kernel, and every pointer to data of an earlier launch goes through
+// pdl_fresh after it: loads through a `__restrict__` argument that the kernel
+// does not write, which the compiler may take for memory that never changes
+// while the kernel runs, were moved up across the wait (wrong results; seen
+// with constant loads in front of the wait, and in an FP64 kernel without).
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

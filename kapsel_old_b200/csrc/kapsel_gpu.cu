@@ -30,6 +30,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/kapsel_gpu.h"
@@ -39,6 +40,7 @@
 #include "obl_kernels.cuh"
 #include "particle_kernels.cuh"
 #include "spectral_kernels.cuh"
+#include "xtile_kernels.cuh"
 #include "yz_kernels.cuh"
 #include "zwarp_kernels.cuh"
 
@@ -177,12 +179,20 @@ __global__ void k_col_pass(Geo g, const Cx<R> *twn, int logn, int n, const Cx<R>
 template <typename R>
 __global__ void k_z_c2r_full(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ in, R *__restrict__ out, double scale);
 
-// Kernel launch on `st`, optionally with programmatic stream serialization
-// (the kernel may start while its predecessor drains; it waits in pdl_begin).
+// How a step's kernels are launched: with programmatic stream serialization
+// (a kernel may start while its predecessor drains; it waits in pdl_begin),
+// and with a preferred split of the SM's memory into shared memory and L1 in
+// percent (-1: the driver's choice per kernel).
+struct Launch {
+  bool pdl;
+  int carve;
+  Launch(bool p = false, int c = -1) : pdl(p), carve(c) {}
+};
+// Kernel launch on `st`; `cluster` blocks along x form a cluster.
 template <typename... KArgs, typename... Args>
-void launch_k(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-              Args... args) {
-  if (!pdl) {
+void launch_kc(int cluster, Launch how, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+               Args... args) {
+  if (!how.pdl && how.carve < 0 && cluster == 1) {
     kern<<<grid, block, smem, st>>>(args...);
     return;
   }
@@ -191,12 +201,29 @@ void launch_k(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t sm
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[3];
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 0;
+  if (how.pdl) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (how.carve >= 0) {
+    at[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[cfg.numAttrs++].val.sharedMemCarveout = how.carve;
+  }
+  if (cluster > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs].val.clusterDim.x = cluster;
+    at[cfg.numAttrs].val.clusterDim.y = 1;
+    at[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
   cudaLaunchKernelEx(&cfg, kern, args...);
+}
+template <typename... KArgs, typename... Args>
+void launch_k(Launch how, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+              Args... args) {
+  launch_kc(1, how, kern, grid, block, smem, st, args...);
 }
 
 // ---------------------------------------------------------------------------
@@ -211,8 +238,6 @@ struct BoxBase {
   short4 *cells = nullptr;  // stencil offsets of the particle kernels (pp.S of them)
   double *uk_dc = nullptr;
   int *status = nullptr;
-  double *partial_p = nullptr;  // [Np][PCL][18] partial force sums
-  int *arrivals = nullptr;    // [Np] blocks done per particle (0 between launches)
   double *noise_dev[2] = {nullptr, nullptr};
   double *noise_host[2] = {nullptr, nullptr};
   cudaEvent_t noise_ev[2] = {nullptr, nullptr};
@@ -403,12 +428,6 @@ struct BoxBase {
 constexpr int kXZThreads = KAPSEL_XZ_THREADS, kXAdvThreads = KAPSEL_XADV_THREADS,
               kXForceThreads = KAPSEL_XFORCE_THREADS;
 
-// warps per block of the fused y/z plane kernels (FP32 fields; 4 measured
-// faster than 6 and 8 at 128^3: three 64 KB blocks per SM hold all 384
-// planes in one wave)
-#ifndef KAPSEL_YZ_NW
-#define KAPSEL_YZ_NW 4
-#endif
 
 template <typename R>
 struct Box : BoxBase {
@@ -428,91 +447,101 @@ struct Box : BoxBase {
   // (the Lees-Edwards step scatters phi and phi u_p into the whole of phiup)
   R *force() const { return phiup + npts(); }
 
-  // x passes with compile-time NX for NX = 32..256 (the runtime-NX kernels otherwise)
-  template <int LX, int XS>
-  int x_setup_s() {
-    KCHECK(allow_smem(k_x_zeta_to_u<R, KCX, LX, XS>, smem_xu));
-    KCHECK(allow_smem(k_x_advect_update<R, KCX, 0, LX, XS>, smem_xadv));
-    KCHECK(allow_smem(k_x_advect_update<R, KCX, 1, LX, XS>, smem_xadv));
-    KCHECK(allow_smem(k_x_force_to_zeta<R, KCX, LX, 0, XS>, smem_xf));
-    KCHECK(allow_smem(k_x_force_to_zeta<R, KCX, LX, 1, XS>, smem_xf));
-    return 0;
+  // calls f with the log2 of a line length as a compile-time constant
+  template <typename F>
+  static void with_len(int l, F f) {
+    switch (l) {
+      case 4: f(std::integral_constant<int, 4>()); break;
+      case 5: f(std::integral_constant<int, 5>()); break;
+      case 6: f(std::integral_constant<int, 6>()); break;
+      case 7: f(std::integral_constant<int, 7>()); break;
+      default: f(std::integral_constant<int, 8>());
+    }
   }
+  // x passes: the warp-level kernels, or with xsplit the block-level ones in
+  // the other radix split (NX = 16..128)
   template <int LX>
   int x_setup() {
-    const int rc = x_setup_s<LX, 0>();
-    return rc ? rc : x_setup_s<LX, 1>();
+    using T = XT<R, LX>;
+    KCHECK(allow_smem(k_xw_zeta_to_u<R, LX>, T::smem(3)));
+    KCHECK(allow_smem(k_xw_advect<R, LX, 0>, T::smem(5, 2)));
+    KCHECK(allow_smem(k_xw_advect<R, LX, 1>, T::smem(5, 2)));
+    KCHECK(allow_smem(k_xw_force<R, LX, 0>, T::smem(3, 2)));
+    KCHECK(allow_smem(k_xw_force<R, LX, 1>, T::smem(3, 2)));
+    if constexpr (LX < 8) {
+      KCHECK(allow_smem(k_x_zeta_to_u<R, KCX, LX, 1>, smem_xu));
+      KCHECK(allow_smem(k_x_advect_update<R, KCX, 0, LX, 1>, smem_xadv));
+      KCHECK(allow_smem(k_x_advect_update<R, KCX, 1, LX, 1>, smem_xadv));
+      KCHECK(allow_smem(k_x_force_to_zeta<R, KCX, LX, 0, 1>, smem_xf));
+      KCHECK(allow_smem(k_x_force_to_zeta<R, KCX, LX, 1, 1>, smem_xf));
+    }
+    return 0;
   }
-  // the x-pass launches, with the radix split of this context (xsplit)
+  // grid of a warp-level x pass over the retained kz of geometry gg
+  template <int LX, bool FULL = false>
+  static dim3 gxw(const Geo &gg) {
+    return dim3((gg.TZ + XT<R, LX, FULL>::CW - 1) / XT<R, LX, FULL>::CW, gg.KYc);
+  }
   template <int LX>
-  void xz_l(bool pdl, const Cx<R> *z, const double *u, Cx<R> *out) {
-    if (xsplit)
-      launch_k(pdl, k_x_zeta_to_u<R, KCX, LX, 1>, gx(), dim3(kXZThreads), smem_xu, stream, g, tw, z, u, out);
-    else
-      launch_k(pdl, k_x_zeta_to_u<R, KCX, LX, 0>, gx(), dim3(kXZThreads), smem_xu, stream, g, tw, z, u, out);
+  void xz_l(Launch pdl, const Cx<R> *z, const double *u, Cx<R> *out) {
+    if constexpr (LX < 8)
+      if (xsplit) {
+        launch_k(pdl, k_x_zeta_to_u<R, KCX, LX, 1>, gx(), dim3(kXZThreads), smem_xu, stream, g, tw, z, u, out);
+        return;
+      }
+    launch_k(pdl, k_xw_zeta_to_u<R, LX>, gxw<LX>(g), dim3(3 * XT<R, LX>::TPG), XT<R, LX>::smem(3), stream, g, tw, z, u, out);
   }
   template <int EU, int LX>
-  void xa_l(bool pdl) {
-    if (xsplit)
-      launch_k(pdl, k_x_advect_update<R, KCX, EU, LX, 1>, gx(), dim3(kXAdvThreads), smem_xadv, stream, g, tw, bufA,
-               zeta, uk_dc);
-    else
-      launch_k(pdl, k_x_advect_update<R, KCX, EU, LX, 0>, gx(), dim3(kXAdvThreads), smem_xadv, stream, g, tw, bufA,
-               zeta, uk_dc);
+  void xa_l(Launch pdl) {
+    if constexpr (LX < 8)
+      if (xsplit) {
+        launch_k(pdl, k_x_advect_update<R, KCX, EU, LX, 1>, gx(), dim3(kXAdvThreads), smem_xadv, stream, g, tw, bufA,
+                 zeta, uk_dc);
+        return;
+      }
+    launch_k(pdl, k_xw_advect<R, LX, EU>, gxw<LX>(g), dim3(5 * XT<R, LX>::TPG), XT<R, LX>::smem(5, 2), stream, g, tw, bufA, zeta,
+             uk_dc);
   }
-  template <int LX, int NEXTU = 0>
-  void xf_l(bool pdl, Cx<R> *in) {
-    if (xsplit)
-      launch_k(pdl, k_x_force_to_zeta<R, KCX, LX, NEXTU, 1>, gx(), dim3(kXForceThreads), smem_xf, stream, g, tw, in,
-               zeta, uk_dc);
-    else
-      launch_k(pdl, k_x_force_to_zeta<R, KCX, LX, NEXTU, 0>, gx(), dim3(kXForceThreads), smem_xf, stream, g, tw, in,
-               zeta, uk_dc);
+  template <int LX, int NEXTU>
+  void xf_l(Launch pdl, Cx<R> *in) {
+    if constexpr (LX < 8)
+      if (xsplit) {
+        launch_k(pdl, k_x_force_to_zeta<R, KCX, LX, NEXTU, 1>, gx(), dim3(kXForceThreads), smem_xf, stream, g, tw, in,
+                 zeta, uk_dc);
+        return;
+      }
+    launch_k(pdl, k_xw_force<R, LX, NEXTU>, gxw<LX>(g), dim3(3 * XT<R, LX>::TPG), XT<R, LX>::smem(3, 2), stream, g, tw, in, zeta,
+             uk_dc);
   }
-  void x_zeta(bool pdl, const Cx<R> *z, const double *u, Cx<R> *out) {
-    switch (g.NX) {
-      case 32: xz_l<5>(pdl, z, u, out); return;
-      case 64: xz_l<6>(pdl, z, u, out); return;
-      case 128: xz_l<7>(pdl, z, u, out); return;
-      case 256: xz_l<8>(pdl, z, u, out); return;
-      default: xz_l<0>(pdl, z, u, out);
-    }
+  void x_zeta(Launch pdl, const Cx<R> *z, const double *u, Cx<R> *out) {
+    with_len(g.lx, [&](auto l) { xz_l<l.value>(pdl, z, u, out); });
   }
   template <int EU>
-  void x_advect(bool pdl) {
-    switch (g.NX) {
-      case 32: xa_l<EU, 5>(pdl); return;
-      case 64: xa_l<EU, 6>(pdl); return;
-      case 128: xa_l<EU, 7>(pdl); return;
-      case 256: xa_l<EU, 8>(pdl); return;
-      default: xa_l<EU, 0>(pdl);
-    }
+  void x_advect(Launch pdl) {
+    with_len(g.lx, [&](auto l) { xa_l<EU, l.value>(pdl); });
   }
-  void x_force(bool pdl, Cx<R> *in) {
-    switch (g.NX) {
-      case 32: xf_l<5>(pdl, in); return;
-      case 64: xf_l<6>(pdl, in); return;
-      case 128: xf_l<7>(pdl, in); return;
-      case 256: xf_l<8>(pdl, in); return;
-      default: xf_l<0>(pdl, in);
-    }
+  void x_force(Launch pdl, Cx<R> *in) {
+    with_len(g.lx, [&](auto l) { xf_l<l.value, 0>(pdl, in); });
   }
   // the same, followed on each tile by the next step's first x pass (u_k of
   // the updated zeta into bufA)
-  void x_force_next(bool pdl) {
-    switch (g.NX) {
-      case 32: xf_l<5, 1>(pdl, bufA); return;
-      case 64: xf_l<6, 1>(pdl, bufA); return;
-      case 128: xf_l<7, 1>(pdl, bufA); return;
-      case 256: xf_l<8, 1>(pdl, bufA); return;
-      default: xf_l<0, 1>(pdl, bufA);
-    }
+  void x_force_next(Launch pdl) {
+    with_len(g.lx, [&](auto l) { xf_l<l.value, 1>(pdl, bufA); });
   }
 
-  // warp-level z kernels for NZ = 64, 128, 256 (zw = log2(NZ/2)); 0: block-level
+  // warp-level z kernels for NZ = 32..256 (zw = log2(NZ/2)); 0: block-level
   int nsm = 0;
-  static constexpr int ZNW = sizeof(R) == 4 ? 8 : 4;  // warps per block at most
+  static constexpr int ZNW = 4;  // warps per block (fewer where shared memory does not hold them)
   int zw = 0;
+  template <typename F>
+  static void with_zlen(int lm, F f) {
+    switch (lm) {
+      case 4: f(std::integral_constant<int, 4>()); break;
+      case 5: f(std::integral_constant<int, 5>()); break;
+      case 6: f(std::integral_constant<int, 6>()); break;
+      default: f(std::integral_constant<int, 7>());
+    }
+  }
   // launch shape of a warp-level z kernel
   struct ZPlan {
     int nw = 0, cap = 0;  // warps per block; blocks the GPU holds at once
@@ -539,22 +568,20 @@ struct Box : BoxBase {
   template <int LM>
   int zw_setup() {
     using Z = ZL<LM>;
-    const size_t line = sizeof(Cx<R>) * Z::RW * Z::LS;  // one line group
-    // FP64: the prefetching products kernel; FP32: four line groups per warp
-    const size_t prod = sizeof(R) == 8 ? sizeof(Cx<R>) * (size_t)ZProd<R, LM>::WARP : 4 * line;
-    int rc = zplan(sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW> : k_zw_products<R, LM, ZNW>, prod, zp_p);
-    if (!rc) rc = zplan(k_zw_c2r<R, LM, ZNW>, line, zp_c);
-    if (!rc) rc = zplan(k_zw_r2c<R, LM, ZNW, true, false>, line, zp_f);
+    const size_t ex = ZX<R, LM>::BYTES;  // exchange buffers of a warp
+    int rc = zplan(k_zw_products<R, LM, ZNW>, zw_products_bytes<R, LM>(), zp_p);
+    if (!rc) rc = zplan(k_zw_c2r<R, LM, ZNW>, ex, zp_c);
+    if (!rc) rc = zplan(k_zw_r2c<R, LM, ZNW, true, false>, ex, zp_f);
     if (!rc && prm.eq == KAPSEL_EQ_ELECTROLYTE) {
-      rc = zplan(sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW, true> : k_zw_products<R, LM, ZNW, true>, prod, zp_pu);
-      if (!rc) rc = zplan(k_zw_charge<R, LM, ZNW, false>, line, zp_q);
-      if (!rc) rc = zplan(k_zw_charge<R, LM, ZNW, true>, line, zp_qf);
-      if (!rc) rc = zplan(k_zw_flux<R, LM, ZNW>, 3 * line, zp_fl);
-      if (!rc) rc = zplan(k_zw_coulomb<R, LM, ZNW>, 3 * line, zp_cb);
+      rc = zplan(k_zw_products<R, LM, ZNW, true>, zw_products_bytes<R, LM>(), zp_pu);
+      if (!rc) rc = zplan(k_zw_charge<R, LM, ZNW, false>, ex, zp_q);
+      if (!rc) rc = zplan(k_zw_charge<R, LM, ZNW, true>, ex, zp_qf);
+      if (!rc) rc = zplan(k_zw_flux<R, LM, ZNW>, ex, zp_fl);
+      if (!rc) rc = zplan(k_zw_coulomb<R, LM, ZNW>, ex, zp_cb);
     }
     if (!rc && prm.eq == KAPSEL_EQ_SHEAR_LE) {
-      rc = zplan(k_zw_cross<R, LM, ZNW>, 6 * line, zp_x);
-      if (!rc) rc = zplan(k_zw_obl_force<R, LM, ZNW>, 3 * line, zp_of);
+      rc = zplan(k_zw_cross<R, LM, ZNW>, zw_cross_bytes<R, LM>(), zp_x);
+      if (!rc) rc = zplan(k_zw_obl_force<R, LM, ZNW>, ex, zp_of);
     }
     if (rc) return rc;
     zw = LM;
@@ -569,57 +596,53 @@ struct Box : BoxBase {
 
   // fused y/z plane kernels (pass variant ymode 3): the inverse to u* and the
   // rigidity force as one launch each, for NY = 2^yz_ly (0: not available)
-  static constexpr int YZNW = sizeof(R) == 4 ? KAPSEL_YZ_NW : 4;  // warps per block
+  static constexpr int YZNW = 4;  // warps per block
   int yz_ly = 0;
   size_t yz_sm = 0;
   template <int LY, int LM>
   int yz_setup() {
     const size_t sm = YZ<R, LY, LM>::smem(YZNW);
     if (sm > 227 * 1024) return 0;
-    KCHECK(allow_smem(k_yzw_c2r<R, LY, LM, false, YZNW>, sm));
+    KCHECK(allow_smem(k_yzw_c2r<R, LY, LM, YZNW>, sm));
     KCHECK(allow_smem(k_zyw_r2c<R, LY, LM, true, YZNW>, sm));
     yz_sm = sm;
     yz_ly = LY;
     return 0;
   }
   template <int LY, int LM>
-  void yz_c2r_l(bool pdl, R *out, DPart *pts, int euler) {
+  void yz_c2r_l(Launch pdl, R *out, DPart *pts, int euler) {
     const int posblk = pts ? (Np + YZNW * 32 - 1) / (YZNW * 32) : 0;
-    launch_k(pdl, k_yzw_c2r<R, LY, LM, false, YZNW>, dim3(3 * g.NX + posblk), dim3(YZNW * 32), yz_sm, stream, g, tw,
+    launch_k(pdl, k_yzw_c2r<R, LY, LM, YZNW>, dim3(3 * g.NX + posblk), dim3(YZNW * 32), yz_sm, stream, g, tw,
              (const Cx<R> *)bufA, out, npts(), g.NZ, 3 * g.NX, pp, pts, euler, status);
   }
   template <int LY, int LM>
-  void zy_force_l(bool pdl) {
+  void zy_force_l(Launch pdl) {
     launch_k(pdl, k_zyw_r2c<R, LY, LM, true, YZNW>, dim3(3 * g.NX), dim3(YZNW * 32), yz_sm, stream, g, tw, force(),
              npts(), bufA);
   }
   // bufA (x real, ky compact) -> real fields, with the position update in extra blocks
   template <int LM>
-  void yz_c2r_m(bool pdl, R *out, DPart *pts, int euler) {
+  void yz_c2r_m(Launch pdl, R *out, DPart *pts, int euler) {
     if (yz_ly == 5) yz_c2r_l<5, LM>(pdl, out, pts, euler);
     else if (yz_ly == 6) yz_c2r_l<6, LM>(pdl, out, pts, euler);
     else yz_c2r_l<7, LM>(pdl, out, pts, euler);
   }
-  void yz_c2r(bool pdl, R *out, DPart *pts, int euler) {
-    if (zw == 5) yz_c2r_m<5>(pdl, out, pts, euler);
-    else if (zw == 6) yz_c2r_m<6>(pdl, out, pts, euler);
-    else yz_c2r_m<7>(pdl, out, pts, euler);
+  void yz_c2r(Launch pdl, R *out, DPart *pts, int euler) {
+    with_zlen(zw, [&](auto l) { yz_c2r_m<l.value>(pdl, out, pts, euler); });
   }
   // rigidity force -> its spectra in bufA (x real, ky compact)
   template <int LM>
-  void zy_force_m(bool pdl) {
+  void zy_force_m(Launch pdl) {
     if (yz_ly == 5) zy_force_l<5, LM>(pdl);
     else if (yz_ly == 6) zy_force_l<6, LM>(pdl);
     else zy_force_l<7, LM>(pdl);
   }
-  void zy_force(bool pdl) {
-    if (zw == 5) zy_force_m<5>(pdl);
-    else if (zw == 6) zy_force_m<6>(pdl);
-    else zy_force_m<7>(pdl);
+  void zy_force(Launch pdl) {
+    with_zlen(zw, [&](auto l) { zy_force_m<l.value>(pdl); });
   }
   template <int LM>
-  void zw_products(bool pdl) {
-    launch_k(pdl, sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW> : k_zw_products<R, LM, ZNW>,
+  void zw_products(Launch pdl) {
+    launch_k(pdl, k_zw_products<R, LM, ZNW>,
              dim3(zp_p.grid(zgroups<LM>())), dim3(zp_p.nw * 32), zp_p.sm, stream, g, tw, bufB, (R *)nullptr);
   }
   template <int LM>
@@ -627,47 +650,44 @@ struct Box : BoxBase {
     return g.NX * g.NY / ZL<LM>::RW;
   }
   template <int LM>
-  void zw_c2r(bool pdl, int nc, R *out, DPart *pts, int euler) {
+  void zw_c2r(Launch pdl, int nc, R *out, DPart *pts, int euler) {
     const int nblk = zp_c.grid(nc * zgroups<LM>());
     const int posblk = pts ? (Np + zp_c.nw * 32 - 1) / (zp_c.nw * 32) : 0;
     launch_k(pdl, k_zw_c2r<R, LM, ZNW>, dim3(nblk + posblk), dim3(zp_c.nw * 32), zp_c.sm, stream, g, tw,
              (const Cx<R> *)bufB, out, npts(), g.NZ, nc, nblk, pp, pts, euler, status);
   }
   template <int LM>
-  void zw_force(bool pdl) {
+  void zw_force(Launch pdl) {
     launch_k(pdl, k_zw_r2c<R, LM, ZNW, true, false>, dim3(zp_f.grid(3 * zgroups<LM>())), dim3(zp_f.nw * 32), zp_f.sm,
              stream, g, tw, force(), npts(), bufB, 3);
   }
   // dispatch on the compile-time line length
-  void zdisp_products(bool pdl) {
-    if (zw == 5) zw_products<5>(pdl);
-    else if (zw == 6) zw_products<6>(pdl);
-    else if (zw == 7) zw_products<7>(pdl);
+  void zdisp_products(Launch pdl) {
+    if (zw)
+      with_zlen(zw, [&](auto l) { zw_products<l.value>(pdl); });
     else launch_k(pdl, k_z_products<R>, dim3(gz()), dim3(256), smem_zp, stream, g, tw, bufB);
   }
   // z c2r of nc components in bufB into real fields, with the position update
   // in extra blocks when pts is not null
-  void zdisp_c2r(bool pdl, int nc, R *out, DPart *pts, int euler) {
-    if (zw == 5) zw_c2r<5>(pdl, nc, out, pts, euler);
-    else if (zw == 6) zw_c2r<6>(pdl, nc, out, pts, euler);
-    else if (zw == 7) zw_c2r<7>(pdl, nc, out, pts, euler);
+  void zdisp_c2r(Launch pdl, int nc, R *out, DPart *pts, int euler) {
+    if (zw)
+      with_zlen(zw, [&](auto l) { zw_c2r<l.value>(pdl, nc, out, pts, euler); });
     else {
       const int posblk = pts ? (Np + 255) / 256 : 0;
       launch_k(pdl, k_z_c2r<R>, dim3(gz() + posblk, nc), dim3(256), smem_zc, stream, g, tw, (const Cx<R> *)bufB, out,
                npts(), g.NZ, pp, pts, euler, status);
     }
   }
-  void zdisp_force(bool pdl) {
-    if (zw == 5) zw_force<5>(pdl);
-    else if (zw == 6) zw_force<6>(pdl);
-    else if (zw == 7) zw_force<7>(pdl);
+  void zdisp_force(Launch pdl) {
+    if (zw)
+      with_zlen(zw, [&](auto l) { zw_force<l.value>(pdl); });
     else launch_k(pdl, k_z_force<R>, dim3(gz()), dim3(256), smem_zf, stream, g, tw, force(), bufB);
   }
   // inverse y and z of three spectra in bufA (x real) into real fields: one
   // launch over planes where the plane kernels are on (pass variant y = 3),
   // else two
   bool planes() const { return ymode == 3 && zw && yz_ly; }
-  void inverse3(bool pdl, R *out, DPart *pts = nullptr, int euler = 0) {
+  void inverse3(Launch pdl, R *out, DPart *pts = nullptr, int euler = 0) {
     if (planes()) {
       yz_c2r(pdl, out, pts, euler);
     } else {
@@ -676,7 +696,7 @@ struct Box : BoxBase {
     }
   }
   // forward z and y of the rigidity force into bufA (x real)
-  void forward_force(bool pdl) {
+  void forward_force(Launch pdl) {
     if (planes()) {
       zy_force(pdl);
     } else {
@@ -733,33 +753,36 @@ struct Box : BoxBase {
     if (smem_xadv > mx || smem_xu > mx || smem_y > mx || smem_zp > mx) return KAPSEL_ERANGE;
     {
       int rc = 0;
-      // the warp-level z kernels give one row group to a warp: below about
-      // 16 groups per SM (64^3 and smaller) the block-level kernels, which
-      // spread a row group over a whole block, keep more of the GPU busy
-      const bool zw_ok = (size_t)g.NX * g.NY >= 16384;
-      if (g.NX == 32) rc = x_setup<5>();
-      else if (g.NX == 64) rc = x_setup<6>();
-      else if (g.NX == 128) rc = x_setup<7>();
-      else if (g.NX == 256) rc = x_setup<8>();
+      with_len(g.lx, [&](auto l) { rc = x_setup<l.value>(); });
       if (rc) return rc;
-      if (g.NZ == 64) rc = zw_setup<5>();
-      else if (g.NZ == 128) rc = zw_setup<6>();
-      else if (g.NZ == 256) rc = zw_setup<7>();
+      if (g.NZ >= 32) with_zlen(g.lm, [&](auto l) { rc = zw_setup<l.value>(); });
       if (rc) return rc;
-      // warp-level z kernels by default only where they fill the GPU (the
-      // batch autotuner may choose otherwise per box shape)
+      // The warp-level z kernels wherever they exist, and the y/z plane
+      // kernels wherever a plane fits in shared memory and an SM holds more
+      // than one (steps in us with block-level z passes, with warp-level ones,
+      // with plane kernels: 64^3 FP32 54.2, 48.7, 43.1; FP64 73.4, 61.6, 59.6;
+      // 64x64x128 FP32 74.9, 60.6, 59.8; 32^3 37.8, 35.2, 33.5; 128x128x64
+      // 121, 95, 88; 128^3 FP32 181, 122, 124; FP64 343, 246, 235; 256x128x128
+      // 334, 207, 202; but 128x128x256 309, 208, 219, 64x64x256 107, 72, 75).
+      // The batch autotuner may choose otherwise for a box shape.
       zw_avail = zw;
-      if (!zw_ok) zw = 0;
-      // FP32: the fused y/z plane kernels wherever the warp-level z kernels
-      // run and three plane blocks fit on an SM (128^3 mixed step 0.200 ->
-      // 0.189 ms; 256x128x128 0.335 -> 0.316; at 128x128x256, one block per
-      // SM, 0.377 -> 0.395, so not there); FP64 planes (90 KB at 128^3)
-      // leave one block per SM and run slower than the separate passes
-      if (sizeof(R) == 4 && zw && yz_ly && 3 * yz_sm <= 227 * 1024) ymode = 3;
-    }
-    {
-      const int rc = x_setup<0>();
-      if (rc) return rc;
+      // A step's kernels want different amounts of shared memory, and an SM
+      // changes its split only when it is empty, so that a kernel with
+      // another split cannot start in the tail of the one before it.  In a
+      // small box, whose kernels are all tail, one split for all is faster;
+      // in a larger one the blocks per SM that each kernel's own split gives
+      // it count for more.  Steps in us with each kernel's own split and with
+      // 25, 45 and 70% shared memory: 64^3 FP32 49, 45, 43, 51; FP64 68, 60,
+      // 59, 65; electrolyte 64^3 FP32 194, 152, 173, 171, FP64 280, 216, 226,
+      // 230; Lees-Edwards 64^3 79, 72, 70, 76; 64x64x128 65, 60, 59, 61;
+      // 128x64x128 84, 87, 73, 75; 128^3 125, 153, 133, 124; electrolyte 128^3
+      // 446, 533, 450, 423; Lees-Edwards 128^3 203, 231, 204, 198; but 128^3
+      // FP64 235, 273, 240, 240 and 256^3 1198, 1505, 1248, 1377.
+      if (npts() <= (size_t)1 << 19)
+        carve = prm.eq == KAPSEL_EQ_ELECTROLYTE ? 25 : 45;
+      else if (npts() <= (size_t)1 << 21 && sizeof(R) == 4)
+        carve = 70;
+      if (zw && yz_ly && !(sizeof(R) == 4 && g.NZ == 256)) ymode = 3;
     }
     KCHECK(allow_smem(k_y_pass<R, true, KCY>, smem_y));
     KCHECK(allow_smem(k_y_pass<R, false, KCY>, smem_y));
@@ -782,30 +805,16 @@ struct Box : BoxBase {
   // y-pass tile width: KCY, or KCY/2 when the autotuner found it faster for
   // this box shape (kapsel_batch_create)
   bool use_pdl = true;
-  // warp-level y pass: persistent grid of YNW-warp blocks, two slots per warp
-  static constexpr int YNW = 4;
-  static constexpr int YSLOTS = sizeof(R) == 4 ? 1 : 2;
-  int yw_occ[2][2] = {{0, 0}, {0, 0}};  // blocks per SM, [inverse][full spectrum]
+  int carve = -1;  // see Launch
+  Launch how() const { return Launch(use_pdl, carve); }
   template <bool INV, int LY, bool FULL>
-  void yw_launch(const Geo &gg, int nc, const Cx<R> *in, Cx<R> *out, bool pdl) {
-    using Y = ZL<LY>;
-    auto kern = k_yw_pass<R, INV, LY, FULL, YNW, YSLOTS>;
-    const size_t sm = sizeof(Cx<R>) * YSLOTS * Y::RW * YLines<R, LY>::LS * YNW;
-    int &occ = yw_occ[INV ? 1 : 0][FULL ? 1 : 0];
-    if (!occ) {
-      int dev = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-      allow_smem(kern, sm);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, YNW * 32, sm);
-      occ = std::max(occ, 1);
-    }
-    const int items = nc * gg.NX * ((gg.TZ + Y::RW - 1) / Y::RW);
-    const int grid = std::min((items + YNW - 1) / YNW, occ * nsm);
-    launch_k(pdl, kern, dim3(grid), dim3(YNW * 32), sm, stream, gg, tw, in, out, nc);
+  void yw_launch(const Geo &gg, int nc, const Cx<R> *in, Cx<R> *out, Launch pdl) {
+    constexpr int CW = y_cols<R, LY>();
+    launch_k(pdl, k_yt_pass<R, INV, LY, FULL, CW>, dim3((gg.TZ + CW - 1) / CW, nc * gg.NX), dim3(CW * ZL<LY>::N2), 0,
+             stream, gg, tw, in, out);
   }
   template <bool INV, int LY>
-  void yw(const Geo &gg, int nc, const Cx<R> *in, Cx<R> *out, bool pdl) {
+  void yw(const Geo &gg, int nc, const Cx<R> *in, Cx<R> *out, Launch pdl) {
     if (gg.KYc == gg.NY)
       yw_launch<INV, LY, true>(gg, nc, in, out, pdl);
     else
@@ -814,7 +823,7 @@ struct Box : BoxBase {
   int ymode = 0;   // y pass variant (time_variant)
   int zw_avail = 0;  // warp-level z kernels set up for this NZ (their line-length log), else 0
   template <bool INV>
-  void launch_y(const Geo &gg, int nc, const Cx<R> *in, Cx<R> *out, bool pdl = false) {
+  void launch_y(const Geo &gg, int nc, const Cx<R> *in, Cx<R> *out, Launch pdl = Launch()) {
     if (ymode == 0 || ymode == 3) switch (gg.NY) {
       case 32: yw<INV, 5>(gg, nc, in, out, pdl); return;
       case 64: yw<INV, 6>(gg, nc, in, out, pdl); return;
@@ -919,7 +928,7 @@ struct Box : BoxBase {
   }
 
   // f -> zeta update, launches 11-13
-  void launch_force_to_zeta(bool pdl = false) {
+  void launch_force_to_zeta(Launch pdl = Launch()) {
     forward_force(pdl);
     x_force(pdl, bufA);
   }
@@ -937,7 +946,7 @@ struct Box : BoxBase {
     auto mark = [&]() {
       if (ev) cudaEventRecord(ev[e++], stream);
     };
-    const bool pdl = use_pdl && !ev;  // events between launches break the programmatic chain
+    const Launch pdl = ev ? Launch() : how();  // events between launches break the programmatic chain
     const Cx<R> *czeta = zeta;
     // the fused path starts at the y pass: the previous step's last launch
     // (or ensure_u_spec) left u_k in bufA; profiling times every launch
@@ -971,9 +980,9 @@ struct Box : BoxBase {
       launch_cells();  // neighbour lists of the new positions (large particle counts)
       mark();
       if (nc) launch_nearcontact();  // timed with the position slot when profiling
-      launch_k(pdl, k_particles_hydro_velocity<R>, dim3(Np * pp.hyd_pcl), dim3(pp.hyd_threads), 0, stream, pp, parts,
-               (const R *)ustar, (const short4 *)cells, noise, euler, status, partial_p, arrivals,
-               nc ? nc_corr : (double *)nullptr, ovl);
+      launch_kc(pp.hyd_pcl, pdl, k_particles_hydro_velocity<R>, dim3(Np * pp.hyd_pcl), dim3(pp.hyd_threads), 0,
+                stream, pp, parts, (const R *)ustar, (const short4 *)cells, noise, euler, status,
+                nc ? nc_corr : (double *)nullptr, ovl);
       mark();
       launch_k(pdl, k_particles_scatter<R, true>, dim3(Np * pp.sc_pcl), dim3(256), 0, stream, pp, (const DPart *)parts,
                (const short4 *)cells, force(), (const R *)ustar, status, (const unsigned *)ovl);
@@ -1021,54 +1030,48 @@ struct Box : BoxBase {
   R *obB = nullptr;        // [3][N]: contravariant u on the oblique grid
   double *obst = nullptr;  // degree_oblique, Shear_rate_eff, ... (obl_kernels.cuh)
   OblPar op{};
-  size_t sm_xo6 = 0, sm_xoa = 0, sm_xof = 0;
   template <int LX>
   int obl_x_setup() {
-    KCHECK(allow_smem(k_x_obl_inv<R, KCX, LX>, sm_xo6));
-    KCHECK(allow_smem(k_x_obl_update<R, KCX, 1, LX>, sm_xoa));
-    KCHECK(allow_smem(k_x_obl_update<R, KCX, 0, LX>, sm_xof));
+    using T = XT<R, LX>;
+    KCHECK(allow_smem(k_x_obl_inv<R, LX>, T::smem(6)));
+    KCHECK(allow_smem(k_x_obl_update<R, LX, 1>, T::smem(3, 2)));
+    KCHECK(allow_smem(k_x_obl_update<R, LX, 0>, T::smem(3)));
     return 0;
   }
   // the x passes with compile-time NX: 0 the first inverse, 1 the advection
   // update, 2 the end of the step
   template <int LX>
-  void obl_x_l(bool pdl, int which) {
+  void obl_x_l(Launch pdl, int which) {
+    using T = XT<R, LX>;
     if (which == 0)
-      launch_k(pdl, k_x_obl_inv<R, KCX, LX>, gx(), dim3(256), sm_xo6, stream, g, tw, (const Cx<R> *)zeta,
+      launch_k(pdl, k_x_obl_inv<R, LX>, gxw<LX>(g), dim3(6 * XT<R, LX>::TPG), T::smem(6), stream, g, tw, (const Cx<R> *)zeta,
                (const double *)uk_dc, (const double *)obst, bufA);
     else if (which == 1)
-      launch_k(pdl, k_x_obl_update<R, KCX, 1, LX>, gx(), dim3(256), sm_xoa, stream, g, tw, bufA, zeta, uk_dc,
+      launch_k(pdl, k_x_obl_update<R, LX, 1>, gxw<LX>(g), dim3(3 * XT<R, LX>::TPG), T::smem(3, 2), stream, g, tw, bufA, zeta, uk_dc,
                (const double *)obst);
     else
-      launch_k(pdl, k_x_obl_update<R, KCX, 0, LX>, gx(), dim3(256), sm_xof, stream, g, tw, bufA, zeta, uk_dc,
+      launch_k(pdl, k_x_obl_update<R, LX, 0>, gxw<LX>(g), dim3(3 * XT<R, LX>::TPG), T::smem(3), stream, g, tw, bufA, zeta, uk_dc,
                (const double *)obst);
   }
-  void obl_x(bool pdl, int which) {
-    switch (g.NX) {
-      case 32: obl_x_l<5>(pdl, which); return;
-      case 64: obl_x_l<6>(pdl, which); return;
-      case 128: obl_x_l<7>(pdl, which); return;
-      case 256: obl_x_l<8>(pdl, which); return;
-      default: obl_x_l<0>(pdl, which);
-    }
+  void obl_x(Launch pdl, int which) {
+    with_len(g.lx, [&](auto l) { obl_x_l<l.value>(pdl, which); });
   }
   template <int LM>
-  void zw_cross(bool pdl) {
+  void zw_cross(Launch pdl) {
     launch_k(pdl, k_zw_cross<R, LM, ZNW>, dim3(zp_x.grid(zgroups<LM>())), dim3(zp_x.nw * 32), zp_x.sm, stream, g, tw,
              bufB);
   }
   template <int LM>
-  void zw_obl_force(bool pdl) {
+  void zw_obl_force(Launch pdl) {
     launch_k(pdl, k_zw_obl_force<R, LM, ZNW>, dim3(zp_of.grid(zgroups<LM>())), dim3(zp_of.nw * 32), zp_of.sm, stream,
              g, tw, op, (const double *)obst, (const R *)phiup, (const R *)ustar, (const R *)ob6, bufB);
   }
   // bufB: inverse z of u and the vorticity, u x omega, forward z.  One launch
   // where the warp-level z kernels exist for this NZ.
-  void obl_cross_z(bool pdl) {
+  void obl_cross_z(Launch pdl) {
     const size_t N = npts();
-    if (zw_avail == 5) zw_cross<5>(pdl);
-    else if (zw_avail == 6) zw_cross<6>(pdl);
-    else if (zw_avail == 7) zw_cross<7>(pdl);
+    if (zw_avail)
+      with_zlen(zw_avail, [&](auto l) { zw_cross<l.value>(pdl); });
     else {
       launch_k(pdl, k_z_c2r<R>, dim3(gz(), 6), dim3(256), smem_zc, stream, g, tw, (const Cx<R> *)bufB, ob6, N, g.NZ,
                PPar{}, (DPart *)nullptr, 0, (int *)nullptr);
@@ -1079,12 +1082,10 @@ struct Box : BoxBase {
   }
   // f = up - phi u (Cartesian), u += U2u_oblique(f), forward z into bufB, and
   // phi/up back to zero
-  void obl_force_z(bool pdl) {
+  void obl_force_z(Launch pdl) {
     const size_t N = npts();
     if (zw_avail) {
-      if (zw_avail == 5) zw_obl_force<5>(pdl);
-      else if (zw_avail == 6) zw_obl_force<6>(pdl);
-      else zw_obl_force<7>(pdl);
+      with_zlen(zw_avail, [&](auto l) { zw_obl_force<l.value>(pdl); });
       if (Np > 0)
         launch_k(pdl, k_obl_clear<R>, dim3(Np * PCL), dim3(256), 0, stream, pp, (const DPart *)parts,
                  (const short4 *)cells, (const double *)obst, phiup);
@@ -1105,19 +1106,9 @@ struct Box : BoxBase {
     KCHECK(cudaMemset(ob6, 0, sizeof(R) * 6 * N));
     KCHECK(cudaMemset(obB, 0, sizeof(R) * 3 * N));
     KCHECK(cudaMemset(obst, 0, sizeof(double) * nst));
-    const size_t C = sizeof(Cx<R>);
-    sm_xo6 = C * (g.NX + (size_t)2 * g.KXc * KCX + (size_t)2 * g.NX * 6 * KCX);
-    sm_xoa = C * (g.NX + (size_t)2 * g.KXc * KCX + (size_t)2 * g.NX * 3 * KCX);
-    sm_xof = C * (g.NX + (size_t)2 * g.NX * 3 * KCX);
-    if (sm_xo6 > 227 * 1024 || smem_zc > 227 * 1024) return KAPSEL_ERANGE;
+    if (smem_zc > 227 * 1024) return KAPSEL_ERANGE;
     int rc = 0;
-    switch (g.NX) {
-      case 32: rc = obl_x_setup<5>(); break;
-      case 64: rc = obl_x_setup<6>(); break;
-      case 128: rc = obl_x_setup<7>(); break;
-      case 256: rc = obl_x_setup<8>(); break;
-      default: rc = obl_x_setup<0>();
-    }
+    with_len(g.lx, [&](auto l) { rc = obl_x_setup<l.value>(); });
     if (rc) return rc;
     KCHECK(allow_smem(k_z_r2c<R>, smem_zc));
     op.shear_rate = prm.shear_rate;
@@ -1135,7 +1126,7 @@ struct Box : BoxBase {
 
   // Time_evolution_hydro_OBL (sp_3d_ns.cxx:214-390).
   void launch_step_obl(const double *noise, int euler) {
-    const bool pdl = use_pdl;
+    const Launch pdl = how();
     // NS_solver_slavedEuler_Shear_OBL: u and omega of the truncated zeta, u x omega,
     // forward, shear correction, curl and the slaved-Euler step; then FIX_CELL on
     // uk_dc, u = Zeta_k2u_k_OBL(zeta, uk_dc), A_k2a
@@ -1216,55 +1207,64 @@ struct Box : BoxBase {
     KCHECK(cudaMalloc(&total_solute, sizeof(double) * 2));
     KCHECK(cudaMemset(conc_k, 0, sizeof(Cx<R>) * 2 * nz));
     KCHECK(cudaMemset(scal, 0, sizeof(double) * 8));
-    // one dynamic shared-memory size for every electrolyte launch: the
-    // largest of the x passes (full geometry, 3 components) and z passes
+    // one dynamic shared-memory size for the block-level z and y passes
     const size_t C = sizeof(Cx<R>);
-    const size_t xi = C * (g.NX + (size_t)3 * gF.KXc * KCX + (size_t)2 * g.NX * 3 * KCX);
-    const size_t xf = C * (g.NX + (size_t)2 * g.NX * 3 * KCX);
     const size_t zr = C * (g.M + g.NZ + (size_t)g.M * (ZROWS + 1) + std::max((size_t)g.M * ZROWS, (size_t)ZROWS * (g.M + 2)));
-    sm_el = std::max(std::max(xi, xf), std::max(zr, smem_zc));
-    sm_el = std::max(sm_el, smem_y);
+    sm_el = std::max(std::max(zr, smem_zc), smem_y);
     sm_y_any = sm_el;
     if (sm_el > 227 * 1024) return KAPSEL_ERANGE;
     const int sm = (int)sm_el;
-    KCHECK(allow_smem(k_x_inv_op<R, KCX, XI_IDENT, 2, 2>, sm));
-    KCHECK(allow_smem(k_x_inv_op<R, KCX, XI_GRADDIFF, 1, 3>, sm));
-    KCHECK(allow_smem(k_x_fwd_op<R, KCX, XF_CONCUPD, 3>, sm));
-    KCHECK(allow_smem(k_x_fwd_op<R, KCX, XF_PSI_FULL, 1>, sm));
-    KCHECK(allow_smem(k_x_inv_op<R, KCX, XI_IDENT, 1, 1>, sm));
-    KCHECK(allow_smem(k_x_poisson<R, KCX, 0>, sm));
-    KCHECK(allow_smem(k_x_poisson<R, KCX, 1>, sm));
+    int rc = 0;
+    with_len(g.lx, [&](auto l) { rc = el_x_setup<l.value>(); });
+    if (rc) return rc;
     KCHECK(allow_smem(k_z_r2c<R>, sm));
     KCHECK(allow_smem(k_z_c2r<R>, sm));
     KCHECK(allow_smem(k_y_pass<R, true, KCY>, sm));
     KCHECK(allow_smem(k_y_pass<R, false, KCY>, sm));
     KCHECK(allow_smem(k_y_pass<R, true, KCY / 2>, sm));
     KCHECK(allow_smem(k_y_pass<R, false, KCY / 2>, sm));
-    KCHECK(allow_smem(k_x_advect_update<R, KCX, 1>, smem_xadv));
     return 0;
   }
 
-  dim3 gxF() const { return dim3(gF.KYc, (gF.TZ + KCX - 1) / KCX); }
   dim3 gyF(int nc) const { return dim3(g.NX, nc, (gF.TZ + KCY - 1) / KCY); }
   double ze() const { return prm.surface_charge * 1.0; }  // Surface_charge_e, Elementary_charge = 1
   bool ext_on() const { return prm.e_ext[0] != 0.0 || prm.e_ext[1] != 0.0 || prm.e_ext[2] != 0.0; }
 
   // real c_n = A_k2a_out(conc_k[n]) for both species
-  void el_conc_real(bool pdl = false) {
+  void el_conc_real(Launch pdl = Launch()) {
     const size_t nz = (size_t)g.KXc * g.KYc * g.TS;
-    launch_k(pdl, k_x_inv_op<R, KCX, XI_IDENT, 2, 2>, gx(), dim3(256), sm_xinv(2, 2), stream, g, tw,
-             (const Cx<R> *)conc_k, nz, bufA, KOp{});
+    with_len(g.lx, [&](auto l) {
+      launch_k(pdl, k_xw_inv_op<R, l.value, XI_IDENT, 2, false>, gxw<l.value>(g), dim3(2 * XT<R, l.value>::TPG),
+               XT<R, l.value>::smem(2), stream, g, tw, (const Cx<R> *)conc_k, nz, bufA, XOp{});
+    });
     launch_y<true>(g, 2, bufA, bufB, pdl);
     zdisp_c2r(pdl, 2, creal, nullptr, 0);
   }
-  // dynamic shared memory of the x passes on the retained box
-  size_t sm_xinv(int nin, int nout) const {
-    return sizeof(Cx<R>) * (g.NX + (size_t)nin * g.KXc * KCX + (size_t)2 * g.NX * nout * KCX);
+  template <int LX>
+  int el_x_setup() {
+    using T = XT<R, LX>;
+    using F = XT<R, LX, true>;
+    KCHECK(allow_smem(k_xw_inv_op<R, LX, XI_IDENT, 2, false>, T::smem(2)));
+    KCHECK(allow_smem(k_xw_inv_op<R, LX, XI_GRADDIFF, 3, false>, T::smem(3)));
+    KCHECK(allow_smem(k_xw_inv_op<R, LX, XI_IDENT, 1, true>, F::smem(1)));
+    KCHECK(allow_smem(k_xw_concupd<R, LX>, T::smem(3)));
+    KCHECK(allow_smem(k_xw_psi<R, LX>, F::smem(1)));
+    KCHECK(allow_smem(k_xw_poisson<R, LX, false>, T::smem(3, 3)));
+    KCHECK(allow_smem(k_xw_poisson<R, LX, true>, F::smem(3, 3)));
+    return 0;
   }
-  size_t sm_x3() const { return sizeof(Cx<R>) * (g.NX + (size_t)2 * g.NX * 3 * KCX); }
+  // potential gradient of the charge spectrum in component 0 of buf
+  template <bool FULL>
+  void el_poisson(Launch pdl, const Geo &gg, Cx<R> *buf, const POp &op) {
+    with_len(g.lx, [&](auto l) {
+      using T = XT<R, l.value, FULL>;
+      launch_k(pdl, k_xw_poisson<R, l.value, FULL>, dim3((gg.TZ + 3 * T::CW - 1) / (3 * T::CW), gg.KYc), dim3(3 * T::TPG),
+               T::smem(3, 3), stream, gg, tw, buf, op);
+    });
+  }
   // surface-charge scale s0 = sum|Z_e| / (sum|surf| DX3) from the scatter's
   // sums (operate_electrolyte.cxx:217-241)
-  void el_surface_scale(bool pdl = false) {
+  void el_surface_scale(Launch pdl = Launch()) {
     const double dx3 = prm.dx * prm.dx * prm.dx;
     launch_k(pdl, k_reduce_final, dim3(1), dim3(256), 0, stream, (const double *)partial, Np * PCL, 1, 0,
              fabs(ze()) * Np, (const double *)total_solute, dx3, scal);
@@ -1278,16 +1278,15 @@ struct Box : BoxBase {
   // and z: into component 0 of bufA.  Where the warp-level z kernels exist for
   // this NZ the charge is formed inside the z pass.
   template <int LM, bool FULL>
-  void zw_charge(bool pdl, int use_fac, R *keep, Cx<R> *out) {
+  void zw_charge(Launch pdl, int use_fac, R *keep, Cx<R> *out) {
     const ZPlan &p = FULL ? zp_qf : zp_q;
     launch_k(pdl, k_zw_charge<R, LM, ZNW, FULL>, dim3(p.grid(zgroups<LM>())), dim3(p.nw * 32), p.sm, stream, g, tw,
              (const R *)phiq, (const R *)creal, (const double *)scal, use_fac, prm.valency_p, prm.valency_n, keep, out);
   }
   template <bool FULL>
-  void el_charge_z(bool pdl, int use_fac, R *keep, Cx<R> *out) {
-    if (zw_avail == 5) zw_charge<5, FULL>(pdl, use_fac, keep, out);
-    else if (zw_avail == 6) zw_charge<6, FULL>(pdl, use_fac, keep, out);
-    else if (zw_avail == 7) zw_charge<7, FULL>(pdl, use_fac, keep, out);
+  void el_charge_z(Launch pdl, int use_fac, R *keep, Cx<R> *out) {
+    if (zw_avail)
+      with_zlen(zw_avail, [&](auto l) { zw_charge<l.value, FULL>(pdl, use_fac, keep, out); });
     else {
       const Geo &gg = FULL ? gF : g;
       launch_k(pdl, k_el_charge<R>, dim3(592), dim3(256), 0, stream, npts(), (const R *)phiq, (const R *)creal,
@@ -1298,15 +1297,14 @@ struct Box : BoxBase {
   }
   // inverse z, ion fluxes, forward z of both species in bufB
   template <int LM>
-  void zw_flux(bool pdl, const FluxPar &fp) {
+  void zw_flux(Launch pdl, const FluxPar &fp) {
     launch_k(pdl, k_zw_flux<R, LM, ZNW>, dim3(zp_fl.grid(2 * zgroups<LM>())), dim3(zp_fl.nw * 32), zp_fl.sm, stream, g,
              tw, bufB, (const R *)creal, (const R *)gradr, (const R *)(phiq + 2 * npts()), (const R *)ureal, fp);
   }
-  void el_flux_z(bool pdl, const FluxPar &fp) {
+  void el_flux_z(Launch pdl, const FluxPar &fp) {
     const size_t N = npts(), nB = (size_t)g.NX * g.NY * g.TS;
-    if (zw_avail == 5) zw_flux<5>(pdl, fp);
-    else if (zw_avail == 6) zw_flux<6>(pdl, fp);
-    else if (zw_avail == 7) zw_flux<7>(pdl, fp);
+    if (zw_avail)
+      with_zlen(zw_avail, [&](auto l) { zw_flux<l.value>(pdl, fp); });
     else
       for (int n = 0; n < 2; ++n) {
         Cx<R> *b = bufB + 3 * n * nB;
@@ -1320,14 +1318,13 @@ struct Box : BoxBase {
   }
   // nonlinear-term centre in bufB, u real into ureal
   template <int LM>
-  void zw_products_u(bool pdl) {
-    launch_k(pdl, sizeof(R) == 8 ? k_zw_products_pf<R, LM, ZNW, true> : k_zw_products<R, LM, ZNW, true>,
+  void zw_products_u(Launch pdl) {
+    launch_k(pdl, k_zw_products<R, LM, ZNW, true>,
              dim3(zp_pu.grid(zgroups<LM>())), dim3(zp_pu.nw * 32), zp_pu.sm, stream, g, tw, bufB, ureal);
   }
-  void el_products_z(bool pdl) {
-    if (zw_avail == 5) zw_products_u<5>(pdl);
-    else if (zw_avail == 6) zw_products_u<6>(pdl);
-    else if (zw_avail == 7) zw_products_u<7>(pdl);
+  void el_products_z(Launch pdl) {
+    if (zw_avail)
+      with_zlen(zw_avail, [&](auto l) { zw_products_u<l.value>(pdl); });
     else {
       launch_k(pdl, k_z_c2r<R>, dim3(gz(), 3), dim3(256), sm_el, stream, g, tw, (const Cx<R> *)bufB, ureal, npts(),
                g.NZ, PPar{}, (DPart *)nullptr, 0, (int *)nullptr);
@@ -1341,7 +1338,7 @@ struct Box : BoxBase {
   // fluid_solver.cxx:176-178)
   void launch_el_fluid() {
     const size_t nz = (size_t)g.KXc * g.KYc * g.TS;
-    const bool pdl = use_pdl;
+    const Launch pdl = how();
     const double Nd = (double)npts();
     // Rhs_NS_Nernst_Planck: charge from the current conc and positions
     el_scatter(1);
@@ -1349,8 +1346,8 @@ struct Box : BoxBase {
     el_conc_real(pdl);
     el_charge_z<false>(pdl, 0, nullptr, bufB);
     launch_y<false>(g, 1, bufB, bufA, pdl);
-    const KOp gp{{1.0 / prm.dielectric, 0.0}, {prm.e_ext[0] * Nd, prm.e_ext[1] * Nd, prm.e_ext[2] * Nd}};
-    launch_k(pdl, k_x_poisson<R, KCX, 0>, gx(), dim3(256), sm_x3(), stream, g, tw, bufA, gp);
+    el_poisson<false>(pdl, g, bufA,
+                      POp{1.0 / prm.dielectric, {prm.e_ext[0] * Nd, prm.e_ext[1] * Nd, prm.e_ext[2] * Nd}});
     inverse3(pdl, gradr);
     // Rhs_NS_solute: u, the advection term and the explicit Euler update of zeta
     x_zeta(pdl, zeta, uk_dc, bufA);
@@ -1359,16 +1356,19 @@ struct Box : BoxBase {
     launch_y<false>(g, 5, bufB, bufA, pdl);
     x_advect<1>(pdl);
     // ion fluxes and the Euler update of the concentrations, both species at once
-    const KOp dk{{prm.kbt * prm.onsager_p, prm.kbt * prm.onsager_n}, {0, 0, 0}};
-    dim3 gx2 = gx();
-    gx2.z = 2;
-    launch_k(pdl, k_x_inv_op<R, KCX, XI_GRADDIFF, 1, 3>, gx2, dim3(256), sm_xinv(1, 3), stream, g, tw,
-             (const Cx<R> *)conc_k, nz, bufA, dk);
+    const XOp dk{{prm.kbt * prm.onsager_p, prm.kbt * prm.onsager_n}};
+    auto two = [](dim3 d) { return dim3(d.x, d.y, 2); };
+    with_len(g.lx, [&](auto l) {
+      launch_k(pdl, k_xw_inv_op<R, l.value, XI_GRADDIFF, 3, false>, two(gxw<l.value>(g)), dim3(3 * XT<R, l.value>::TPG),
+               XT<R, l.value>::smem(3), stream, g, tw, (const Cx<R> *)conc_k, nz, bufA, dk);
+    });
     launch_y<true>(g, 6, bufA, bufB, pdl);
     el_flux_z(pdl, FluxPar{{prm.onsager_p, prm.onsager_n}, {prm.valency_p, prm.valency_n}});
     launch_y<false>(g, 6, bufB, bufA, pdl);
-    launch_k(pdl, k_x_fwd_op<R, KCX, XF_CONCUPD, 3>, gx2, dim3(256), sm_x3(), stream, g, tw, (const Cx<R> *)bufA,
-             conc_k, nz, KOp{{prm.dt, 0.0}, {0, 0, 0}});
+    with_len(g.lx, [&](auto l) {
+      launch_k(pdl, k_xw_concupd<R, l.value>, two(gxw<l.value>(g)), dim3(3 * XT<R, l.value>::TPG), XT<R, l.value>::smem(3), stream, g,
+               tw, (const Cx<R> *)bufA, conc_k, nz, prm.dt);
+    });
   }
   // Rescale_solute (solute_rhs.cxx:99-128) at the current positions: the
   // factors total[n] / (sum (1 - phi) c_n DX3) into scal[1..2], conc_k scaled.
@@ -1377,7 +1377,7 @@ struct Box : BoxBase {
   void launch_el_rescale() {
     const size_t N = npts(), nz = (size_t)g.KXc * g.KYc * g.TS;
     const double dx3 = prm.dx * prm.dx * prm.dx;
-    const bool pdl = use_pdl;
+    const Launch pdl = how();
     el_scatter(0);
     el_surface_scale(pdl);
     el_conc_real(pdl);
@@ -1390,21 +1390,20 @@ struct Box : BoxBase {
   // The full (untruncated) potential gradient of Make_Coulomb_force_x_on_fluid
   // (operate_electrolyte.cxx:90-177), y-transformed, into F2; the charge field
   // itself into charge.  use_fac: concentrations times the rescale factors.
-  void el_full_gradient(bool pdl, int use_fac) {
+  void el_full_gradient(Launch pdl, int use_fac) {
     el_charge_z<true>(pdl, use_fac, charge, F2);
     launch_y<false>(gF, 1, F2, F1, pdl);
-    launch_k(pdl, k_x_poisson<R, KCX, 1>, gxF(), dim3(256), sm_x3(), stream, gF, tw, F1,
-             KOp{{1.0 / prm.dielectric, 0.0}, {0, 0, 0}});
+    el_poisson<true>(pdl, gF, F1, POp{1.0 / prm.dielectric, {0, 0, 0}});
     launch_y<true>(gF, 3, F1, F2, pdl);
   }
   // f = charge (-grad psi + E_ext) times `scale`, forward z and y into bufA
   template <int LM>
-  void zw_coulomb(bool pdl, const double *e, double scale) {
-    launch_k(pdl, k_zw_coulomb<R, LM, ZNW>, dim3(zp_cb.grid(zgroups<LM>())), dim3(zp_cb.nw * 32), zp_cb.sm, stream, g,
+  void zw_coulomb(Launch pdl, const double *e, double scale) {
+    launch_k(pdl, k_zw_coulomb<R, LM, ZNW>, dim3(zp_cb.grid(3 * zgroups<LM>())), dim3(zp_cb.nw * 32), zp_cb.sm, stream, g,
              tw, (const Cx<R> *)F2, (const R *)charge, e[0], e[1], e[2], scale, bufB);
   }
   // the same force density into the real field fluxr
-  void el_coulomb_real(bool pdl, double scale) {
+  void el_coulomb_real(Launch pdl, double scale) {
     const size_t N = npts();
     launch_k(pdl, k_z_c2r<R>, dim3(gz(), 3), dim3(256), sm_el, stream, gF, tw, (const Cx<R> *)F2, gradr, N, g.NZ,
              PPar{}, (DPart *)nullptr, 0, (int *)nullptr);
@@ -1412,10 +1411,9 @@ struct Box : BoxBase {
     launch_k(pdl, k_el_coulomb<R>, dim3(592), dim3(256), 0, stream, N, (const R *)charge, (const R *)gradr,
              ext ? prm.e_ext[0] : 0.0, ext ? prm.e_ext[1] : 0.0, ext ? prm.e_ext[2] : 0.0, scale, fluxr);
   }
-  void el_coulomb_forward(bool pdl, double scale) {
-    if (zw_avail == 5) zw_coulomb<5>(pdl, prm.e_ext, scale);
-    else if (zw_avail == 6) zw_coulomb<6>(pdl, prm.e_ext, scale);
-    else if (zw_avail == 7) zw_coulomb<7>(pdl, prm.e_ext, scale);
+  void el_coulomb_forward(Launch pdl, double scale) {
+    if (zw_avail)
+      with_zlen(zw_avail, [&](auto l) { zw_coulomb<l.value>(pdl, prm.e_ext, scale); });
     else {
       el_coulomb_real(pdl, scale);
       launch_k(pdl, k_z_r2c<R>, dim3(gz(), 3), dim3(256), sm_el, stream, g, tw, (const R *)fluxr, g.NZ, npts(), bufB,
@@ -1432,10 +1430,13 @@ struct Box : BoxBase {
     const size_t nfull = (size_t)g.NX * g.NY * gF.TS;
     k_z_r2c<R><<<dim3(gz(), 1), 256, sm_el, stream>>>(gF, tw, charge, g.NZ, N, F2, gF.TZ, gF.TS);
     launch_y<false>(gF, 1, F2, F1);
-    k_x_fwd_op<R, KCX, XF_PSI_FULL, 1><<<gxF(), 256, sm_el, stream>>>(gF, tw, F1, F2, nfull,
-                                                                         KOp{{1.0 / prm.dielectric, 0.0}, {0, 0, 0}});
-    k_hermitian_planes<R><<<592, 256, 0, stream>>>(gF, F2, 1);
-    k_x_inv_op<R, KCX, XI_IDENT, 1, 1><<<gxF(), 256, sm_el, stream>>>(gF, tw, F2, nfull, F1, KOp{});
+    with_len(g.lx, [&](auto l) {
+      using T = XT<R, l.value, true>;
+      const dim3 gr = gxw<l.value, true>(gF);
+      k_xw_psi<R, l.value><<<gr, T::TPG, T::smem(1), stream>>>(gF, tw, F1, F2, 1.0 / prm.dielectric);
+      k_hermitian_planes<R><<<592, 256, 0, stream>>>(gF, F2, 1);
+      k_xw_inv_op<R, l.value, XI_IDENT, 1, true><<<gr, T::TPG, T::smem(1), stream>>>(gF, tw, F2, nfull, F1, XOp{});
+    });
     launch_y<true>(gF, 1, F1, F2);
     k_z_c2r<R><<<dim3(gz(), 1), 256, sm_el, stream>>>(gF, tw, F2, out, N, g.NZ, PPar{}, nullptr, 0, nullptr);
   }
@@ -1477,7 +1478,7 @@ struct Box : BoxBase {
   }
 
   void launch_step_el(int euler) {
-    const bool pdl = use_pdl;
+    const Launch pdl = how();
     launch_el_fluid();
     if (Np > 0) k_particles_position<<<(Np + 127) / 128, 128, 0, stream>>>(pp, parts, euler, status);
     launch_cells();
@@ -1492,9 +1493,9 @@ struct Box : BoxBase {
     // u (real), then the particle part of the step
     inverse3(pdl, ustar);
     if (Np > 0) {
-      launch_k(pdl, k_particles_hydro_velocity<R>, dim3(Np * pp.hyd_pcl), dim3(pp.hyd_threads), 0, stream, pp, parts,
-               (const R *)ustar, (const short4 *)cells, (const double *)nullptr, euler, status, partial_p, arrivals,
-               (double *)nullptr, ovl);
+      launch_kc(pp.hyd_pcl, pdl, k_particles_hydro_velocity<R>, dim3(Np * pp.hyd_pcl), dim3(pp.hyd_threads), 0,
+                stream, pp, parts, (const R *)ustar, (const short4 *)cells, (const double *)nullptr, euler, status,
+                (double *)nullptr, ovl);
       launch_k(pdl, k_particles_scatter<R, true>, dim3(Np * pp.sc_pcl), dim3(256), 0, stream, pp, (const DPart *)parts,
                (const short4 *)cells, force(), (const R *)ustar, status, (const unsigned *)ovl);
       launch_force_to_zeta(pdl);
@@ -2368,10 +2369,21 @@ int kapsel_gpu_create(const kapsel_params *p, kapsel_ctx **out) {
   // 159 with 64; 256 at 128^3: 15.7, 17.6, 23.6, 36).  The scatter's blocks
   // each find the particle's neighbours first, so with enough particles to
   // fill the GPU one block does all its points (336 us with four, 250 with
-  // two, 215 with one at 256^3; 14.9, 13.2, 15.4 at 128^3).
+  // two, 215 with one at 256^3; 14.9, 13.2, 15.4 at 128^3).  The line between
+  // few and some lies where blocks of 1024 threads, one to an SM, no longer
+  // run at once (128 particles at 128^3: 118 us a step against 122).
   pp.hyd_pcl = 1;
-  pp.hyd_threads = b->Np >= 1024 ? 128 : b->Np >= 128 ? 512 : 1024;
-  pp.sc_pcl = b->Np >= 1024 ? 1 : b->Np >= 128 ? 2 : PCL;
+  pp.hyd_threads = b->Np >= 1024 ? 128 : b->Np > 148 ? 512 : 1024;
+  pp.sc_pcl = b->Np >= 1024 ? 1 : b->Np > 148 ? 2 : PCL;
+  // In FP64 the profile's arithmetic fills the few SMs that so few particles
+  // use: a cluster of eight blocks each (64^3, 16 particles: 59.6 -> 55.3 us a
+  // step; electrolyte, 8: 217 -> 211.  In FP32 43.1 -> 43.3: the cluster's two
+  // barriers take what the shorter loop gives).
+  if (p->precision == KAPSEL_FP64 && b->Np <= 32) {
+    pp.hyd_pcl = 8;
+    pp.hyd_threads = 256;
+    pp.sc_pcl = 8;
+  }
   // a neighbour's centre is within two supports, a point within one
   const double reach = 3.0 * (p->a + 0.5 * p->a_xi) + 4.0;
   pp.near_wrap = std::min(g.NX, std::min(g.NY, g.NZ)) < 2.0 * reach ? 1 : 0;
@@ -2410,13 +2422,10 @@ int kapsel_gpu_create(const kapsel_params *p, kapsel_ctx **out) {
     rc = b->setup_cells(rl);
     if (rc) return rc;
   }
-  if (b->Np > 0 && b->Np <= 1024 && !b->cl_on && pp.hyd_pcl == 1) {
+  if (b->Np > 0 && b->Np <= 1024 && !b->cl_on) {
     if (cudaMalloc(&b->ovl, sizeof(unsigned) * 32 * (size_t)b->Np) != cudaSuccess) return KAPSEL_ENOMEM;
     cudaMemset(b->ovl, 0, sizeof(unsigned) * 32 * (size_t)b->Np);
   }
-  if (cudaMalloc(&b->partial_p, sizeof(double) * 18 * HYD_PCL_MAX * np1) != cudaSuccess) return KAPSEL_ENOMEM;
-  if (cudaMalloc(&b->arrivals, sizeof(int) * np1) != cudaSuccess) return KAPSEL_ENOMEM;
-  cudaMemset(b->arrivals, 0, sizeof(int) * np1);
   for (int s = 0; s < 2; ++s) {
     if (cudaMalloc(&b->noise_dev[s], sizeof(double) * 6 * np1) != cudaSuccess) return KAPSEL_ENOMEM;
     if (cudaMallocHost(&b->noise_host[s], sizeof(double) * 6 * np1) != cudaSuccess) return KAPSEL_ENOMEM;
@@ -2450,8 +2459,6 @@ int kapsel_gpu_destroy(kapsel_ctx *ctx) {
     cudaFree(b->cells);
     cudaFree(b->uk_dc);
     cudaFree(b->status);
-    cudaFree(b->partial_p);
-    cudaFree(b->arrivals);
     cudaFree(b->nc_feat);
     cudaFree(b->nc_frames);
     cudaFree(b->nc_pairs);
@@ -2796,16 +2803,17 @@ static int calc_fr_impl(kapsel_ctx *ctx, double *fr, bool gravity) {
   b->launch_cells();
   PPar p = b->pp;
   p.S = 0;           // no hydro gather
+  p.hyd_pcl = 1;
   p.thermostat = 0;  // no kick
   p.frozen = 0;
   if (!gravity) p.grav = 0.0;
   // u is never read with S == 0
   if (b->prm.precision == KAPSEL_FP64)
     k_particles_hydro_velocity<double><<<b->Np * p.hyd_pcl, p.hyd_threads, 0, b->stream>>>(p, scratch, nullptr, b->cells, nullptr, 1,
-                                                                           b->status, b->partial_p, b->arrivals);
+                                                                           b->status, nullptr, nullptr);
   else
     k_particles_hydro_velocity<float><<<b->Np * p.hyd_pcl, p.hyd_threads, 0, b->stream>>>(p, scratch, nullptr, b->cells, nullptr, 1,
-                                                                          b->status, b->partial_p, b->arrivals);
+                                                                          b->status, nullptr, nullptr);
   std::vector<DPart> h(b->Np);
   cudaMemcpyAsync(h.data(), scratch, sizeof(DPart) * b->Np, cudaMemcpyDeviceToHost, b->stream);
   if (cudaStreamSynchronize(b->stream) != cudaSuccess) return KAPSEL_ECUDA;
@@ -2904,15 +2912,16 @@ int kapsel_gpu_md_velocity(kapsel_ctx *ctx, const double *f_hydro, const double 
   b->launch_cells();
   PPar p = b->pp;
   p.S = 0;
+  p.hyd_pcl = 1;
   p.thermostat = 0;
   p.frozen = 0;
   if (!rc) {
     if (b->prm.precision == KAPSEL_FP64)
       k_particles_hydro_velocity<double><<<b->Np * p.hyd_pcl, p.hyd_threads, 0, b->stream>>>(
-          p, b->parts, nullptr, b->cells, nullptr, euler ? 1 : 0, b->status, b->partial_p, b->arrivals, corr);
+          p, b->parts, nullptr, b->cells, nullptr, euler ? 1 : 0, b->status, corr, nullptr);
     else
       k_particles_hydro_velocity<float><<<b->Np * p.hyd_pcl, p.hyd_threads, 0, b->stream>>>(
-          p, b->parts, nullptr, b->cells, nullptr, euler ? 1 : 0, b->status, b->partial_p, b->arrivals, corr);
+          p, b->parts, nullptr, b->cells, nullptr, euler ? 1 : 0, b->status, corr, nullptr);
     if (cudaGetLastError() != cudaSuccess) rc = KAPSEL_ECUDA;
   }
   if (!rc) rc = check_status(b);

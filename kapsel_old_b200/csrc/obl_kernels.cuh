@@ -29,6 +29,7 @@
 
 #include "particle_kernels.cuh"
 #include "spectral_kernels.cuh"
+#include "xtile_kernels.cuh"
 #include "zwarp_kernels.cuh"
 
 namespace kapsel {
@@ -94,68 +95,47 @@ __device__ __forceinline__ void obl_zeta_to_u(int KXi, int kz, R kx, R ky, R kzr
 // k = 0 from uk_dc) and the contravariant vorticity (Zeta_k2omega_k_OBL), for
 // the advection term (Zeta_k2u_cpuky / Zeta_k2omega_OBL, operate_omega.h:
 // 144-172).  IK2 and the metric use degree_oblique at the start of the step.
-// out I1: [6][NX][KYc][TS].  grid (KYc, ceil(TZ/KC)).
-template <typename R, int KC, int LX = 0>
-__global__ void __launch_bounds__(256) k_x_obl_inv(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ zeta,
+// out I1: [6][NX][KYc][TS].  grid (ceil(TZ/CW), KYc), six groups.
+template <typename R, int LX>
+__global__ void __launch_bounds__(6 * XT<R, LX>::TPG, XT<R, LX>::blocks(6)) k_x_obl_inv(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ zeta,
                                                    const double *__restrict__ uk_dc, const double *__restrict__ st,
                                                    Cx<R> *__restrict__ out) {
+  using T = XT<R, LX>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  const int NXv = LX > 0 ? (1 << LX) : g.NX, LXv = LX > 0 ? LX : g.lx;
-  constexpr int W = 6 * KC;
-  Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
-  Cx<R> *Zt = twx + NXv;            // [2][KXc][KC]
-  Cx<R> *U = Zt + 2 * g.KXc * KC;   // [NX][6*KC]
-  Cx<R> *scr = U + NXv * W;
-  const int iy = blockIdx.x;
-  const int kz0 = blockIdx.y * KC;
-  const int ncol = min(KC, g.TZ - kz0);
-  const size_t zplane = (size_t)g.KXc * g.KYc * g.TS;
-  load_twiddles(twx, tw.x, NXv);
   zeta = pdl_fresh(zeta);
   uk_dc = pdl_fresh(uk_dc);
   st = pdl_fresh(st);
-  for (int it = threadIdx.x; it < 2 * g.KXc * KC; it += blockDim.x) {
-    const int col = it % KC, rest = it / KC, ix = rest % g.KXc, c = rest / g.KXc;
-    if (col < ncol) cp_async_cx(Zt + it, zeta + c * zplane + ((size_t)ix * g.KYc + iy) * g.TS + kz0 + col);
-  }
+  const int grp = T::group();
+  Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + grp * T::EX;
+  Cx<R> *S = reinterpret_cast<Cx<R> *>(smem_raw);  // [6][KXc][CW], a group's buffer each
+  const int iy = blockIdx.y, kz0 = blockIdx.x * T::CW, ncol = min(T::CW, g.TZ - kz0);
+  const size_t zplane = (size_t)T::KXc * g.KYc * g.TS, at = (size_t)iy * g.TS + kz0, row = (size_t)g.KYc * g.TS;
   const double deg = st[OB_DEG];
-  cp_async_wait_all();
-  __syncthreads();
   const int KYi = signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY);
   const R ky = R(g.wave[1] * KYi);
-  for (int it = threadIdx.x; it < NXv * KC; it += blockDim.x) {
-    const int col = it % KC, i = it / KC;
+  x_modes<R, LX>(kz0, ncol, [&](int ix, int KXi, int col, int kz) {
+    const Cx<R> *z = zeta + ix * row + at + col;
+    const Cx<R> z0 = z[0], z1 = z[zplane];
+    const R kx = R(g.wave[0] * KXi), kzr = R(g.wave[2] * kz);
+    const double k2 = obl_k2(g, deg, KXi, KYi, kz);
+    const R ik2 = k2 > 0.0 ? R(1.0 / k2) : R(0);
     Cx<R> o[6];
+    obl_zeta_to_u(KXi, kz, kx, ky, kzr, ik2, R(deg), z0, z1, o);
+    if (KXi == 0 && KYi == 0 && kz == 0)
+      for (int d = 0; d < 3; ++d) o[d] = {R(uk_dc[d]), R(0)};
+    obl_omega(KXi, kz, kx, ky, kzr, z0, z1, o + 3);
 #pragma unroll
-    for (int c = 0; c < 6; ++c) o[c] = {R(0), R(0)};
-    const int KXi = signed_k(i, NXv);
-    if (col < ncol && abs(KXi) < g.TX) {
-      const int ix = KXi >= 0 ? KXi : KXi + g.KXc;
-      const int kz = kz0 + col;
-      const R kx = R(g.wave[0] * KXi), kzr = R(g.wave[2] * kz);
-      const Cx<R> z0 = Zt[ix * KC + col], z1 = Zt[(g.KXc + ix) * KC + col];
-      const double k2 = obl_k2(g, deg, KXi, KYi, kz);
-      const R ik2 = k2 > 0.0 ? R(1.0 / k2) : R(0);
-      obl_zeta_to_u(KXi, kz, kx, ky, kzr, ik2, R(deg), z0, z1, o);
-      if (KXi == 0 && KYi == 0 && kz == 0) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) o[d] = {R(uk_dc[d]), R(0)};
-      }
-      obl_omega(KXi, kz, kx, ky, kzr, z0, z1, o + 3);
-    }
-#pragma unroll
-    for (int c = 0; c < 6; ++c) U[i * W + c * KC + col] = o[c];
-  }
+    for (int c = 0; c < 6; ++c) S[c * T::EX + ix * T::CW + col] = o[c];
+  });
   __syncthreads();
-  fft2_smem<R, -1, W, LX>(U, scr, LXv, 1, W, twx);
-  for (int it = threadIdx.x; it < 6 * NXv * KC; it += blockDim.x) {
-    const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LXv;
-    if (col < ncol) out[(((size_t)c * NXv + x) * g.KYc + iy) * g.TS + kz0 + col] = U[x * W + c * KC + col];
-  }
+  Cx<R> v[ZL<LX>::N1];
+  x_get<R, LX>(ex, v);
+  xfft<R, LX, -1>(v, ex, tw.x);
+  x_store<R, LX>(out + (size_t)grp * T::NX * row + at, row, ncol, v);
 }
 
-// x passes of three spectra on one tile of (ky, kz chunk), in place on buf
+// x passes of three spectra on one tile of (ky, kz columns), in place on buf
 // (I1 layout), with the update of zeta between them:
 //   ADV = 1: buf = the advection term u x omega.  A -= 2 S_eff (1, deg, 0) u^y_k
 //            (operate_omega.cxx:155-164; u^y_k of the zeta at the start of the
@@ -170,78 +150,60 @@ __global__ void __launch_bounds__(256) k_x_obl_inv(Geo g, Twiddles<R> tw, const 
 //            (operate_omega.cxx:222-263), contra2co (fft_wrapper.h:327-361),
 //            U_k2zeta_k_OBL with uk_dc = co2contra(u_co(0)) (fft_wrapper.cxx:
 //            341-406), all with the updated degree_oblique.
-// grid (KYc, ceil(TZ/KC)).
-template <typename R, int KC, int ADV, int LX = 0>
-__global__ void __launch_bounds__(256) k_x_obl_update(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ buf,
-                                                      Cx<R> *__restrict__ zeta, double *__restrict__ uk_dc,
-                                                      const double *__restrict__ st) {
+// grid (ceil(TZ/CW), KYc), three groups.
+template <typename R, int LX, int ADV>
+__global__ void __launch_bounds__(3 * XT<R, LX>::TPG, XT<R, LX>::blocks(3)) k_x_obl_update(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ buf,
+                                                     Cx<R> *__restrict__ zeta, double *__restrict__ uk_dc,
+                                                     const double *__restrict__ st) {
+  using T = XT<R, LX>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double uks[2][3];  // uk_dc at the start, and after FIX_CELL
   pdl_begin();
-  const int NXv = LX > 0 ? (1 << LX) : g.NX, LXv = LX > 0 ? LX : g.lx;
-  constexpr int W = 3 * KC;
-  Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
-  Cx<R> *Pb = twx + NXv;             // [NX][3*KC]
-  Cx<R> *scr = Pb + NXv * W;
-  Cx<R> *Zs = scr + NXv * W;         // [2][KXc][KC] (ADV only)
-  __shared__ double uks[2][3];       // uk_dc at the start, and after FIX_CELL
-  const int iy = blockIdx.x;
-  const int kz0 = blockIdx.y * KC;
-  const int ncol = min(KC, g.TZ - kz0);
-  const size_t cstr = (size_t)NXv * g.KYc * g.TS;
-  const size_t zplane = (size_t)g.KXc * g.KYc * g.TS;
-  load_twiddles(twx, tw.x, NXv);
   buf = pdl_fresh(buf);
   zeta = pdl_fresh(zeta);
   uk_dc = pdl_fresh(uk_dc);
   st = pdl_fresh(st);
-  for (int it = threadIdx.x; it < 3 * NXv * KC; it += blockDim.x) {
-    const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LXv;
-    Cx<R> *d = Pb + x * W + c * KC + col;
-    if (col < ncol)
-      cp_async_cx(d, buf + c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col);
-    else
-      *d = {R(0), R(0)};
-  }
+  const int grp = T::group();
+  Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + grp * T::EX;
+  Cx<R> *S = reinterpret_cast<Cx<R> *>(smem_raw);  // [3][KXc][CW], a group's buffer each; then u
+  Cx<R> *Zs = S + 3 * T::EX;                       // [2][KXc][CW] (ADV only)
+  const int iy = blockIdx.y, kz0 = blockIdx.x * T::CW, ncol = min(T::CW, g.TZ - kz0);
+  const size_t zplane = (size_t)T::KXc * g.KYc * g.TS, at = (size_t)iy * g.TS + kz0, row = (size_t)g.KYc * g.TS;
+  const size_t cstr = (size_t)T::NX * row;
+  Cx<R> v[ZL<LX>::N1];
+  x_load<R, LX>(buf + grp * cstr + at, row, ncol, v);
   if (ADV) {
-    for (int it = threadIdx.x; it < 2 * g.KXc * KC; it += blockDim.x) {
-      const int col = it % KC, rest = it / KC, ix = rest % g.KXc, c = rest / g.KXc;
-      if (col < ncol) cp_async_cx(Zs + it, zeta + c * zplane + ((size_t)ix * g.KYc + iy) * g.TS + kz0 + col);
-    }
-    if (iy == 0 && blockIdx.y == 0 && threadIdx.x < 3) {
-      const double v = uk_dc[threadIdx.x];
-      uks[0][threadIdx.x] = v;
-      uks[1][threadIdx.x] = g.fix_cell[threadIdx.x] ? 0.0 : v;
+    x_stage_zeta<R, LX>(Zs, zeta, zplane, row, at, ncol);
+    if (iy == 0 && blockIdx.x == 0 && threadIdx.x < 3) {
+      const double u0 = uk_dc[threadIdx.x];
+      uks[0][threadIdx.x] = u0;
+      uks[1][threadIdx.x] = g.fix_cell[threadIdx.x] ? 0.0 : u0;
       uk_dc[threadIdx.x] = uks[1][threadIdx.x];
     }
   }
   const double deg = st[OB_DEG], s_eff = ADV ? st[OB_SRATE] : 0.0;
+  xfft<R, LX, 1>(v, ex, tw.x);
+  x_put<R, LX>(ex, v);
   cp_async_wait_all();
   __syncthreads();
-  fft2_smem<R, 1, W, LX>(Pb, scr, LXv, 1, W, twx);
   const R degr = R(deg);
   const int KYi = signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY);
   const R ky = R(g.wave[1] * KYi);
-  for (int it = threadIdx.x; it < g.KXc * KC; it += blockDim.x) {
-    const int col = it % KC, ix = it / KC;
-    if (col >= ncol) continue;
-    const int KXi = ix < g.TX ? ix : ix - g.KXc;
-    const int i = KXi >= 0 ? KXi : KXi + NXv;
-    const int kz = kz0 + col;
-    const size_t o = ((size_t)ix * g.KYc + iy) * g.TS + kz;
-    const Cx<R> *p = Pb + i * W + col;
+  x_modes<R, LX>(kz0, ncol, [&](int ix, int KXi, int col, int kz) {
+    Cx<R> *z = zeta + ix * row + at + col, *p = S + ix * T::CW + col;
     const R kx = R(g.wave[0] * KXi), kzr = R(g.wave[2] * kz);
     const double k2 = obl_k2(g, deg, KXi, KYi, kz);
     const R ik2 = k2 > 0.0 ? R(1.0 / k2) : R(0);
     const bool k0 = (KXi == 0 && KYi == 0 && kz == 0);
     if (ADV) {
-      Cx<R> z0 = Zs[ix * KC + col], z1 = Zs[(g.KXc + ix) * KC + col];
+      Cx<R> z0 = Zs[ix * T::CW + col], z1 = Zs[T::MODES + ix * T::CW + col];
       Cx<R> uo[3];
       obl_zeta_to_u(KXi, kz, kx, ky, kzr, ik2, degr, z0, z1, uo);
       const R uy_re = k0 ? R(uks[0][1]) : uo[1].x, uy_im = k0 ? R(0) : uo[1].y;
       const R s2 = R(2.0 * s_eff), s2d = R(2.0 * s_eff * deg);
       const Cx<R> a0 = {p[0].x - s2 * uy_re, p[0].y - s2 * uy_im};
-      const Cx<R> a1 = {p[KC].x - s2d * uy_re, p[KC].y - s2d * uy_im};
-      const Cx<R> a2 = p[2 * KC];
+      const Cx<R> a1 = {p[T::EX].x - s2d * uy_re, p[T::EX].y - s2d * uy_im};
+      const Cx<R> a2 = p[2 * T::EX];
       Cx<R> w[3];
       w[0] = {ky * a2.y - kzr * a1.y, -(ky * a2.x - kzr * a1.x)};
       w[1] = {kzr * a0.y - kx * a2.y, -(kzr * a0.x - kx * a2.x)};
@@ -262,12 +224,14 @@ __global__ void __launch_bounds__(256) k_x_obl_update(Geo g, Twiddles<R> tw, Cx<
       const R c1 = R(1.0 / g.nu) * ik2;
       z0 = {z0.x + dmy * (z0.x - c1 * f0.x), z0.y + dmy * (z0.y - c1 * f0.y)};
       z1 = {z1.x + dmy * (z1.x - c1 * f1.x), z1.y + dmy * (z1.y - c1 * f1.y)};
-      zeta[o] = z0;
-      zeta[zplane + o] = z1;
-      Zs[ix * KC + col] = z0;
-      Zs[(g.KXc + ix) * KC + col] = z1;
+      z[0] = z0;
+      z[zplane] = z1;
+      Cx<R> u[3];
+      obl_zeta_to_u(KXi, kz, kx, ky, kzr, ik2, degr, z0, z1, u);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) p[d * T::EX] = k0 ? Cx<R>{R(uks[1][d]), R(0)} : u[d];
     } else {
-      Cx<R> u0 = p[0], u1 = p[KC], u2 = p[2 * KC];
+      Cx<R> u0 = p[0], u1 = p[T::EX], u2 = p[2 * T::EX];
       const R kxc = (R(1) + degr * degr) * kx - degr * ky;
       const R kyc = -degr * kx + ky;
       const Cx<R> dm = {ik2 * (u0.x * kx + u1.x * ky + u2.x * kzr), ik2 * (u0.y * kx + u1.y * ky + u2.y * kzr)};
@@ -283,14 +247,14 @@ __global__ void __launch_bounds__(256) k_x_obl_update(Geo g, Twiddles<R> tw, Cx<
       w[1] = {kzr * c0.y - kx * c2.y, -(kzr * c0.x - kx * c2.x)};
       w[2] = {kx * c1.y - ky * c0.y, -(kx * c1.x - ky * c0.x)};
       if (KXi != 0) {
-        zeta[o] = w[1];
-        zeta[zplane + o] = w[2];
+        z[0] = w[1];
+        z[zplane] = w[2];
       } else if (kz != 0) {
-        zeta[o] = w[1];
-        zeta[zplane + o] = w[0];
+        z[0] = w[1];
+        z[zplane] = w[0];
       } else {
-        zeta[o] = w[0];
-        zeta[zplane + o] = w[2];
+        z[0] = w[0];
+        z[zplane] = w[2];
       }
       if (k0) {
         // co2contra_single of the real parts (fft_wrapper.h:412-423)
@@ -300,34 +264,12 @@ __global__ void __launch_bounds__(256) k_x_obl_update(Geo g, Twiddles<R> tw, Cx<
         uk_dc[2] = (double)c2.x;
       }
     }
-  }
+  });
   if (!ADV) return;
   __syncthreads();
-  for (int it = threadIdx.x; it < NXv * KC; it += blockDim.x) {
-    const int col = it % KC, i = it / KC;
-    Cx<R> u[3] = {{R(0), R(0)}, {R(0), R(0)}, {R(0), R(0)}};
-    const int KXi = signed_k(i, NXv);
-    if (col < ncol && abs(KXi) < g.TX) {
-      const int ix = KXi >= 0 ? KXi : KXi + g.KXc;
-      const int kz = kz0 + col;
-      const R kx = R(g.wave[0] * KXi), kzr = R(g.wave[2] * kz);
-      const double k2 = obl_k2(g, deg, KXi, KYi, kz);
-      const R ik2 = k2 > 0.0 ? R(1.0 / k2) : R(0);
-      obl_zeta_to_u(KXi, kz, kx, ky, kzr, ik2, degr, Zs[ix * KC + col], Zs[(g.KXc + ix) * KC + col], u);
-      if (KXi == 0 && KYi == 0 && kz == 0) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) u[d] = {R(uks[1][d]), R(0)};
-      }
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) Pb[i * W + d * KC + col] = u[d];
-  }
-  __syncthreads();
-  fft2_smem<R, -1, W, LX>(Pb, scr, LXv, 1, W, twx);
-  for (int it = threadIdx.x; it < 3 * NXv * KC; it += blockDim.x) {
-    const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LXv;
-    if (col < ncol) buf[c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col] = Pb[x * W + c * KC + col];
-  }
+  x_get<R, LX>(ex, v);
+  xfft<R, LX, -1>(v, ex, tw.x);
+  x_store<R, LX>(buf + grp * cstr + at, row, ncol, v);
 }
 
 // ---------------------------------------------------------------------------
@@ -801,44 +743,61 @@ __global__ void __launch_bounds__(256) k_obl_clear(PPar p, const DPart *__restri
 // Inverse z of u and omega (components 0..2 and 3..5 of io), u x omega
 // (operate_omega.cxx:131-150), forward z into components 0..2.  None of the
 // nine real fields is stored (as three block-level launches over them this
-// took 60 + 14 + 30 us at 128^3 in FP32).
+// took 60 + 14 + 30 us at 128^3 in FP32).  Six components of 64 bytes or more
+// per lane do not fit the registers and wait in shared memory, each lane at
+// its own place.
+template <typename R, int LM>
+__host__ __device__ constexpr bool zw_cross_park() {
+  return sizeof(R) * ZL<LM>::N1 >= 64;
+}
+template <typename R, int LM>
+__host__ __device__ constexpr size_t zw_cross_bytes() {
+  return ZX<R, LM>::BYTES + (zw_cross_park<R, LM>() ? sizeof(Cx<R>) * 6 * 32 * ZL<LM>::N1 : 0);
+}
 template <typename R, int LM, int NW>
 __global__ void __launch_bounds__(NW * 32) k_zw_cross(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ io) {
   using Z = ZL<LM>;
-  constexpr int GL = Z::RW * Z::LS, NI = Z::RW * Z::M / 32;
+  constexpr bool PARK = zw_cross_park<R, LM>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * 6 * GL;
-  Cx<R> wi[Z::N1], wk[Z::KW];
-  wfft_twiddles<R, LM, -1>(tw.m, wi);
-  wpre_twiddles<R, LM>(tw.z, wk);
   io = pdl_fresh(io);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw + warp * zw_cross_bytes<R, LM>());
+  Cx<R> *park = ex + ZX<R, LM>::ELEMS;  // [6][N1][32]
+  int turn = 0;
+  Cx<R> w[Z::N1], wz[Z::N1];
+  wfft_twiddles<R, LM>(tw.m, w);
+  wpack_twiddles<R, LM>(tw.z, wz);
   const size_t rows = (size_t)g.NX * g.NY, cstr = rows * Z::TS;
   const int ngroups = (int)(rows / Z::RW);
   const R sc = R(g.inv_n);
   for (int grp = blockIdx.x * nw + warp; grp < ngroups; grp += gridDim.x * nw) {
-    Cx<R> *row = io + (size_t)grp * Z::RW * Z::TS;
+    Cx<R> *line = io + ((size_t)grp * Z::RW + wl<LM>()) * Z::TS;
+    Cx<R> u[PARK ? 1 : 6][Z::N1];
 #pragma unroll
-    for (int c = 0; c < 6; ++c)
-      for (int rr = 0; rr < Z::RW; ++rr) wpack_c2r<R, LM>(row + c * cstr + rr * Z::TS, buf + c * GL + rr * Z::LS, wk);
-    __syncwarp();
+    for (int c = 0; c < 6; ++c) {
+      Cx<R>(&v)[Z::N1] = u[PARK ? 0 : c];
+      wpack_c2r<R, LM>(line + c * cstr, v, wz);
+      wfft<R, LM, -1>(v, ex, turn, w);
 #pragma unroll
-    for (int c = 0; c < 6; ++c) wfft<R, LM, -1>(buf + c * GL, wi);
-#pragma unroll 2
-    for (int h = 0; h < NI; ++h) {
-      const int i = lane + 32 * h, at = (i >> LM) * Z::LS + zpos<LM>(i & (Z::M - 1));
-      Cx<R> v[6];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) v[c] = cscale(buf[c * GL + at], sc);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const int a = (d + 1) % 3, b = (d + 2) % 3;
-        buf[d * GL + at] = {v[a].x * v[3 + b].x - v[b].x * v[3 + a].x, v[a].y * v[3 + b].y - v[b].y * v[3 + a].y};
+      for (int n1 = 0; n1 < Z::N1; ++n1) {
+        v[n1] = cscale(v[n1], sc);
+        if (PARK) park[(c * Z::N1 + n1) * 32 + lane] = v[n1];
       }
     }
-    __syncwarp();
-    zw_forward3<R, LM>(buf, GL, tw, row, cstr);
+    auto get = [&](int c, int n1) -> Cx<R> { return PARK ? park[(c * Z::N1 + n1) * 32 + lane] : u[PARK ? 0 : c][n1]; };
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int a = (d + 1) % 3, b = (d + 2) % 3;
+      Cx<R> p[Z::N1];
+#pragma unroll
+      for (int n1 = 0; n1 < Z::N1; ++n1) {
+        const Cx<R> ua = get(a, n1), ub = get(b, n1), wa = get(3 + a, n1), wb = get(3 + b, n1);
+        p[n1] = {ua.x * wb.x - ub.x * wa.x, ua.y * wb.y - ub.y * wa.y};
+      }
+      wfft<R, LM, 1>(p, ex, turn, w);
+      wunpack_r2c<R, LM>(p, line + d * cstr, wz, tw.z);
+    }
   }
 }
 
@@ -854,15 +813,19 @@ __global__ void __launch_bounds__(NW * 32) k_zw_obl_force(Geo g, Twiddles<R> tw,
                                                           Cx<R> *__restrict__ out) {
   using Z = ZL<LM>;
   using V2 = typename Vec2<R>::T;
-  constexpr int GL = Z::RW * Z::LS, HR = Z::M / 32;  // element pairs per lane and row
+  constexpr int B = 4;  // element pairs whose loads are in flight together
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
   st = pdl_fresh(st);
   phiup = pdl_fresh(phiup);
   ucart = pdl_fresh(ucart);
   uobl = pdl_fresh(uobl);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  Cx<R> *buf = reinterpret_cast<Cx<R> *>(smem_raw) + (size_t)warp * 3 * GL;
+  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
+  int turn = 0;
+  Cx<R> w[Z::N1], wz[Z::N1];
+  wfft_twiddles<R, LM>(tw.m, w);
+  wpack_twiddles<R, LM>(tw.z, wz);
   const double deg = st[OB_DEG];
   const bool remap = st[OB_REMAP] != 0.0;
   const size_t rows = (size_t)g.NX * g.NY, n = rows * Z::NZ, cstr = rows * Z::TS;
@@ -888,31 +851,32 @@ __global__ void __launch_bounds__(NW * 32) k_zw_obl_force(Geo g, Twiddles<R> tw,
     for (int d = 0; d < 3; ++d) f[d] = V2{up[d].x * i0 - p0 * us[d].x, up[d].y * i1 - p1 * us[d].y};
   };
   for (int grp = blockIdx.x * nw + warp; grp < ngroups; grp += gridDim.x * nw) {
-    const int row0 = grp * Z::RW, i = row0 / g.NY;
-#pragma unroll 1
-    for (int rr = 0; rr < Z::RW; ++rr) {
-      const int j = (row0 + rr) & (g.NY - 1);
-      double sign = (double)(j - o.NY / 2);
-      if (!(sign == 0)) sign = sign / fabs(sign);
-      const double jd = (double)(j - o.NY / 2);
-      const int io = (int)((double)(int)(sign * deg * jd) * sign);
-      const double alpha = (deg * jd - (double)io) * sign, beta = 1. - alpha;
-      const int iob = (i + io) & (o.NX - 1);
-      const int iobp = (iob + (int)sign) & (o.NX - 1);
-      const size_t s = ((size_t)iob * o.NY + j) * Z::NZ, sp = ((size_t)iobp * o.NY + j) * Z::NZ;
-      const size_t su = obl_source_row(o, remap, i, j) * Z::NZ;
-      V2 pa[HR], pb[HR], u[HR][3];
+    const int row = grp * Z::RW + wl<LM>(), i = row / g.NY, j = row & (g.NY - 1);
+    double sign = (double)(j - o.NY / 2);
+    if (!(sign == 0)) sign = sign / fabs(sign);
+    const double jd = (double)(j - o.NY / 2);
+    const int sh = (int)((double)(int)(sign * deg * jd) * sign);
+    const double alpha = (deg * jd - (double)sh) * sign, beta = 1. - alpha;
+    const int iob = (i + sh) & (o.NX - 1);
+    const int iobp = (iob + (int)sign) & (o.NX - 1);
+    const size_t at = 2 * wt<LM>();
+    const size_t s = ((size_t)iob * o.NY + j) * Z::NZ + at, sp = ((size_t)iobp * o.NY + j) * Z::NZ + at;
+    const size_t su = obl_source_row(o, remap, i, j) * Z::NZ + at;
+    Cx<R> v[3][Z::N1];
 #pragma unroll
-      for (int h = 0; h < HR; ++h) {
-        const int k = 2 * (lane + 32 * h);
+    for (int n0 = 0; n0 < Z::N1; n0 += B) {
+      V2 pa[B], pb[B], u[B][3];
+#pragma unroll
+      for (int h = 0; h < B; ++h) {
+        const int k = 2 * Z::N2 * (n0 + h);
         pa[h] = *reinterpret_cast<const V2 *>(phiup + s + k);
         pb[h] = *reinterpret_cast<const V2 *>(phiup + sp + k);
 #pragma unroll
         for (int d = 0; d < 3; ++d) u[h][d] = *reinterpret_cast<const V2 *>(uobl + d * n + su + k);
       }
 #pragma unroll
-      for (int h = 0; h < HR; ++h) {
-        const int m = lane + 32 * h, k = 2 * m;
+      for (int h = 0; h < B; ++h) {
+        const int k = 2 * Z::N2 * (n0 + h);
         if (remap) {
           u[h][0].x += u[h][1].x;
           u[h][0].y += u[h][1].y;
@@ -938,11 +902,14 @@ __global__ void __launch_bounds__(NW * 32) k_zw_obl_force(Geo g, Twiddles<R> tw,
           }
         }
 #pragma unroll
-        for (int d = 0; d < 3; ++d) buf[d * GL + rr * Z::LS + zpos<LM>(m)] = {u[h][d].x, u[h][d].y};
+        for (int d = 0; d < 3; ++d) v[d][n0 + h] = {u[h][d].x, u[h][d].y};
       }
     }
-    __syncwarp();
-    zw_forward3<R, LM>(buf, GL, tw, out + (size_t)row0 * Z::TS, cstr);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      wfft<R, LM, 1>(v[d], ex, turn, w);
+      wunpack_r2c<R, LM>(v[d], out + d * cstr + (size_t)row * Z::TS, wz, tw.z);
+    }
   }
 }
 

@@ -2,6 +2,7 @@
 // in every mode; only the fields they read or scatter into follow R.
 #pragma once
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "fft_device.cuh"
@@ -36,7 +37,7 @@ struct PPar {
   int thermostat;
   double noise_v, noise_o;  // fluct.cxx:13-19
   int frozen;               // positions and velocities held; forces still measured
-  int hyd_pcl;              // gather blocks per particle (at most HYD_PCL_MAX)
+  int hyd_pcl;              // gather blocks per particle (a cluster; at most 8)
   int hyd_threads;          // threads per gather block (at most 1024)
   int sc_pcl;               // scatter blocks per particle
   int near_wrap;            // a neighbour's offsets may pass half the box (small grids)
@@ -281,26 +282,27 @@ __device__ void block_reduce(KSum (&v)[NV], double *sh /* [2*NV][32] */) {
 // thermostat kick of Add_random_force_thermostat (fluct.cxx:10-36) from a
 // precomputed table of its normals.
 // The scatters run PCL blocks per particle.  The gather runs p.hyd_pcl
-// blocks of p.hyd_threads threads per particle.  With one block per particle
-// the block's sums are the particle's and thread 0 updates it; with several,
-// each block stores its partial sums and the block that finishes last (a
-// per-particle arrival counter) adds the partials in a fixed order -- the
-// result does not depend on block scheduling -- and updates the particle.
+// blocks of p.hyd_threads threads per particle: a cluster, whose first block
+// adds the others' sums from their shared memory (in a fixed order) and
+// updates the particle.
 constexpr int PCL = 4;
-constexpr int HYD_PCL_MAX = 8;
 
+// Compiled for blocks of 1024 threads, that is 64 registers: a few values
+// spill, but with the 100 registers that smaller blocks would leave it, half
+// the blocks are resident (256 particles at 128^3: 15.7 -> 18.5 us).
 template <typename R>
 __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart *__restrict__ parts,
                                                                   const R *__restrict__ u, const short4 *__restrict__ cells,
                                                                   const double *__restrict__ noise, int euler,
                                                                   int *__restrict__ status,
-                                                                  double *__restrict__ partial,
-                                                                  int *__restrict__ arrivals,
                                                                   double *__restrict__ nc_corr = nullptr,
                                                                   unsigned *__restrict__ ovl = nullptr) {
   __shared__ double sh[2 * 9 * 32];
-  __shared__ int last;
   pdl_begin();
+  parts = pdl_fresh(parts);
+  u = pdl_fresh(u);
+  noise = pdl_fresh(noise);
+  if (nc_corr) nc_corr = pdl_fresh(nc_corr);
   const int n = blockIdx.x / p.hyd_pcl;
   const int rank = blockIdx.x % p.hyd_pcl;
   const int stride = p.hyd_pcl * blockDim.x;
@@ -425,8 +427,6 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
     }
   }
   if (p.lj_on) {
-    int mc[3];
-    for (int d = 0; d < 3; ++d) mc[d] = (int)(xp[d] / p.lc_r);
     // candidates: the neighbour list (every pair within the LJ cutoff is on
     // it) or all particles
     const int *lst = p.nbl ? p.nbl + (size_t)n * (NBL_MAX + 1) : nullptr;
@@ -435,25 +435,28 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
       const int j = lst ? lst[1 + t] : t;
       if (j == n) continue;
       const DPart &o = parts[j];
-      int mult = 1;
       double x12[3], r2 = 0.0;
       for (int d = 0; d < 3; ++d) {
-        // times the cell-list scan (md_force.cxx:72-121) meets this pair
-        const int cj = (int)(o.x[d] / p.lc_r);
-        int cnt = 0;
-        for (int off = -1; off <= 1; ++off) {
-          int c = mc[d] + off;
-          if (c < 0) c = p.lc[d] - 1;
-          if (c > p.lc[d] - 1) c = 0;
-          cnt += (c == cj);
-        }
-        mult *= cnt;
         x12[d] = o.x[d] - xp[d];
         x12[d] -= nint_d(x12[d] * p.invL[d]) * p.L[d];
         r2 += x12[d] * x12[d];
       }
       const double rij = sqrt(r2);
-      if (mult > 0 && rij < p.lj_cut) {
+      if (!(rij < p.lj_cut)) continue;
+      // times the cell-list scan (md_force.cxx:72-121) meets this pair
+      int mult = 1;
+      for (int d = 0; d < 3; ++d) {
+        const int mc = (int)(xp[d] / p.lc_r), cj = (int)(o.x[d] / p.lc_r);
+        int cnt = 0;
+        for (int off = -1; off <= 1; ++off) {
+          int c = mc + off;
+          if (c < 0) c = p.lc[d] - 1;
+          if (c > p.lc[d] - 1) c = 0;
+          cnt += (c == cj);
+        }
+        mult *= cnt;
+      }
+      if (mult > 0) {
         // Lennard_Jones_f (interaction.h:156-181)
         const double s = p.lj_dia / rij;
         double dmy = (s * s) * (s * s) * (s * s);
@@ -464,12 +467,12 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
       }
     }
   }
-  if (ovl && p.hyd_pcl == 1 && !p.nbl) {
+  if (ovl && !p.nbl) {
     // the overlap candidates of this particle for the scatter that follows
     // (centre distance below 2 (RADIUS + HXI)), as a bit per particle: one
     // word per 32 candidates, written by the warp that tested them
     const double lim = 2.0 * (p.RADIUS + p.HXI), lim2 = lim * lim;
-    for (int base = 0; base < p.Np; base += blockDim.x) {
+    for (int base = rank * blockDim.x; base < p.Np; base += stride) {
       const int j = base + threadIdx.x;
       bool near = false;
       if (j < p.Np && j != n) {
@@ -485,7 +488,20 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
       if ((threadIdx.x & 31) == 0 && base + (threadIdx.x & ~31) < p.Np) ovl[(size_t)n * 32 + (j >> 5)] = bal;
     }
   }
-  KSum acc[9];
+  // thread d ends the step of component d: its operands are on their way
+  // while the sums are added up
+  const int d = threadIdx.x;
+  const bool tail = rank == 0 && d < 3;
+  double v0 = 0.0, o0 = 0.0, frp = 0.0, g0 = 0.0, g1 = 0.0;
+  if (tail) {
+    v0 = a.v[d];
+    o0 = a.omega[d];
+    frp = a.fr_prev[d];
+    if (p.thermostat) {
+      g0 = noise[6 * (size_t)n + d];
+      g1 = noise[6 * (size_t)n + 3 + d];
+    }
+  }
   if constexpr (sizeof(R) == 4) {
     // each batch of a thread's hydro terms is summed in float; from there up
     // every sum is double (thread and warp sums plain, the sum over the warps
@@ -507,92 +523,66 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
       }
     }
     __syncthreads();
-    if (threadIdx.x == 0)
-#pragma unroll
-      for (int i = 0; i < 9; ++i) acc[i] = {sh[(2 * i) * 32], sh[(2 * i + 1) * 32]};
   } else {
+    KSum acc[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) acc[i] = {a9[i], 0.0};
     block_reduce<9>(acc, sh);
   }
-  KSum tot[9];
-  if (p.hyd_pcl == 1) {
-    // one block per particle: its sums are the particle's
-    if (threadIdx.x != 0) return;
-    for (int i = 0; i < 9; ++i) tot[i] = acc[i];
-  } else {
-    if (threadIdx.x == 0) {
-      double *pp = partial + ((size_t)n * p.hyd_pcl + rank) * 18;
-      for (int i = 0; i < 9; ++i) {
-        pp[2 * i] = acc[i].s;
-        pp[2 * i + 1] = acc[i].c;
+  // value i of the block: sh[2 i * 32] + sh[(2 i + 1) * 32]
+  if (p.hyd_pcl > 1) {
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    cl.sync();
+    if (rank == 0 && threadIdx.x < 9) {
+      const int i = threadIdx.x;
+      KSum t{sh[(2 * i) * 32], sh[(2 * i + 1) * 32]};
+      for (int q = 1; q < p.hyd_pcl; ++q) {
+        const double *o = cl.map_shared_rank(sh, q);
+        t.add(o[(2 * i) * 32]);
+        t.c += o[(2 * i + 1) * 32];
       }
-      __threadfence();
-      last = (atomicAdd(arrivals + n, 1) == p.hyd_pcl - 1);
+      sh[(2 * i) * 32] = t.s;
+      sh[(2 * i + 1) * 32] = t.c;
     }
-    __syncthreads();
-    if (!last || threadIdx.x != 0) return;
-    __threadfence();
-    arrivals[n] = 0;
-    for (int i = 0; i < 9; ++i) tot[i] = {0.0, 0.0};
-    for (int q = 0; q < p.hyd_pcl; ++q) {
-      const volatile double *pq = partial + ((size_t)n * p.hyd_pcl + q) * 18;
-      for (int i = 0; i < 9; ++i) {
-        tot[i].add(pq[2 * i]);
-        tot[i].c += pq[2 * i + 1];
-      }
-    }
+    cl.sync();  // the other blocks stay until their sums are read
   }
-  double fh[3], th[3], fr[3];
-  for (int d = 0; d < 3; ++d) {
-    fh[d] = p.fh_coef * (tot[d].s + tot[d].c);
-    th[d] = p.rotation ? p.fh_coef * (tot[3 + d].s + tot[3 + d].c) : 0.0;
-    fr[d] = tot[6 + d].s + tot[6 + d].c;
-  }
-  fr[p.gdir] -= p.grav;
+  if (!tail) return;
+  auto sum = [&](int i) { return sh[(2 * i) * 32] + sh[(2 * i + 1) * 32]; };
+  double fh = p.fh_coef * sum(d);
+  double th = p.rotation ? p.fh_coef * sum(3 + d) : 0.0;
+  double fr = sum(6 + d);
+  if (d == p.gdir) fr -= p.grav;
   if (nc_corr) {
     // learned near-contact correction of this step's hydrodynamic force/torque
-    for (int d = 0; d < 3; ++d) {
-      fh[d] += nc_corr[6 * (size_t)n + d];
-      if (p.rotation) th[d] += nc_corr[6 * (size_t)n + 3 + d];
-      nc_corr[6 * (size_t)n + d] = 0.0;
-      nc_corr[6 * (size_t)n + 3 + d] = 0.0;
-    }
+    double *nc = nc_corr + 6 * (size_t)n + d;
+    fh += nc[0];
+    if (p.rotation) th += nc[3];
+    nc[0] = 0.0;
+    nc[3] = 0.0;
   }
-  if (p.frozen) {
-    for (int d = 0; d < 3; ++d) {
-      a.fr_prev[d] = fr[d];
-      a.f_hydro_prev[d] = fh[d];
-      a.t_hydro_prev[d] = th[d];
-    }
-    return;
-  }
+  a.fr_prev[d] = fr;
+  a.f_hydro_prev[d] = fh;
+  a.t_hydro_prev[d] = th;
+  if (p.frozen) return;
   const double hdt = 0.5 * p.dt;
-  for (int d = 0; d < 3; ++d) {
-    a.v_old[d] = a.v[d];
-    a.omega_old[d] = a.omega[d];
-    if (euler) {
-      const double dmy = p.dt * p.IMASS, dmy_rot = p.dt * p.IMOI;
-      a.v[d] += dmy * (fh[d] + fr[d]);
-      a.omega[d] += dmy_rot * th[d];
-    } else {
-      const double dmy = hdt * p.IMASS, dmy_rot = hdt * p.IMOI;
-      a.v[d] += dmy * (2.0 * fh[d] + fr[d] + a.fr_prev[d]);
-      a.omega[d] += dmy_rot * 2.0 * th[d];
-    }
-    a.fr_prev[d] = fr[d];
-    a.f_hydro_prev[d] = fh[d];
-    a.t_hydro_prev[d] = th[d];
+  a.v_old[d] = v0;
+  a.omega_old[d] = o0;
+  if (euler) {
+    const double dmy = p.dt * p.IMASS, dmy_rot = p.dt * p.IMOI;
+    v0 += dmy * (fh + fr);
+    o0 += dmy_rot * th;
+  } else {
+    const double dmy = hdt * p.IMASS, dmy_rot = hdt * p.IMOI;
+    v0 += dmy * (2.0 * fh + fr + frp);
+    o0 += dmy_rot * 2.0 * th;
   }
   if (p.thermostat) {
-    const double *g = noise + 6 * (size_t)n;
-    for (int d = 0; d < 3; ++d) {
-      a.v[d] += g[d] * p.noise_v * p.IMASS;
-      if (p.rotation) a.omega[d] += g[3 + d] * p.noise_o * p.IMOI;
-    }
+    v0 += g0 * p.noise_v * p.IMASS;
+    if (p.rotation) o0 += g1 * p.noise_o * p.IMOI;
   }
-  for (int d = 0; d < 3; ++d)
-    if (!isfinite(a.v[d]) || !isfinite(a.omega[d])) atomicExch(status, -5);
+  a.v[d] = v0;
+  a.omega[d] = o0;
+  if (!isfinite(v0) || !isfinite(o0)) atomicExch(status, -5);
 }
 
 // ---------------------------------------------------------------------------
@@ -751,6 +741,9 @@ __global__ void __launch_bounds__(256) k_particles_scatter(PPar p, const DPart *
                                                            const unsigned *__restrict__ ovl = nullptr) {
   __shared__ NbShared nb[NB_MAX];
   pdl_begin();
+  parts = pdl_fresh(parts);
+  ustar = pdl_fresh(ustar);
+  if (ovl) ovl = pdl_fresh(ovl);
   const int n = blockIdx.x / p.sc_pcl;
   const int stride = p.sc_pcl * blockDim.x;
   const int first = (blockIdx.x % p.sc_pcl) * blockDim.x + threadIdx.x;

@@ -38,13 +38,55 @@ __device__ __forceinline__ void dft4(Cx<R> *v) {
   v[3] = csub(t1, t3);
 }
 
-// exp(SIGN 2 pi i k / 16), k = 0..7, from cos/sin of multiples of pi/8
+// Twiddle product with its roundings spelt out, so that kernels that do the
+// same transform give the same bits however the compiler fuses around it.
+__device__ __forceinline__ Cx<float> cmul_tw(Cx<float> a, Cx<float> w) {
+  return {fmaf(a.x, w.x, -__fmul_rn(a.y, w.y)), fmaf(a.x, w.y, __fmul_rn(a.y, w.x))};
+}
+__device__ __forceinline__ Cx<double> cmul_tw(Cx<double> a, Cx<double> w) {
+  return {fma(a.x, w.x, -__dmul_rn(a.y, w.y)), fma(a.x, w.y, __dmul_rn(a.y, w.x))};
+}
+
+// Radix-2 butterfly a = e + w o, b = e - w o with w = exp(SIGN 2 pi i k / 16).
+// w = c + i s is taken out as its larger part: with t = s/c,
+// w o = c ((x - t y) + i (y + t x)), and the outer factor goes into the
+// additions, so the butterfly is six fused multiply-adds (Linzer and Feig
+// 1993) where the product and two additions take eight operations; w = 1
+// and w = i need no product.  A 16-point network is 148 operations
+// instead of 180, an 8-point one 52 instead of 60.
 template <typename R, int SIGN>
-__device__ __forceinline__ Cx<R> w16(int k) {
-  const R c1 = R(0.92387953251128675613), s1 = R(0.38268343236508977173), h = R(0.70710678118654752440);
-  const R cs[8] = {R(1), c1, h, s1, R(0), -s1, -h, -c1};
-  const R sn[8] = {R(0), s1, h, c1, R(1), c1, h, s1};
-  return {cs[k], R(SIGN) * sn[k]};
+__device__ __forceinline__ void bfly16(int k, Cx<R> e, Cx<R> o, Cx<R> &a, Cx<R> &b) {
+  if (k == 0) {
+    a = cadd(e, o);
+    b = csub(e, o);
+    return;
+  }
+  if (k == 4) {
+    const Cx<R> t = mul_si<R, SIGN>(o);
+    a = cadd(e, t);
+    b = csub(e, t);
+    return;
+  }
+  // tan(pi/8) and the parts of w for k = 1, 2, 3 (and 8 - k)
+  const R tn = R(0.41421356237309504880), c1 = R(0.92387953251128675613), h = R(0.70710678118654752440);
+  const bool cosine = k <= 2 || k >= 6;              // |c| >= |s|
+  const R t = (k == 2 || k == 6) ? R(1) : tn;        // |smaller| / |larger|
+  const R m = (k == 2 || k == 6) ? h : c1;           // |larger|
+  const bool neg = k > 4;                            // c < 0
+  Cx<R> p;
+  if (cosine) {  // w o = c (o + (s/c) i o)
+    const R q = neg ? -t : t, sq = R(SIGN) * q;
+    p = {fma(-sq, o.y, o.x), fma(sq, o.x, o.y)};
+    const R c = neg ? -m : m;
+    a = {fma(c, p.x, e.x), fma(c, p.y, e.y)};
+    b = {fma(-c, p.x, e.x), fma(-c, p.y, e.y)};
+  } else {  // w o = s i (o - (c/s) i o)
+    const R q = neg ? -t : t, sq = R(SIGN) * q;  // c/s
+    p = {fma(sq, o.y, o.x), fma(-sq, o.x, o.y)};
+    const R c = R(SIGN) * m;  // s
+    a = {fma(-c, p.y, e.x), fma(c, p.x, e.y)};
+    b = {fma(c, p.y, e.x), fma(-c, p.x, e.y)};
+  }
 }
 
 template <typename R, int SIGN>
@@ -53,11 +95,7 @@ __device__ __forceinline__ void dft8(Cx<R> *v) {
   dft4<R, SIGN>(e);
   dft4<R, SIGN>(o);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const Cx<R> t = k == 0 ? o[0] : cmul(o[k], w16<R, SIGN>(2 * k));
-    v[k] = cadd(e[k], t);
-    v[k + 4] = csub(e[k], t);
-  }
+  for (int k = 0; k < 4; ++k) bfly16<R, SIGN>(2 * k, e[k], o[k], v[k], v[k + 4]);
 }
 
 template <typename R, int SIGN>
@@ -71,11 +109,7 @@ __device__ __forceinline__ void dft16(Cx<R> *v) {
   dft8<R, SIGN>(e);
   dft8<R, SIGN>(o);
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const Cx<R> t = k == 0 ? o[0] : cmul(o[k], w16<R, SIGN>(k));
-    v[k] = cadd(e[k], t);
-    v[k + 8] = csub(e[k], t);
-  }
+  for (int k = 0; k < 8; ++k) bfly16<R, SIGN>(k, e[k], o[k], v[k], v[k + 8]);
 }
 
 template <typename R, int SIGN>

@@ -97,6 +97,8 @@ __global__ void __launch_bounds__(256) k_x_zeta_to_u(Geo g, Twiddles<R> tw, cons
                                                      const double *__restrict__ uk_dc, Cx<R> *__restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
+  zeta = pdl_fresh(zeta);
+  uk_dc = pdl_fresh(uk_dc);
   const int NXv = LX > 0 ? (1 << LX) : g.NX, LXv = LX > 0 ? LX : g.lx;
   constexpr int W = 3 * KC;
   Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
@@ -157,6 +159,7 @@ __global__ void __launch_bounds__(256, 3) k_y_pass(Geo g, Twiddles<R> tw, const 
                                                 Cx<R> *__restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
+  in = pdl_fresh(in);
   Cx<R> *twy = reinterpret_cast<Cx<R> *>(smem_raw);
   Cx<R> *Y = twy + g.NY;      // [NY rows][KC]
   Cx<R> *scr = Y + g.NY * KC;  // FFT scratch
@@ -234,6 +237,7 @@ template <typename R>
 __global__ void __launch_bounds__(256) k_z_products(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ io) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
+  io = pdl_fresh(io);
   const int M = g.M;
   constexpr int NV = ZROWS * 3, NQ = ZROWS * 5;
   constexpr int EV = NV + 1, EQ = NQ + 1;  // odd element strides: conflict-free columns
@@ -303,6 +307,7 @@ __global__ void __launch_bounds__(256) k_z_c2r(Geo g, Twiddles<R> tw, const Cx<R
                                                DPart *__restrict__ parts, int euler, int *__restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
+  in = pdl_fresh(in);
   const int nrow_blocks = (g.NX * g.NY) / ZROWS;
   if ((int)blockIdx.x >= nrow_blocks) {
     const int n = ((int)blockIdx.x - nrow_blocks) * blockDim.x + threadIdx.x;
@@ -355,6 +360,7 @@ __global__ void __launch_bounds__(256) k_z_force(Geo g, Twiddles<R> tw, R *__res
                                                  Cx<R> *__restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
+  force = pdl_fresh(force);
   const int M = g.M;
   constexpr int NS = ZROWS * 3, ES = NS + 1;
   Cx<R> *twm = reinterpret_cast<Cx<R> *>(smem_raw);
@@ -428,6 +434,7 @@ __global__ void __launch_bounds__(256) k_z_r2c(Geo g, Twiddles<R> tw, const R *_
                                                size_t in_cstride, Cx<R> *__restrict__ out, int nkeep, int ostride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
+  in = pdl_fresh(in);
   const int M = g.M;
   constexpr int ES = ZROWS + 1;
   Cx<R> *twm = reinterpret_cast<Cx<R> *>(smem_raw);
@@ -547,6 +554,9 @@ __global__ void __launch_bounds__(256) k_x_advect_update(Geo g, Twiddles<R> tw, 
                                                          Cx<R> *__restrict__ zeta, double *__restrict__ uk_dc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
+  buf = pdl_fresh(buf);
+  zeta = pdl_fresh(zeta);
+  uk_dc = pdl_fresh(uk_dc);
   const int NXv = LX > 0 ? (1 << LX) : g.NX, LXv = LX > 0 ? LX : g.lx;
   constexpr int W5 = 5 * KC, W3 = 3 * KC;
   Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
@@ -657,6 +667,22 @@ __global__ void __launch_bounds__(256) k_x_advect_update(Geo g, Twiddles<R> tw, 
   }
 }
 
+// Reduced vorticity of the solenoidal part of one mode of the force:
+// Solenoidal_uk (operate_omega.cxx:186-219), then omega = -i k x f.
+template <typename R>
+__device__ __forceinline__ void force_mode_zeta(int KXi, int KYi, R kx, R ky, R kzr, R IK2, Cx<R> f0, Cx<R> f1,
+                                                Cx<R> f2, Cx<R> &z0, Cx<R> &z1) {
+  const Cx<R> dk = {IK2 * (f0.x * kx + f1.x * ky + f2.x * kzr), IK2 * (f0.y * kx + f1.y * ky + f2.y * kzr)};
+  f0 = {f0.x - dk.x * kx, f0.y - dk.y * kx};
+  f1 = {f1.x - dk.x * ky, f1.y - dk.y * ky};
+  f2 = {f2.x - dk.x * kzr, f2.y - dk.y * kzr};
+  Cx<R> w[3];
+  w[0] = cmul_mi(Cx<R>{ky * f2.x - kzr * f1.x, ky * f2.y - kzr * f1.y});
+  w[1] = cmul_mi(Cx<R>{kzr * f0.x - kx * f2.x, kzr * f0.y - kx * f2.y});
+  w[2] = cmul_mi(Cx<R>{kx * f1.x - ky * f0.x, kx * f1.y - ky * f0.y});
+  select_zeta(KXi, KYi, w, z0, z1);
+}
+
 // ---------------------------------------------------------------------------
 // x pass, forward, of the rigidity force f fused with the end of the step:
 // 2/3 truncation (implicit), Solenoidal_uk (operate_omega.cxx:186-219) and
@@ -674,6 +700,9 @@ __global__ void __launch_bounds__(256) k_x_force_to_zeta(Geo g, Twiddles<R> tw, 
                                                          Cx<R> *__restrict__ zeta, double *__restrict__ uk_dc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
+  buf = pdl_fresh(buf);
+  zeta = pdl_fresh(zeta);
+  uk_dc = pdl_fresh(uk_dc);
   const int NXv = LX > 0 ? (1 << LX) : g.NX, LXv = LX > 0 ? LX : g.lx;
   constexpr int W3 = 3 * KC;
   Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
@@ -736,17 +765,8 @@ __global__ void __launch_bounds__(256) k_x_force_to_zeta(Geo g, Twiddles<R> tw, 
     }
     const R K2 = kx * kx + ky * ky + kzr * kzr;
     const R IK2 = R(1) / K2;
-    const Cx<R> dk = {IK2 * (f0.x * kx + f1.x * ky + f2.x * kzr), IK2 * (f0.y * kx + f1.y * ky + f2.y * kzr)};
-    f0 = {f0.x - dk.x * kx, f0.y - dk.y * kx};
-    f1 = {f1.x - dk.x * ky, f1.y - dk.y * ky};
-    f2 = {f2.x - dk.x * kzr, f2.y - dk.y * kzr};
-    // omega = -i k x f
-    Cx<R> w[3];
-    w[0] = cmul_mi(Cx<R>{ky * f2.x - kzr * f1.x, ky * f2.y - kzr * f1.y});
-    w[1] = cmul_mi(Cx<R>{kzr * f0.x - kx * f2.x, kzr * f0.y - kx * f2.y});
-    w[2] = cmul_mi(Cx<R>{kx * f1.x - ky * f0.x, kx * f1.y - ky * f0.y});
     Cx<R> z0, z1;
-    select_zeta(KXi, KYi, w, z0, z1);
+    force_mode_zeta(KXi, KYi, kx, ky, kzr, IK2, f0, f1, f2, z0, z1);
     const size_t o = ((size_t)ix * g.KYc + iy) * g.TS + kz;
     z0 = cadd(Zs[ix * KC + col], z0);
     z1 = cadd(Zs[(g.KXc + ix) * KC + col], z1);
