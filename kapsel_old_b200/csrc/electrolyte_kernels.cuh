@@ -482,7 +482,6 @@ __global__ void __launch_bounds__(NW * 32) k_zw_charge(Geo g, Twiddles<R> tw, co
   scal = pdl_fresh(scal);
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
-  int turn = 0;
   Cx<R> w[Z::N1], wz[Z::N1];
   wfft_twiddles<R, LM>(tw.m, w);
   wpack_twiddles<R, LM>(tw.z, wz);
@@ -507,7 +506,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_charge(Geo g, Twiddles<R> tw, co
       if (charge) *reinterpret_cast<V2 *>(charge + o) = q;
       v[n1] = {q.x, q.y};
     }
-    wfft<R, LM, 1>(v, ex, turn, w);
+    wfft<R, LM, 1>(v, ex, w);
     wunpack_r2c<R, LM, NK>(v, out + row * OS, wz, tw.z);
   }
 }
@@ -534,7 +533,6 @@ __global__ void __launch_bounds__(NW * 32) k_zw_flux(Geo g, Twiddles<R> tw, Cx<R
   u = pdl_fresh(u);
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
-  int turn = 0;
   Cx<R> w[Z::N1], wz[Z::N1];
   wfft_twiddles<R, LM>(tw.m, w);
   wpack_twiddles<R, LM>(tw.z, wz);
@@ -550,7 +548,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_flux(Geo g, Twiddles<R> tw, Cx<R
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       wpack_c2r<R, LM>(line + c * cstr, f[c], wz);
-      wfft<R, LM, -1>(f[c], ex, turn, w);
+      wfft<R, LM, -1>(f[c], ex, w);
     }
 #pragma unroll
     for (int n1 = 0; n1 < Z::N1; ++n1) {
@@ -586,7 +584,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_flux(Geo g, Twiddles<R> tw, Cx<R
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      wfft<R, LM, 1>(f[c], ex, turn, w);
+      wfft<R, LM, 1>(f[c], ex, w);
       wunpack_r2c<R, LM>(f[c], line + c * cstr, wz, tw.z);
     }
   }
@@ -608,7 +606,6 @@ __global__ void __launch_bounds__(NW * 32) k_zw_coulomb(Geo g, Twiddles<R> tw, c
   charge = pdl_fresh(charge);
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
-  int turn = 0;
   Cx<R> w[Z::N1], wz[Z::N1];
   wfft_twiddles<R, LM>(tw.m, w);
   wpack_twiddles<R, LM>(tw.z, wz);
@@ -625,7 +622,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_coulomb(Geo g, Twiddles<R> tw, c
 #pragma unroll
     for (int n1 = 0; n1 < Z::N1; ++n1)
       q[n1] = *reinterpret_cast<const V2 *>(charge + row * Z::NZ + 2 * (wt<LM>() + Z::N2 * n1));
-    wfft<R, LM, -1>(v, ex, turn, w);
+    wfft<R, LM, -1>(v, ex, w);
 #pragma unroll
     for (int n1 = 0; n1 < Z::N1; ++n1) {
       R fx = -(v[n1].x * sc), fy = -(v[n1].y * sc);
@@ -633,7 +630,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_coulomb(Geo g, Twiddles<R> tw, c
       fy += e;
       v[n1] = {(q[n1].x * fx) * R(scale), (q[n1].y * fy) * R(scale)};
     }
-    wfft<R, LM, 1>(v, ex, turn, w);
+    wfft<R, LM, 1>(v, ex, w);
     wunpack_r2c<R, LM>(v, out + (c * rows + row) * Z::TS, wz, tw.z);
   }
 }

@@ -340,7 +340,7 @@ struct BoxBase {
   // factorisation of NX (fft2_n1_sel); time_variant times the current one
   int xsplit = 0;
   virtual bool xsplit_ok(int xs) const = 0;
-  virtual void set_xsplit(int xs) = 0;
+  virtual int set_xsplit(int xs) = 0;
   // the step runs the fused y/z plane kernels (k_yzw_c2r, k_zyw_r2c)
   virtual bool fused_yz() const { return false; }
   virtual int alloc_el() = 0;
@@ -468,6 +468,10 @@ struct Box : BoxBase {
     KCHECK(allow_smem(k_xw_advect<R, LX, 1>, T::smem(5, 2)));
     KCHECK(allow_smem(k_xw_force<R, LX, 0>, T::smem(3, 2)));
     KCHECK(allow_smem(k_xw_force<R, LX, 1>, T::smem(3, 2)));
+    return 0;
+  }
+  template <int LX>
+  int x_setup_block() {
     if constexpr (LX < 8) {
       KCHECK(allow_smem(k_x_zeta_to_u<R, KCX, LX, 1>, smem_xu));
       KCHECK(allow_smem(k_x_advect_update<R, KCX, 0, LX, 1>, smem_xadv));
@@ -596,28 +600,30 @@ struct Box : BoxBase {
 
   // fused y/z plane kernels (pass variant ymode 3): the inverse to u* and the
   // rigidity force as one launch each, for NY = 2^yz_ly (0: not available)
-  static constexpr int YZNW = 4;  // warps per block
   int yz_ly = 0;
   size_t yz_sm = 0;
   template <int LY, int LM>
   int yz_setup() {
-    const size_t sm = YZ<R, LY, LM>::smem(YZNW);
+    constexpr int NW = YZ<R, LY, LM>::NW;
+    const size_t sm = YZ<R, LY, LM>::smem();
     if (sm > 227 * 1024) return 0;
-    KCHECK(allow_smem(k_yzw_c2r<R, LY, LM, YZNW>, sm));
-    KCHECK(allow_smem(k_zyw_r2c<R, LY, LM, true, YZNW>, sm));
+    KCHECK(allow_smem(k_yzw_c2r<R, LY, LM, NW>, sm));
+    KCHECK(allow_smem(k_zyw_r2c<R, LY, LM, true, NW>, sm));
     yz_sm = sm;
     yz_ly = LY;
     return 0;
   }
   template <int LY, int LM>
   void yz_c2r_l(Launch pdl, R *out, DPart *pts, int euler) {
-    const int posblk = pts ? (Np + YZNW * 32 - 1) / (YZNW * 32) : 0;
-    launch_k(pdl, k_yzw_c2r<R, LY, LM, YZNW>, dim3(3 * g.NX + posblk), dim3(YZNW * 32), yz_sm, stream, g, tw,
+    constexpr int NW = YZ<R, LY, LM>::NW;
+    const int posblk = pts ? (Np + NW * 32 - 1) / (NW * 32) : 0;
+    launch_k(pdl, k_yzw_c2r<R, LY, LM, NW>, dim3(3 * g.NX + posblk), dim3(NW * 32), yz_sm, stream, g, tw,
              (const Cx<R> *)bufA, out, npts(), g.NZ, 3 * g.NX, pp, pts, euler, status);
   }
   template <int LY, int LM>
   void zy_force_l(Launch pdl) {
-    launch_k(pdl, k_zyw_r2c<R, LY, LM, true, YZNW>, dim3(3 * g.NX), dim3(YZNW * 32), yz_sm, stream, g, tw, force(),
+    constexpr int NW = YZ<R, LY, LM>::NW;
+    launch_k(pdl, k_zyw_r2c<R, LY, LM, true, NW>, dim3(3 * g.NX), dim3(NW * 32), yz_sm, stream, g, tw, force(),
              npts(), bufA);
   }
   // bufA (x real, ky compact) -> real fields, with the position update in extra blocks
@@ -842,8 +848,11 @@ struct Box : BoxBase {
   }
   size_t sm_y_any = 0;
   bool xsplit_ok(int xs) const override { return xs == 0 || (xs == 1 && g.NX >= 8 && g.NX <= 128); }
-  void set_xsplit(int xs) override {
-    if (xs == xsplit) return;
+  int set_xsplit(int xs) override {
+    if (xs == xsplit) return 0;
+    int rc = 0;
+    if (xs) with_len(g.lx, [&](auto l) { rc = x_setup_block<l.value>(); });
+    if (rc) return rc;
     xsplit = xs;
     // bufA's u_k was formed with the other split; the captured graphs hold
     // the other launches
@@ -853,6 +862,7 @@ struct Box : BoxBase {
         cudaGraphExecDestroy(graph[s]);
         graph[s] = nullptr;
       }
+    return 0;
   }
   bool variant_ok(int zmode, int ymode_) const override {
     if (prm.eq != KAPSEL_EQ_NAVIER_STOKES || zmode < 0 || zmode > 1 || ymode_ < 0 || ymode_ > 3) return false;
@@ -3125,7 +3135,7 @@ int kapsel_batch_create(kapsel_ctx *const *boxes, int n, int autotune, kapsel_ba
         float best = 0.f;
         for (int xs = 0; xs < 2; ++xs) {
           if (!x->xsplit_ok(xs)) continue;
-          x->set_xsplit(xs);
+          if (x->set_xsplit(xs)) continue;
           for (int zm = 0; zm < 2; ++zm)
             for (int ym = 0; ym < 4; ++ym) {
               if (!x->variant_ok(zm, ym)) continue;
@@ -3139,7 +3149,7 @@ int kapsel_batch_create(kapsel_ctx *const *boxes, int n, int autotune, kapsel_ba
         }
         chosen.push_back({key, {zp, yp, xp}});
       }
-      x->set_xsplit(xp);
+      if (x->set_xsplit(xp)) return KAPSEL_ECUDA;
       x->set_variant(zp, yp);
     }
     b->variants.clear();
@@ -3247,8 +3257,7 @@ int kapsel_gpu_set_x_split(kapsel_ctx *ctx, int split) {
   BoxBase *x = ctx->box.get();
   if (!x->xsplit_ok(split)) return KAPSEL_EINVAL;
   if (cudaStreamSynchronize(x->stream) != cudaSuccess) return KAPSEL_ECUDA;
-  x->set_xsplit(split);
-  return 0;
+  return x->set_xsplit(split);
 }
 
 int kapsel_gpu_set_pass_variant(kapsel_ctx *ctx, int zmode, int ymode) {

@@ -764,7 +764,6 @@ __global__ void __launch_bounds__(NW * 32) k_zw_cross(Geo g, Twiddles<R> tw, Cx<
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw + warp * zw_cross_bytes<R, LM>());
   Cx<R> *park = ex + ZX<R, LM>::ELEMS;  // [6][N1][32]
-  int turn = 0;
   Cx<R> w[Z::N1], wz[Z::N1];
   wfft_twiddles<R, LM>(tw.m, w);
   wpack_twiddles<R, LM>(tw.z, wz);
@@ -778,7 +777,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_cross(Geo g, Twiddles<R> tw, Cx<
     for (int c = 0; c < 6; ++c) {
       Cx<R>(&v)[Z::N1] = u[PARK ? 0 : c];
       wpack_c2r<R, LM>(line + c * cstr, v, wz);
-      wfft<R, LM, -1>(v, ex, turn, w);
+      wfft<R, LM, -1>(v, ex, w);
 #pragma unroll
       for (int n1 = 0; n1 < Z::N1; ++n1) {
         v[n1] = cscale(v[n1], sc);
@@ -795,7 +794,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_cross(Geo g, Twiddles<R> tw, Cx<
         const Cx<R> ua = get(a, n1), ub = get(b, n1), wa = get(3 + a, n1), wb = get(3 + b, n1);
         p[n1] = {ua.x * wb.x - ub.x * wa.x, ua.y * wb.y - ub.y * wa.y};
       }
-      wfft<R, LM, 1>(p, ex, turn, w);
+      wfft<R, LM, 1>(p, ex, w);
       wunpack_r2c<R, LM>(p, line + d * cstr, wz, tw.z);
     }
   }
@@ -822,7 +821,6 @@ __global__ void __launch_bounds__(NW * 32) k_zw_obl_force(Geo g, Twiddles<R> tw,
   uobl = pdl_fresh(uobl);
   const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
-  int turn = 0;
   Cx<R> w[Z::N1], wz[Z::N1];
   wfft_twiddles<R, LM>(tw.m, w);
   wpack_twiddles<R, LM>(tw.z, wz);
@@ -907,7 +905,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_obl_force(Geo g, Twiddles<R> tw,
     }
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      wfft<R, LM, 1>(v[d], ex, turn, w);
+      wfft<R, LM, 1>(v[d], ex, w);
       wunpack_r2c<R, LM>(v[d], out + d * cstr + (size_t)row * Z::TS, wz, tw.z);
     }
   }

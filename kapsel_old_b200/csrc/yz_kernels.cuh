@@ -30,7 +30,12 @@ struct YZ {
   static constexpr int EX = EX_Y > EX_Z ? EX_Y : EX_Z;    // per-warp exchange buffers
   static constexpr int NB = (Z::TZ + Y::RW - 1) / Y::RW;  // kz column batches
   static constexpr int NG = NY / Z::RW;                   // z row groups
-  static size_t smem(int nw) { return sizeof(Cx<R>) * ((size_t)NY * PS + (size_t)nw * EX); }
+  // warps per block: the blocks an SM holds are few (two to three at 128 x 128
+  // in FP32, one in FP64), so the large planes take eight (128^3 FP32 step with
+  // 4 and 8: 125 and 120 us; FP64 235 and 230); the small ones have no work for
+  // more than four (128x128x64 85 and 87; 64x64x128 FP64 67 and 69)
+  static constexpr int NW = NG >= 32 ? 8 : 4;
+  static size_t smem() { return sizeof(Cx<R>) * ((size_t)NY * PS + (size_t)NW * EX); }
 };
 
 // Inverse y, then z c2r, of planes (c, x) = blockIdx.x < nplanes:
@@ -57,7 +62,6 @@ __global__ void __launch_bounds__(NW * 32) k_yzw_c2r(Geo g, Twiddles<R> tw, cons
   const int warp = threadIdx.x >> 5;
   Cx<R> *plane = reinterpret_cast<Cx<R> *>(smem_raw);
   Cx<R> *ex = plane + P::NY * P::PS + warp * P::EX;
-  int turn = 0;
   const int pl = blockIdx.x;  // c * NX + x
   const int c = pl / g.NX;
   {
@@ -74,13 +78,12 @@ __global__ void __launch_bounds__(NW * 32) k_yzw_c2r(Geo g, Twiddles<R> tw, cons
 #pragma unroll
       for (int n1 = 0; n1 < Y::N1; ++n1) v[n1] = next[n1];
       if (b + NW < P::NB) load(b + NW);
-      wfft<R, LY, -1>(v, ex, turn, w);
+      wfft<R, LY, -1>(v, ex, w);
       const int col = b * Y::RW + wl<LY>();
       yw_store<R, LY, false, false>(plane + col, P::PS, col < Z::TZ, v);
     }
   }
   __syncthreads();
-  turn = 0;
   Cx<R> w[Z::N1], wz[Z::N1];
   wfft_twiddles<R, LM>(tw.m, w);
   wpack_twiddles<R, LM>(tw.z, wz);
@@ -90,7 +93,7 @@ __global__ void __launch_bounds__(NW * 32) k_yzw_c2r(Geo g, Twiddles<R> tw, cons
     const int row = grp * Z::RW + wl<LM>();
     Cx<R> v[Z::N1];
     wpack_c2r<R, LM>(plane + row * P::PS, v, wz);
-    wfft<R, LM, -1>(v, ex, turn, w);
+    wfft<R, LM, -1>(v, ex, w);
     wstore_real<R, LM>(v, dst + (size_t)row * out_pitch, sc);
   }
 }
@@ -111,7 +114,6 @@ __global__ void __launch_bounds__(NW * 32) k_zyw_r2c(Geo g, Twiddles<R> tw, R *_
   const int warp = threadIdx.x >> 5;
   Cx<R> *plane = reinterpret_cast<Cx<R> *>(smem_raw);
   Cx<R> *ex = plane + P::NY * P::PS + warp * P::EX;
-  int turn = 0;
   const int pl = blockIdx.x;  // c * NX + x
   const int c = pl / g.NX, x = pl - c * g.NX;
   {
@@ -135,19 +137,18 @@ __global__ void __launch_bounds__(NW * 32) k_zyw_r2c(Geo g, Twiddles<R> tw, R *_
           src[(size_t)grp * Z::RW * Z::M + Z::N2 * n1] = V2{R(0), R(0)};
       }
       if (grp + NW < P::NG) load(grp + NW);
-      wfft<R, LM, 1>(v, ex, turn, w);
+      wfft<R, LM, 1>(v, ex, w);
       wunpack_r2c<R, LM>(v, plane + (grp * Z::RW + wl<LM>()) * P::PS, wz, tw.z);
     }
   }
   __syncthreads();
-  turn = 0;
   Cx<R> w[Y::N1];
   wfft_twiddles<R, LY>(tw.y, w);
   for (int b = warp; b < P::NB; b += NW) {
     const int col = b * Y::RW + wl<LY>();
     Cx<R> v[Y::N1];
     yw_load<R, LY, false, false>(plane + col, P::PS, col < Z::TZ, v);
-    wfft<R, LY, 1>(v, ex, turn, w);
+    wfft<R, LY, 1>(v, ex, w);
     yw_store<R, LY, true, false>(out + (size_t)pl * YGeo<LY, false>::KYc * g.TS + col, g.TS, col < Z::TZ, v);
   }
 }

@@ -19,16 +19,18 @@
 // transform.  The kernels before this kept lines in shared memory between the
 // steps (6 accesses for an inverse, 7 for a forward transform) and ran into
 // the shared-memory pipe, 80% busy at 256^3.  Per launch, before and after:
-// products at 128^3 32.9 -> 20.3 us in FP32, 55 -> 37 in FP64, at 256^3 230 ->
-// 143 (76 at the memory rate; with 255 registers eight warps are resident on an
-// SM and wait for their rows); c2r at 256^3 76 (51), where the L1 pipe is 95%
-// busy: a warp's load touches four rows, 64 bytes of each.
+// products at 128^3 32.9 -> 20.5 us in FP32, 55 -> 36 in FP64, at 256^3 230 ->
+// 150 (76 at the memory rate; with 255 registers eight warps are resident on an
+// SM and wait for their rows; with the twiddles in shared memory and 168
+// registers 138, but FP64 377 -> 387, other lengths unchanged).  c2r at 256^3
+// 76 -> 68 (51) when A[M-k] came from the partner lane instead of a second
+// load: the L1 pipe was 95% busy, a warp's load touching four rows, 64 bytes of
+// each.
 //
 // Lanes are l-fastest (lane = t RW + l).  The exchange buffer
 // gives line l the offset l LS and row k1 the stride N2 + 1, with LS chosen so
 // that each bank wavefront (16 lanes of 8 bytes, 8 of 16) hits distinct banks
-// in both directions.  Two buffers take turns, so one warp barrier per
-// transform is enough.  z lengths are M = 16..128 (NZ = 32..256).
+// in both directions.  z lengths are M = 16..128 (NZ = 32..256).
 #pragma once
 
 #include "spectral_kernels.cuh"
@@ -45,14 +47,14 @@ struct ZL {
   static_assert(LM >= 4 && LM <= 8 && N1 >= N2, "line length");
 };
 
-// Exchange buffers of a warp: two of RW lines of N1 rows of N2 values.
+// Exchange buffer of a warp: RW lines of N1 rows of N2 values.
 template <typename R, int LM>
 struct ZX {
   using Z = ZL<LM>;
   static constexpr int W = sizeof(R) == 4 ? 16 : 8;  // elements per bank wavefront
   static constexpr int PL = Z::N1 * (Z::N2 + 1);
   static constexpr int LS = PL + ((W / Z::RW - PL % W) + W) % W;  // LS mod W = W / RW
-  static constexpr int BUF = Z::RW * LS, ELEMS = 2 * BUF;
+  static constexpr int ELEMS = Z::RW * LS;
   static constexpr size_t BYTES = sizeof(Cx<R>) * ELEMS;
 };
 
@@ -77,16 +79,15 @@ __device__ __forceinline__ void wpack_twiddles(const Cx<R> *__restrict__ twz, Cx
   for (int n1 = 0; n1 < ZL<LM>::N1; ++n1) wz[n1] = twz[wt<LM>() + ZL<LM>::N2 * n1];
 }
 
-// Transform of the warp's RW lines; `turn` alternates the exchange buffers
-// (every transform of the warp flips it).
-template <typename R, int LM, int SIGN>
-__device__ __forceinline__ void wfft(Cx<R> (&v)[ZL<LM>::N1], Cx<R> *ex, int &turn, const Cx<R> (&w)[ZL<LM>::N1]) {
+// Transform of the warp's RW lines; w[k1] are the lane's phase-1 twiddles.
+template <typename R, int LM, int SIGN, typename W>
+__device__ __forceinline__ void wfft(Cx<R> (&v)[ZL<LM>::N1], Cx<R> *ex, const W &w) {
   using Z = ZL<LM>;
   using X = ZX<R, LM>;
   const int t = wt<LM>();
-  Cx<R> *b = ex + turn * X::BUF + wl<LM>() * X::LS;
-  turn ^= 1;
+  Cx<R> *b = ex + wl<LM>() * X::LS;
   dft_small<R, SIGN>(v, Z::N1);
+  __syncwarp();  // the warp's last transform has read the buffer
   b[t] = v[0];
 #pragma unroll
   for (int k1 = 1; k1 < Z::N1; ++k1) b[k1 * (Z::N2 + 1) + t] = cmul_tw(v[k1], SIGN > 0 ? w[k1] : cconj(w[k1]));
@@ -102,25 +103,6 @@ __device__ __forceinline__ void wfft(Cx<R> (&v)[ZL<LM>::N1], Cx<R> *ex, int &tur
   }
 }
 
-// c2r packing of the lane's elements of one row A[k], k < NK (global or
-// shared): Z[k] = (A[k] + conj A[M-k]) + i (A[k] - conj A[M-k]) w_NZ^{-k}.
-template <typename R, int LM, int NK = ZL<LM>::TZ>
-__device__ __forceinline__ void wpack_c2r(const Cx<R> *A, Cx<R> (&v)[ZL<LM>::N1], const Cx<R> (&wz)[ZL<LM>::N1]) {
-  using Z = ZL<LM>;
-  const int t = wt<LM>();
-  const Cx<R> zero = {R(0), R(0)};
-  Cx<R> a[Z::N1], b[Z::N1];
-#pragma unroll
-  for (int n1 = 0; n1 < Z::N1; ++n1) {
-    const int k = t + Z::N2 * n1;
-    a[n1] = k < NK ? A[k] : zero;
-    b[n1] = Z::M - k < NK ? cconj(A[Z::M - k]) : zero;
-  }
-#pragma unroll
-  for (int n1 = 0; n1 < Z::N1; ++n1)
-    v[n1] = cadd(cadd(a[n1], b[n1]), cmul_pi(cmul(csub(a[n1], b[n1]), cconj(wz[n1]))));
-}
-
 __device__ __forceinline__ Cx<float> shfl_cx(Cx<float> v, int src) {
   return {__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
 }
@@ -128,12 +110,36 @@ __device__ __forceinline__ Cx<double> shfl_cx(Cx<double> v, int src) {
   return {__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
 }
 
+// c2r packing of the lane's elements of one row A[k], k < NK (global or
+// shared): Z[k] = (A[k] + conj A[M-k]) + i (A[k] - conj A[M-k]) w_NZ^{-k}.
+// A[M-k] is element N1-1-n1 of lane N2-t (of the lane itself, shifted by one,
+// at t = 0).  Every lane of the warp calls it.
+template <typename R, int LM, int NK = ZL<LM>::TZ, typename W>
+__device__ __forceinline__ void wpack_c2r(const Cx<R> *A, Cx<R> (&v)[ZL<LM>::N1], const W &wz) {
+  using Z = ZL<LM>;
+  const int t = wt<LM>(), src = (((Z::N2 - t) & (Z::N2 - 1)) << Z::LR) + wl<LM>();
+  const Cx<R> zero = {R(0), R(0)};
+  Cx<R> a[Z::N1];
+#pragma unroll
+  for (int n1 = 0; n1 < Z::N1; ++n1) {
+    const int k = t + Z::N2 * n1;
+    a[n1] = k < NK ? A[k] : zero;
+  }
+  const Cx<R> top = NK == Z::M + 1 && t == 0 ? A[Z::M] : zero;
+#pragma unroll
+  for (int n1 = 0; n1 < Z::N1; ++n1) {
+    const Cx<R> p = Z::N2 * (Z::N1 - 1 - n1) < NK ? shfl_cx(a[Z::N1 - 1 - n1], src) : zero;
+    const Cx<R> b = cconj(t == 0 ? (n1 == 0 ? top : a[(Z::N1 - n1) & (Z::N1 - 1)]) : p);
+    v[n1] = cadd(cadd(a[n1], b), cmul_pi(cmul(csub(a[n1], b), cconj(wz[n1]))));
+  }
+}
+
 // r2c unpacking of a transformed line to dst[k], k < NK:
 // A[k] = (Z[k] + conj Z[M-k])/2 - i/2 (Z[k] - conj Z[M-k]) w_NZ^k.  Z[M-k] is
 // element N1-1-n1 of lane N2-t (of the lane itself, shifted by one, at t = 0).
 // Every lane of the warp calls it; `put` is off for rows that do not exist.
-template <typename R, int LM, int NK = ZL<LM>::TZ>
-__device__ __forceinline__ void wunpack_r2c(const Cx<R> (&v)[ZL<LM>::N1], Cx<R> *dst, const Cx<R> (&wz)[ZL<LM>::N1],
+template <typename R, int LM, int NK = ZL<LM>::TZ, typename W>
+__device__ __forceinline__ void wunpack_r2c(const Cx<R> (&v)[ZL<LM>::N1], Cx<R> *dst, const W &wz,
                                             const Cx<R> *__restrict__ twz) {
   using Z = ZL<LM>;
   const int t = wt<LM>(), src = (((Z::N2 - t) & (Z::N2 - 1)) << Z::LR) + wl<LM>();
@@ -199,7 +205,6 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products(Geo g, Twiddles<R> tw, 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw + warp * zw_products_bytes<R, LM>());
   Cx<R> *park = ex + ZX<R, LM>::ELEMS;  // [3][N1][32]
-  int turn = 0;
   Cx<R> w[Z::N1], wz[Z::N1];
   wfft_twiddles<R, LM>(tw.m, w);
   wpack_twiddles<R, LM>(tw.z, wz);
@@ -215,7 +220,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products(Geo g, Twiddles<R> tw, 
     for (int c = 0; c < 3; ++c) {
       Cx<R>(&v)[Z::N1] = u[PARK ? 0 : c];
       wpack_c2r<R, LM>(line + c * cstr, v, wz);
-      wfft<R, LM, -1>(v, ex, turn, w);
+      wfft<R, LM, -1>(v, ex, w);
 #pragma unroll
       for (int n1 = 0; n1 < Z::N1; ++n1) v[n1] = cscale(v[n1], sc);
       if (STORE) wstore_real<R, LM>(v, ureal + (c * rows + row) * Z::NZ, R(1));
@@ -235,7 +240,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products(Geo g, Twiddles<R> tw, 
         const Cx<R> x = get(a, n1), y = get(b, n1);
         p[n1] = q < 3 ? Cx<R>{x.x * y.x, x.y * y.y} : Cx<R>{(x.x - y.x) * (x.x + y.x), (x.y - y.y) * (x.y + y.y)};
       }
-      wfft<R, LM, 1>(p, ex, turn, w);
+      wfft<R, LM, 1>(p, ex, w);
       wunpack_r2c<R, LM>(p, line + q * cstr, wz, tw.z);
     }
   }
@@ -261,7 +266,6 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
   }
   const int warp = threadIdx.x >> 5;
   Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
-  int turn = 0;
   Cx<R> w[Z::N1], wz[Z::N1];
   wfft_twiddles<R, LM>(tw.m, w);
   wpack_twiddles<R, LM>(tw.z, wz);
@@ -273,7 +277,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
     const size_t row = (size_t)(task - c * ngroups) * Z::RW + wl<LM>();
     Cx<R> v[Z::N1];
     wpack_c2r<R, LM>(in + (c * rows + row) * Z::TS, v, wz);
-    wfft<R, LM, -1>(v, ex, turn, w);
+    wfft<R, LM, -1>(v, ex, w);
     wstore_real<R, LM>(v, out + c * out_cstride + row * out_pitch, sc);
   }
 }
@@ -294,7 +298,6 @@ __global__ void __launch_bounds__(NW * 32) k_zw_r2c(Geo g, Twiddles<R> tw, R *__
   in = pdl_fresh(in);
   const int warp = threadIdx.x >> 5;
   Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
-  int turn = 0;
   Cx<R> w[Z::N1], wz[Z::N1];
   wfft_twiddles<R, LM>(tw.m, w);
   wpack_twiddles<R, LM>(tw.z, wz);
@@ -313,7 +316,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_r2c(Geo g, Twiddles<R> tw, R *__
       v[n1] = {x[n1].x, x[n1].y};
       if (CLEAR && (x[n1].x != R(0) || x[n1].y != R(0))) src[Z::N2 * n1] = V2{R(0), R(0)};
     }
-    wfft<R, LM, 1>(v, ex, turn, w);
+    wfft<R, LM, 1>(v, ex, w);
     wunpack_r2c<R, LM, NK>(v, out + (c * rows + row) * OS, wz, tw.z);
   }
 }
