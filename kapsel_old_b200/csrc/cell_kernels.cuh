@@ -40,6 +40,8 @@ __device__ __forceinline__ void cell_coords(const double *x, const CellPar &c, i
 
 __global__ void k_cell_count(PPar p, CellPar c, const DPart *__restrict__ parts, int *__restrict__ cellof,
                              int *__restrict__ count) {
+  pdl_begin();
+  parts = pdl_fresh(parts);
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= p.Np) return;
   int ci[3];
@@ -50,18 +52,25 @@ __global__ void k_cell_count(PPar p, CellPar c, const DPart *__restrict__ parts,
 }
 
 // Exclusive scan of the per-cell counts (one block of 1024 threads): start
-// and cursor, and the counts cleared for the next build.
+// and cursor, and the counts cleared for the next build.  One round of the
+// block takes eight neighbouring cells a thread, since a round's barriers and
+// loads are what it costs (9000 cells, one a thread: 14.5 us).
+constexpr int SCAN_CELLS = 8;
 __global__ void __launch_bounds__(1024) k_cell_scan(CellPar c, int *__restrict__ count, int *__restrict__ start,
                                                     int *__restrict__ cursor) {
   __shared__ int wsum[32];
-  __shared__ int carry;
+  pdl_begin();
+  count = pdl_fresh(count);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < c.ncell; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    const int v = i < c.ncell ? count[i] : 0;
-    int incl = v;
+  int carry = 0;  // cells' counts before this round, the same in every thread
+  for (int base = 0; base < c.ncell; base += SCAN_CELLS * blockDim.x) {
+    const int i0 = base + SCAN_CELLS * threadIdx.x;
+    int v[SCAN_CELLS], sum = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_CELLS; ++k) v[k] = i0 + k < c.ncell ? count[i0 + k] : 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_CELLS; ++k) sum += v[k];
+    int incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -69,23 +78,31 @@ __global__ void __launch_bounds__(1024) k_cell_scan(CellPar c, int *__restrict__
     }
     if (lane == 31) wsum[warp] = incl;
     __syncthreads();
-    int before = carry;
-    for (int w = 0; w < warp; ++w) before += wsum[w];
-    if (i < c.ncell) {
-      const int ex = before + incl - v;
-      start[i] = ex;
-      cursor[i] = ex;
-      count[i] = 0;
+    int w = wsum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += t;
     }
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) carry += wsum[w];
-    __syncthreads();
+    const int warps_before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+    int ex = carry + (warp > 0 ? warps_before : 0) + incl - sum;
+#pragma unroll
+    for (int k = 0; k < SCAN_CELLS; ++k)
+      if (i0 + k < c.ncell) {
+        start[i0 + k] = ex;
+        cursor[i0 + k] = ex;
+        count[i0 + k] = 0;
+        ex += v[k];
+      }
+    carry += __shfl_sync(0xffffffffu, w, 31);
+    __syncthreads();  // wsum is written again
   }
   if (threadIdx.x == 0) start[c.ncell] = carry;
 }
 
 __global__ void k_cell_fill(PPar p, const int *__restrict__ cellof, int *__restrict__ cursor, int *__restrict__ list) {
+  pdl_begin();
+  cellof = pdl_fresh(cellof);
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= p.Np) return;
   list[atomicAdd(cursor + cellof[n], 1)] = n;
@@ -93,6 +110,9 @@ __global__ void k_cell_fill(PPar p, const int *__restrict__ cellof, int *__restr
 
 // Members of each cell in increasing particle index (a cell holds a few).
 __global__ void k_cell_sort(CellPar c, const int *__restrict__ start, int *__restrict__ list) {
+  pdl_begin();
+  start = pdl_fresh(start);
+  list = pdl_fresh(list);
   const int cell = blockIdx.x * blockDim.x + threadIdx.x;
   if (cell >= c.ncell) return;
   const int b = start[cell], e = start[cell + 1];
@@ -110,14 +130,22 @@ __global__ void k_cell_sort(CellPar c, const int *__restrict__ start, int *__res
 // Neighbour list of each particle: count, then up to NBL_MAX indices in
 // increasing order, of the particles within the list range (minimum image).
 // More neighbours than NBL_MAX: KAPSEL_ERANGE in the status word.  One warp
-// per particle: the lanes test a cell's members together and append the
-// hits in cell order (ballot), then each lane places its entries by rank.
+// per particle: the lanes read the bounds of the (up to 27) neighbouring cells
+// together, share the members of all of them out among themselves, append the
+// hits (ballot), then each lane places its entries by rank.  The chain of
+// dependent loads is what it costs, and cell after cell it was 27 times as long
+// (8600 particles at 256^3, the five launches with the position update, timed
+// alone: 82 -> 54 us; the step, with the launches chained, 1154 -> 1131).
 constexpr int NBL_WARPS = 4;  // particles per block
 __global__ void __launch_bounds__(NBL_WARPS * 32) k_neighbor_lists(PPar p, CellPar c, const DPart *__restrict__ parts,
                                                                    const int *__restrict__ start,
                                                                    const int *__restrict__ list, int *__restrict__ nbl,
                                                                    int *__restrict__ status) {
   __shared__ int cand[NBL_WARPS][NBL_MAX];
+  pdl_begin();
+  parts = pdl_fresh(parts);
+  start = pdl_fresh(start);
+  list = pdl_fresh(list);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = blockIdx.x * NBL_WARPS + warp;
   if (n >= p.Np) return;  // a whole warp: no later block-wide barrier
@@ -125,43 +153,58 @@ __global__ void __launch_bounds__(NBL_WARPS * 32) k_neighbor_lists(PPar p, CellP
   const double xn[3] = {parts[n].x[0], parts[n].x[1], parts[n].x[2]};
   int ci[3];
   cell_coords(xn, c, ci);
-  int cnt = 0;
-  for (int ox = -1; ox <= 1; ++ox) {
-    // each distinct neighbouring cell once (fewer than 3 cells on an axis)
-    if ((c.lc[0] == 1 && ox != 0) || (c.lc[0] == 2 && ox == -1)) continue;
-    const int cx = (ci[0] + ox + c.lc[0]) % c.lc[0];
-    for (int oy = -1; oy <= 1; ++oy) {
-      if ((c.lc[1] == 1 && oy != 0) || (c.lc[1] == 2 && oy == -1)) continue;
-      const int cy = (ci[1] + oy + c.lc[1]) % c.lc[1];
-      for (int oz = -1; oz <= 1; ++oz) {
-        if ((c.lc[2] == 1 && oz != 0) || (c.lc[2] == 2 && oz == -1)) continue;
-        const int cz = (ci[2] + oz + c.lc[2]) % c.lc[2];
-        const int cell = (cx * c.lc[1] + cy) * c.lc[2] + cz;
-        const int b = start[cell], e = start[cell + 1];
-        for (int k0 = b; k0 < e; k0 += 32) {
-          const int k = k0 + lane;
-          int j = -1;
-          bool hit = false;
-          if (k < e) {
-            j = list[k];
-            if (j != n) {
-              double s = 0.0;
+  // lane q < 27: cell (ox, oy, oz); each distinct neighbouring cell once
+  // (fewer than 3 cells on an axis)
+  int first = 0, len = 0;
+  if (lane < 27) {
+    const int o[3] = {lane / 9 - 1, lane / 3 % 3 - 1, lane % 3 - 1};
+    int cc[3];
+    bool use = true;
 #pragma unroll
-              for (int d = 0; d < 3; ++d) {
-                double dd = parts[j].x[d] - xn[d];
-                dd -= nint_d(dd * p.invL[d]) * p.L[d];
-                s += dd * dd;
-              }
-              hit = s < c.r2list;
-            }
-          }
-          const unsigned bal = __ballot_sync(0xffffffffu, hit);
-          const int pos = cnt + __popc(bal & ((1u << lane) - 1u));
-          if (hit && pos < NBL_MAX) cw[pos] = j;
-          cnt += __popc(bal);
+    for (int d = 0; d < 3; ++d) {
+      if ((c.lc[d] == 1 && o[d] != 0) || (c.lc[d] == 2 && o[d] == -1)) use = false;
+      cc[d] = (ci[d] + o[d] + c.lc[d]) % c.lc[d];
+    }
+    if (use) {
+      const int cell = (cc[0] * c.lc[1] + cc[1]) * c.lc[2] + cc[2];
+      first = start[cell];
+      len = start[cell + 1] - first;
+    }
+  }
+  int incl = len;  // members of the cells up to this lane's
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  const int base = first - (incl - len), total = __shfl_sync(0xffffffffu, incl, 31);
+  int cnt = 0;
+  for (int t0 = 0; t0 < total; t0 += 32) {
+    const int t = t0 + lane;
+    int q = 0;  // cells that end at or before member t
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+      if (__shfl_sync(0xffffffffu, incl, q + s - 1) <= t) q += s;
+    const int at = __shfl_sync(0xffffffffu, base, q) + t;
+    int j = -1;
+    bool hit = false;
+    if (t < total) {
+      j = list[at];
+      if (j != n) {
+        double s = 0.0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          double dd = parts[j].x[d] - xn[d];
+          dd -= nint_d(dd * p.invL[d]) * p.L[d];
+          s += dd * dd;
         }
+        hit = s < c.r2list;
       }
     }
+    const unsigned bal = __ballot_sync(0xffffffffu, hit);
+    const int pos = cnt + __popc(bal & ((1u << lane) - 1u));
+    if (hit && pos < NBL_MAX) cw[pos] = j;
+    cnt += __popc(bal);
   }
   __syncwarp();
   if (cnt > NBL_MAX) {

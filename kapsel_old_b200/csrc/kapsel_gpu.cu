@@ -309,14 +309,15 @@ struct BoxBase {
   }
   // the lists of the current positions (five launches), before any kernel
   // that reads them
-  void launch_cells() {
+  void launch_cells(Launch how = Launch()) {
     if (!cl_on || Np == 0) return;
-    k_cell_count<<<(Np + 255) / 256, 256, 0, stream>>>(pp, clp, parts, cl_cellof, cl_count);
-    k_cell_scan<<<1, 1024, 0, stream>>>(clp, cl_count, cl_start, cl_cursor);
-    k_cell_fill<<<(Np + 255) / 256, 256, 0, stream>>>(pp, cl_cellof, cl_cursor, cl_list);
-    k_cell_sort<<<(clp.ncell + 255) / 256, 256, 0, stream>>>(clp, cl_start, cl_list);
-    k_neighbor_lists<<<(Np + NBL_WARPS - 1) / NBL_WARPS, NBL_WARPS * 32, 0, stream>>>(pp, clp, parts, cl_start,
-                                                                                   cl_list, nbl, status);
+    const int nb = (Np + 255) / 256;
+    launch_k(how, k_cell_count, dim3(nb), dim3(256), 0, stream, pp, clp, (const DPart *)parts, cl_cellof, cl_count);
+    launch_k(how, k_cell_scan, dim3(1), dim3(1024), 0, stream, clp, cl_count, cl_start, cl_cursor);
+    launch_k(how, k_cell_fill, dim3(nb), dim3(256), 0, stream, pp, (const int *)cl_cellof, cl_cursor, cl_list);
+    launch_k(how, k_cell_sort, dim3((clp.ncell + 255) / 256), dim3(256), 0, stream, clp, (const int *)cl_start, cl_list);
+    launch_k(how, k_neighbor_lists, dim3((Np + NBL_WARPS - 1) / NBL_WARPS), dim3(NBL_WARPS * 32), 0, stream, pp, clp,
+             (const DPart *)parts, (const int *)cl_start, (const int *)cl_list, nbl, status);
   }
   void free_cells() {
     cudaFree(cl_count);
@@ -987,7 +988,7 @@ struct Box : BoxBase {
     mark();
     if (Np > 0) {
       if (!fuse_pos) k_particles_position<<<(Np + 127) / 128, 128, 0, stream>>>(pp, parts, euler, status);
-      launch_cells();  // neighbour lists of the new positions (large particle counts)
+      launch_cells(pdl);  // neighbour lists of the new positions (large particle counts)
       mark();
       if (nc) launch_nearcontact();  // timed with the position slot when profiling
       launch_kc(pp.hyd_pcl, pdl, k_particles_hydro_velocity<R>, dim3(Np * pp.hyd_pcl), dim3(pp.hyd_threads), 0,
