@@ -95,6 +95,9 @@ def kernel_bytes(cfg, R: int):
         # fused y/z plane kernels: the y pass's intermediate stays on chip
         "k_yzw_c2r": 3 * I1 + 3 * N * R,
         "k_zyw_force": 7 * N * R + 3 * I1,
+        # the same pair where the scatter has formed the force (its stencil's
+        # points are counted with the scatter)
+        "k_zyw_r2c": 3 * N * R + 3 * I1,
     }
 
 

@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(1024) k_cell_scan(CellPar c, int *__restrict__
   pdl_begin();
   count = pdl_fresh(count);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int carry = 0;  // cells' counts before this round, the same in every thread
+  int carry = 0;  // counts before this pass of the loop, the same in every thread
   for (int base = 0; base < c.ncell; base += SCAN_CELLS * blockDim.x) {
     const int i0 = base + SCAN_CELLS * threadIdx.x;
     int v[SCAN_CELLS], sum = 0;

@@ -2,21 +2,23 @@
 // sequence, CUDA graph replay and the C ABI declared in include/kapsel_gpu.h.
 //
 // One SPM step (Time_evolution_hydro, sp_3d_ns.cxx:61-212, Navier_Stokes
-// branch) is 12 launches (13 kernels; 8 runs in extra blocks of 7), each
-// after the first launched with programmatic stream serialization:
-//   1 k_x_zeta_to_u        truncated zeta -> u_k -> inverse x
-//   2 k_y_pass<inv>        inverse y (3 comps)
-//   3 k_z_products         inverse z, 5 products, forward z
-//   4 k_y_pass<fwd>        forward y (5 comps)
-//   5 k_x_advect_update    forward x, Omega, slaved Euler, FIX_CELL, u*_k, inverse x
-//   6 k_y_pass<inv>        inverse y (3 comps)
-//   7 k_z_c2r              inverse z -> u* (real)
-//   8 (k_z_c2r blocks)     AB2 / Euler positions and orientations
+// branch) is 12 launches (8 runs in extra blocks of 7) chained with
+// programmatic stream serialization.  A steady step leaves out 1, which the
+// last step's 13 has done; where the y/z plane kernels run, 6 + 7 are
+// k_yzw_c2r and 11 + 12 k_zyw_r2c.
+//   1 k_xw_zeta_to_u       truncated zeta -> u_k -> inverse x
+//   2 k_yt_pass            inverse y (3 comps)
+//   3 k_zw_products        inverse z, 5 products, forward z
+//   4 k_yt_pass            forward y (5 comps)
+//   5 k_xw_advect          forward x, Omega, slaved Euler, FIX_CELL, u*_k, inverse x
+//   6 k_yt_pass            inverse y (3 comps)
+//   7 k_zw_c2r             inverse z -> u* (real)
+//   8 (blocks of 7)        AB2 / Euler positions and orientations
 //   9 k_particles_hydro_velocity  hydro force+torque gather, LJ, gravity, velocity, thermostat
 //  10 k_particles_scatter  phi, phi*u_p, clamp, f = up - phi u*
-//  11 k_z_force            forward z of f, f cleared
-//  12 k_y_pass<fwd>        forward y (3 comps)
-//  13 k_x_force_to_zeta    forward x, solenoidal projection, zeta += zeta(f), uk_dc += f(0)
+//  11 k_zw_r2c             forward z of f, f cleared
+//  12 k_yt_pass            forward y (3 comps)
+//  13 k_xw_force           forward x, solenoidal projection, zeta += zeta(f), uk_dc += f(0), next u_k
 // The 20 3D FFTs of the reference become 14 pruned ones because
 // U2zeta_k(u* + f_sol) = trunc(zeta) + U_k2zeta_k(f_sol) (linearity).
 #include <cuda_runtime.h>
