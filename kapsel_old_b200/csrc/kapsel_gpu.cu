@@ -785,12 +785,15 @@ struct Box : BoxBase {
       // 59, 65; electrolyte 64^3 FP32 194, 152, 173, 171, FP64 280, 216, 226,
       // 230; Lees-Edwards 64^3 79, 72, 70, 76; 64x64x128 65, 60, 59, 61;
       // 128x64x128 84, 87, 73, 75; 128^3 125, 153, 133, 124; electrolyte 128^3
-      // 446, 533, 450, 423; Lees-Edwards 128^3 203, 231, 204, 198; but 128^3
-      // FP64 235, 273, 240, 240 and 256^3 1198, 1505, 1248, 1377.
+      // 446, 533, 450, 423; Lees-Edwards 128^3 203, 231, 204, 198.  With each
+      // kernel's own, 70 and 80%: 256x128x128 201, 197, 202; 128x128x256 207,
+      // 206, 208; 256^3 1135, 1138, 1180; FP64 128x64x128 129, 121, 121;
+      // 128x128x64 144, 145, 145; 128^3 229, 233, 229; electrolyte 128^3 824,
+      // 773, 790; Lees-Edwards 128^3 344, 341, 345.
       if (npts() <= (size_t)1 << 19)
         carve = prm.eq == KAPSEL_EQ_ELECTROLYTE ? 25 : 45;
-      else if (npts() <= (size_t)1 << 21 && sizeof(R) == 4)
-        carve = 70;
+      else if (npts() <= (size_t)1 << (sizeof(R) == 4 ? 22 : 21))
+        carve = sizeof(R) == 8 && prm.eq == KAPSEL_EQ_NAVIER_STOKES ? 80 : 70;
       if (zw && yz_ly && !(sizeof(R) == 4 && g.NZ == 256)) ymode = 3;
     }
     KCHECK(allow_smem(k_y_pass<R, true, KCY>, smem_y));
