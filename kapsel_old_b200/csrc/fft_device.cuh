@@ -133,6 +133,9 @@ __device__ __forceinline__ void cp_async_cx(Cx<R> *smem, const Cx<R> *gmem) {
 // does not write, which the compiler may take for memory that never changes
 // while the kernel runs, were moved up across the wait (wrong results; seen
 // with constant loads in front of the wait, and in an FP64 kernel without).
+// For the same reason no `__ldg` of such data: its read-only path is allowed
+// only for memory that nothing writes while the kernel is resident, and this
+// kernel is resident while the launch before it writes.
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
       for (int k = 0; k < GB; ++k)
         if (ph[k] != 0.f)
 #pragma unroll
-          for (int d = 0; d < 3; ++d) ug[k][d] = (float)__ldg(u + d * npts + im[k]);
+          for (int d = 0; d < 3; ++d) ug[k][d] = (float)u[d * npts + im[k]];
 #pragma unroll
       for (int k = 0; k < GB; ++k) {
         if (ph[k] == 0.f) continue;
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(1024) k_particles_hydro_velocity(PPar p, DPart
         // the profile's exponentials
         if (dist < p.RADIUS + p.HXI) {
 #pragma unroll
-          for (int d = 0; d < 3; ++d) ug[k][d] = (double)__ldg(u + d * npts + im);
+          for (int d = 0; d < 3; ++d) ug[k][d] = (double)u[d * npts + im];
           ph[k] = (double)prof_phi<R>(dist, p);
         }
       }

@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(256) k_z_c2r(Geo g, Twiddles<R> tw, const Cx<R
   const int nrow_blocks = (g.NX * g.NY) / ZROWS;
   if ((int)blockIdx.x >= nrow_blocks) {
     const int n = ((int)blockIdx.x - nrow_blocks) * blockDim.x + threadIdx.x;
-    if (blockIdx.y == 0 && parts && n < pp.Np) position_update_one(pp, parts, n, euler, status);
+    if (blockIdx.y == 0 && parts && n < pp.Np) position_update_one(pp, pdl_fresh(parts), n, euler, status);
     return;
   }
   const int M = g.M;

@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
   in = pdl_fresh(in);
   if ((int)blockIdx.x >= nblk) {
     const int n = ((int)blockIdx.x - nblk) * blockDim.x + threadIdx.x;
-    if (parts && n < pp.Np) position_update_one(pp, parts, n, euler, status);
+    if (parts && n < pp.Np) position_update_one(pp, pdl_fresh(parts), n, euler, status);
     return;
   }
   const int warp = threadIdx.x >> 5;
