@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products(Geo g, Twiddles<R> tw, 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
   io = pdl_fresh(io);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw + warp * zw_products_bytes<R, LM>());
   Cx<R> *park = ex + ZX<R, LM>::ELEMS;  // [3][N1][32]
   Cx<R> w[Z::N1], wz[Z::N1];
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_products(Geo g, Twiddles<R> tw, 
   const size_t cstr = rows * Z::TS;
   const int ngroups = (int)(rows / Z::RW);
   const R sc = R(g.inv_n);
-  for (int grp = blockIdx.x * NW + warp; grp < ngroups; grp += gridDim.x * NW) {
+  for (int grp = blockIdx.x * nw + warp; grp < ngroups; grp += gridDim.x * nw) {
     const size_t row = (size_t)grp * Z::RW + wl<LM>();
     Cx<R> *line = io + row * Z::TS;
     Cx<R> u[PARK ? 1 : 3][Z::N1];
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
     if (parts && n < pp.Np) position_update_one(pp, pdl_fresh(parts), n, euler, status);
     return;
   }
-  const int warp = threadIdx.x >> 5;
+  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
   Cx<R> w[Z::N1], wz[Z::N1];
   wfft_twiddles<R, LM>(tw.m, w);
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
   const size_t rows = (size_t)g.NX * g.NY;
   const int ngroups = (int)(rows / Z::RW);
   const R sc = R(g.inv_n);
-  for (int task = blockIdx.x * NW + warp; task < ncomp * ngroups; task += nblk * NW) {
+  for (int task = blockIdx.x * nw + warp; task < ncomp * ngroups; task += nblk * nw) {
     const int c = task / ngroups;
     const size_t row = (size_t)(task - c * ngroups) * Z::RW + wl<LM>();
     Cx<R> v[Z::N1];
@@ -296,14 +296,14 @@ __global__ void __launch_bounds__(NW * 32) k_zw_r2c(Geo g, Twiddles<R> tw, R *__
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
   in = pdl_fresh(in);
-  const int warp = threadIdx.x >> 5;
+  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   Cx<R> *ex = reinterpret_cast<Cx<R> *>(smem_raw) + warp * ZX<R, LM>::ELEMS;
   Cx<R> w[Z::N1], wz[Z::N1];
   wfft_twiddles<R, LM>(tw.m, w);
   wpack_twiddles<R, LM>(tw.z, wz);
   const size_t rows = (size_t)g.NX * g.NY;
   const int ngroups = (int)(rows / Z::RW);
-  for (int task = blockIdx.x * NW + warp; task < ncomp * ngroups; task += gridDim.x * NW) {
+  for (int task = blockIdx.x * nw + warp; task < ncomp * ngroups; task += gridDim.x * nw) {
     const int c = task / ngroups;
     const size_t row = (size_t)(task - c * ngroups) * Z::RW + wl<LM>();
     V2 *src = reinterpret_cast<V2 *>(in + c * in_cstride + row * Z::NZ) + wt<LM>();

@@ -70,3 +70,14 @@ def test_earlier_launches_data_is_read_through_fresh_pointers(k):
         if not m or m.group(1) == "cells" or not ("const" in p or "DPart" in p):
             continue
         assert re.search(rf"pdl_fresh\({m.group(1)}\)", body), f"{name}: {m.group(1)}"
+
+
+def test_kernels_of_planned_block_sizes_stride_by_the_block_they_run_in():
+    """zplan launches fewer warps than the template's NW where shared memory does
+    not hold them: a kernel that strode by NW would then leave rows out."""
+    src = dict(_sources())["kapsel_gpu.cu"]
+    planned = set(re.findall(r"zplan\((k_\w+)<", src))
+    assert {"k_zw_products", "k_zw_c2r", "k_zw_cross", "k_zw_flux"} <= planned
+    for _, name, _, body in kernels():
+        if name in planned:
+            assert "blockDim.x >> 5" in body and not re.search(r"\bNW\b", body), name
