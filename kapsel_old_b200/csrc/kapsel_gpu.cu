@@ -3474,12 +3474,12 @@ int kapsel_nc_create(const float *params, kapsel_nc **out) {
 
 int kapsel_nc_destroy(kapsel_nc *nc) {
   if (!nc) return KAPSEL_EINVAL;
+  if (nc->rows) cudaFreeAsync(nc->rows, nc->stream);
   cudaStreamSynchronize(nc->stream);
   cudaFree(nc->params);
   cudaFree(nc->grad);
   cudaFree(nc->m);
   cudaFree(nc->v);
-  cudaFree(nc->rows);
   cudaStreamDestroy(nc->stream);
   delete nc;
   return 0;
@@ -3514,17 +3514,28 @@ static int nc_status(kapsel_nc *nc) {
   return nc_clear(nc, st);
 }
 
-// device rows for n samples: inputs, targets or outputs, column weights
+// device rows for n samples: inputs, targets or outputs, column weights.  They
+// are taken and given back in the order of the object's stream: cudaMalloc and
+// cudaFree wait for all streams, a box being stepped by another thread among
+// them.  Half as much again as the object had, so that calls that grow a little
+// each time do not all pay for new memory.
 static int nc_rows(kapsel_nc *nc, int n) {
   if ((size_t)n <= nc->rows_cap) return 0;
-  cudaFree(nc->rows);
+  auto bytes = [](size_t k) { return sizeof(float) * ((nc::IN + nc::OUT) * k + nc::OUT); };
+  size_t want = std::max((size_t)n, nc->rows_cap + nc->rows_cap / 2);
+  if (nc->rows) cudaFreeAsync(nc->rows, nc->stream);
   nc->rows = nullptr;
   nc->rows_cap = 0;
-  if (cudaMalloc(&nc->rows, sizeof(float) * ((nc::IN + nc::OUT) * (size_t)n + nc::OUT)) != cudaSuccess) {
+  if (cudaMallocAsync(&nc->rows, bytes(want), nc->stream) != cudaSuccess) {
     cudaGetLastError();
-    return KAPSEL_ENOMEM;
+    want = (size_t)n;
+    if (cudaMallocAsync(&nc->rows, bytes(want), nc->stream) != cudaSuccess) {
+      cudaGetLastError();
+      nc->rows = nullptr;
+      return KAPSEL_ENOMEM;
+    }
   }
-  nc->rows_cap = (size_t)n;
+  nc->rows_cap = want;
   return 0;
 }
 

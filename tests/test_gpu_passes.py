@@ -155,3 +155,30 @@ def test_network_calls_of_changing_size():
         (ga, la), (gb, lb) = kept.gradient(x, y, w), fresh.gradient(x, y, w)
         # the same products, added by atomics in any order
         assert rel(ga, gb) < 1e-5 and abs(la - lb) < 1e-5 * abs(lb)
+
+
+def test_network_rows_grow_without_waiting_for_other_streams():
+    """A call with more rows than any before takes its memory in its own stream's
+    order: it is back while another stream's work (a device-side sleep of about
+    half a second, here) is still running."""
+    import torch
+
+    from kapsel_old_b200 import nearcontact as nc
+
+    rng = np.random.Generator(np.random.PCG64(8))
+    x, w = rng.normal(size=(4096, 16)).astype(np.float32), np.ones(16, np.float32)
+    net = nc.NearContactNet(nc.init_params(3))
+    other, done = torch.cuda.Stream(), torch.cuda.Event()
+    net.gradient(x[:64], x[:64], w)
+    net.forward(x[:64])
+    with torch.cuda.stream(other):
+        torch.cuda._sleep(1000)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(other):
+        torch.cuda._sleep(10 ** 9)
+        done.record()
+    net.gradient(x[:2048], x[:2048], w)
+    net.forward(x)
+    still_running = not done.query()
+    torch.cuda.synchronize()
+    assert still_running
