@@ -133,3 +133,23 @@ def test_block_level_x_passes_of_sixteen_points(np_xyz, precision):
     a.step(4)
     b.step(4, graph=True)
     assert rel(b.zeta(), a.zeta()) < (1e-5 if precision else 1e-12)
+
+
+@pytest.mark.parametrize("np_xyz,precision,planes", [
+    ((6, 6, 8), 0, False),  # 192 planes of one four-warp block an SM: a last wave of 44
+    ((5, 6, 8), 0, True), ((7, 6, 8), 0, True),  # one wave; a last wave of 88
+    ((6, 5, 8), 0, True), ((6, 7, 7), 0, True),  # two blocks an SM; eight warps
+    ((6, 6, 6), 1, True), ((6, 6, 8), 1, False)])
+def test_where_the_plane_kernels_are_the_default(np_xyz, precision, planes):
+    import kapsel_old_b200 as kg
+
+    cfg = {"eq": "Navier_Stokes", "np_xyz": np_xyz, "a": 3.0, "a_xi": 2.0, "kbt": 0.0, "dt": 0.01,
+           "particles": [{"x": (9.0, 9.0, 9.0)}]}
+    s = kg.Simulation(cfg, precision=precision)
+    assert (s.step_kernel_names()[6] == "k_yzw_c2r") == planes
+    # either way the other form is there and gives the same bits
+    s.step(2)
+    t = kg.Simulation(cfg, precision=precision)
+    assert t.L.kapsel_gpu_set_pass_variant(t.h, 0, 0 if planes else 3) == 0
+    t.step(2)
+    assert np.array_equal(s.zeta(), t.zeta())
