@@ -476,11 +476,11 @@ struct Box : BoxBase {
   template <int LX>
   int x_setup_block() {
     if constexpr (LX < 8) {
-      KCHECK(allow_smem(k_x_zeta_to_u<R, KCX, LX, 1>, smem_xu));
-      KCHECK(allow_smem(k_x_advect_update<R, KCX, 0, LX, 1>, smem_xadv));
-      KCHECK(allow_smem(k_x_advect_update<R, KCX, 1, LX, 1>, smem_xadv));
-      KCHECK(allow_smem(k_x_force_to_zeta<R, KCX, LX, 0, 1>, smem_xf));
-      KCHECK(allow_smem(k_x_force_to_zeta<R, KCX, LX, 1, 1>, smem_xf));
+      KCHECK(allow_smem(k_x_zeta_to_u<R, KCX, LX>, smem_xu));
+      KCHECK(allow_smem(k_x_advect_update<R, KCX, 0, LX>, smem_xadv));
+      KCHECK(allow_smem(k_x_advect_update<R, KCX, 1, LX>, smem_xadv));
+      KCHECK(allow_smem(k_x_force_to_zeta<R, KCX, LX, 0>, smem_xf));
+      KCHECK(allow_smem(k_x_force_to_zeta<R, KCX, LX, 1>, smem_xf));
     }
     return 0;
   }
@@ -493,7 +493,7 @@ struct Box : BoxBase {
   void xz_l(Launch pdl, const Cx<R> *z, const double *u, Cx<R> *out) {
     if constexpr (LX < 8)
       if (xsplit) {
-        launch_k(pdl, k_x_zeta_to_u<R, KCX, LX, 1>, gx(), dim3(kXZThreads), smem_xu, stream, g, tw, z, u, out);
+        launch_k(pdl, k_x_zeta_to_u<R, KCX, LX>, gx(), dim3(kXZThreads), smem_xu, stream, g, tw, z, u, out);
         return;
       }
     launch_k(pdl, k_xw_zeta_to_u<R, LX>, gxw<LX>(g), dim3(3 * XT<R, LX>::TPG), XT<R, LX>::smem(3), stream, g, tw, z, u, out);
@@ -502,7 +502,7 @@ struct Box : BoxBase {
   void xa_l(Launch pdl) {
     if constexpr (LX < 8)
       if (xsplit) {
-        launch_k(pdl, k_x_advect_update<R, KCX, EU, LX, 1>, gx(), dim3(kXAdvThreads), smem_xadv, stream, g, tw, bufA,
+        launch_k(pdl, k_x_advect_update<R, KCX, EU, LX>, gx(), dim3(kXAdvThreads), smem_xadv, stream, g, tw, bufA,
                  zeta, uk_dc);
         return;
       }
@@ -513,7 +513,7 @@ struct Box : BoxBase {
   void xf_l(Launch pdl, Cx<R> *in) {
     if constexpr (LX < 8)
       if (xsplit) {
-        launch_k(pdl, k_x_force_to_zeta<R, KCX, LX, NEXTU, 1>, gx(), dim3(kXForceThreads), smem_xf, stream, g, tw, in,
+        launch_k(pdl, k_x_force_to_zeta<R, KCX, LX, NEXTU>, gx(), dim3(kXForceThreads), smem_xf, stream, g, tw, in,
                  zeta, uk_dc);
         return;
       }
@@ -578,7 +578,7 @@ struct Box : BoxBase {
     const size_t ex = ZX<R, LM>::BYTES;  // exchange buffers of a warp
     int rc = zplan(k_zw_products<R, LM, ZNW>, zw_products_bytes<R, LM>(), zp_p);
     if (!rc) rc = zplan(k_zw_c2r<R, LM, ZNW>, ex, zp_c);
-    if (!rc) rc = zplan(k_zw_r2c<R, LM, ZNW, true, false>, ex, zp_f);
+    if (!rc) rc = zplan(k_zw_r2c<R, LM, ZNW>, ex, zp_f);
     if (!rc && prm.eq == KAPSEL_EQ_ELECTROLYTE) {
       rc = zplan(k_zw_products<R, LM, ZNW, true>, zw_products_bytes<R, LM>(), zp_pu);
       if (!rc) rc = zplan(k_zw_charge<R, LM, ZNW, false>, ex, zp_q);
@@ -612,7 +612,7 @@ struct Box : BoxBase {
     const size_t sm = YZ<R, LY, LM>::smem();
     if (sm > 227 * 1024) return 0;
     KCHECK(allow_smem(k_yzw_c2r<R, LY, LM, NW>, sm));
-    KCHECK(allow_smem(k_zyw_r2c<R, LY, LM, true, NW>, sm));
+    KCHECK(allow_smem(k_zyw_r2c<R, LY, LM, NW>, sm));
     KCHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&yz_occ, k_yzw_c2r<R, LY, LM, NW>, NW * 32, sm));
     yz_occ = std::max(yz_occ, 1);
     yz_warps = yz_occ * NW;
@@ -630,7 +630,7 @@ struct Box : BoxBase {
   template <int LY, int LM>
   void zy_force_l(Launch pdl) {
     constexpr int NW = YZ<R, LY, LM>::NW;
-    launch_k(pdl, k_zyw_r2c<R, LY, LM, true, NW>, dim3(3 * g.NX), dim3(NW * 32), yz_sm, stream, g, tw, force(),
+    launch_k(pdl, k_zyw_r2c<R, LY, LM, NW>, dim3(3 * g.NX), dim3(NW * 32), yz_sm, stream, g, tw, force(),
              npts(), bufA);
   }
   // bufA (x real, ky compact) -> real fields, with the position update in extra blocks
@@ -671,7 +671,7 @@ struct Box : BoxBase {
   }
   template <int LM>
   void zw_force(Launch pdl) {
-    launch_k(pdl, k_zw_r2c<R, LM, ZNW, true, false>, dim3(zp_f.grid(3 * zgroups<LM>())), dim3(zp_f.nw * 32), zp_f.sm,
+    launch_k(pdl, k_zw_r2c<R, LM, ZNW>, dim3(zp_f.grid(3 * zgroups<LM>())), dim3(zp_f.nw * 32), zp_f.sm,
              stream, g, tw, force(), npts(), bufB, 3);
   }
   // dispatch on the compile-time line length
@@ -1257,7 +1257,6 @@ struct Box : BoxBase {
     return 0;
   }
 
-  dim3 gyF(int nc) const { return dim3(g.NX, nc, (gF.TZ + KCY - 1) / KCY); }
   double ze() const { return prm.surface_charge * 1.0; }  // Surface_charge_e, Elementary_charge = 1
   bool ext_on() const { return prm.e_ext[0] != 0.0 || prm.e_ext[1] != 0.0 || prm.e_ext[2] != 0.0; }
 

@@ -132,15 +132,13 @@ __device__ __forceinline__ int fft2_n1(int logn) {
   return 1 << (l1 > 4 ? 4 : l1);
 }
 
-// SPLIT = 1 takes the other factorisation of the same length (both factors
-// 2..16): 8 = 2 x 4, 16 = 8 x 2, 32 = 4 x 8, 64 = 16 x 4, 128 = 16 x 8;
-// 256 has only 16 x 16.  Which one is faster depends on the line count and
-// the precision; the batch autotuner times both.
+// SPLIT = 1, the block-level x passes (NX = 16..128), takes the other
+// factorisation of the same length: 16 = 8 x 2, 32 = 4 x 8, 64 = 16 x 4, 128 =
+// 16 x 8.
 template <int SPLIT>
 __device__ __forceinline__ int fft2_n1_sel(int logn) {
   if (SPLIT == 0) return fft2_n1(logn);
   switch (logn) {
-    case 3: return 2;
     case 4: return 8;
     case 5: return 4;
     default: return 16;

@@ -92,14 +92,14 @@ __device__ __forceinline__ void select_zeta(int KXi, int KYi, const Cx<R> w[3], 
 // ---------------------------------------------------------------------------
 // x pass, inverse: zeta -> u_k (Zeta_k2u_k) -> inverse x transform.
 // grid (KYc, ceil(TZ/KC)), out I1[3][NX][KYc][TZ].
-template <typename R, int KC, int LX = 0, int XS = 0>
+template <typename R, int KC, int LX>
 __global__ void __launch_bounds__(256) k_x_zeta_to_u(Geo g, Twiddles<R> tw, const Cx<R> *__restrict__ zeta,
                                                      const double *__restrict__ uk_dc, Cx<R> *__restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
   zeta = pdl_fresh(zeta);
   uk_dc = pdl_fresh(uk_dc);
-  const int NXv = LX > 0 ? (1 << LX) : g.NX, LXv = LX > 0 ? LX : g.lx;
+  constexpr int NXv = 1 << LX;
   constexpr int W = 3 * KC;
   Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
   Cx<R> *Zt = twx + NXv;          // [2][KXc][KC] staged zeta tile
@@ -142,9 +142,9 @@ __global__ void __launch_bounds__(256) k_x_zeta_to_u(Geo g, Twiddles<R> tw, cons
     U[i * W + 2 * KC + col] = u[2];
   }
   __syncthreads();
-  fft2_smem<R, -1, W, LX, XS>(U, scr, LXv, 1, W, twx);
+  fft2_smem<R, -1, W, LX, 1>(U, scr, LX, 1, W, twx);
   for (int it = threadIdx.x; it < 3 * NXv * KC; it += blockDim.x) {
-    const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LXv;
+    const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LX;
     if (col < ncol)
       out[(((size_t)c * NXv + x) * g.KYc + iy) * g.TS + kz0 + col] = U[x * W + c * KC + col];
   }
@@ -549,7 +549,7 @@ __device__ __forceinline__ void store_pair(Cx<R> *o, const Cx<R> *p, int left) {
 // NSsolute_solver_Euler (Add_zeta_viscous_term then Field_solver_Euler,
 // fluid_solver.cxx:122-135, operate_omega.cxx:172-184) instead of the slaved
 // step, and no u* output (the electrolyte rebuilds u after the Coulomb force).
-template <typename R, int KC, int EULER = 0, int LX = 0, int XS = 0>
+template <typename R, int KC, int EULER, int LX>
 __global__ void __launch_bounds__(256) k_x_advect_update(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ buf,
                                                          Cx<R> *__restrict__ zeta, double *__restrict__ uk_dc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(256) k_x_advect_update(Geo g, Twiddles<R> tw, 
   buf = pdl_fresh(buf);
   zeta = pdl_fresh(zeta);
   uk_dc = pdl_fresh(uk_dc);
-  const int NXv = LX > 0 ? (1 << LX) : g.NX, LXv = LX > 0 ? LX : g.lx;
+  constexpr int NXv = 1 << LX;
   constexpr int W5 = 5 * KC, W3 = 3 * KC;
   Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
   Cx<R> *Zs = twx + NXv;               // [2][KXc][KC] zeta tile (updated in place)
@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(256) k_x_advect_update(Geo g, Twiddles<R> tw, 
   if constexpr (sizeof(R) == 4 && KC % 2 == 0) {
     constexpr int KP = KC / 2;
     for (int it = threadIdx.x; it < 5 * NXv * KP; it += blockDim.x) {
-      const int col = 2 * (it % KP), rest = it / KP, x = rest & (NXv - 1), c = rest >> LXv;
+      const int col = 2 * (it % KP), rest = it / KP, x = rest & (NXv - 1), c = rest >> LX;
       stage_pair(Pb + x * W5 + c * KC + col, buf + c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col,
                  ncol - col);
     }
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(256) k_x_advect_update(Geo g, Twiddles<R> tw, 
     }
   } else {
     for (int it = threadIdx.x; it < 5 * NXv * KC; it += blockDim.x) {
-      const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LXv;
+      const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LX;
       Cx<R> *d = Pb + x * W5 + c * KC + col;
       if (col < ncol)
         cp_async_cx(d, buf + c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col);
@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(256) k_x_advect_update(Geo g, Twiddles<R> tw, 
   }
   cp_async_wait_all();
   __syncthreads();
-  fft2_smem<R, 1, W5, LX, XS>(Pb, scr, LXv, 1, W5, twx);
+  fft2_smem<R, 1, W5, LX, 1>(Pb, scr, LX, 1, W5, twx);
   const int KYi = signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY);
   const R ky = R(g.wave[1] * KYi);
   for (int it = threadIdx.x; it < g.KXc * KC; it += blockDim.x) {
@@ -651,17 +651,17 @@ __global__ void __launch_bounds__(256) k_x_advect_update(Geo g, Twiddles<R> tw, 
     Pb[i * W3 + 2 * KC + col] = u[2];
   }
   __syncthreads();
-  fft2_smem<R, -1, W3, LX, XS>(Pb, scr, LXv, 1, W3, twx);
+  fft2_smem<R, -1, W3, LX, 1>(Pb, scr, LX, 1, W3, twx);
   if constexpr (sizeof(R) == 4 && KC % 2 == 0) {
     constexpr int KP = KC / 2;
     for (int it = threadIdx.x; it < 3 * NXv * KP; it += blockDim.x) {
-      const int col = 2 * (it % KP), rest = it / KP, x = rest & (NXv - 1), c = rest >> LXv;
+      const int col = 2 * (it % KP), rest = it / KP, x = rest & (NXv - 1), c = rest >> LX;
       store_pair(buf + c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col, Pb + x * W3 + c * KC + col,
                  ncol - col);
     }
   } else {
     for (int it = threadIdx.x; it < 3 * NXv * KC; it += blockDim.x) {
-      const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LXv;
+      const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LX;
       if (col < ncol) buf[c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col] = Pb[x * W3 + c * KC + col];
     }
   }
@@ -695,7 +695,7 @@ __device__ __forceinline__ void force_mode_zeta(int KXi, int KYi, R kx, R ky, R 
 // u_k = Zeta_k2u_k(zeta, uk_dc) of the updated values and the inverse x
 // transform, written over buf (as k_x_zeta_to_u writes it, with the same
 // arithmetic), so the next step starts at its y pass.
-template <typename R, int KC, int LX = 0, int NEXTU = 0, int XS = 0>
+template <typename R, int KC, int LX, int NEXTU>
 __global__ void __launch_bounds__(256) k_x_force_to_zeta(Geo g, Twiddles<R> tw, Cx<R> *__restrict__ buf,
                                                          Cx<R> *__restrict__ zeta, double *__restrict__ uk_dc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(256) k_x_force_to_zeta(Geo g, Twiddles<R> tw, 
   buf = pdl_fresh(buf);
   zeta = pdl_fresh(zeta);
   uk_dc = pdl_fresh(uk_dc);
-  const int NXv = LX > 0 ? (1 << LX) : g.NX, LXv = LX > 0 ? LX : g.lx;
+  constexpr int NXv = 1 << LX;
   constexpr int W3 = 3 * KC;
   Cx<R> *twx = reinterpret_cast<Cx<R> *>(smem_raw);
   Cx<R> *Zs = twx + NXv;          // [2][KXc][KC]
@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(256) k_x_force_to_zeta(Geo g, Twiddles<R> tw, 
   if constexpr (sizeof(R) == 4 && KC % 2 == 0) {
     constexpr int KP = KC / 2;
     for (int it = threadIdx.x; it < 3 * NXv * KP; it += blockDim.x) {
-      const int col = 2 * (it % KP), rest = it / KP, x = rest & (NXv - 1), c = rest >> LXv;
+      const int col = 2 * (it % KP), rest = it / KP, x = rest & (NXv - 1), c = rest >> LX;
       stage_pair(Pb + x * W3 + c * KC + col, buf + c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col,
                  ncol - col);
     }
@@ -729,7 +729,7 @@ __global__ void __launch_bounds__(256) k_x_force_to_zeta(Geo g, Twiddles<R> tw, 
     }
   } else {
     for (int it = threadIdx.x; it < 3 * NXv * KC; it += blockDim.x) {
-      const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LXv;
+      const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LX;
       Cx<R> *d = Pb + x * W3 + c * KC + col;
       if (col < ncol)
         cp_async_cx(d, buf + c * cstr + ((size_t)x * g.KYc + iy) * g.TS + kz0 + col);
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(256) k_x_force_to_zeta(Geo g, Twiddles<R> tw, 
   }
   cp_async_wait_all();
   __syncthreads();
-  fft2_smem<R, 1, W3, LX, XS>(Pb, scr, LXv, 1, W3, twx);
+  fft2_smem<R, 1, W3, LX, 1>(Pb, scr, LX, 1, W3, twx);
   const int KYi = signed_k(full_from_compact(iy, g.TY, g.KYc, g.NY), g.NY);
   const R ky = R(g.wave[1] * KYi);
   for (int it = threadIdx.x; it < g.KXc * KC; it += blockDim.x) {
@@ -803,17 +803,17 @@ __global__ void __launch_bounds__(256) k_x_force_to_zeta(Geo g, Twiddles<R> tw, 
     Pb[i * W3 + 2 * KC + col] = u[2];
   }
   __syncthreads();
-  fft2_smem<R, -1, W3, LX, XS>(Pb, scr, LXv, 1, W3, twx);
+  fft2_smem<R, -1, W3, LX, 1>(Pb, scr, LX, 1, W3, twx);
   if constexpr (sizeof(R) == 4 && KC % 2 == 0) {
     constexpr int KP = KC / 2;
     for (int it = threadIdx.x; it < 3 * NXv * KP; it += blockDim.x) {
-      const int col = 2 * (it % KP), rest = it / KP, x = rest & (NXv - 1), c = rest >> LXv;
+      const int col = 2 * (it % KP), rest = it / KP, x = rest & (NXv - 1), c = rest >> LX;
       store_pair(buf + (((size_t)c * NXv + x) * g.KYc + iy) * g.TS + kz0 + col, Pb + x * W3 + c * KC + col,
                  ncol - col);
     }
   } else {
     for (int it = threadIdx.x; it < 3 * NXv * KC; it += blockDim.x) {
-      const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LXv;
+      const int col = it % KC, rest = it / KC, x = rest & (NXv - 1), c = rest >> LX;
       if (col < ncol) buf[(((size_t)c * NXv + x) * g.KYc + iy) * g.TS + kz0 + col] = Pb[x * W3 + c * KC + col];
     }
   }

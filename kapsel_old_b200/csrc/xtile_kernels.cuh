@@ -136,9 +136,9 @@ __device__ __forceinline__ void x_get(const Cx<R> *tile, Cx<R> (&v)[ZL<LX>::N1])
 
 // The modes of a tile, shared by the block's threads: f(ix, KXi, col, kz) for
 // every retained kx and existing column.
-template <typename R, int LX, typename F, bool FULL = false>
+template <typename R, int LX, typename F>
 __device__ __forceinline__ void x_modes(int kz0, int ncol, F f) {
-  using T = XT<R, LX, FULL>;
+  using T = XT<R, LX>;
   for (int it = threadIdx.x; it < T::MODES; it += blockDim.x) {
     const int col = it & (T::CW - 1), ix = it / T::CW;
     if (col < ncol) f(ix, ix < T::TX ? ix : ix - T::KXc, col, kz0 + col);

@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(NW * 32) k_yzw_c2r(Geo g, Twiddles<R> tw, cons
     // transformed
     const Cx<R> *src = in + (size_t)pl * YGeo<LY, false>::KYc * g.TS + wl<LY>();
     auto load = [&](int b) {
-      yw_load<R, LY, true, false>(src + b * Y::RW, g.TS, b * Y::RW + wl<LY>() < Z::TZ, next);
+      yw_load<R, LY, true>(src + b * Y::RW, g.TS, b * Y::RW + wl<LY>() < Z::TZ, next);
     };
     if (warp < P::NB) load(warp);
     for (int b = warp; b < P::NB; b += NW) {
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(NW * 32) k_yzw_c2r(Geo g, Twiddles<R> tw, cons
       if (b + NW < P::NB) load(b + NW);
       wfft<R, LY, -1>(v, ex, w);
       const int col = b * Y::RW + wl<LY>();
-      yw_store<R, LY, false, false>(plane + col, P::PS, col < Z::TZ, v);
+      yw_store<R, LY, false>(plane + col, P::PS, col < Z::TZ, v);
     }
   }
   __syncthreads();
@@ -100,8 +100,8 @@ __global__ void __launch_bounds__(NW * 32) k_yzw_c2r(Geo g, Twiddles<R> tw, cons
 
 // Forward z, then forward y, of plane (c, x) = blockIdx.x of real fields
 // in[c][NX][NY][NZ] (planes in_cstride apart) -> out [c][NX][KYc][TS], as
-// k_zw_r2c followed by the forward k_yt_pass.  CLEAR as in k_zw_r2c.
-template <typename R, int LY, int LM, bool CLEAR, int NW>
+// k_zw_r2c followed by the forward k_yt_pass, and set back to zero as there.
+template <typename R, int LY, int LM, int NW>
 __global__ void __launch_bounds__(NW * 32) k_zyw_r2c(Geo g, Twiddles<R> tw, R *__restrict__ in, size_t in_cstride,
                                                      Cx<R> *__restrict__ out) {
   using P = YZ<R, LY, LM>;
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(NW * 32) k_zyw_r2c(Geo g, Twiddles<R> tw, R *_
 #pragma unroll
       for (int n1 = 0; n1 < Z::N1; ++n1) {
         v[n1] = {next[n1].x, next[n1].y};
-        if (CLEAR && (v[n1].x != R(0) || v[n1].y != R(0)))
+        if (v[n1].x != R(0) || v[n1].y != R(0))
           src[(size_t)grp * Z::RW * Z::M + Z::N2 * n1] = V2{R(0), R(0)};
       }
       if (grp + NW < P::NG) load(grp + NW);
@@ -147,9 +147,9 @@ __global__ void __launch_bounds__(NW * 32) k_zyw_r2c(Geo g, Twiddles<R> tw, R *_
   for (int b = warp; b < P::NB; b += NW) {
     const int col = b * Y::RW + wl<LY>();
     Cx<R> v[Y::N1];
-    yw_load<R, LY, false, false>(plane + col, P::PS, col < Z::TZ, v);
+    yw_load<R, LY, false>(plane + col, P::PS, col < Z::TZ, v);
     wfft<R, LY, 1>(v, ex, w);
-    yw_store<R, LY, true, false>(out + (size_t)pl * YGeo<LY, false>::KYc * g.TS + col, g.TS, col < Z::TZ, v);
+    yw_store<R, LY, true>(out + (size_t)pl * YGeo<LY, false>::KYc * g.TS + col, g.TS, col < Z::TZ, v);
   }
 }
 

@@ -137,7 +137,7 @@ __device__ __forceinline__ void wpack_c2r(const Cx<R> *A, Cx<R> (&v)[ZL<LM>::N1]
 // r2c unpacking of a transformed line to dst[k], k < NK:
 // A[k] = (Z[k] + conj Z[M-k])/2 - i/2 (Z[k] - conj Z[M-k]) w_NZ^k.  Z[M-k] is
 // element N1-1-n1 of lane N2-t (of the lane itself, shifted by one, at t = 0).
-// Every lane of the warp calls it; `put` is off for rows that do not exist.
+// Every lane of the warp calls it.
 template <typename R, int LM, int NK = ZL<LM>::TZ, typename W>
 __device__ __forceinline__ void wunpack_r2c(const Cx<R> (&v)[ZL<LM>::N1], Cx<R> *dst, const W &wz,
                                             const Cx<R> *__restrict__ twz) {
@@ -282,17 +282,15 @@ __global__ void __launch_bounds__(NW * 32) k_zw_c2r(Geo g, Twiddles<R> tw, const
   }
 }
 
-// Forward z of real fields in[c][rows][NZ] (planes in_cstride apart), kz < TZ
-// kept, or all M + 1 (FULL), -> out [c][rows][TS].  Tasks (component, row
-// group).  CLEAR: the field is set back to zero where it was not (the rigidity
-// force, which only the points under a particle's profile carry, is all zero
-// again for the next scatter).
-template <typename R, int LM, int NW, bool CLEAR, bool FULL>
+// Forward z of the rigidity force in[c][rows][NZ] (planes in_cstride apart), kz
+// < TZ kept -> out [c][rows][TS].  Tasks (component, row group).  The force,
+// which only the points under a particle's profile carry, is set back to zero
+// where it was not, for the next scatter.
+template <typename R, int LM, int NW>
 __global__ void __launch_bounds__(NW * 32) k_zw_r2c(Geo g, Twiddles<R> tw, R *__restrict__ in, size_t in_cstride,
                                                     Cx<R> *__restrict__ out, int ncomp) {
   using Z = ZL<LM>;
   using V2 = typename Vec2<R>::T;
-  constexpr int NK = FULL ? Z::M + 1 : Z::TZ, OS = (NK + 3) & ~3;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_begin();
   in = pdl_fresh(in);
@@ -314,10 +312,10 @@ __global__ void __launch_bounds__(NW * 32) k_zw_r2c(Geo g, Twiddles<R> tw, R *__
 #pragma unroll
     for (int n1 = 0; n1 < Z::N1; ++n1) {
       v[n1] = {x[n1].x, x[n1].y};
-      if (CLEAR && (x[n1].x != R(0) || x[n1].y != R(0))) src[Z::N2 * n1] = V2{R(0), R(0)};
+      if (x[n1].x != R(0) || x[n1].y != R(0)) src[Z::N2 * n1] = V2{R(0), R(0)};
     }
     wfft<R, LM, 1>(v, ex, w);
-    wunpack_r2c<R, LM, NK>(v, out + (c * rows + row) * OS, wz, tw.z);
+    wunpack_r2c<R, LM>(v, out + (c * rows + row) * Z::TS, wz, tw.z);
   }
 }
 
@@ -336,21 +334,21 @@ struct YGeo {
 };
 // elements j = t + N2 n1 of column col (element j at row(j) * stride); zero
 // for columns and rows that do not exist
-template <typename R, int LY, bool COMPACT, bool FULLY>
+template <typename R, int LY, bool COMPACT>
 __device__ __forceinline__ void yw_load(const Cx<R> *src, int stride, bool ok, Cx<R> (&v)[ZL<LY>::N1]) {
   using Y = ZL<LY>;
 #pragma unroll
   for (int n1 = 0; n1 < Y::N1; ++n1) {
-    const int j = wt<LY>() + Y::N2 * n1, r = COMPACT ? YGeo<LY, FULLY>::row(j) : j;
+    const int j = wt<LY>() + Y::N2 * n1, r = COMPACT ? YGeo<LY, false>::row(j) : j;
     v[n1] = ok && r >= 0 ? src[(size_t)r * stride] : Cx<R>{R(0), R(0)};
   }
 }
-template <typename R, int LY, bool COMPACT, bool FULLY>
+template <typename R, int LY, bool COMPACT>
 __device__ __forceinline__ void yw_store(Cx<R> *dst, int stride, bool ok, const Cx<R> (&v)[ZL<LY>::N1]) {
   using Y = ZL<LY>;
 #pragma unroll
   for (int n1 = 0; n1 < Y::N1; ++n1) {
-    const int j = wt<LY>() + Y::N2 * n1, r = COMPACT ? YGeo<LY, FULLY>::row(j) : j;
+    const int j = wt<LY>() + Y::N2 * n1, r = COMPACT ? YGeo<LY, false>::row(j) : j;
     if (ok && r >= 0) dst[(size_t)r * stride] = v[n1];
   }
 }
