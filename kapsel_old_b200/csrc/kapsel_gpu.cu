@@ -605,7 +605,7 @@ struct Box : BoxBase {
   // rigidity force as one launch each, for NY = 2^yz_ly (0: not available)
   int yz_ly = 0;
   size_t yz_sm = 0;
-  int yz_occ = 0, yz_warps = 0;  // blocks and warps of them that an SM holds
+  int yz_occ = 0;  // blocks that an SM holds
   template <int LY, int LM>
   int yz_setup() {
     constexpr int NW = YZ<R, LY, LM>::NW;
@@ -615,7 +615,6 @@ struct Box : BoxBase {
     KCHECK(allow_smem(k_zyw_r2c<R, LY, LM, NW>, sm));
     KCHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&yz_occ, k_yzw_c2r<R, LY, LM, NW>, NW * 32, sm));
     yz_occ = std::max(yz_occ, 1);
-    yz_warps = yz_occ * NW;
     yz_sm = sm;
     yz_ly = LY;
     return 0;
@@ -776,15 +775,15 @@ struct Box : BoxBase {
       // with plane kernels: 64^3 FP32 54.2, 48.7, 43.1; FP64 73.4, 61.6, 59.6;
       // 64x64x128 FP32 74.9, 60.6, 59.8; 32^3 37.8, 35.2, 33.5; 128x128x64
       // 121, 95, 88; 128^3 FP32 181, 122, 124; FP64 343, 246, 235; 256x128x128
-      // 334, 207, 202).  Not in FP32 with NZ = 256 (128x128x256 309, 208, 219;
-      // 64x64x256 107, 72, 75).  Nor where an SM holds fewer than eight warps
-      // of planes (FP64 with 64 x 256: one block of four) and their waves are
-      // together less than three quarters full: nothing runs beside such a
-      // block when few are left (FP64 without and with planes: 64x64x256, 192
-      // planes, 133, 144; 32x64x256, 128x and 256x, of one, three and six
-      // waves, 80.4, 79.7, 231, 231 and 444, 439; with 32 x 256, two blocks an
-      // SM, 64x32x256 81, 77 and 128x32x256 143, 138; with 128 x 128, one of
-      // eight warps, 64x128x128 123.7, 124.1).  The batch autotuner may choose
+      // 334, 207, 202).  Not in FP32 with NZ = 256, where neither wins
+      // throughout (without and with planes: 16x64x256 50, 53; 64x64x256 82, 79;
+      // 128x64x256 122, 124; 16x128x256 56, 64; 64x128x256 121, 125; 128x and
+      // 256x 201, 202 and 397, 395; with NY = 32 51, 52 for NX = 16, but 85, 77
+      // for 128).  Nor where an SM holds one plane and the waves of planes
+      // are together less than three quarters full: nothing runs beside the
+      // planes of the last wave (FP64 with 64 x 256 and 128 x 128, NX = 16..256:
+      // 63, 70; 78.7, 78.4; 132, 136; 233, 232; 454, 441; and 60, 63; 78.6, 78.0;
+      // 122, 124; 221, 211; 410, 393).  The batch autotuner may choose
       // otherwise for a box shape.
       zw_avail = zw;
       // A step's kernels want different amounts of shared memory, and an SM
@@ -808,7 +807,7 @@ struct Box : BoxBase {
         carve = sizeof(R) == 8 && prm.eq == KAPSEL_EQ_NAVIER_STOKES ? 80 : 70;
       if (zw && yz_ly && !(sizeof(R) == 4 && g.NZ == 256)) {
         const int cap = yz_occ * nsm, waves = (3 * g.NX + cap - 1) / cap;
-        if (yz_warps >= 8 || waves == 1 || 12 * g.NX >= 3 * waves * cap) ymode = 3;
+        if (yz_occ > 1 || 12 * g.NX >= 3 * waves * cap) ymode = 3;
       }
     }
     KCHECK(allow_smem(k_y_pass<R, true, KCY>, smem_y));

@@ -136,9 +136,10 @@ def test_block_level_x_passes_of_sixteen_points(np_xyz, precision):
 
 
 @pytest.mark.parametrize("np_xyz,precision,planes", [
-    ((6, 6, 8), 0, False),  # 192 planes of one four-warp block an SM: a last wave of 44
-    ((5, 6, 8), 0, True), ((7, 6, 8), 0, True),  # one wave; a last wave of 88
-    ((6, 5, 8), 0, True), ((6, 7, 7), 0, True),  # two blocks an SM; eight warps
+    # one plane an SM: half a wave, 1.3 waves, 2.6 waves
+    ((5, 6, 8), 0, False), ((6, 6, 8), 0, False), ((7, 6, 8), 0, True),
+    ((4, 7, 7), 0, False), ((6, 7, 7), 0, False), ((7, 7, 7), 0, True),
+    ((6, 5, 8), 0, True), ((4, 6, 7), 0, True),  # more than one
     ((6, 6, 6), 1, True), ((6, 6, 8), 1, False)])
 def test_where_the_plane_kernels_are_the_default(np_xyz, precision, planes):
     import kapsel_old_b200 as kg
