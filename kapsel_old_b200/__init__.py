@@ -497,10 +497,9 @@ class Batch:
 
     def variants(self) -> list:
         """The autotuner's choice per box shape: (NX, NY, NZ, z variant,
-        y variant, x split); z 0 warp-level / 1 block-level, y 0 warp-level /
-        1 block-level wide tile / 2 block-level narrow tile / 3 warp-level
-        with the fused y/z plane kernels, x split 0 default / 1 the other
-        radix factorisation of NX."""
+        y variant, x split); z 0 warp-level / 1 block-level, y 0 register tile /
+        1 block-level wide tile / 2 block-level narrow tile / 3 as 0 with the
+        fused y/z plane kernels, x split 0 register tiles / 1 block-level."""
         self.L.kapsel_batch_variants.argtypes = [_VP, _IP, ctypes.c_int]
         buf = (ctypes.c_int * (6 * 64))()
         n = self.L.kapsel_batch_variants(self.h, buf, 64)

@@ -1,14 +1,17 @@
-// Shared-memory FFT building blocks for the pruned 3D real transforms.
+// Complex arithmetic, copies and launch chaining that all passes share, and the
+// in-place transform of the routine-level full spectra.
 //
 // The reference transforms a whole NX*NY*NZ_ field with Ooura's row-column
 // rdft3d (fftsg3d.c:560-642) behind A2a_k / A_k2a (fft_wrapper.h:432-631).
-// Here a 3D transform is split into three batched 1D passes (x, y, z); each
-// pass stages a tile of lines in shared memory and runs an in-place
-// decimation-in-time FFT on it: bit-reversed load, one radix-2 stage when
-// log2(N) is odd, then merged radix-2^2 (radix-4) stages, one barrier per
-// stage.  The sign convention is the reference's: forward exp(+i theta),
-// inverse exp(-i theta), no scaling (the 1/N of A_k2a is applied by the
-// caller at the real-space end).
+// Here a 3D transform is split into three batched 1D passes (x, y, z).  The
+// steps' passes hold lines in registers (zwarp_kernels.cuh, xtile_kernels.cuh)
+// or, in the block-level variants, do two register networks with shared memory
+// between (rfft_device.cuh).  fft_inplace below serves the entry points that
+// transform whole spectra, A_k2a and Solenoidal_u among them: a tile of lines
+// in shared memory, bit-reversed load, one radix-2 stage when log2(N) is odd,
+// then merged radix-2^2 (radix-4) stages, one barrier per stage.  The sign
+// convention is the reference's: forward exp(+i theta), inverse exp(-i theta),
+// no scaling (the 1/N of A_k2a is applied by the caller at the real-space end).
 #pragma once
 
 #include <cuda_runtime.h>

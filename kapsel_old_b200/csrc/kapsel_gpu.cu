@@ -333,14 +333,15 @@ struct BoxBase {
 
   virtual int alloc() = 0;
   // pass variants of the batch autotuner: z passes warp-level (0) or
-  // block-level (1); y pass warp-level (0), block-level with the wide (1) or
-  // the narrow (2) kz tile.  time_variant runs `reps` steps of this box's
-  // workload with a variant on a copy of its state and restores the state.
+  // block-level (1); y pass on register tiles (0), block-level with the wide
+  // (1) or the narrow (2) kz tile, or as 0 with the y/z plane kernels (3).
+  // time_variant runs `reps` steps of this box's workload with a variant on a
+  // copy of its state and restores the state.
   virtual float time_variant(int zmode, int ymode, int reps) = 0;
   virtual void set_variant(int zmode, int ymode) = 0;
   virtual bool variant_ok(int zmode, int ymode) const = 0;
-  // radix split of the block-level x transforms: 0 the default, 1 the other
-  // factorisation of NX (fft2_n1_sel); time_variant times the current one
+  // x passes: 0 register tiles, 1 block-level (NX = 16..128); time_variant
+  // times the current ones
   int xsplit = 0;
   virtual bool xsplit_ok(int xs) const = 0;
   virtual int set_xsplit(int xs) = 0;
@@ -461,8 +462,8 @@ struct Box : BoxBase {
       default: f(std::integral_constant<int, 8>());
     }
   }
-  // x passes: the warp-level kernels, or with xsplit the block-level ones in
-  // the other radix split (NX = 16..128)
+  // x passes: the register tiles, or with xsplit the block-level kernels (NX =
+  // 16..128)
   template <int LX>
   int x_setup() {
     using T = XT<R, LX>;
@@ -484,7 +485,7 @@ struct Box : BoxBase {
     }
     return 0;
   }
-  // grid of a warp-level x pass over the retained kz of geometry gg
+  // grid of a register-tile x pass over the retained kz of geometry gg
   template <int LX, bool FULL = false>
   static dim3 gxw(const Geo &gg) {
     return dim3((gg.TZ + XT<R, LX, FULL>::CW - 1) / XT<R, LX, FULL>::CW, gg.KYc);
@@ -794,7 +795,9 @@ struct Box : BoxBase {
       // it count for more.  Steps in us with each kernel's own split and with
       // 25, 45 and 70% shared memory: 64^3 FP32 49, 45, 43, 51; FP64 68, 60,
       // 59, 65; electrolyte 64^3 FP32 194, 152, 173, 171, FP64 280, 216, 226,
-      // 230; Lees-Edwards 64^3 79, 72, 70, 76; 64x64x128 65, 60, 59, 61;
+      // 230, 32^3 FP32 124, 118, 116, 117, FP64 147, 135, 133, 141, 128x64x32
+      // 222, 162, 196, 210 and 300, 221, 233, 248, 64x64x128 218, 184, 191, 199
+      // and 293, 265, 251, 259; Lees-Edwards 64^3 79, 72, 70, 76; 64x64x128 65, 60, 59, 61;
       // 128x64x128 84, 87, 73, 75; 128^3 125, 153, 133, 124; electrolyte 128^3
       // 446, 533, 450, 423; Lees-Edwards 128^3 203, 231, 204, 198.  With each
       // kernel's own, 70 and 80%: 256x128x128 201, 197, 202; 128x128x256 207,
@@ -2399,8 +2402,8 @@ int kapsel_gpu_create(const kapsel_params *p, kapsel_ctx **out) {
   // each find the particle's neighbours first, so with enough particles to
   // fill the GPU one block does all its points (336 us with four, 250 with
   // two, 215 with one at 256^3; 14.9, 13.2, 15.4 at 128^3).  The line between
-  // few and some lies where blocks of 1024 threads, one to an SM, no longer
-  // run at once (128 particles at 128^3: 118 us a step against 122).
+  // few and some lies where blocks of 1024 threads, one to each of the 148 SMs,
+  // no longer run at once (128 particles at 128^3: 118 us a step against 122).
   pp.hyd_pcl = 1;
   pp.hyd_threads = b->Np >= 1024 ? 128 : b->Np > 148 ? 512 : 1024;
   pp.sc_pcl = b->Np >= 1024 ? 1 : b->Np > 148 ? 2 : PCL;

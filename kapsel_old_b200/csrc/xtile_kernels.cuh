@@ -25,7 +25,8 @@
 namespace kapsel {
 
 // Tile geometry.  Columns: 64 bytes of a row in FP32 as long as the five groups
-// of k_xw_advect are 320 threads, and 64 bytes in FP64 (8 and 4 columns:
+// of k_xw_advect are 320 threads, and 64 bytes in FP64; below NX = 64 eight
+// columns in either, so that a group is whole warps (8 and 4 columns:
 // electrolyte at 128^3 432 and 481 us, 64x64x128 step 60.8 and 65.3; with 640
 // threads at NX = 256 k_xw_advect takes 141 us, with 320 it takes 131).
 template <typename R, int LX>
