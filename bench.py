@@ -19,7 +19,8 @@ the timed region is bracketed by a barrier and the max over ranks is used.
 
 Reference arm: the unmodified KAPSEL sources built by oracle/Makefile
 (oracle/_ref, OpenMP loops on all host cores) timed by wall clock on the same
-workload, min(K, 30) steps after min(W, 10) warm-up steps; rank 0 only.
+workload, min(K, 30) steps after min(W, 10) warm-up steps; rank 0 only.  Where
+that build is not there the arm says so and times nothing.
 """
 from __future__ import annotations
 
@@ -654,7 +655,12 @@ def cpu_baseline_batch(boxes):
 
 def run_reference(args, world: int = 1):
     from kapsel_old_b200 import workload
+    from oracle import ref
 
+    if not os.path.exists(os.path.join(ref.REF_DIR, "kapsel_ref_omp")):
+        return {"impl": "reference",
+                "unavailable": "no build of the KAPSEL sources here (oracle/_ref/kapsel_ref_omp; `make -C oracle` "
+                               "makes it where they are)"}
     cfg = workload.mixed_128_256()
     steps = max(1, min(args.steps, REF_MAX_STEPS))
     # the warm-up the caller asked for (as the GPU arm takes it), at most 10
